@@ -523,10 +523,8 @@ struct nn_cg_plan {
     } as;
 };
 
-void nn_cg_plan_destroy(nn_cg_plan* pl)
+static void cg_free(nn_cg_plan* pl)
 {
-    if (!pl) return;
-    if (pl->ctx) cudaStreamSynchronize(pl->ctx->stream);
     for (int q = 0; q < 2; ++q) {
         nn_release(pl->r[q]);
         nn_release(pl->w[q]);
@@ -537,6 +535,13 @@ void nn_cg_plan_destroy(nn_cg_plan* pl)
     nn_release(pl->partials);
     nn_release(pl->ticket);
     nn_release(pl->flags);
+}
+
+void nn_cg_plan_destroy(nn_cg_plan* pl)
+{
+    if (!pl) return;
+    if (pl->ctx) cudaStreamSynchronize(pl->ctx->stream);
+    cg_free(pl);
     for (auto e : pl->ev_a) cudaEventDestroy(e);
     for (auto e : pl->ev_b) cudaEventDestroy(e);
     if (pl->as.e0) cudaEventDestroy(pl->as.e0);
@@ -546,12 +551,47 @@ void nn_cg_plan_destroy(nn_cg_plan* pl)
     nn_ctx_release(ctx);
 }
 
+// The plan's vectors, scalars and tensor maps, allocated once.
+static nn_status cg_vectors(nn_cg_plan* pl)
+{
+    if (pl->flags) return NN_OK;
+    nn_ctx* ctx = pl->ctx;
+    const size_t G = (size_t)pl->G;
+    const int max_tiles = ((pl->nx + TX - 1) / TX) * ((pl->ny + TY - 1) / TY) * ((pl->nz + 3) / 4);  // zc >= 4
+    const int nparts = std::max(max_tiles, pl->init_blocks);
+    nn_status st = NN_OK;
+    for (int q = 0; q < 2 && st == NN_OK; ++q) {
+        st = nn_alloc(ctx, &pl->r[q], G);
+        if (st == NN_OK) st = nn_alloc(ctx, &pl->w[q], G);
+        if (st == NN_OK) st = nn_alloc(ctx, &pl->s[q], G);
+    }
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->p, G);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->scal, C_COUNT);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->partials, (size_t)3 * nparts);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->ticket, 1);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->flags, 4);
+    for (int q = 0; q < 2 && st == NN_OK; ++q)
+        if (!make_map(&pl->map_r[q], pl->r[q], pl->nx, pl->ny, pl->nz, true) ||
+            !make_map(&pl->map_w[q], pl->w[q], pl->nx, pl->ny, pl->nz, true) ||
+            !make_map(&pl->map_s[q], pl->s[q], pl->nx, pl->ny, pl->nz, true))
+            st = NN_ERR_UNSUPPORTED;
+    if (st == NN_OK && !make_map(&pl->map_p, pl->p, pl->nx, pl->ny, pl->nz, false)) st = NN_ERR_UNSUPPORTED;
+    if (st == NN_OK && pl->D &&
+        (!make_map(&pl->map_d, const_cast<float*>(pl->D), pl->nx, pl->ny, pl->nz, true) ||
+         !make_map(&pl->map_m, const_cast<float*>(pl->invdv), pl->nx, pl->ny, pl->nz, true)))
+        st = NN_ERR_UNSUPPORTED;
+    if (st == NN_OK) st = nn_cuda_check(ctx, cudaMemsetAsync(pl->ticket, 0, sizeof(unsigned int), ctx->stream), "memset");
+    if (st != NN_OK) cg_free(pl);
+    return st;
+}
+
 // The TMA path needs rows that are a multiple of 16 bytes (nx % 4 == 0),
 // 16-byte aligned D and 1/diag, and a driver exposing cuTensorMapEncodeTiled;
 // otherwise it reports UNSUPPORTED and the caller keeps the two-kernel PCG.
 // D and invdv (both null for constant coefficients) stay owned by the caller.
+// lazy: the vectors are allocated at the first use.
 nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D,
-                            const float* invdv, nn_cg_plan** out)
+                            const float* invdv, bool lazy, nn_cg_plan** out)
 {
     *out = nullptr;
     if (nx % 4 != 0 || nx < 4 || ny < 1 || nz < 1 || !encode_fn()) return NN_ERR_UNSUPPORTED;
@@ -569,30 +609,7 @@ nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, d
     pl->D = D;
     pl->invdv = invdv;
     pl->init_blocks = nn_grid_for(ctx, pl->G, CG_THREADS, 8);
-    const size_t G = (size_t)pl->G;
-    const int max_tiles = ((nx + TX - 1) / TX) * ((ny + TY - 1) / TY) * ((nz + 3) / 4);  // zc >= 4
-    const int nparts = std::max(max_tiles, pl->init_blocks);
-    nn_status st = NN_OK;
-    for (int q = 0; q < 2 && st == NN_OK; ++q) {
-        st = nn_alloc(ctx, &pl->r[q], G);
-        if (st == NN_OK) st = nn_alloc(ctx, &pl->w[q], G);
-        if (st == NN_OK) st = nn_alloc(ctx, &pl->s[q], G);
-    }
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->p, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->scal, C_COUNT);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->partials, (size_t)3 * nparts);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->ticket, 1);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->flags, 4);
-    for (int q = 0; q < 2 && st == NN_OK; ++q)
-        if (!make_map(&pl->map_r[q], pl->r[q], nx, ny, nz, true) ||
-            !make_map(&pl->map_w[q], pl->w[q], nx, ny, nz, true) ||
-            !make_map(&pl->map_s[q], pl->s[q], nx, ny, nz, true))
-            st = NN_ERR_UNSUPPORTED;
-    if (st == NN_OK && !make_map(&pl->map_p, pl->p, nx, ny, nz, false)) st = NN_ERR_UNSUPPORTED;
-    if (st == NN_OK && D &&
-        (!make_map(&pl->map_d, const_cast<float*>(D), nx, ny, nz, true) ||
-         !make_map(&pl->map_m, const_cast<float*>(invdv), nx, ny, nz, true)))
-        st = NN_ERR_UNSUPPORTED;
+    nn_status st = lazy ? NN_OK : cg_vectors(pl);
     if (st == NN_OK) {
         cudaError_t e = D ? cudaFuncSetAttribute(k_cg_iter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  Layout<true>::SMEM_BYTES)
@@ -627,7 +644,6 @@ nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, d
             }
         }
     }
-    if (st == NN_OK) st = nn_cuda_check(ctx, cudaMemsetAsync(pl->ticket, 0, sizeof(unsigned int), ctx->stream), "memset");
     if (st != NN_OK) {
         nn_cg_plan_destroy(pl);
         return st;
@@ -725,6 +741,7 @@ nn_status nn_cg_async_begin(nn_cg_plan* pl, const float* d_b, float* d_x, double
                             cudaStream_t cs)
 {
     nn_ctx* ctx = pl->ctx;
+    NN_TRY(cg_vectors(pl));
     if (((uintptr_t)d_x & 15) || !make_map(&pl->as.map_x, d_x, pl->nx, pl->ny, pl->nz, false))
         return nn_fail(ctx, NN_ERR_INVALID_ARG, "nn_cg_async_begin: x must be a 16-byte aligned device vector");
     if (!pl->as.e0) NN_CUDA(ctx, cudaEventCreate(&pl->as.e0));
@@ -787,6 +804,7 @@ nn_status nn_cg_run(nn_cg_plan* pl, const float* d_b, float* d_x, double rtol, i
 {
     nn_ctx* ctx = pl->ctx;
     cudaStream_t cs = ctx->stream;
+    NN_TRY(cg_vectors(pl));
     NN_CUDA(ctx, cudaMemsetAsync(pl->ticket, 0, sizeof(unsigned int), cs));  // clean after an aborted solve
     CUtensorMap map_x;  // the caller's solution vector
     if (((uintptr_t)d_x & 15) || !make_map(&map_x, d_x, pl->nx, pl->ny, pl->nz, false))
@@ -855,6 +873,7 @@ nn_status nn_cg_plan_autotune(nn_cg_plan* pl, const float* d_b, float* d_x, int 
     nn_ctx* ctx = pl->ctx;
     cudaStream_t cs = ctx->stream;
     if (iters < 1) return NN_ERR_INVALID_ARG;
+    NN_TRY(cg_vectors(pl));
     CUtensorMap map_x;
     if (((uintptr_t)d_x & 15) || !make_map(&map_x, d_x, pl->nx, pl->ny, pl->nz, false))
         return nn_fail(ctx, NN_ERR_INVALID_ARG, "nn_cg_plan_autotune: x must be a 16-byte aligned device vector");

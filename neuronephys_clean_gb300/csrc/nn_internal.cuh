@@ -232,9 +232,19 @@ nn_status nn_bpcg_async_begin(nn_bpcg* bp, const float* d_b, float* d_x, double 
 nn_status nn_bpcg_async_finish(nn_bpcg* bp, int* h_iters, int* max_iters, int* unconverged);
 int nn_bpcg_cells_per_block(const nn_bpcg* bp);
 
+// resident CG: the whole solve in one kernel (nn_rcg.cu)
+struct nn_rcg_plan;
+nn_status nn_rcg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D,
+                             nn_rcg_plan** out);
+void nn_rcg_plan_destroy(nn_rcg_plan* pl);
+void nn_rcg_set_timing(nn_rcg_plan* pl, bool on);
+void nn_rcg_last_timing(const nn_rcg_plan* pl, float* ms, int* iters);
+nn_status nn_rcg_begin(nn_rcg_plan* pl, const float* d_b, float* d_x, double rtol, int max_iter, cudaStream_t cs);
+nn_status nn_rcg_finish(nn_rcg_plan* pl, cudaStream_t cs, int* iters, double* relres, int* converged);
+
 struct nn_cg_plan;
 nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D,
-                            const float* invdv, nn_cg_plan** out);
+                            const float* invdv, bool lazy, nn_cg_plan** out);
 void nn_cg_plan_destroy(nn_cg_plan* pl);
 nn_status nn_cg_run(nn_cg_plan* pl, const float* d_b, float* d_x, double rtol, int max_iter, int* iters,
                     double* relres, int* converged);

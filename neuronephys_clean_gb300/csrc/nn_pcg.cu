@@ -41,15 +41,24 @@ struct nn_pcg {
     int last_iters = 0;
     // single-kernel TMA iteration (nx % 4 == 0, aligned D); null: two-kernel path
     nn_cg_plan* fast = nullptr;
+    // whole solve in one kernel, for grids that fit on the chip; null: a
+    // launch per iteration (or two)
+    nn_rcg_plan* res = nullptr;
+    cudaStream_t res_stream = nullptr;  // stream of the resident solve in progress
 };
 
 void nn_pcg_set_timing(nn_pcg* pc, bool on)
 {
     pc->timing = on;
     if (pc->fast) nn_cg_set_timing(pc->fast, on);
+    if (pc->res) nn_rcg_set_timing(pc->res, on);
 }
 void nn_pcg_last_timing(const nn_pcg* pc, float* ms, int* iters)
 {
+    if (pc->res) {
+        nn_rcg_last_timing(pc->res, ms, iters);
+        return;
+    }
     if (pc->fast) {
         nn_cg_last_timing(pc->fast, ms, iters);
         return;
@@ -293,6 +302,25 @@ Op make_op(const nn_pcg* pc)
 }
 }  // namespace
 
+// Vectors, scalars and flags of the two-kernel iteration.
+static nn_status two_kernel_vectors(nn_pcg* pc)
+{
+    nn_ctx* ctx = pc->ctx;
+    const size_t G = (size_t)pc->G;
+    NN_TRY(nn_alloc(ctx, &pc->r, G));
+    NN_TRY(nn_alloc(ctx, &pc->p0, G));
+    NN_TRY(nn_alloc(ctx, &pc->p1, G));
+    NN_TRY(nn_alloc(ctx, &pc->Ap, G));
+    NN_TRY(nn_alloc(ctx, &pc->scal, S_COUNT));
+    NN_TRY(nn_alloc(ctx, &pc->partials, (size_t)3 * pc->nblocks));
+    NN_TRY(nn_alloc(ctx, &pc->ticket, 1));
+    NN_TRY(nn_alloc(ctx, &pc->flags, 2));
+    NN_CUDA(ctx, cudaMemsetAsync(pc->ticket, 0, sizeof(unsigned int), ctx->stream));
+    NN_CUDA(ctx, cudaMemsetAsync(pc->p0, 0, sizeof(float) * G, ctx->stream));
+    NN_CUDA(ctx, cudaMemsetAsync(pc->p1, 0, sizeof(float) * G, ctx->stream));
+    return NN_OK;
+}
+
 extern "C" nn_status nn_pcg_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta,
                                    const float* d_Dcell, nn_pcg** out)
 {
@@ -309,22 +337,12 @@ extern "C" nn_status nn_pcg_create(nn_ctx* ctx, int nx, int ny, int nz, double a
     pc->inv_diag_const = (float)(1.0 / (1.0 + beta + 6.0 * alpha));
     pc->nblocks = nn_grid_for(ctx, pc->G, PCG_THREADS, 8);
     const size_t G = (size_t)pc->G;
-    nn_status st = nn_alloc(ctx, &pc->r, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &pc->p0, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &pc->p1, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &pc->Ap, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &pc->scal, S_COUNT);
-    if (st == NN_OK) st = nn_alloc(ctx, &pc->partials, (size_t)3 * pc->nblocks);
-    if (st == NN_OK) st = nn_alloc(ctx, &pc->ticket, 1);
-    if (st == NN_OK) st = nn_alloc(ctx, &pc->flags, 2);
+    nn_status st = NN_OK;
     if (st == NN_OK && d_Dcell) st = nn_alloc(ctx, &pc->invd, G);
     if (st != NN_OK) {
         nn_pcg_destroy(pc);
         return st;
     }
-    cudaMemsetAsync(pc->ticket, 0, sizeof(unsigned int), ctx->stream);
-    cudaMemsetAsync(pc->p0, 0, sizeof(float) * G, ctx->stream);
-    cudaMemsetAsync(pc->p1, 0, sizeof(float) * G, ctx->stream);
     if (d_Dcell) {
         Op o = make_op(pc);
         k_pcg_invdiag<<<pc->nblocks, PCG_THREADS, 0, ctx->stream>>>(o, pc->invd);
@@ -332,11 +350,18 @@ extern "C" nn_status nn_pcg_create(nn_ctx* ctx, int nx, int ny, int nz, double a
     }
     st = nn_cuda_check(ctx, cudaGetLastError(), "nn_pcg_create");
     if (st == NN_OK && !std::getenv("NN_PCG_TWO_KERNEL")) {
-        // the single-kernel TMA iteration where supported
-        nn_status fs = nn_cg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, pc->invd, &pc->fast);
+        // the resident solve where the grid fits, and the single-kernel TMA
+        // iteration where supported (beside the resident solve only the tile
+        // autotuner uses it, which allocates its vectors then)
+        nn_status fs = nn_rcg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, &pc->res);
         if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
+        if (st == NN_OK) {
+            fs = nn_cg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, pc->invd, pc->res != nullptr, &pc->fast);
+            if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
+        }
         ctx->last_error.clear();
     }
+    if (st == NN_OK && !pc->res && !pc->fast) st = two_kernel_vectors(pc);
     if (st != NN_OK) {
         nn_pcg_destroy(pc);
         return st;
@@ -352,6 +377,7 @@ extern "C" nn_status nn_pcg_destroy(nn_pcg* pc)
     nn_release(pc->r); nn_release(pc->p0); nn_release(pc->p1); nn_release(pc->Ap); nn_release(pc->scal);
     nn_release(pc->partials); nn_release(pc->ticket); nn_release(pc->flags); nn_release(pc->invd);
     if (pc->fast) nn_cg_plan_destroy(pc->fast);
+    if (pc->res) nn_rcg_plan_destroy(pc->res);
     for (auto e : pc->ev_a) cudaEventDestroy(e);
     for (auto e : pc->ev_b) cudaEventDestroy(e);
     nn_ctx* ctx = pc->ctx;
@@ -367,31 +393,6 @@ extern "C" nn_status nn_pcg_apply(nn_pcg* pc, const float* d_x, float* d_y)
     Op o = make_op(pc);
     k_pcg_apply<<<pc->nblocks, PCG_THREADS, 0, ctx->stream>>>(o, d_x, d_y);
     NN_CHECK_LAUNCH(ctx, "k_pcg_apply");
-    return NN_OK;
-}
-
-// Enqueue the whole solve without host synchronisation: init + max_iter
-// iteration pairs, each a no-op once the device flag says converged.  Used
-// inside captured simulation periods.
-nn_status nn_pcg_enqueue(nn_pcg* pc, const float* d_b, float* d_x, double rtol, int max_iter)
-{
-    nn_ctx* ctx = pc->ctx;
-    cudaStream_t s = ctx->stream;
-    Op o = make_op(pc);
-    const double rtol2 = rtol * rtol;
-    k_pcg_init<<<pc->nblocks, PCG_THREADS, 0, s>>>(o, d_b, d_x, pc->r, pc->scal, pc->partials, pc->ticket, pc->flags,
-                                                    rtol2);
-    NN_CHECK_LAUNCH(ctx, "k_pcg_init");
-    for (int it = 0; it < max_iter; ++it) {
-        float* p_old = (it & 1) ? pc->p1 : pc->p0;
-        float* p_new = (it & 1) ? pc->p0 : pc->p1;
-        k_pcg_dir_apply<<<pc->nblocks, PCG_THREADS, 0, s>>>(o, pc->r, p_old, p_new, pc->Ap, pc->scal, pc->partials,
-                                                             pc->ticket, pc->flags);
-        NN_CHECK_LAUNCH(ctx, "k_pcg_dir_apply");
-        k_pcg_update<<<pc->nblocks, PCG_THREADS, 0, s>>>(o, d_x, pc->r, p_new, pc->Ap, pc->scal, pc->partials,
-                                                          pc->ticket, pc->flags, rtol2, max_iter);
-        NN_CHECK_LAUNCH(ctx, "k_pcg_update");
-    }
     return NN_OK;
 }
 
@@ -456,20 +457,6 @@ nn_status nn_pcg_run(nn_pcg* pc, const float* d_b, float* d_x, double rtol, int 
     return NN_OK;
 }
 
-nn_status nn_pcg_stats(nn_pcg* pc, int* iters, double* relres, int* converged)
-{
-    nn_ctx* ctx = pc->ctx;
-    int h_flags[2];
-    double h_scal[S_COUNT];
-    NN_CUDA(ctx, cudaMemcpyAsync(h_flags, pc->flags, sizeof h_flags, cudaMemcpyDeviceToHost, ctx->stream));
-    NN_CUDA(ctx, cudaMemcpyAsync(h_scal, pc->scal, sizeof h_scal, cudaMemcpyDeviceToHost, ctx->stream));
-    NN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (iters) *iters = h_flags[1];
-    if (relres) *relres = h_scal[S_BB] > 0 ? std::sqrt(h_scal[S_RR] / h_scal[S_BB]) : 0.0;
-    if (converged) *converged = h_flags[0] == 1;
-    return NN_OK;
-}
-
 extern "C" nn_status nn_pcg_solve(nn_pcg* pc, const float* d_b, float* d_x, double rtol, int max_iter, int* iters,
                                   double* relres)
 {
@@ -512,27 +499,40 @@ extern "C" nn_status nn_pcg_kernel_time(nn_pcg* pc, float* ms, int* iters)
     return NN_OK;
 }
 
-// Asynchronous solve on a stream (single-kernel path only; UNSUPPORTED
-// otherwise): n iterations enqueued now, the rest and the outcome at finish.
+// Asynchronous solve on a stream (UNSUPPORTED with the two-kernel PCG): the
+// whole solve, or n iterations of it, enqueued now, the rest and the outcome
+// at finish.
 nn_status nn_pcg_async_begin(nn_pcg* pc, const float* d_b, float* d_x, double rtol, int max_iter, int n,
                              cudaStream_t cs)
 {
+    if (pc->res) {
+        pc->res_stream = cs;
+        return nn_rcg_begin(pc->res, d_b, d_x, rtol, max_iter, cs);
+    }
     if (!pc->fast) return NN_ERR_UNSUPPORTED;
     return nn_cg_async_begin(pc->fast, d_b, d_x, rtol, max_iter, n, cs);
 }
 
 nn_status nn_pcg_async_finish(nn_pcg* pc, int* iters, double* relres, int* converged)
 {
+    if (pc->res) return nn_rcg_finish(pc->res, pc->res_stream, iters, relres, converged);
     if (!pc->fast) return NN_ERR_UNSUPPORTED;
     return nn_cg_async_finish(pc->fast, iters, relres, converged);
 }
 
-bool nn_pcg_async_supported(const nn_pcg* pc) { return pc->fast != nullptr; }
+bool nn_pcg_async_supported(const nn_pcg* pc) { return pc->fast != nullptr || pc->res != nullptr; }
 
-// The single-kernel TMA iteration when the grid allows it, else two kernels.
+// The resident solve when the grid fits, the single-kernel TMA iteration when
+// its rows allow it, else two kernels.
 nn_status nn_pcg_run_best(nn_pcg* pc, const float* d_b, float* d_x, double rtol, int max_iter, int* iters,
                           double* relres, int* converged)
 {
+    if (pc->res) {
+        if (pc->fast && ((uintptr_t)d_x & 15))
+            return nn_fail(pc->ctx, NN_ERR_INVALID_ARG, "PCG: x must be a 16-byte aligned device vector");
+        NN_TRY(nn_rcg_begin(pc->res, d_b, d_x, rtol, max_iter, pc->ctx->stream));
+        return nn_rcg_finish(pc->res, pc->ctx->stream, iters, relres, converged);
+    }
     if (pc->fast) return nn_cg_run(pc->fast, d_b, d_x, rtol, max_iter, iters, relres, converged);
     return nn_pcg_run(pc, d_b, d_x, rtol, max_iter, iters, relres, converged);
 }

@@ -1,0 +1,822 @@
+// Resident preconditioned CG: the whole solve in one kernel, for grids whose
+// vectors fit in the registers and shared memory of the GPU.
+//
+// Same operator and recurrences as nn_cg.cu (7-point backward Euler, Jacobi
+// preconditioner, Chronopoulos and Gear's one-reduction form), written in the
+// scaled residual u = M r, with w' = M A u and s' = M s:
+//   s' = w' + b s'    p = u + b p    x += a p    u -= a s'    w' = M A u
+//   g = (r, u) = (u, u/M),  d = (w, u) = (w'/M, u),  rho = (r, r)
+// so that the preconditioner is needed only inside the stencil pass, where
+// the diagonal is the sum of the face coefficients at hand.
+//
+// What bounds it.  A launch per iteration (nn_cg.cu) moves ten vectors through
+// L2 and pays a grid's start, tail and reduction: 22 us an iteration at 128^3,
+// 5 us at 32^3, and 54 us at 97 x 83 x 150 in the two-kernel form of nn_pcg.cu
+// (rows that no TMA box can hold).  Here nothing but the bricks' faces and the
+// three sums leaves the SM: an iteration costs one exchange between the blocks
+// (3 us) and the arithmetic on the block's own cells.  Measured per iteration:
+// 2.8 us at 32^3, 3.4 at 48^3, 3.9 at 64^3, 9 at 128^3 (solve to 1e-6: 2.13 ms
+// -> 0.87), 9.3 at 97 x 83 x 150 with a cell field (9.8 ms -> 1.8).
+//
+// Layout.  A block owns a brick of whole x rows, by x bz of them.  A thread
+// owns one quad of four x cells in each of the brick's bz planes, so p and
+// s' stay in registers (8 bz of them) and the z neighbours pass from plane to
+// plane; u (and the cell field) lie in shared memory with a one-cell halo, w'
+// in a private slot per thread.  x is read by nothing during the solve: it
+// stays in L2 and takes two directions every second iteration, loaded while
+// the block waits for the others (in registers it spilled).  The halo keeps its own copy of s', so a block needs only
+// w' of its neighbours' faces, which are published together with the partial
+// sums: one exchange an iteration.
+//
+// Exchange.  Every published 64-bit word carries 32 bits of data and a 32-bit
+// tag (the iteration number), and a reader polls the word until the tag is
+// the one it waits for.  So data and signal travel together: no fence, no
+// counter, no second round trip.  Two buffers alternate; a block writes
+// iteration i + 2 only after it has read every block's sums of i + 1, which
+// each block publishes after its last read of i.  The blocks wait on one
+// another, so the launch is cooperative; every poll is bounded.
+#include <algorithm>
+#include <cmath>
+
+#include "nn_hh.cuh"
+#include "nn_internal.cuh"
+
+namespace {
+constexpr int RT = 512;               // most threads of a block
+constexpr int POLL_LIMIT = 1 << 22;   // some seconds
+constexpr int MAX_BLOCKS = 160;
+
+typedef unsigned long long u64;
+
+__device__ __forceinline__ void st_tagged(ulonglong2* p, uint32_t a, uint32_t b, uint32_t tag)
+{
+    const u64 t = (u64)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | a), "l"(t | b) : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_tagged(const ulonglong2* p)
+{
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+// four values in one 32-byte sector
+struct Tagged4 {
+    u64 w[4];
+};
+__device__ __forceinline__ void st_tagged4(Tagged4* p, const float (&v)[4], uint32_t tag)
+{
+    const u64 t = (u64)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(t | __float_as_uint(v[0])),
+                 "l"(t | __float_as_uint(v[1])), "l"(t | __float_as_uint(v[2])), "l"(t | __float_as_uint(v[3]))
+                 : "memory");
+}
+__device__ __forceinline__ Tagged4 ld_tagged4(const Tagged4* p)
+{
+    Tagged4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3])
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ bool tagged(const Tagged4& v, uint32_t tag)
+{
+    return (uint32_t)(v.w[0] >> 32) == tag && (uint32_t)(v.w[1] >> 32) == tag && (uint32_t)(v.w[2] >> 32) == tag &&
+           (uint32_t)(v.w[3] >> 32) == tag;
+}
+__device__ __forceinline__ bool tagged(const ulonglong2& v, uint32_t tag)
+{
+    return (uint32_t)(v.x >> 32) == tag && (uint32_t)(v.y >> 32) == tag;
+}
+
+// Sums and scalars as unevaluated pairs of floats (48 bits).  The addends are
+// FP32 warp sums, so FP64 would carry no more information, and its chains of
+// dependent additions and divisions are slow on this chip: an iteration on
+// 8^3 cells took 5.1 us with FP64 sums and scalars and takes 3.1 us with pairs
+// (the solutions' errors against FP64 are the same).  Sums are kept scaled by
+// SUM_SCALE, so that adding thousands of warps does not overflow.
+struct Pair {
+    float h, l;
+};
+constexpr float SUM_SCALE = 1.0f / 4096.0f;
+
+__device__ __forceinline__ Pair pair_norm(float h, float l)
+{
+    const float s = __fadd_rn(h, l);
+    return {s, __fsub_rn(l, __fsub_rn(s, h))};
+}
+__device__ __forceinline__ Pair pair_add(const Pair& x, const Pair& y)
+{
+    const float s = __fadd_rn(x.h, y.h), t = __fsub_rn(s, x.h);
+    const float e = __fadd_rn(__fsub_rn(x.h, __fsub_rn(s, t)), __fsub_rn(y.h, t));
+    return pair_norm(s, __fadd_rn(e, __fadd_rn(x.l, y.l)));
+}
+__device__ __forceinline__ Pair pair_mul(const Pair& x, const Pair& y)
+{
+    const float p = __fmul_rn(x.h, y.h);
+    return pair_norm(p, __fmaf_rn(x.l, y.h, __fmaf_rn(x.h, y.l, __fmaf_rn(x.h, y.h, -p))));
+}
+__device__ __forceinline__ Pair pair_div(const Pair& x, const Pair& y)
+{
+    const float q = __fdividef(x.h, y.h);
+    const float r = __fadd_rn(__fmaf_rn(-q, y.h, x.h), __fmaf_rn(-q, y.l, x.l));
+    return pair_norm(q, __fdividef(r, y.h));
+}
+__device__ __forceinline__ Pair pair_shfl(const Pair& x, int o)
+{
+    return {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
+}
+
+struct RcgArgs {
+    int nx, ny, nz;
+    int by, bz, nyb, nb;       // brick, bricks along y, bricks in all
+    int quads, pitch, hq;      // quads a row, shared row pitch, halo quads of a brick
+    float op_alpha, onepb, invd;
+    float half_ia;             // 1 / (2 alpha)
+    Pair diag;                 // constant coefficients: 1 / invd
+    Pair rtol2;
+    const float* b;
+    float* x;
+    const float* D;
+    float4* xw;                // x during the solve: [block][plane][thread]
+    ulonglong2* rec;           // [2][nb][4]: tagged pairs g, d, rho, (b, b)
+    Tagged4* halo;             // [2][nb][hq]: tagged w' of a brick's faces
+    unsigned* epoch;           // first tag of the next solve
+    double* scal;              // out: rho, (b, b)
+    int* flags;                // out: [0] 1 converged, 2 max_iter, 3 error  [1] iterations  [2] a wait gave up
+    int max_iter;
+};
+
+// The four x cells of a thread in one plane, as two packed pairs (nn_hh.cuh).
+typedef nn_vf<2> V2;
+struct Quad {
+    V2 a, b;
+};
+__device__ __forceinline__ Quad quad_ld(const float* p)
+{
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    return {{{v.x, v.y}}, {{v.z, v.w}}};
+}
+__device__ __forceinline__ void quad_st(float* p, const Quad& q)
+{
+    *reinterpret_cast<float4*>(p) = make_float4(q.a.v[0], q.a.v[1], q.b.v[0], q.b.v[1]);
+}
+__device__ __forceinline__ Quad quad_ldcg(const float4* p)  // kept where it stands in the program
+{
+    Quad q;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(q.a.v[0]), "=f"(q.a.v[1]), "=f"(q.b.v[0]), "=f"(q.b.v[1])
+                 : "l"(p)
+                 : "memory");
+    return q;
+}
+__device__ __forceinline__ Quad quad_zero() { return {{{0, 0}}, {{0, 0}}}; }
+__device__ __forceinline__ float& at(Quad& q, int e) { return e < 2 ? q.a.v[e] : q.b.v[e - 2]; }
+__device__ __forceinline__ float at(const Quad& q, int e) { return e < 2 ? q.a.v[e] : q.b.v[e - 2]; }
+
+template <int NZ, bool HET>
+__global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
+{
+    extern __shared__ float4 smem4[];
+    __shared__ float ws[4][RT / 32];
+    __shared__ Pair wp[4][8];
+    __shared__ float sc_alpha, sc_beta;
+    __shared__ int sc_stop, sc_fail;
+    const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int jb = blockIdx.x % a.nyb, kb = blockIdx.x / a.nyb;
+    const int y0 = jb * a.by, z0 = kb * a.bz;
+    const int byn = min(a.by, a.ny - y0), bzn = min(a.bz, a.nz - z0);
+    const int rows = a.by + 2, psz = rows * a.pitch;  // shared plane
+    float* U = reinterpret_cast<float*>(smem4);
+    float* Ds = U + (HET ? (a.bz + 2) * psz : 0);
+    float4* W = reinterpret_cast<float4*>(Ds + (a.bz + 2) * psz);
+    float4* SH = W + a.bz * T;
+    float4* WH = SH + a.hq;
+    int2* HT = reinterpret_cast<int2*>(WH + a.hq);  // per halo quad: shared place, face slot it comes from (-1: none)
+    const int q = tid % a.quads, j = tid / a.quads;
+    const bool act = j < byn;
+    const int i0 = 4 * q;
+    const int ub = psz + (min(j, a.by - 1) + 1) * a.pitch + 4 + i0;  // own quad in plane 0
+    const int64_t gsz = (int64_t)a.nx * a.ny;
+    const int64_t g0 = i0 + (int64_t)a.nx * (y0 + j) + gsz * z0;
+    const bool full = i0 + 4 <= a.nx;
+    const uint32_t base = *reinterpret_cast<volatile unsigned*>(a.epoch);
+    // halo duty is on all warps but the first (there are two or more), which
+    // polls the sums
+    const int ht = tid - 32, hstep = T - 32, nw = T >> 5;
+    const int yq = a.bz * a.quads, zq = a.by * a.quads;  // halo quads: y-, y+ (yq each), z-, z+ (zq each)
+
+    // halo quad h: its place in shared memory, the brick and face slot it
+    // comes from (-1: outside the grid or the brick), the first cell's index
+    auto halo_at = [&](int h, int& sm, int& src, int& slot, int64_t& g) {
+        int f, r;
+        if (h < 2 * yq) { f = h >= yq; r = h - f * yq; }
+        else { f = 2 + (h - 2 * yq >= zq); r = h - 2 * yq - (f - 2) * zq; }
+        const int line = r / a.quads, hx = r - line * a.quads;
+        int lj, lk;
+        if (f < 2) {
+            lk = line;
+            lj = f ? byn : -1;
+            src = f ? (jb + 1 < a.nyb ? (int)blockIdx.x + 1 : -1) : (jb > 0 ? (int)blockIdx.x - 1 : -1);
+            slot = (f ? 0 : yq) + r;
+            if (lk >= bzn) src = -1;
+        } else {
+            lj = line;
+            lk = f == 3 ? bzn : -1;
+            src = f == 3 ? (z0 + a.bz < a.nz ? (int)blockIdx.x + a.nyb : -1) : (kb > 0 ? (int)blockIdx.x - a.nyb : -1);
+            slot = 2 * yq + (f == 3 ? 0 : zq) + r;
+            if (lj >= byn) src = -1;
+        }
+        sm = (lk + 1) * psz + (lj + 1) * a.pitch + 4 + 4 * hx;
+        g = 4 * hx + (int64_t)a.nx * (y0 + lj) + gsz * (z0 + lk);
+    };
+
+    Quad P[NZ], S[NZ];
+#pragma unroll
+    for (int k = 0; k < NZ; ++k) P[k] = S[k] = quad_zero();
+    float4* xw = a.xw + (size_t)blockIdx.x * a.bz * T + tid;  // the thread's x
+
+    // ---- load x with halo; with a cell field, v = 1 / (2 alpha D): the face
+    // coefficient alpha 2 D D' / (D + D') is 1 / (v + v'), and a copy of the
+    // cell's own v outside the grid gives the boundary face alpha D
+    for (int c = tid; c < (a.bz + 2) * psz / 4; c += T) reinterpret_cast<float4*>(U)[c] = make_float4(0, 0, 0, 0);
+    if (tid == 0) sc_fail = 0;
+    __syncthreads();
+    bool poison = false;  // two neighbours with D = 0: their face coefficient is 0 / 0
+    if (act) {
+#pragma unroll
+        for (int k = 0; k < NZ; ++k) {
+            if (k >= bzn) break;
+            Quad x = quad_zero(), v = quad_zero();
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (i0 + e < a.nx) {
+                    const int64_t c = g0 + k * gsz + e;
+                    at(x, e) = a.x[c];
+                    if (HET) {
+                        const float d = a.D[c];
+                        at(v, e) = __fdiv_rn(a.half_ia, d);
+                        if (d == 0.0f)
+                            poison |= (i0 + e > 0 && a.D[c - 1] == 0.0f) || (i0 + e < a.nx - 1 && a.D[c + 1] == 0.0f) ||
+                                      (y0 + j > 0 && a.D[c - a.nx] == 0.0f) ||
+                                      (y0 + j < a.ny - 1 && a.D[c + a.nx] == 0.0f) ||
+                                      (z0 + k > 0 && a.D[c - gsz] == 0.0f) || (z0 + k < a.nz - 1 && a.D[c + gsz] == 0.0f);
+                    }
+                }
+            quad_st(U + ub + k * psz, x);
+            quad_st(reinterpret_cast<float*>(xw + k * T), x);
+            if (HET) {
+                float* row = Ds + ub + k * psz;
+                quad_st(row, v);
+                if (q == 0) row[-1] = v.a.v[0];
+                if (q == a.quads - 1) row[a.nx - i0] = row[a.nx - i0 - 1];
+            }
+        }
+    }
+    for (int h = tid; h < a.hq; h += T) {
+        int sm, src, slot;
+        int64_t g;
+        halo_at(h, sm, src, slot, g);
+        SH[h] = make_float4(0, 0, 0, 0);
+        HT[h] = make_int2(sm, src < 0 ? -1 : src * a.hq + slot);
+        const int lj = h < 2 * yq ? 0 : (h - 2 * yq) % zq / a.quads, lk = h < 2 * yq ? h % yq / a.quads : 0;
+        if (lj >= byn || lk >= bzn) continue;
+        const int hx = (sm - 4) % a.pitch;  // x of the quad's first cell
+        // the brick's own cell beside a cell outside the grid
+        const int64_t in = h < yq ? a.nx : h < 2 * yq ? -(int64_t)a.nx : h < 2 * yq + zq ? gsz : -gsz;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (hx + e >= a.nx) break;
+            if (src >= 0) U[sm + e] = a.x[g + e];
+            if (HET) Ds[sm + e] = __fdiv_rn(a.half_ia, a.D[src >= 0 ? g + e : g + in + e]);
+        }
+    }
+    __syncthreads();
+
+    // ---- stencil over the thread's column: out(k, u, A u, diag) per plane
+    const V2 onepb = vb<2>(a.onepb), alpha2 = vb<2>(a.op_alpha), six = vb<2>(6.0f), minus = vb<2>(-1.0f);
+    const bool edge_l = lane == 0 || q == 0, edge_r = lane == 31 || q == a.quads - 1;
+    // all threads take part (x neighbours pass between lanes); those without
+    // a quad read their clamped row and call nothing
+    auto column = [&](auto out) {
+        Quad um = quad_ld(U + ub - psz), uc = quad_ld(U + ub), vc, cz;
+        if (HET) {
+            const Quad vm = quad_ld(Ds + ub - psz);
+            vc = quad_ld(Ds + ub);
+            cz = {vrcp(vadd(vc.a, vm.a)), vrcp(vadd(vc.b, vm.b))};
+        }
+#pragma unroll
+        for (int k = 0; k < NZ; ++k) {
+            if (k >= bzn) break;
+            const float* u = U + ub + k * psz;
+            const Quad ym = quad_ld(u - a.pitch), yp = quad_ld(u + a.pitch), un = quad_ld(u + psz);
+            float xl = __shfl_up_sync(0xffffffffu, uc.b.v[1], 1), xr = __shfl_down_sync(0xffffffffu, uc.a.v[0], 1);
+            if (edge_l) xl = u[-1];
+            if (edge_r) xr = u[4];
+            Quad A, dg;
+            if (!HET) {
+                V2 na{{xl + uc.a.v[1], uc.a.v[0] + uc.b.v[0]}}, nb{{uc.a.v[1] + uc.b.v[1], uc.b.v[0] + xr}};
+                na = vadd(vadd(vadd(vadd(na, ym.a), yp.a), um.a), un.a);
+                nb = vadd(vadd(vadd(vadd(nb, ym.b), yp.b), um.b), un.b);
+                // 6 u - (neighbours) before alpha: a coefficient 1 + beta + 6 alpha
+                // rounded to FP32 would shift the mass term by 6 alpha 2^-24
+                A = {vfma(alpha2, vfma(six, uc.a, vmul(minus, na)), vmul(onepb, uc.a)),
+                     vfma(alpha2, vfma(six, uc.b, vmul(minus, nb)), vmul(onepb, uc.b))};
+            } else {
+                const float* d = Ds + ub + k * psz;
+                const Quad vm = quad_ld(d - a.pitch), vp = quad_ld(d + a.pitch), vn = quad_ld(d + psz);
+                float dl = __shfl_up_sync(0xffffffffu, vc.b.v[1], 1), dr = __shfl_down_sync(0xffffffffu, vc.a.v[0], 1);
+                if (edge_l) dl = d[-1];
+                if (edge_r) dr = d[4];
+                // x faces: coefficients and fluxes of the quad's five faces
+                const float c0 = nn_rcp(dl + vc.a.v[0]), c1 = nn_rcp(vc.a.v[0] + vc.a.v[1]);
+                const float c2 = nn_rcp(vc.a.v[1] + vc.b.v[0]), c3 = nn_rcp(vc.b.v[0] + vc.b.v[1]);
+                const float c4 = nn_rcp(vc.b.v[1] + dr);
+                const float f0 = c0 * (uc.a.v[0] - xl), f1 = c1 * (uc.a.v[0] - uc.a.v[1]);
+                const float f2 = c2 * (uc.a.v[1] - uc.b.v[0]), f3 = c3 * (uc.b.v[0] - uc.b.v[1]);
+                const float f4 = c4 * (uc.b.v[1] - xr);
+                auto half = [&](const V2& cx, const V2& fx, const V2& u0, const V2& ym1, const V2& yp1, const V2& um1,
+                                const V2& un1, const V2& v0, const V2& vm1, const V2& vp1, const V2& vn1, V2& czh,
+                                V2& A1, V2& d1) {
+                    const V2 cm = vrcp(vadd(v0, vm1)), cp = vrcp(vadd(v0, vp1)), cn = vrcp(vadd(v0, vn1));
+                    V2 acc = vfma(cm, vsub(u0, ym1), fx);
+                    acc = vfma(cp, vsub(u0, yp1), acc);
+                    acc = vfma(czh, vsub(u0, um1), acc);
+                    acc = vfma(cn, vsub(u0, un1), acc);
+                    A1 = vfma(onepb, u0, acc);
+                    d1 = vadd(vadd(vadd(vadd(vadd(cx, cm), cp), czh), cn), onepb);
+                    czh = cn;
+                };
+                half({{c0 + c1, c1 + c2}}, {{f0 + f1, f2 - f1}}, uc.a, ym.a, yp.a, um.a, un.a, vc.a, vm.a, vp.a, vn.a,
+                     cz.a, A.a, dg.a);
+                half({{c2 + c3, c3 + c4}}, {{f3 - f2, f4 - f3}}, uc.b, ym.b, yp.b, um.b, un.b, vc.b, vm.b, vp.b, vn.b,
+                     cz.b, A.b, dg.b);
+                vc = vn;
+            }
+            if (act) out(k, uc, A, dg);
+            um = uc;
+            uc = un;
+        }
+    };
+    // the four values of plane k on the brick's faces, for the neighbours
+    const bool face[4] = {act && j == 0 && jb > 0, act && j == byn - 1 && jb + 1 < a.nyb, kb > 0, z0 + a.bz < a.nz};
+    auto publish = [&](int k, const Quad& v, uint32_t tag) {
+        Tagged4* f = a.halo + ((size_t)(tag & 1) * a.nb + blockIdx.x) * a.hq;
+        const float c[4] = {v.a.v[0], v.a.v[1], v.b.v[0], v.b.v[1]};
+        auto put = [&](int slot) { st_tagged4(f + slot, c, tag); };
+        if (face[0]) put(k * a.quads + q);
+        if (face[1]) put(yq + k * a.quads + q);
+        if (k == 0 && face[2]) put(2 * yq + j * a.quads + q);
+        if (k == bzn - 1 && face[3]) put(2 * yq + zq + j * a.quads + q);
+    };
+    // the neighbours' faces into out(h, shared place, values); RB quads in flight
+    auto receive = [&](uint32_t tag, auto out) {
+        constexpr int RB = 2;  // (three spill)
+        if (ht < 0) return;
+        const Tagged4* f = a.halo + (size_t)(tag & 1) * a.nb * a.hq;
+        for (int h = ht; h < a.hq; h += RB * hstep) {
+            int2 at[RB];
+            Tagged4 v[RB];
+#pragma unroll
+            for (int m = 0; m < RB; ++m) {
+                at[m] = h + m * hstep < a.hq ? HT[h + m * hstep] : make_int2(0, -1);
+                if (at[m].y >= 0) v[m] = ld_tagged4(f + at[m].y);
+            }
+#pragma unroll
+            for (int m = 0; m < RB; ++m) {
+                if (at[m].y < 0) continue;
+                int it = 0;
+                while (!tagged(v[m], tag)) {
+                    if (++it > POLL_LIMIT || *(volatile int*)&sc_fail) {
+                        sc_fail = 1;
+                        break;
+                    }
+                    v[m] = ld_tagged4(f + at[m].y);
+                }
+                out(h + m * hstep, at[m].x,
+                    make_float4(__uint_as_float((uint32_t)v[m].w[0]), __uint_as_float((uint32_t)v[m].w[1]),
+                                __uint_as_float((uint32_t)v[m].w[2]), __uint_as_float((uint32_t)v[m].w[3])));
+            }
+        }
+    };
+    auto vmask = [&](Quad& v) {  // zeros in the cells past the row's end
+        if (!full)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (i0 + e >= a.nx) at(v, e) = 0.0f;
+    };
+
+    // ---- u0 = M (b - A x0)
+    float acc_b = 0.0f;
+    const V2 idg = vb<2>(a.invd);
+    column([&](int k, const Quad&, const Quad& A, const Quad& dg) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (i0 + e < a.nx) {
+                const float bv = a.b[g0 + k * gsz + e];
+                at(S[k], e) = HET ? __fdividef(bv - at(A, e), at(dg, e)) : (bv - at(A, e)) * a.invd;
+                if (poison) at(S[k], e) = nanf("");
+                acc_b += bv * bv;
+            }
+        publish(k, S[k], base + 1);
+    });
+    __syncthreads();
+    if (act) {
+#pragma unroll
+        for (int k = 0; k < NZ; ++k) {
+            if (k >= bzn) break;
+            quad_st(U + ub + k * psz, S[k]);
+            S[k] = quad_zero();
+        }
+    }
+    receive(base + 1, [&](int, int sm, float4 v) { *reinterpret_cast<float4*>(U + sm) = v; });
+
+    uint32_t tag = base + 2;
+    Pair gamma{0, 0}, alpha{0, 0}, bb{0, 0}, rr{0, 0};  // thread 0
+    int it = -1, stop = 0;
+    float al_prev = 0.0f;
+    bool owed = false;  // x lacks the last direction, al_prev P
+    for (;; ++tag) {
+        __syncthreads();
+        if (sc_fail) break;
+        // ---- w' = M A u, the sums and the faces
+        V2 ag{{0, 0}}, ad{{0, 0}}, ar{{0, 0}};
+        column([&](int k, const Quad& u, const Quad& A, const Quad& dg) {
+            Quad w, r;
+            if (HET) {
+                w = {vmul(A.a, vrcp(dg.a)), vmul(A.b, vrcp(dg.b))};
+                r = {vmul(u.a, dg.a), vmul(u.b, dg.b)};
+                vmask(w);
+                vmask(r);
+            } else {
+                w = {vmul(A.a, idg), vmul(A.b, idg)};
+                r = u;
+                vmask(w);
+            }
+            publish(k, w, tag);
+            quad_st(reinterpret_cast<float*>(W + k * T + tid), w);
+            ag = vfma(r.b, u.b, vfma(r.a, u.a, ag));
+            if (HET) {
+                Quad m = A;
+                vmask(m);
+                ad = vfma(m.b, u.b, vfma(m.a, u.a, ad));
+                ar = vfma(r.b, r.b, vfma(r.a, r.a, ar));
+            } else {
+                ad = vfma(A.b, u.b, vfma(A.a, u.a, ad));
+            }
+        });
+        // block sums: FP32 within a warp, pairs across warps and blocks
+        const float v0 = nn_warp_sumf(ag.v[0] + ag.v[1]), v1 = nn_warp_sumf(ad.v[0] + ad.v[1]);
+        const float v2 = HET ? nn_warp_sumf(ar.v[0] + ar.v[1]) : 0.0f;
+        const float v3 = it < 0 ? nn_warp_sumf(acc_b) : 0.0f;
+        if (lane == 0) {
+            ws[0][warp] = v0;
+            ws[1][warp] = v1;
+            ws[2][warp] = v2;
+            ws[3][warp] = v3;
+        }
+        __syncthreads();
+        const int hl = lane & 15, up = lane >> 4;  // lanes 0-15: g, rho; 16-31: d, (b, b)
+        const int np = (HET || it < 0) ? 2 : 1;    // pairs of sums to exchange: {g, d} and {rho, (b, b)}
+        ulonglong2* rec = a.rec + 4 * (size_t)(tag & 1) * a.nb;
+        if (warp == 0)
+            for (int pr = 0; pr < np; ++pr) {
+                Pair s0{hl < nw ? ws[2 * pr + up][hl] * SUM_SCALE : 0.0f, 0.0f};
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) s0 = pair_add(s0, pair_shfl(s0, o));
+                if (hl == 0)
+                    st_tagged(rec + 4 * blockIdx.x + 2 * pr + up, __float_as_uint(s0.h), __float_as_uint(s0.l), tag);
+            }
+        // x takes two directions every second iteration: loaded here, behind
+        // the wait
+        Quad X[NZ];
+        if (owed && act)
+#pragma unroll
+            for (int k = 0; k < NZ; ++k)
+                if (k < bzn) X[k] = quad_ldcg(xw + k * T);
+        receive(tag, [&](int h, int, float4 v) { WH[h] = v; });
+        // every block adds all blocks' sums in the same order: a record a
+        // thread, then warps, then the first warp
+        for (int c0 = 32 * warp; c0 < a.nb; c0 += T) {
+            const int c = c0 + lane;
+            Pair t[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+            if (c < a.nb) {
+                ulonglong2 v[4];
+#pragma unroll
+                for (int w = 0; w < 4; ++w)
+                    if (w < 2 * np) v[w] = ld_tagged(rec + 4 * c + w);
+#pragma unroll
+                for (int w = 0; w < 4; ++w)
+                    if (w < 2 * np) {
+                        int n = 0;
+                        while (!tagged(v[w], tag)) {
+                            if (++n > POLL_LIMIT || *(volatile int*)&sc_fail) {
+                                sc_fail = 1;
+                                break;
+                            }
+                            v[w] = ld_tagged(rec + 4 * c + w);
+                        }
+                        t[w] = Pair{__uint_as_float((uint32_t)v[w].x), __uint_as_float((uint32_t)v[w].y)};
+                    }
+            }
+            __syncwarp();
+            for (int pr = 0; pr < np; ++pr) {
+                const Pair t0 = pr ? t[2] : t[0], t1 = pr ? t[3] : t[1];
+                Pair r = pair_add(up ? t1 : t0, pair_shfl(up ? t0 : t1, 16));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) r = pair_add(r, pair_shfl(r, o));
+                if (hl == 0) wp[2 * pr + up][c0 >> 5] = r;
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // lane 8 w + i: sum w of the group of blocks i
+            const int w = lane >> 3, i = lane & 7, groups = (a.nb + 31) >> 5;
+            Pair r = i < groups && w < 2 * np ? wp[w][i] : Pair{0, 0};
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) r = pair_add(r, pair_shfl(r, o));
+            const Pair d = pair_shfl(r, 8), r2 = pair_shfl(r, 16), r3 = pair_shfl(r, 24);  // lane 0's
+            if (lane == 0) {
+                const Pair g = HET ? r : pair_mul(r, a.diag);  // constant coefficients: r = diag u
+                rr = HET ? r2 : pair_mul(g, a.diag);
+                if (it < 0) bb = r3;
+                const Pair lim = pair_mul(a.rtol2, bb);
+                const bool met = rr.h < lim.h || (rr.h == lim.h && rr.l <= lim.l);
+                Pair al{0, 0}, be{0, 0};
+                if (it < 0) {
+                    if (d.h != 0.0f) al = pair_div(g, d);
+                    stop = met ? 1 : a.max_iter <= 0 ? 2 : 0;
+                } else {
+                    be = pair_div(g, gamma);
+                    const Pair m = pair_div(pair_mul(be, g), alpha);
+                    const Pair den = pair_add(d, Pair{-m.h, -m.l});
+                    if (den.h != 0.0f) al = pair_div(g, den);
+                    stop = met ? 1 : it + 1 >= a.max_iter ? 2 : !(isfinite(al.h) && isfinite(be.h)) ? 3 : 0;
+                }
+                sc_alpha = al.h;
+                sc_beta = be.h;
+                sc_stop = stop;
+                gamma = g;
+                alpha = al;
+            }
+        }
+        __syncthreads();
+        ++it;
+        if (sc_fail || sc_stop) break;
+        // ---- s', p, x, u (own cells and halo)
+        const float al = sc_alpha, be = sc_beta;
+        if (act) {
+            const V2 al2 = vb<2>(al), nal2 = vb<2>(-al), be2 = vb<2>(be), ap2 = vb<2>(al_prev);
+#pragma unroll
+            for (int k = 0; k < NZ; ++k) {
+                if (k >= bzn) break;
+                float* up = U + ub + k * psz;
+                const Quad w = quad_ld(reinterpret_cast<const float*>(W + k * T + tid)), u = quad_ld(up);
+                S[k] = {vfma(be2, S[k].a, w.a), vfma(be2, S[k].b, w.b)};
+                quad_st(up, {vfma(nal2, S[k].a, u.a), vfma(nal2, S[k].b, u.b)});
+                const Quad p{vfma(be2, P[k].a, u.a), vfma(be2, P[k].b, u.b)};
+                if (owed) {
+                    const Quad x{vfma(ap2, P[k].a, X[k].a), vfma(ap2, P[k].b, X[k].b)};
+                    quad_st(reinterpret_cast<float*>(xw + k * T), {vfma(al2, p.a, x.a), vfma(al2, p.b, x.b)});
+                }
+                P[k] = p;
+            }
+        }
+        al_prev = al;
+        owed = !owed;
+        if (ht >= 0)
+            for (int h = ht; h < a.hq; h += hstep) {
+                const int2 at = HT[h];
+                if (at.y < 0) continue;
+                const float4 w = WH[h];
+                float4 s = SH[h];
+                s = make_float4(w.x + be * s.x, w.y + be * s.y, w.z + be * s.z, w.w + be * s.w);
+                SH[h] = s;
+                float4* up = reinterpret_cast<float4*>(U + at.x);
+                const float4 u = *up;
+                *up = make_float4(u.x - al * s.x, u.y - al * s.y, u.z - al * s.z, u.w - al * s.w);
+            }
+    }
+    if (act) {
+#pragma unroll
+        for (int k = 0; k < NZ; ++k) {
+            if (k >= bzn) break;
+            Quad x = quad_ldcg(xw + k * T);
+            if (owed) x = {vfma(vb<2>(al_prev), P[k].a, x.a), vfma(vb<2>(al_prev), P[k].b, x.b)};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (i0 + e < a.nx) a.x[g0 + k * gsz + e] = at(x, e);
+        }
+    }
+    if (tid == 0) {
+        if (sc_fail) {
+            a.flags[2] = 1;
+            a.flags[0] = 3;
+        } else if (blockIdx.x == 0) {
+            a.flags[0] = stop;
+            a.flags[1] = it;
+            a.flags[2] = 0;
+            a.scal[0] = ((double)rr.h + rr.l) / SUM_SCALE;
+            a.scal[1] = ((double)bb.h + bb.l) / SUM_SCALE;
+            *a.epoch = tag + 2;
+        }
+    }
+}
+
+template <bool HET>
+const void* kernel_of(int nz)
+{
+    switch (nz) {
+        case 1: return (const void*)k_rcg<1, HET>;
+        case 2: return (const void*)k_rcg<2, HET>;
+        case 3: return (const void*)k_rcg<3, HET>;
+        case 4: return (const void*)k_rcg<4, HET>;
+        case 5: return (const void*)k_rcg<5, HET>;
+        case 6: return HET ? nullptr : (const void*)k_rcg<6, false>;
+        case 7: return HET ? nullptr : (const void*)k_rcg<7, false>;
+        default: return nullptr;
+    }
+}
+}  // namespace
+
+static Pair split(double v)
+{
+    const float h = (float)v;
+    return {h, (float)(v - (double)h)};
+}
+
+struct nn_rcg_plan {
+    nn_ctx* ctx = nullptr;
+    RcgArgs a{};
+    const void* kernel = nullptr;
+    int threads = 0;
+    size_t smem = 0, rec_bytes = 0, halo_bytes = 0;
+    bool timing = false;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    float last_ms = 0.0f;
+    int last_iters = 0;
+};
+
+void nn_rcg_plan_destroy(nn_rcg_plan* pl)
+{
+    if (!pl) return;
+    if (pl->ctx) cudaStreamSynchronize(pl->ctx->stream);
+    nn_release(pl->a.xw);
+    nn_release(pl->a.rec);
+    nn_release(pl->a.halo);
+    nn_release(pl->a.epoch);
+    nn_release(pl->a.scal);
+    nn_release(pl->a.flags);
+    if (pl->e0) cudaEventDestroy(pl->e0);
+    if (pl->e1) cudaEventDestroy(pl->e1);
+    nn_ctx* ctx = pl->ctx;
+    delete pl;
+    nn_ctx_release(ctx);
+}
+
+static nn_status rcg_reset(nn_rcg_plan* pl, cudaStream_t cs)
+{
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->a.rec, 0, pl->rec_bytes, cs));
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->a.halo, 0, pl->halo_bytes, cs));
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->a.epoch, 0, sizeof(unsigned), cs));
+    return NN_OK;
+}
+
+// Brick of the grid: the (by, bz) whose blocks fit the chip (one a SM, threads
+// and shared memory) at the least estimated cycles of an iteration.  Measured
+// on bricks of 8 to 512 quads a plane: a plane costs about 600 cycles of
+// latency and 1.3 a quad, 1.6 times that with a cell field; a round of halo
+// loads (two a thread, the first warp has none) about 600.
+static bool rcg_shape(const nn_ctx* ctx, bool het, RcgArgs& a, int& threads, size_t& smem)
+{
+    const int quads = (a.nx + 3) / 4, limit = std::min(ctx->num_sms, MAX_BLOCKS);
+    const int nzmax = het ? 5 : 7;
+    if (quads > RT) return false;
+    double best = 0.0;
+    for (int by = 1; by <= std::min(a.ny, RT / quads); ++by)
+        for (int bz = 1; bz <= std::min(a.nz, nzmax); ++bz) {
+            const int nyb = (a.ny + by - 1) / by;
+            const int64_t nb = (int64_t)nyb * ((a.nz + bz - 1) / bz);
+            if (nb > limit) continue;
+            // a thread polls one block's sums, and spare warps share the halo
+            const int Q = quads * by, T = std::max(192, (Q + 31) / 32 * 32);
+            const int pitch = 4 * quads + 8, hq = 2 * quads * (by + bz);
+            const size_t sm = (size_t)(bz + 2) * (by + 2) * pitch * 4 * (het ? 2 : 1) +
+                              ((size_t)bz * T + 2 * (size_t)hq) * 16 + (size_t)hq * 8;
+            if (sm > 225 * 1024) continue;
+            const double cost = (het ? 1.6 : 1.0) * bz * (600.0 + 1.3 * Q) +
+                                600.0 * ((hq + 2 * (T - 32) - 1) / (2 * (T - 32))) + 3.0 * nb;
+            if (best > 0.0 && cost >= best) continue;
+            best = cost;
+            a.by = by; a.bz = bz; a.nyb = nyb; a.nb = (int)nb;
+            a.quads = quads; a.pitch = pitch; a.hq = hq;
+            threads = T;
+            smem = sm;
+        }
+    return best > 0.0;
+}
+
+// NN_ERR_UNSUPPORTED when the grid does not fit (the caller keeps its other
+// solvers).  D stays owned by the caller and is read at each solve.
+nn_status nn_rcg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D,
+                             nn_rcg_plan** out)
+{
+    *out = nullptr;
+    RcgArgs a{};
+    a.nx = nx; a.ny = ny; a.nz = nz;
+    int threads = 0, coop = 0;
+    size_t smem = 0;
+    if (!rcg_shape(ctx, D != nullptr, a, threads, smem)) return NN_ERR_UNSUPPORTED;
+    const void* kernel = D ? kernel_of<true>(a.bz) : kernel_of<false>(a.bz);
+    if (!kernel) return NN_ERR_UNSUPPORTED;
+    NN_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+    NN_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024));
+    int per_sm = 0;
+    NN_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    if (!coop || per_sm < 1) return NN_ERR_UNSUPPORTED;
+    a.op_alpha = (float)alpha;
+    a.onepb = (float)(1.0 + beta);
+    a.invd = (float)(1.0 / (1.0 + beta + 6.0 * alpha));
+    a.half_ia = (float)(0.5 / alpha);
+    a.diag = split(1.0 / (double)a.invd);
+    a.D = D;
+    nn_rcg_plan* pl = new nn_rcg_plan();
+    pl->ctx = ctx;
+    nn_ctx_retain(ctx);
+    pl->a = a;
+    pl->kernel = kernel;
+    pl->threads = threads;
+    pl->smem = smem;
+    pl->rec_bytes = sizeof(ulonglong2) * 8 * (size_t)a.nb;
+    pl->halo_bytes = sizeof(Tagged4) * 2 * (size_t)a.nb * a.hq;
+    nn_status st = nn_alloc(ctx, &pl->a.rec, 8 * (size_t)a.nb);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->a.xw, (size_t)a.nb * a.bz * threads);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->a.halo, 2 * (size_t)a.nb * a.hq);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->a.epoch, 1);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->a.scal, 2);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->a.flags, 4);
+    if (st == NN_OK) st = rcg_reset(pl, ctx->stream);
+    if (st != NN_OK) {
+        nn_rcg_plan_destroy(pl);
+        return st;
+    }
+    // solves may run on other streams
+    st = nn_cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "nn_rcg_plan_create");
+    if (st != NN_OK) {
+        nn_rcg_plan_destroy(pl);
+        return st;
+    }
+    *out = pl;
+    return NN_OK;
+}
+
+void nn_rcg_set_timing(nn_rcg_plan* pl, bool on) { pl->timing = on; }
+void nn_rcg_last_timing(const nn_rcg_plan* pl, float* ms, int* iters)
+{
+    *ms = pl->last_ms;
+    *iters = pl->last_iters;
+}
+
+// The whole solve on stream cs (x: initial guess in, solution out).
+nn_status nn_rcg_begin(nn_rcg_plan* pl, const float* d_b, float* d_x, double rtol, int max_iter, cudaStream_t cs)
+{
+    nn_ctx* ctx = pl->ctx;
+    pl->a.b = d_b;
+    pl->a.x = d_x;
+    pl->a.rtol2 = split(rtol * rtol);
+    pl->a.max_iter = max_iter;
+    if (pl->timing && !pl->e0) {
+        NN_CUDA(ctx, cudaEventCreate(&pl->e0));
+        NN_CUDA(ctx, cudaEventCreate(&pl->e1));
+    }
+    if (pl->timing) NN_CUDA(ctx, cudaEventRecord(pl->e0, cs));
+    void* args[] = {&pl->a};
+    NN_CUDA(ctx, cudaLaunchCooperativeKernel(pl->kernel, dim3(pl->a.nb), dim3(pl->threads), args, pl->smem, cs));
+    ctx->launches++;
+    if (pl->timing) NN_CUDA(ctx, cudaEventRecord(pl->e1, cs));
+    return NN_OK;
+}
+
+nn_status nn_rcg_finish(nn_rcg_plan* pl, cudaStream_t cs, int* iters, double* relres, int* converged)
+{
+    nn_ctx* ctx = pl->ctx;
+    int h_flags[4] = {0, 0, 0, 0};
+    double h_scal[2] = {0.0, 0.0};
+    NN_CUDA(ctx, cudaMemcpyAsync(h_flags, pl->a.flags, sizeof h_flags, cudaMemcpyDeviceToHost, cs));
+    NN_CUDA(ctx, cudaMemcpyAsync(h_scal, pl->a.scal, sizeof h_scal, cudaMemcpyDeviceToHost, cs));
+    NN_CUDA(ctx, cudaStreamSynchronize(cs));
+    if (h_flags[2]) {
+        NN_TRY(rcg_reset(pl, cs));
+        NN_CUDA(ctx, cudaMemsetAsync(pl->a.flags, 0, sizeof h_flags, cs));
+        NN_CUDA(ctx, cudaStreamSynchronize(cs));
+        return nn_fail(ctx, NN_ERR_TIMEOUT, "k_rcg: a block's wait for its neighbours gave up");
+    }
+    if (pl->timing) {
+        NN_CUDA(ctx, cudaEventElapsedTime(&pl->last_ms, pl->e0, pl->e1));
+        pl->last_iters = h_flags[1];
+    }
+    if (iters) *iters = h_flags[1];
+    if (relres) *relres = h_scal[1] > 0 ? std::sqrt(h_scal[0] / h_scal[1]) : 0.0;
+    if (converged) *converged = h_flags[0] == 1;
+    return NN_OK;
+}
