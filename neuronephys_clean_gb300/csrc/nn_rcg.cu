@@ -40,6 +40,7 @@
 
 #include "nn_hh.cuh"
 #include "nn_internal.cuh"
+#include "nn_pair.cuh"
 
 namespace {
 constexpr int RT = 512;               // most threads of a block
@@ -95,33 +96,8 @@ __device__ __forceinline__ bool tagged(const ulonglong2& v, uint32_t tag)
 // 8^3 cells took 5.1 us with FP64 sums and scalars and takes 3.1 us with pairs
 // (the solutions' errors against FP64 are the same).  Sums are kept scaled by
 // SUM_SCALE, so that adding thousands of warps does not overflow.
-struct Pair {
-    float h, l;
-};
 constexpr float SUM_SCALE = 1.0f / 4096.0f;
 
-__device__ __forceinline__ Pair pair_norm(float h, float l)
-{
-    const float s = __fadd_rn(h, l);
-    return {s, __fsub_rn(l, __fsub_rn(s, h))};
-}
-__device__ __forceinline__ Pair pair_add(const Pair& x, const Pair& y)
-{
-    const float s = __fadd_rn(x.h, y.h), t = __fsub_rn(s, x.h);
-    const float e = __fadd_rn(__fsub_rn(x.h, __fsub_rn(s, t)), __fsub_rn(y.h, t));
-    return pair_norm(s, __fadd_rn(e, __fadd_rn(x.l, y.l)));
-}
-__device__ __forceinline__ Pair pair_mul(const Pair& x, const Pair& y)
-{
-    const float p = __fmul_rn(x.h, y.h);
-    return pair_norm(p, __fmaf_rn(x.l, y.h, __fmaf_rn(x.h, y.l, __fmaf_rn(x.h, y.h, -p))));
-}
-__device__ __forceinline__ Pair pair_div(const Pair& x, const Pair& y)
-{
-    const float q = __fdividef(x.h, y.h);
-    const float r = __fadd_rn(__fmaf_rn(-q, y.h, x.h), __fmaf_rn(-q, y.l, x.l));
-    return pair_norm(q, __fdividef(r, y.h));
-}
 __device__ __forceinline__ Pair pair_shfl(const Pair& x, int o)
 {
     return {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};

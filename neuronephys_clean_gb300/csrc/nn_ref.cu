@@ -9,6 +9,7 @@
 
 #include "nn_hh.cuh"
 #include "nn_internal.cuh"
+#include "nn_pair.cuh"
 
 // =============================================================== leapfrog ==
 
@@ -29,6 +30,9 @@ extern "C" void nn_leapfrog_params_reference(nn_leapfrog_params* p, int variant)
 }
 
 namespace {
+// small blocks: a network of 15k neurons then spreads over most of the chip
+constexpr int LF_THREADS = 64;
+
 struct LFVars { float* v[NN_HH_NUM_VARS]; };
 
 // Leapfrog_HH (src/ephys.cu:28-96), evaluated in the precision the
@@ -45,21 +49,136 @@ struct LFVars { float* v[NN_HH_NUM_VARS]; };
 // lies within 1e-9 of zero, fused or not (the neighbouring floats give
 // 3.8e-7), so the test is an FP32 compare, off the FP64 pipe that bounds
 // this kernel.
-__device__ __forceinline__ float lf_rate_am(float V)
+__device__ __noinline__ float lf_rate_am(float V)
 {
     if (V == -35.0f) return 1.0f;
     return (float)((3.5 + 0.1 * V) / (1 - exp(-3.5 - 0.1 * V)));
 }
 
-__device__ __forceinline__ float lf_rate_an(float V)
+__device__ __noinline__ float lf_rate_an(float V)
 {
     if (V == -50.0f) return 0.1f;
     return (float)((-0.5 - 0.01 * V) / (exp(-5 - 0.1 * V) - 1));
 }
 
-// One neuron's step (zi: its standard-normal noise draw).
+__device__ __noinline__ float lf_rate_bh(float V) { return (float)(1 / (exp(-3 - 0.1 * V) + 1)); }
+
+// The same roundings without the FP64 pipe.  It issues one warp instruction
+// in 16 cycles, and the five FP64 expressions of a neuron (three exponentials
+// and four divisions among them) held the step at 181 us per million neurons (38 us now, 78 % issue-active).
+// Here they are evaluated in pairs of floats to about 2^-43; where the result
+// lies so near the midpoint of two floats (2^-39 relative) that this cannot
+// say how FP64 rounds, and close to the two singularities, where the FP64
+// expression itself cancels, the FP64 expression is evaluated after all
+// (A. Ziv, "Fast evaluation of elementary mathematical functions with
+// correctly rounded last bit", ACM TOMS 17, 1991).  All three exponentials
+// are e^{-V/10} times a constant; that one is table-driven (P. T. P. Tang,
+// "Table-driven implementation of the exponential function in IEEE
+// floating-point arithmetic", ACM TOMS 15, 1989): 2^(j/32) sits in lane j of
+// the warp and comes by shuffle, the remainder |s| <= ln 2 / 64 by its series.
+
+// 2^(j/32) as pairs
+__device__ const Pair lf_exp_table[32] = {
+    {0x1p+0f, 0.0f}, {0x1.059b0ep+0f, -0x1.9d4f52p-25f}, {0x1.0b5586p+0f, 0x1.9f3122p-25f}, {0x1.11301ep+0f, -0x1.fdb496p-25f},
+    {0x1.172b84p+0f, -0x1.c15742p-27f}, {0x1.1d4874p+0f, -0x1.d2e8cap-25f}, {0x1.2387a6p+0f, 0x1.ceac48p-25f}, {0x1.29e9ep+0f, -0x1.5c0424p-25f},
+    {0x1.306fep+0f, 0x1.4636e2p-25f}, {0x1.371a74p+0f, -0x1.18aac6p-25f}, {0x1.3dea64p+0f, 0x1.824684p-25f}, {0x1.44e086p+0f, 0x1.8624b4p-30f},
+    {0x1.4bfdaep+0f, -0x1.593abcp-25f}, {0x1.5342b6p+0f, -0x1.2c561p-25f}, {0x1.5ab07ep+0f, -0x1.5bd5ecp-27f}, {0x1.6247ecp+0f, -0x1.f8b55p-25f},
+    {0x1.6a09e6p+0f, 0x1.9fcef4p-26f}, {0x1.71f75ep+0f, 0x1.1d8beep-25f}, {0x1.7a1148p+0f, -0x1.829fdp-25f}, {0x1.82589ap+0f, -0x1.accc7cp-26f},
+    {0x1.8ace54p+0f, 0x1.15506ep-27f}, {0x1.93737cp+0f, -0x1.e64744p-25f}, {0x1.9c4918p+0f, 0x1.51f848p-27f}, {0x1.a5503cp+0f, -0x1.b83b54p-25f},
+    {0x1.ae89fap+0f, -0x1.a94b14p-26f}, {0x1.b7f77p+0f, -0x1.a09438p-25f}, {0x1.c199bep+0f, -0x1.3d56b2p-27f}, {0x1.cb720ep+0f, -0x1.8837ccp-27f},
+    {0x1.d5818ep+0f, -0x1.822dbcp-27f}, {0x1.dfc974p+0f, -0x1.908c94p-25f}, {0x1.ea4afap+0f, 0x1.52486cp-27f}, {0x1.f50766p+0f, -0x1.246ebp-26f}};
+
+// e^{-V/10} with 0.1 as the double 0.1, |V| <= 400; all lanes of the warp.
+// tab: lane j's table entry; x receives V/10.
+__device__ __forceinline__ Pair lf_exp_tenth(float V, const Pair& tab, Pair& x)
+{
+    const float ph = __fmul_rn(0x1.99999ap-4f, V);
+    x = pair_norm(ph, __fmaf_rn(-0x1.99999ap-30f, V, __fmaf_rn(0x1.99999ap-4f, V, -ph)));
+    const float n = rintf(x.h * -0x1.715476p+5f);  // 32 / ln 2
+    // s = -x - n ln2/32: the first 13 bits of ln2/32 make an exact product and
+    // an exact difference, two more floats the rest
+    const float a = __fmaf_rn(-n, 0x1.62ep-6f, -x.h);
+    const float c = __fmul_rn(n, 0x1.0bfbe8p-20f), e = __fmaf_rn(n, 0x1.0bfbe8p-20f, -c);
+    Pair s = pair_two_sum(a, -c);
+    s = pair_norm(s.h, __fsub_rn(__fsub_rn(s.l, e), __fmaf_rn(n, 0x1.cf79acp-45f, x.l)));
+    // e^s - 1 = s + s^2/2 + s^3 (1/6 + s/24 + s^2/120)
+    const float h2 = __fmul_rn(s.h, s.h), l2 = __fmaf_rn(2.0f * s.h, s.l, __fmaf_rn(s.h, s.h, -h2));
+    const float cub = h2 * s.h * (1.0f / 6.0f + s.h * (1.0f / 24.0f + s.h * (1.0f / 120.0f)));
+    const Pair m = pair_add(s, Pair{0.5f * h2, __fadd_rn(0.5f * l2, cub)});
+    const int k = (int)n;
+    const Pair t{__shfl_sync(0xffffffffu, tab.h, k & 31), __shfl_sync(0xffffffffu, tab.l, k & 31)};
+    const Pair r = pair_add(t, pair_mul(t, m));
+    const float p2 = __int_as_float((127 + (k >> 5)) << 23);
+    return {r.h * p2, r.l * p2};
+}
+
+// a / (1 - e^{-a}) = 1 + a/2 + a^2/12 - a^4/720 + a^6/30240 - ... for |a| < 0.35
+__device__ __forceinline__ Pair lf_series(const Pair& a)
+{
+    const Pair z = pair_mul(a, a), z2 = pair_mul(z, z);
+    const float y = z.h;
+    const float rest =
+        y * y * y * (1.0f / 30240.0f + y * (-1.0f / 1209600.0f + y * (1.0f / 47900160.0f + y * -5.28419014e-10f)));
+    const Pair t = pair_add(pair_mul(z, Pair{0x1.555556p-4f, -0x1.555556p-29f}),    // 1/12
+                            pair_mul(z2, Pair{-0x1.6c16c2p-10f, 0x1.27d27ep-35f}));  // -1/720
+    const Pair r = pair_add(pair_add(Pair{1.0f, 0.0f}, Pair{0.5f * a.h, 0.5f * a.l}), t);
+    return pair_norm(r.h, __fadd_rn(r.l, rest));
+}
+
+// Whether every value within 2^-39 (relative) of h + l rounds to h.
+__device__ __forceinline__ bool lf_rounds(const Pair& r) { return __fmaf_rn(r.l, 1.0f + 0x1p-13f, r.h) == r.h; }
+
+// alpha_m, alpha_n and beta_h of the reference's expressions (all lanes).
+__device__ __forceinline__ void lf_rates(float V, const Pair& tab, float& am, float& an, float& bh)
+{
+    const bool in = fabsf(V) <= 400.0f;
+    Pair x;
+    const Pair e = lf_exp_tenth(in ? V : 0.0f, tab, x);
+    const Pair e1 = pair_mul(e, Pair{0x1.eec102p-6f, -0x1.c6c026p-32f});  // e^{-3.5 - V/10}
+    const Pair e2 = pair_mul(e, Pair{0x1.b993fep-8f, 0x1.aa6ec4p-41f});   // e^{-5 - V/10}
+    const Pair e3 = pair_mul(e, Pair{0x1.97db0cp-5f, 0x1.99d616p-30f});   // e^{-3 - V/10}
+    const Pair a1 = pair_add(Pair{3.5f, 0.0f}, x), a2 = pair_add(Pair{5.0f, 0.0f}, x);
+    const Pair m = fabsf(a1.h) < 0.35f ? lf_series(a1)
+                                       : pair_div(a1, pair_add(Pair{1.0f, 0.0f}, Pair{-e1.h, -e1.l}));
+    // numerator 0.5 + 0.01 V with the double 0.01: a2/10 - 3.47e-19 V
+    Pair n;
+    if (fabsf(a2.h) < 0.35f) {
+        const Pair f = lf_series(a2);
+        n = pair_mul(f, Pair{0x1.99999ap-4f, -0x1.99999ap-30f});
+        n = pair_norm(n.h, __fadd_rn(n.l, __fdividef(-3.46944695e-19f * V * f.h, a2.h)));
+    } else {
+        const float ph = __fmul_rn(0x1.47ae14p-7f, V);
+        const Pair q = pair_norm(ph, __fmaf_rn(0x1.eb851ep-33f, V, __fmaf_rn(0x1.47ae14p-7f, V, -ph)));
+        n = pair_div(pair_add(Pair{0.5f, 0.0f}, q), pair_add(Pair{1.0f, 0.0f}, Pair{-e2.h, -e2.l}));
+    }
+    const Pair h = pair_div(Pair{1.0f, 0.0f}, pair_add(e3, Pair{1.0f, 0.0f}));
+    am = m.h;
+    an = n.h;
+    bh = h.h;
+    if (!(in && lf_rounds(m) && fabsf(a1.h) > 0x1p-12f)) am = lf_rate_am(V);
+    if (!(in && lf_rounds(n) && fabsf(a2.h) > 0x1p-12f)) an = lf_rate_an(V);
+    if (!(in && lf_rounds(h))) bh = lf_rate_bh(V);
+}
+
+// (float)(0.07 * e) and (float)(Tmax / (1.0 + e)) of a float e >= 0
+__device__ __noinline__ float lf_seven_fp64(float e) { return (float)(0.07 * e); }
+__device__ __noinline__ float lf_sigmoid_fp64(float Tmax, float e) { return (float)(Tmax / (1.0 + e)); }
+__device__ __forceinline__ float lf_seven(float e)
+{
+    const Pair r = pair_mulf(Pair{0x1.1eb852p-4f, -0x1.47ae14p-32f}, e);
+    return e > 1e-25f && e < 1e30f && lf_rounds(r) ? r.h : lf_seven_fp64(e);
+}
+__device__ __forceinline__ float lf_sigmoid(float Tmax, float e)
+{
+    const Pair r = pair_div(Pair{Tmax, 0.0f}, pair_two_sum(1.0f, e));
+    return e < 1e15f && fabsf(Tmax) > 1e-10f && fabsf(Tmax) < 1e10f && lf_rounds(r) ? r.h : lf_sigmoid_fp64(Tmax, e);
+}
+
+// One neuron's step (zi: its standard-normal noise draw; tab: the lane's entry
+// of the exponential's table).  All lanes of the warp take part; those with
+// store unset compute a neuron that is there and write nothing.
 __device__ __forceinline__ void lf_neuron(const LFVars& s, int i, float timestep, const nn_leapfrog_params& p,
-                                          float zi)
+                                          float zi, const Pair& tab, bool store)
 {
     {
         const float local_in = s.v[NN_HH_LOCAL_IN][i], local_num_in = s.v[NN_HH_LOCAL_COUNT][i];
@@ -69,12 +188,11 @@ __device__ __forceinline__ void lf_neuron(const LFVars& s, int i, float timestep
         const float V = s.v[NN_HH_V][i], M = s.v[NN_HH_M][i], N = s.v[NN_HH_N][i], H = s.v[NN_HH_H][i];
         const float local_Y = s.v[NN_HH_LOCAL_Y][i], IY = s.v[NN_HH_IY][i], EY = s.v[NN_HH_EY][i];
 
-        const float Am = lf_rate_am(V);
-        const float An = lf_rate_an(V);
-        const float Ah = (float)(0.07 * expf(-V / 20 - 3));
+        float Am, An, Bh;
+        lf_rates(V, tab, Am, An, Bh);
+        const float Ah = lf_seven(expf(-V / 20 - 3));
         const float Bm = 4 * expf(-(V + 60) / 18);
-        const float Bn = (float)(0.125 * expf(-(V + 60) / 80));
-        const float Bh = (float)(1 / (exp(-3 - 0.1 * V) + 1));
+        const float Bn = 0.125f * expf(-(V + 60) / 80);  // a power of two: no rounding of its own
 
         const float new_M = (Am * timestep + (1 - timestep / 2 * (Am + Bm)) * M) / (timestep / 2 * (Am + Bm) + 1);
         const float new_N = (An * timestep + (1 - timestep / 2 * (An + Bn)) * N) / (timestep / 2 * (An + Bn) + 1);
@@ -117,6 +235,8 @@ __device__ __forceinline__ void lf_neuron(const LFVars& s, int i, float timestep
         float num = __fmaf_rn(E, timestep, __fmul_rn(__fadd_rn(white_noise, appcur), timestep));
         num = __fmaf_rn(__fmaf_rn(-half_dt, G, 1.0f), V, num);
         const float nV = __fdiv_rn(num, __fmaf_rn(half_dt, G, 1.0f));
+        const float out = lf_sigmoid(p.Tmax, expf(-(nV - p.Vt) / p.Kp));
+        if (!store) return;
         s.v[NN_HH_V][i] = nV;
         s.v[NN_HH_M][i] = new_M;
         s.v[NN_HH_N][i] = new_N;
@@ -124,32 +244,25 @@ __device__ __forceinline__ void lf_neuron(const LFVars& s, int i, float timestep
         s.v[NN_HH_LOCAL_Y][i] = new_local_Y;
         s.v[NN_HH_IY][i] = new_IY;
         s.v[NN_HH_EY][i] = new_EY;
-        const float out = (float)(p.Tmax / (1.0 + expf(-(nV - p.Vt) / p.Kp)));
         s.v[NN_HH_LOCAL_OUTPUT][i] = out;
         s.v[NN_HH_IOUTPUT][i] = out;
         s.v[NN_HH_EOUTPUT][i] = out;
     }
 }
 
-// A thread steps the neuron pair (2k, 2k + 1), which shares one draw of the
-// counter-based noise stream (the pair's two Box-Muller outputs).
+// A neuron per thread.  It draws its pair's two Box-Muller outputs and takes
+// its own: the draw costs 6 % more instructions than a pair per thread would,
+// and a network of 15k neurons has twice the warps to hide its latency with.
 template <bool EXT_Z>
-__global__ void __launch_bounds__(256) k_leapfrog(LFVars s, int n, float timestep, nn_leapfrog_params p,
-                                                  uint64_t seed, uint64_t step, const float* __restrict__ z)
+__global__ void __launch_bounds__(LF_THREADS) k_leapfrog(LFVars s, int n, float timestep, nn_leapfrog_params p,
+                                                         uint64_t seed, uint64_t step, const float* __restrict__ z)
 {
-    const int pairs = (n + 1) >> 1;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < pairs; k += gridDim.x * blockDim.x) {
-        const int i0 = 2 * k;
-        const bool two = i0 + 1 < n;
-        float z0, z1;
-        if (EXT_Z) {
-            z0 = z[i0];
-            z1 = two ? z[i0 + 1] : 0.0f;
-        } else {
-            nn_normal_pair(seed, (uint32_t)k, step, z0, z1);
-        }
-        lf_neuron(s, i0, timestep, p, z0);
-        if (two) lf_neuron(s, i0 + 1, timestep, p, z1);
+    const int lane = threadIdx.x & 31;
+    const Pair tab = lf_exp_table[lane];
+    // whole warps: lanes past the last neuron repeat it
+    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const int i = min(i0 + lane, n - 1);
+        lf_neuron(s, i, timestep, p, EXT_Z ? z[i] : nn_normal(seed, (uint32_t)i, step), tab, i0 + lane < n);
     }
 }
 
@@ -163,9 +276,9 @@ nn_status leapfrog_launch(nn_ctx* ctx, float* const* vars, int n, float dt, cons
         if (!vars[q]) return nn_fail(ctx, NN_ERR_INVALID_ARG, "%s: sim_vars[%d] is NULL", what, q);
         s.v[q] = vars[q];
     }
-    const int grid = nn_grid_for(ctx, ((int64_t)n + 1) / 2, 256, 64);
-    if (d_z) k_leapfrog<true><<<grid, 256, 0, ctx->stream>>>(s, n, dt, *p, seed, step, d_z);
-    else k_leapfrog<false><<<grid, 256, 0, ctx->stream>>>(s, n, dt, *p, seed, step, nullptr);
+    const int grid = nn_grid_for(ctx, n, LF_THREADS, 64);
+    if (d_z) k_leapfrog<true><<<grid, LF_THREADS, 0, ctx->stream>>>(s, n, dt, *p, seed, step, d_z);
+    else k_leapfrog<false><<<grid, LF_THREADS, 0, ctx->stream>>>(s, n, dt, *p, seed, step, nullptr);
     NN_CHECK_LAUNCH(ctx, "k_leapfrog");
     return NN_OK;
 }
