@@ -764,15 +764,15 @@ struct nn_paracrine {
     float* w8 = nullptr;
     float* u = nullptr;          // density
     float* Ax = nullptr;         // scatter accumulator
-    float *lap = nullptr, *x = nullptr, *b = nullptr, *r = nullptr, *pv = nullptr, *Ap = nullptr;
+    float *un = nullptr, *x = nullptr, *b = nullptr, *r = nullptr, *p0 = nullptr, *p1 = nullptr, *Ap = nullptr;
     float* at_neurons = nullptr;    // density_at_neurons
     float* generated = nullptr;     // density_generated_at_neurons
     float* g_out = nullptr;         // d_g_paracrine (caller's)
     double* scal = nullptr;         // [0]=rr [1]=pAp [2]=rr_new
-    double* partials = nullptr;
-    unsigned int* ticket = nullptr;
-    int* done = nullptr;            // convergence flag
-    int nparts = 0;
+    double* partials = nullptr;     // [2][nparts]
+    unsigned int* bar = nullptr;    // grid barrier of k_cn_solve
+    int* done = nullptr;            // [0] outcome [1] iterations [2] a wait gave up
+    int nparts = 0;                 // blocks of k_cn_solve
 };
 
 extern "C" void nn_paracrine_ref_params_default(nn_paracrine_ref_params* p)
@@ -864,152 +864,162 @@ __global__ void k_fine(int n, const int* list, const int* count, float* gen, flo
     }
 }
 
-// zero-padded 3x3x3 correlation (af::convolve3 with AF_CONV_DEFAULT), x fastest
-__global__ void k_conv27(const float* in, float* out, int nx, int ny, int nz, Stencil27 K, const int* done)
+// The whole Crank-Nicolson solve (update_density, src/paracrine.cu:63-134) in
+// one cooperative launch: density += deposits, right-hand side and initial
+// guess from its Laplacian, up to max_iter CG iterations, commit.  As separate
+// launches it was 106 kernels of 2.6-4 us each whatever the iteration count
+// (about 4 are needed); here an iteration is two passes over the block's cells
+// (vectors in L2) and two grid barriers.  The direction p = r + beta p is
+// formed at the 27 neighbours as they are read (p alternates between two
+// buffers), which saves a third barrier.
+//
+// Barrier: a counter that every block adds to, behind a fence; each block's
+// first thread polls it (bounded).  Sums: FP64 per thread, block partials,
+// added by every block in the same order after the barrier.
+constexpr int CN_THREADS = 512;
+constexpr int CN_POLLS = 1 << 22;  // some seconds
+
+struct CnArgs {
+    int nx, ny, nz, max_iter;
+    int64_t G;
+    Stencil27 L, A;
+    float a, bb, c, d;         // x0 = a u + bb lap, b = c u + d lap
+    float tol;
+    const float* dep;          // deposits
+    float *u, *un, *x, *b, *r, *p0, *p1, *Ap;
+    double* scal;              // out: [0] rr of the last direction [1] pAp [2] rr
+    double* partials;          // [2][blocks]
+    unsigned* bar;
+    int* done;                 // out: [0] 1 converged, 2 nothing to do  [1] iterations  [2] a wait gave up
+};
+
+template <class I>
+__global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
 {
-    if (done && *done) return;
-    const int64_t G = (int64_t)nx * ny * nz;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < G; c += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(c % nx);
-        const int j = (int)((c / nx) % ny);
-        const int k = (int)(c / ((int64_t)nx * ny));
+    __shared__ double ws[CN_THREADS / 32];
+    __shared__ double total;
+    __shared__ int fail;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const I stride = (I)gridDim.x * CN_THREADS, c0 = (I)blockIdx.x * CN_THREADS + tid, G = (I)q.G;
+    unsigned phase = 0;
+    if (tid == 0) fail = 0;
+    __syncthreads();
+    // grid barrier; with sum set, the grid total of v in `total`
+    auto barrier = [&](bool sum, double v) {
+        double* part = q.partials + (phase & 1) * gridDim.x;
+        if (sum) {
+            v = nn_warp_sum(v);
+            if (lane == 0) ws[w] = v;
+        }
+        __syncthreads();
+        ++phase;
+        if (tid == 0) {
+            if (sum) {
+                double s = 0.0;
+                for (int k = 0; k < CN_THREADS / 32; ++k) s += ws[k];
+                part[blockIdx.x] = s;
+            }
+            __threadfence();
+            atomicAdd(q.bar, 1u);
+            int n = 0;
+            while (*(volatile unsigned*)q.bar < phase * gridDim.x)
+                if (++n > CN_POLLS) {
+                    fail = 1;
+                    break;
+                }
+            __threadfence();
+        }
+        __syncthreads();
+        if (sum && w == 0) {
+            double s = 0.0;
+            for (unsigned k = lane; k < gridDim.x; k += 32) s += ((volatile double*)part)[k];
+            s = nn_warp_sum(s);
+            if (lane == 0) total = s;
+        }
+        __syncthreads();
+    };
+    // zero-padded 3x3x3 correlation (af::convolve3 with AF_CONV_DEFAULT), x fastest
+    auto conv = [&](I c, const Stencil27& K, auto val) {
+        const int i = (int)(c % (I)q.nx), j = (int)((c / (I)q.nx) % (I)q.ny), k = (int)(c / ((I)q.nx * (I)q.ny));
         float acc = 0.0f;
 #pragma unroll
-        for (int dz = -1; dz <= 1; ++dz) {
-            const int kk = k + dz;
-            if (kk < 0 || kk >= nz) continue;
+        for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
-            for (int dy = -1; dy <= 1; ++dy) {
-                const int jj = j + dy;
-                if (jj < 0 || jj >= ny) continue;
+            for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
                 for (int dx = -1; dx <= 1; ++dx) {
-                    const int ii = i + dx;
-                    if (ii < 0 || ii >= nx) continue;
-                    acc += K.k[(dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)] * in[ii + (int64_t)nx * (jj + (int64_t)ny * kk)];
+                    const int ii = i + dx, jj = j + dy, kk = k + dz;
+                    if (ii < 0 || ii >= q.nx || jj < 0 || jj >= q.ny || kk < 0 || kk >= q.nz) continue;
+                    acc += K.k[(dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)] * val((I)ii + (I)q.nx * ((I)jj + (I)q.ny * (I)kk));
                 }
-            }
+        return acc;
+    };
+    // written by other blocks during this launch: read past L1
+    auto cg = [](const float* p) { return __ldcg(p); };
+
+    for (I c = c0; c < G; c += stride) {
+        auto val = [&](I n) { return q.u[n] + q.dep[n]; };
+        const float lap = conv(c, q.L, val), un = val(c);
+        q.un[c] = un;
+        q.x[c] = q.a * un + q.bb * lap;
+        q.b[c] = q.c * un + q.d * lap;
+    }
+    barrier(false, 0.0);
+    double acc = 0.0;
+    for (I c = c0; c < G; c += stride) {
+        const float rv = q.b[c] - conv(c, q.A, [&](I n) { return cg(q.x + n); });
+        q.r[c] = rv;
+        acc += (double)rv * rv;
+    }
+    barrier(true, acc);
+    double rr = total, pap = 0.0, rr_new = 0.0;
+    int done = rr < (double)q.tol ? 2 : 0, it = 0;
+    float beta = 0.0f;
+    float *p_old = q.p1, *p_new = q.p0;
+    while (!done && it < q.max_iter && !fail) {
+        acc = 0.0;
+        for (I c = c0; c < G; c += stride) {
+            auto val = [&](I n) { return it ? cg(q.r + n) + beta * cg(p_old + n) : cg(q.r + n); };
+            const float pv = val(c), ap = conv(c, q.A, val);
+            p_new[c] = pv;
+            q.Ap[c] = ap;
+            acc += (double)pv * ap;
         }
-        out[c] = acc;
+        barrier(true, acc);
+        pap = total;
+        const float alpha = (float)(rr / pap);
+        acc = 0.0;
+        for (I c = c0; c < G; c += stride) {
+            q.x[c] += alpha * p_new[c];
+            const float rv = q.r[c] - alpha * q.Ap[c];
+            q.r[c] = rv;
+            acc += (double)rv * rv;
+        }
+        barrier(true, acc);
+        rr_new = total;
+        ++it;
+        if (rr_new < (double)q.tol) {
+            done = 1;
+        } else {
+            beta = (float)(rr_new / rr);
+            rr = rr_new;
+            float* t = p_old;
+            p_old = p_new;
+            p_new = t;
+        }
     }
-}
-
-__global__ void k_add(float* u, const float* a, int64_t G)
-{
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < G; q += (int64_t)gridDim.x * blockDim.x)
-        u[q] += a[q];
-}
-
-// x = a*u + b*lap ; y = c*u + d*lap
-__global__ void k_cn_init(const float* u, const float* lap, float* x, float* b, int64_t G, float a, float bb, float c,
-                          float d)
-{
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < G; q += (int64_t)gridDim.x * blockDim.x) {
-        x[q] = a * u[q] + bb * lap[q];
-        b[q] = c * u[q] + d * lap[q];
+    // density = x unless the initial residual already met the tolerance (src/paracrine.cu:114-116)
+    for (I c = c0; c < G; c += stride) q.u[c] = done == 2 ? q.un[c] : q.x[c];
+    if (tid == 0) {
+        if (fail) q.done[2] = 1;
+        if (blockIdx.x == 0) {
+            q.done[0] = done;
+            q.done[1] = it;
+            q.scal[0] = rr;
+            q.scal[1] = pap;
+            q.scal[2] = rr_new;
+        }
     }
-}
-
-// Finish a grid-wide FP64 sum: block partial -> last block reduces in a fixed order.
-__device__ bool last_block_reduce(double v, double* partials, unsigned int* ticket, double* result)
-{
-    __shared__ double ws[32];
-    __shared__ bool is_last;
-    v = nn_warp_sum(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) ws[w] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += ws[q];
-        partials[blockIdx.x] = s;
-        __threadfence();
-        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!is_last) return false;
-    // the last block sums the partials with all its threads (fixed order)
-    __threadfence();
-    double s = 0.0;
-    for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) s += ((volatile double*)partials)[q];
-    s = nn_warp_sum(s);
-    __syncthreads();
-    if (lane == 0) ws[w] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += ws[q];
-        *result = t;
-        *ticket = 0;
-    }
-    __syncthreads();
-    return true;
-}
-
-// r = b - Ax ; p = r ; rr = (r, r); done = rr < tol
-__global__ void k_cn_residual(const float* b, const float* Ax, float* r, float* p, int64_t G, double* partials,
-                              unsigned int* ticket, double* scal, int* done, float tol)
-{
-    double acc = 0.0;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < G; q += (int64_t)gridDim.x * blockDim.x) {
-        const float rv = b[q] - Ax[q];
-        r[q] = rv;
-        p[q] = rv;
-        acc += (double)rv * rv;
-    }
-    if (last_block_reduce(acc, partials, ticket, &scal[0]) && threadIdx.x == 0) *done = scal[0] < (double)tol ? 2 : 0;
-}
-
-// pAp = (p, Ap)
-__global__ void k_cn_pap(const float* p, const float* Ap, int64_t G, double* partials, unsigned int* ticket,
-                         double* scal, const int* done)
-{
-    if (*done) return;
-    double acc = 0.0;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < G; q += (int64_t)gridDim.x * blockDim.x)
-        acc += (double)p[q] * Ap[q];
-    last_block_reduce(acc, partials, ticket, &scal[1]);
-}
-
-// x += a p ; r -= a Ap ; rr_new = (r, r); converged -> done; else p = r + beta p (next kernel)
-__global__ void k_cn_update(float* x, float* r, const float* p, const float* Ap, int64_t G, double* partials,
-                            unsigned int* ticket, double* scal, int* done, float tol, int* iters)
-{
-    if (*done) return;
-    const float alpha = (float)(scal[0] / scal[1]);
-    double acc = 0.0;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < G; q += (int64_t)gridDim.x * blockDim.x) {
-        x[q] += alpha * p[q];
-        const float rv = r[q] - alpha * Ap[q];
-        r[q] = rv;
-        acc += (double)rv * rv;
-    }
-    if (last_block_reduce(acc, partials, ticket, &scal[2]) && threadIdx.x == 0) {
-        *iters += 1;
-        if (scal[2] < (double)tol) *done = 1;
-    }
-}
-
-__global__ void k_cn_direction(float* p, const float* r, int64_t G, double* scal, const int* done)
-{
-    if (*done) return;
-    const float beta = (float)(scal[2] / scal[0]);
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < G; q += (int64_t)gridDim.x * blockDim.x)
-        p[q] = r[q] + beta * p[q];
-}
-
-__global__ void k_cn_roll(double* scal, const int* done)
-{
-    if (*done) return;
-    scal[0] = scal[2];
-}
-
-// data = x unless the initial residual already met the tolerance (src/paracrine.cu:114-116)
-__global__ void k_cn_commit(float* u, const float* x, int64_t G, const int* done)
-{
-    if (*done == 2) return;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < G; q += (int64_t)gridDim.x * blockDim.x)
-        u[q] = x[q];
 }
 }  // namespace
 
@@ -1027,14 +1037,14 @@ extern "C" nn_status nn_paracrine_ref_create(nn_ctx* ctx, const nn_paracrine_ref
     pm->G = (int64_t)p->nx * p->ny * p->nz;
     pm->g_out = d_g_paracrine;
     const size_t G = (size_t)pm->G, N = (size_t)(n > 0 ? n : 1);
-    pm->nparts = nn_grid_for(ctx, pm->G, 256, 4);
+    pm->nparts = nn_grid_for(ctx, pm->G, CN_THREADS, 1);  // co-resident: one block a SM at most
     nn_status st = NN_OK;
 #define PM_ALLOC(ptr, cnt) if (st == NN_OK) st = nn_alloc(ctx, &pm->ptr, cnt)
     PM_ALLOC(idx8, 8 * N); PM_ALLOC(w8, 8 * N);
-    PM_ALLOC(u, G); PM_ALLOC(Ax, G); PM_ALLOC(lap, G); PM_ALLOC(x, G); PM_ALLOC(b, G);
-    PM_ALLOC(r, G); PM_ALLOC(pv, G); PM_ALLOC(Ap, G);
+    PM_ALLOC(u, G); PM_ALLOC(Ax, G); PM_ALLOC(un, G); PM_ALLOC(x, G); PM_ALLOC(b, G);
+    PM_ALLOC(r, G); PM_ALLOC(p0, G); PM_ALLOC(p1, G); PM_ALLOC(Ap, G);
     PM_ALLOC(at_neurons, N); PM_ALLOC(generated, N);
-    PM_ALLOC(scal, 4); PM_ALLOC(partials, (size_t)pm->nparts); PM_ALLOC(ticket, 1); PM_ALLOC(done, 2);
+    PM_ALLOC(scal, 4); PM_ALLOC(partials, 2 * (size_t)pm->nparts); PM_ALLOC(bar, 1); PM_ALLOC(done, 3);
 #undef PM_ALLOC
     if (st != NN_OK) {
         nn_paracrine_destroy(pm);
@@ -1044,7 +1054,7 @@ extern "C" nn_status nn_paracrine_ref_create(nn_ctx* ctx, const nn_paracrine_ref
     cudaMemsetAsync(pm->u, 0, sizeof(float) * G, s);
     cudaMemsetAsync(pm->generated, 0, sizeof(float) * N, s);
     cudaMemsetAsync(pm->at_neurons, 0, sizeof(float) * N, s);
-    cudaMemsetAsync(pm->ticket, 0, sizeof(unsigned int), s);
+    cudaMemsetAsync(pm->done, 0, 3 * sizeof(int), s);
     if (n > 0) {
         k_trilinear<<<nn_grid_for(ctx, n, 256, 16), 256, 0, s>>>(n, d_x, d_y, d_z, p->nx, p->ny, p->nz, p->h, pm->idx8,
                                                                   pm->w8);
@@ -1067,10 +1077,11 @@ extern "C" nn_status nn_paracrine_destroy(nn_paracrine* pm)
 {
     if (!pm) return NN_OK;
     if (pm->ctx) cudaStreamSynchronize(pm->ctx->stream);
-    nn_release(pm->idx8); nn_release(pm->w8); nn_release(pm->u); nn_release(pm->Ax); nn_release(pm->lap);
-    nn_release(pm->x); nn_release(pm->b); nn_release(pm->r); nn_release(pm->pv); nn_release(pm->Ap);
+    nn_release(pm->idx8); nn_release(pm->w8); nn_release(pm->u); nn_release(pm->Ax); nn_release(pm->un);
+    nn_release(pm->x); nn_release(pm->b); nn_release(pm->r); nn_release(pm->p0); nn_release(pm->p1);
+    nn_release(pm->Ap);
     nn_release(pm->at_neurons); nn_release(pm->generated); nn_release(pm->scal); nn_release(pm->partials);
-    nn_release(pm->ticket); nn_release(pm->done);
+    nn_release(pm->bar); nn_release(pm->done);
     nn_ctx* ctx = pm->ctx;
     delete pm;
     nn_ctx_release(ctx);
@@ -1098,7 +1109,6 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
     cudaStream_t s = ctx->stream;
     const auto& p = pm->p;
     const int64_t G = pm->G;
-    const int gb = pm->nparts;
     const int nb = nn_grid_for(ctx, pm->n, 256, 16);
     // scatter_to_grid: Ax = G^T generated; density += Ax (src/paracrine.cu:276-287)
     NN_CUDA(ctx, cudaMemsetAsync(pm->Ax, 0, sizeof(float) * (size_t)G, s));
@@ -1117,35 +1127,25 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
         A.k[q] = (float)(-0.5 * p.D * dt * lq);
     }
     A.k[13] = (float)((double)A.k[13] + 1.0 + 0.5 * dt * p.decay);
-    k_add<<<gb, 256, 0, s>>>(pm->u, pm->Ax, G);  // density += Ax
-    NN_CHECK_LAUNCH(ctx, "k_add");
-    k_conv27<<<gb, 256, 0, s>>>(pm->u, pm->lap, p.nx, p.ny, p.nz, L, nullptr);
-    NN_CHECK_LAUNCH(ctx, "k_conv27(L)");
     const double c = p.quirk_rhs ? h : dt;
-    k_cn_init<<<gb, 256, 0, s>>>(pm->u, pm->lap, pm->x, pm->b, G, (float)(1.0 - dt * p.decay), (float)(dt * p.D),
-                                 (float)(1.0 - c * p.decay / 2.0), (float)(c * p.D / 2.0));
-    NN_CHECK_LAUNCH(ctx, "k_cn_init");
-    k_conv27<<<gb, 256, 0, s>>>(pm->x, pm->Ap, p.nx, p.ny, p.nz, A, nullptr);
-    NN_CHECK_LAUNCH(ctx, "k_conv27(A x0)");
-    NN_CUDA(ctx, cudaMemsetAsync(pm->done, 0, 2 * sizeof(int), s));
-    k_cn_residual<<<gb, 256, 0, s>>>(pm->b, pm->Ap, pm->r, pm->pv, G, pm->partials, pm->ticket, pm->scal, pm->done,
-                                     p.abs_tol);
-    NN_CHECK_LAUNCH(ctx, "k_cn_residual");
-    for (int it = 0; it < p.max_iter; ++it) {
-        k_conv27<<<gb, 256, 0, s>>>(pm->pv, pm->Ap, p.nx, p.ny, p.nz, A, pm->done);
-        NN_CHECK_LAUNCH(ctx, "k_conv27(A p)");
-        k_cn_pap<<<gb, 256, 0, s>>>(pm->pv, pm->Ap, G, pm->partials, pm->ticket, pm->scal, pm->done);
-        NN_CHECK_LAUNCH(ctx, "k_cn_pap");
-        k_cn_update<<<gb, 256, 0, s>>>(pm->x, pm->r, pm->pv, pm->Ap, G, pm->partials, pm->ticket, pm->scal, pm->done,
-                                       p.abs_tol, pm->done + 1);
-        NN_CHECK_LAUNCH(ctx, "k_cn_update");
-        k_cn_direction<<<gb, 256, 0, s>>>(pm->pv, pm->r, G, pm->scal, pm->done);
-        NN_CHECK_LAUNCH(ctx, "k_cn_direction");
-        k_cn_roll<<<1, 1, 0, s>>>(pm->scal, pm->done);
-        NN_CHECK_LAUNCH(ctx, "k_cn_roll");
-    }
-    k_cn_commit<<<gb, 256, 0, s>>>(pm->u, pm->x, G, pm->done);
-    NN_CHECK_LAUNCH(ctx, "k_cn_commit");
+    CnArgs q{p.nx, p.ny, p.nz, p.max_iter, G, L, A};
+    q.a = (float)(1.0 - dt * p.decay);
+    q.bb = (float)(dt * p.D);
+    q.c = (float)(1.0 - c * p.decay / 2.0);
+    q.d = (float)(c * p.D / 2.0);
+    q.tol = p.abs_tol;
+    q.dep = pm->Ax;
+    q.u = pm->u; q.un = pm->un; q.x = pm->x; q.b = pm->b; q.r = pm->r;
+    q.p0 = pm->p0; q.p1 = pm->p1; q.Ap = pm->Ap;
+    q.scal = pm->scal;
+    q.partials = pm->partials;
+    q.bar = pm->bar;
+    q.done = pm->done;
+    NN_CUDA(ctx, cudaMemsetAsync(pm->bar, 0, sizeof(unsigned), s));
+    void* args[] = {&q};
+    NN_CUDA(ctx, cudaLaunchCooperativeKernel(G <= INT32_MAX / 2 ? (const void*)k_cn_solve<int> : (const void*)k_cn_solve<int64_t>,
+                                             dim3(pm->nparts), dim3(CN_THREADS), args, 0, s));
+    ctx->launches++;
     // interpolate, reset sources, copy out (src/paracrine.cuh:259-264)
     if (pm->n > 0) {
         k_interp<<<nb, 256, 0, s>>>(pm->n, pm->idx8, pm->w8, pm->u, G, pm->at_neurons, pm->g_out);
@@ -1153,7 +1153,7 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
         NN_CUDA(ctx, cudaMemsetAsync(pm->generated, 0, sizeof(float) * (size_t)pm->n, s));
     }
     if (std::getenv("NN_DEBUG_PARACRINE")) {
-        int h_done[2];
+        int h_done[3];
         double h_scal[3];
         std::vector<float> hu((size_t)G), hx((size_t)G), hax((size_t)G);
         cudaMemcpyAsync(h_done, pm->done, sizeof h_done, cudaMemcpyDeviceToHost, s);
@@ -1168,11 +1168,15 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
                 h_done[0], h_done[1], h_scal[0], h_scal[1], h_scal[2], su, sx, sa);
     }
     if (iters || final_rr) {
-        int h_done[2];
+        int h_done[3];
         double h_scal[3];
-        NN_CUDA(ctx, cudaMemcpyAsync(h_done, pm->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        NN_CUDA(ctx, cudaMemcpyAsync(h_done, pm->done, sizeof h_done, cudaMemcpyDeviceToHost, s));
         NN_CUDA(ctx, cudaMemcpyAsync(h_scal, pm->scal, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
         NN_CUDA(ctx, cudaStreamSynchronize(s));
+        if (h_done[2]) {
+            NN_CUDA(ctx, cudaMemsetAsync(pm->done, 0, 3 * sizeof(int), s));
+            return nn_fail(ctx, NN_ERR_TIMEOUT, "k_cn_solve: a grid barrier gave up");
+        }
         if (iters) *iters = h_done[1];
         if (final_rr) *final_rr = (float)(h_done[1] == 0 ? h_scal[0] : (h_done[0] == 1 ? h_scal[2] : h_scal[0]));
     }
