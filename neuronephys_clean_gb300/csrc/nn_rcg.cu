@@ -37,6 +37,7 @@
 // another, so the launch is cooperative; every poll is bounded.
 #include <algorithm>
 #include <cmath>
+#include <map>
 
 #include "nn_hh.cuh"
 #include "nn_internal.cuh"
@@ -150,16 +151,18 @@ __device__ __forceinline__ Quad quad_zero() { return {{{0, 0}}, {{0, 0}}}; }
 __device__ __forceinline__ float& at(Quad& q, int e) { return e < 2 ? q.a.v[e] : q.b.v[e - 2]; }
 __device__ __forceinline__ float at(const Quad& q, int e) { return e < 2 ? q.a.v[e] : q.b.v[e - 2]; }
 
+// One solve by the a.nb blocks that call this with ranks 0 .. a.nb - 1, first
+// tag base + 1.  Returns the last tag used; fail: a wait gave up.
 template <int NZ, bool HET>
-__global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
+__device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, const uint32_t base, float4* smem4,
+                                              bool& fail)
 {
-    extern __shared__ float4 smem4[];
     __shared__ float ws[4][RT / 32];
     __shared__ Pair wp[4][8];
     __shared__ float sc_alpha, sc_beta;
     __shared__ int sc_stop, sc_fail;
     const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    const int jb = blockIdx.x % a.nyb, kb = blockIdx.x / a.nyb;
+    const int jb = rank % a.nyb, kb = rank / a.nyb;
     const int y0 = jb * a.by, z0 = kb * a.bz;
     const int byn = min(a.by, a.ny - y0), bzn = min(a.bz, a.nz - z0);
     const int rows = a.by + 2, psz = rows * a.pitch;  // shared plane
@@ -176,7 +179,6 @@ __global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
     const int64_t gsz = (int64_t)a.nx * a.ny;
     const int64_t g0 = i0 + (int64_t)a.nx * (y0 + j) + gsz * z0;
     const bool full = i0 + 4 <= a.nx;
-    const uint32_t base = *reinterpret_cast<volatile unsigned*>(a.epoch);
     // halo duty is on all warps but the first (there are two or more), which
     // polls the sums
     const int ht = tid - 32, hstep = T - 32, nw = T >> 5;
@@ -193,13 +195,13 @@ __global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
         if (f < 2) {
             lk = line;
             lj = f ? byn : -1;
-            src = f ? (jb + 1 < a.nyb ? (int)blockIdx.x + 1 : -1) : (jb > 0 ? (int)blockIdx.x - 1 : -1);
+            src = f ? (jb + 1 < a.nyb ? rank + 1 : -1) : (jb > 0 ? rank - 1 : -1);
             slot = (f ? 0 : yq) + r;
             if (lk >= bzn) src = -1;
         } else {
             lj = line;
             lk = f == 3 ? bzn : -1;
-            src = f == 3 ? (z0 + a.bz < a.nz ? (int)blockIdx.x + a.nyb : -1) : (kb > 0 ? (int)blockIdx.x - a.nyb : -1);
+            src = f == 3 ? (z0 + a.bz < a.nz ? rank + a.nyb : -1) : (kb > 0 ? rank - a.nyb : -1);
             slot = 2 * yq + (f == 3 ? 0 : zq) + r;
             if (lj >= byn) src = -1;
         }
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
     Quad P[NZ], S[NZ];
 #pragma unroll
     for (int k = 0; k < NZ; ++k) P[k] = S[k] = quad_zero();
-    float4* xw = a.xw + (size_t)blockIdx.x * a.bz * T + tid;  // the thread's x
+    float4* xw = a.xw + (size_t)rank * a.bz * T + tid;  // the thread's x
 
     // ---- load x with halo; with a cell field, v = 1 / (2 alpha D): the face
     // coefficient alpha 2 D D' / (D + D') is 1 / (v + v'), and a copy of the
@@ -337,7 +339,7 @@ __global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
     // the four values of plane k on the brick's faces, for the neighbours
     const bool face[4] = {act && j == 0 && jb > 0, act && j == byn - 1 && jb + 1 < a.nyb, kb > 0, z0 + a.bz < a.nz};
     auto publish = [&](int k, const Quad& v, uint32_t tag) {
-        Tagged4* f = a.halo + ((size_t)(tag & 1) * a.nb + blockIdx.x) * a.hq;
+        Tagged4* f = a.halo + ((size_t)(tag & 1) * a.nb + rank) * a.hq;
         const float c[4] = {v.a.v[0], v.a.v[1], v.b.v[0], v.b.v[1]};
         auto put = [&](int slot) { st_tagged4(f + slot, c, tag); };
         if (face[0]) put(k * a.quads + q);
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) s0 = pair_add(s0, pair_shfl(s0, o));
                 if (hl == 0)
-                    st_tagged(rec + 4 * blockIdx.x + 2 * pr + up, __float_as_uint(s0.h), __float_as_uint(s0.l), tag);
+                    st_tagged(rec + 4 * rank + 2 * pr + up, __float_as_uint(s0.h), __float_as_uint(s0.l), tag);
             }
         // x takes two directions every second iteration: loaded here, behind
         // the wait
@@ -584,18 +586,127 @@ __global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
                 if (i0 + e < a.nx) a.x[g0 + k * gsz + e] = at(x, e);
         }
     }
+    fail = sc_fail;
     if (tid == 0) {
-        if (sc_fail) {
+        if (fail) {
             a.flags[2] = 1;
             a.flags[0] = 3;
-        } else if (blockIdx.x == 0) {
+        } else if (rank == 0) {
             a.flags[0] = stop;
             a.flags[1] = it;
             a.flags[2] = 0;
             a.scal[0] = ((double)rr.h + rr.l) / SUM_SCALE;
             a.scal[1] = ((double)bb.h + bb.l) / SUM_SCALE;
-            *a.epoch = tag + 2;
         }
+    }
+    return tag;
+}
+
+template <int NZ, bool HET>
+__global__ void __launch_bounds__(RT, 1) k_rcg(const RcgArgs a)
+{
+    extern __shared__ float4 smem4[];
+    bool fail;
+    const uint32_t base = *reinterpret_cast<volatile unsigned*>(a.epoch);
+    const uint32_t tag = rcg_solve<NZ, HET>(a, blockIdx.x, base, smem4, fail);
+    if (!fail && blockIdx.x == 0 && threadIdx.x == 0) *a.epoch = tag + 2;
+}
+
+// Many independent solves in one launch (the fields of a batch of networks).
+// The blocks are split into groups; a group solves the instances of its list
+// one after another.  Before each it exchanges a tag that says every block has
+// left the previous solve (its buffers may be written again) and carries the
+// last tag used, since a block without a brick in a solve has not counted its
+// iterations.
+struct RcgGroup {
+    int first, count, width;   // its instances in the list, its blocks
+    int64_t rec, halo, xw;     // its parts of the buffers
+};
+struct RcgBatchArgs {
+    const RcgArgs* inst;       // per instance: shape and operator
+    const int64_t* off;        // first cell of each instance
+    const int2* block;         // per block: group, rank
+    const RcgGroup* group;
+    const int* list;
+    const float* b;
+    float* x;
+    ulonglong2* start;         // [2][blocks]: tags of the exchange before a solve
+    uint32_t seq;              // first of those tags
+    unsigned* epoch;           // per group
+    double* scal;              // [instances][2]
+    int* flags;                // [instances][4]
+    Pair rtol2;
+    int max_iter;
+};
+
+template <int NZ>
+__global__ void __launch_bounds__(RT, 1) k_rcg_batch(const RcgBatchArgs B)
+{
+    extern __shared__ float4 smem4[];
+    __shared__ RcgArgs a;
+    __shared__ unsigned last;
+    __shared__ int gave_up;
+    const int tid = threadIdx.x, rank = B.block[blockIdx.x].y, first = (int)blockIdx.x - rank;
+    const RcgGroup g = B.group[B.block[blockIdx.x].x];
+    unsigned* epoch = B.epoch + B.block[blockIdx.x].x;
+    uint32_t tag = *reinterpret_cast<volatile unsigned*>(epoch);
+    if (tid == 0) gave_up = 0;
+    for (int k = 0; k < g.count; ++k) {
+        const uint32_t s = B.seq + k;
+        ulonglong2* slot = B.start + (size_t)(s & 1) * gridDim.x + first;
+        __syncthreads();
+        if (tid == 0) {
+            last = 0;
+            const int q = B.list[g.first + k];
+            a = B.inst[q];
+            a.b = B.b + B.off[q];
+            a.x = B.x + B.off[q];
+            a.flags = B.flags + 4 * q;
+            a.scal = B.scal + 2 * q;
+            a.rtol2 = B.rtol2;
+            a.max_iter = B.max_iter;
+            st_tagged(slot + rank, tag, 0, s);
+        }
+        __syncthreads();
+        if (tid < g.width) {
+            int n = 0;
+            ulonglong2 v = ld_tagged(slot + tid);
+            while (!tagged(v, s)) {
+                if (++n > POLL_LIMIT) {
+                    gave_up = 1;
+                    break;
+                }
+                v = ld_tagged(slot + tid);
+            }
+            atomicMax(&last, (unsigned)v.x);
+        }
+        __syncthreads();
+        if (gave_up) {
+            if (tid == 0) {
+                a.flags[2] = 1;
+                a.flags[0] = 3;
+            }
+            return;
+        }
+        tag = last;
+        bool fail = false;
+        if (rank < a.nb) tag = rcg_solve<NZ, false>(a, rank, tag, smem4, fail);
+        if (fail) return;
+    }
+    // the group's blocks have all read it: they have been through the last start
+    if (rank == 0 && tid == 0) *epoch = tag + 2;
+}
+
+const void* batch_kernel_of(int nz)
+{
+    switch (nz) {
+        case 1: return (const void*)k_rcg_batch<1>;
+        case 2: return (const void*)k_rcg_batch<2>;
+        case 3: return (const void*)k_rcg_batch<3>;
+        case 4: return (const void*)k_rcg_batch<4>;
+        case 5: return (const void*)k_rcg_batch<5>;
+        case 6: return (const void*)k_rcg_batch<6>;
+        default: return (const void*)k_rcg_batch<7>;
     }
 }
 
@@ -619,6 +730,15 @@ static Pair split(double v)
 {
     const float h = (float)v;
     return {h, (float)(v - (double)h)};
+}
+
+static void rcg_operator(RcgArgs& a, double alpha, double beta)
+{
+    a.op_alpha = (float)alpha;
+    a.onepb = (float)(1.0 + beta);
+    a.invd = (float)(1.0 / (1.0 + beta + 6.0 * alpha));
+    a.half_ia = (float)(0.5 / alpha);
+    a.diag = split(1.0 / (double)a.invd);
 }
 
 struct nn_rcg_plan {
@@ -663,11 +783,13 @@ static nn_status rcg_reset(nn_rcg_plan* pl, cudaStream_t cs)
 // on bricks of 8 to 512 quads a plane: a plane costs about 600 cycles of
 // latency and 1.3 a quad, 1.6 times that with a cell field; a round of halo
 // loads (two a thread, the first warp has none) about 600.
-static bool rcg_shape(const nn_ctx* ctx, bool het, RcgArgs& a, int& threads, size_t& smem)
+// limit: blocks to use at most; all_threads: blocks of RT threads.  Returns the
+// estimate, 0 where nothing fits.
+static double rcg_shape(int limit, bool het, bool all_threads, RcgArgs& a, int& threads, size_t& smem)
 {
-    const int quads = (a.nx + 3) / 4, limit = std::min(ctx->num_sms, MAX_BLOCKS);
+    const int quads = (a.nx + 3) / 4;
     const int nzmax = het ? 5 : 7;
-    if (quads > RT) return false;
+    if (quads > RT) return 0.0;
     double best = 0.0;
     for (int by = 1; by <= std::min(a.ny, RT / quads); ++by)
         for (int bz = 1; bz <= std::min(a.nz, nzmax); ++bz) {
@@ -675,7 +797,7 @@ static bool rcg_shape(const nn_ctx* ctx, bool het, RcgArgs& a, int& threads, siz
             const int64_t nb = (int64_t)nyb * ((a.nz + bz - 1) / bz);
             if (nb > limit) continue;
             // a thread polls one block's sums, and spare warps share the halo
-            const int Q = quads * by, T = std::max(192, (Q + 31) / 32 * 32);
+            const int Q = quads * by, T = all_threads ? RT : std::max(192, (Q + 31) / 32 * 32);
             const int pitch = 4 * quads + 8, hq = 2 * quads * (by + bz);
             const size_t sm = (size_t)(bz + 2) * (by + 2) * pitch * 4 * (het ? 2 : 1) +
                               ((size_t)bz * T + 2 * (size_t)hq) * 16 + (size_t)hq * 8;
@@ -689,7 +811,7 @@ static bool rcg_shape(const nn_ctx* ctx, bool het, RcgArgs& a, int& threads, siz
             threads = T;
             smem = sm;
         }
-    return best > 0.0;
+    return best;
 }
 
 // NN_ERR_UNSUPPORTED when the grid does not fit (the caller keeps its other
@@ -702,7 +824,8 @@ nn_status nn_rcg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, 
     a.nx = nx; a.ny = ny; a.nz = nz;
     int threads = 0, coop = 0;
     size_t smem = 0;
-    if (!rcg_shape(ctx, D != nullptr, a, threads, smem)) return NN_ERR_UNSUPPORTED;
+    if (rcg_shape(std::min(ctx->num_sms, MAX_BLOCKS), D != nullptr, false, a, threads, smem) == 0.0)
+        return NN_ERR_UNSUPPORTED;
     const void* kernel = D ? kernel_of<true>(a.bz) : kernel_of<false>(a.bz);
     if (!kernel) return NN_ERR_UNSUPPORTED;
     NN_CUDA(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
@@ -710,11 +833,7 @@ nn_status nn_rcg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, 
     int per_sm = 0;
     NN_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     if (!coop || per_sm < 1) return NN_ERR_UNSUPPORTED;
-    a.op_alpha = (float)alpha;
-    a.onepb = (float)(1.0 + beta);
-    a.invd = (float)(1.0 / (1.0 + beta + 6.0 * alpha));
-    a.half_ia = (float)(0.5 / alpha);
-    a.diag = split(1.0 / (double)a.invd);
+    rcg_operator(a, alpha, beta);
     a.D = D;
     nn_rcg_plan* pl = new nn_rcg_plan();
     pl->ctx = ctx;
@@ -794,5 +913,252 @@ nn_status nn_rcg_finish(nn_rcg_plan* pl, cudaStream_t cs, int* iters, double* re
     if (iters) *iters = h_flags[1];
     if (relres) *relres = h_scal[1] > 0 ? std::sqrt(h_scal[0] / h_scal[1]) : 0.0;
     if (converged) *converged = h_flags[0] == 1;
+    return NN_OK;
+}
+
+// ------------------------------------------------------------------ batches --
+
+struct nn_rcg_batch {
+    nn_ctx* ctx = nullptr;
+    int n_inst = 0, blocks = 0, longest = 0;
+    const void* kernel = nullptr;
+    size_t smem = 0;
+    RcgBatchArgs B{};
+    RcgArgs* inst = nullptr;
+    int64_t* off = nullptr;
+    int2* block = nullptr;
+    RcgGroup* group = nullptr;
+    int* list = nullptr;
+    ulonglong2* rec = nullptr;
+    Tagged4* halo = nullptr;
+    float4* xw = nullptr;
+    size_t n_rec = 0, n_halo = 0, groups = 0;
+};
+
+void nn_rcg_batch_destroy(nn_rcg_batch* pl)
+{
+    if (!pl) return;
+    if (pl->ctx) cudaStreamSynchronize(pl->ctx->stream);
+    nn_release(pl->inst); nn_release(pl->off); nn_release(pl->block); nn_release(pl->group); nn_release(pl->list);
+    nn_release(pl->rec); nn_release(pl->halo); nn_release(pl->xw);
+    nn_release(pl->B.start); nn_release(pl->B.epoch); nn_release(pl->B.scal); nn_release(pl->B.flags);
+    nn_ctx* ctx = pl->ctx;
+    delete pl;
+    nn_ctx_release(ctx);
+}
+
+static nn_status batch_reset(nn_rcg_batch* pl, cudaStream_t cs)
+{
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->rec, 0, sizeof(ulonglong2) * pl->n_rec, cs));
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->halo, 0, sizeof(Tagged4) * pl->n_halo, cs));
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->B.start, 0, sizeof(ulonglong2) * 2 * (size_t)pl->blocks, cs));
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->B.epoch, 0, sizeof(unsigned) * pl->groups, cs));
+    pl->B.seq = 1;
+    return NN_OK;
+}
+
+// Groups and their lists: columns of blocks, filled with instances from the
+// largest side down so that no column is estimated to run longer than a bound;
+// the least bound for which the columns fit the chip, by bisection.  An
+// instance's estimate is the cycles of an iteration on the column's blocks
+// times its side, to which its iterations are about proportional.
+// NN_ERR_UNSUPPORTED when an instance does not fit.
+nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const int64_t* off, double alpha_unit,
+                              double beta, nn_rcg_batch** out)
+{
+    *out = nullptr;
+    const int sms = std::min(ctx->num_sms, MAX_BLOCKS);
+    struct Shape {
+        double cost = 0.0;
+        RcgArgs a{};
+        size_t smem = 0;
+    };
+    std::map<std::pair<int, int>, Shape> shapes;  // (side, blocks)
+    auto shape = [&](int side, int width) -> const Shape& {
+        Shape& s = shapes[{side, width}];
+        if (s.cost == 0.0) {
+            int threads = 0;
+            s.a.nx = s.a.ny = s.a.nz = side;
+            s.cost = rcg_shape(width, false, true, s.a, threads, s.smem) * side;
+            if (s.cost == 0.0) s.cost = -1.0;
+        }
+        return s;
+    };
+    static const int widths[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 14, 16, 19, 22, 25, 30, 38, 50, 76, 152};
+    std::vector<int> order((size_t)n_inst);
+    for (int b = 0; b < n_inst; ++b) order[(size_t)b] = b;
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return sides[p] > sides[q]; });
+    struct Column {
+        int width;
+        double height;
+        std::vector<int> list;
+    };
+    std::vector<Column> cols;
+    auto pack = [&](double bound) {
+        cols.clear();
+        int used = 0;
+        for (int b : order) {
+            Column* best = nullptr;
+            double left = 0.0;
+            for (Column& c : cols) {
+                const double cost = shape(sides[b], c.width).cost, rest = bound - c.height - cost;
+                if (cost > 0.0 && rest >= 0.0 && (!best || rest < left)) {
+                    best = &c;
+                    left = rest;
+                }
+            }
+            if (!best) {
+                for (int w : widths) {
+                    if (w > sms - used) return false;
+                    const double cost = shape(sides[b], w).cost;
+                    if (cost > 0.0 && cost <= bound) {
+                        used += w;
+                        cols.push_back({w, 0.0, {}});
+                        best = &cols.back();
+                        break;
+                    }
+                }
+                if (!best) return false;
+            }
+            best->height += shape(sides[b], best->width).cost;
+            best->list.push_back(b);
+        }
+        return true;
+    };
+    double hi = 0.0;
+    for (int b : order) {
+        const double c = shape(sides[b], widths[18] <= sms ? widths[18] : 76).cost;
+        if (c <= 0.0) return NN_ERR_UNSUPPORTED;
+        hi += c;
+    }
+    double lo = 0.0;
+    if (!pack(hi)) return NN_ERR_UNSUPPORTED;
+    for (int q = 0; q < 14; ++q) {
+        const double mid = 0.5 * (lo + hi);
+        (pack(mid) ? hi : lo) = mid;
+    }
+    if (!pack(hi)) return NN_ERR_UNSUPPORTED;
+
+    nn_rcg_batch* pl = new nn_rcg_batch();
+    pl->ctx = ctx;
+    nn_ctx_retain(ctx);
+    pl->n_inst = n_inst;
+    pl->groups = cols.size();
+    std::vector<RcgArgs> inst((size_t)n_inst);
+    std::vector<RcgGroup> group;
+    std::vector<int2> block;
+    std::vector<int> list;
+    int nz = 1;
+    size_t n_xw = 0;
+    for (const Column& c : cols) {
+        RcgGroup g{(int)list.size(), (int)c.list.size(), c.width, (int64_t)pl->n_rec, (int64_t)pl->n_halo, (int64_t)n_xw};
+        size_t halo = 0, xw = 0;
+        for (int b : c.list) {
+            const Shape& s = shape(sides[b], c.width);
+            RcgArgs a = s.a;
+            rcg_operator(a, alpha_unit * sides[b] * sides[b], beta);
+            nz = std::max(nz, a.bz);
+            pl->smem = std::max(pl->smem, s.smem);
+            halo = std::max(halo, 2 * (size_t)a.nb * a.hq);
+            xw = std::max(xw, (size_t)a.nb * a.bz * RT);
+            inst[(size_t)b] = a;
+            list.push_back(b);
+        }
+        for (int r = 0; r < c.width; ++r) block.push_back({(int)group.size(), r});
+        pl->n_rec += 8 * (size_t)c.width;
+        pl->n_halo += halo;
+        n_xw += xw;
+        pl->longest = std::max(pl->longest, g.count);
+        group.push_back(g);
+    }
+    pl->blocks = (int)block.size();
+    pl->kernel = batch_kernel_of(nz);
+    const size_t N = (size_t)n_inst;
+    nn_status st = nn_alloc(ctx, &pl->rec, pl->n_rec);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->halo, pl->n_halo);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->xw, n_xw);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->inst, N);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->off, N);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->block, block.size());
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->group, group.size());
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->list, list.size());
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.start, 2 * (size_t)pl->blocks);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.epoch, group.size());
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.scal, 2 * N);
+    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.flags, 4 * N);
+    if (st == NN_OK)
+        for (const RcgGroup& g : group)
+            for (int k = 0; k < g.count; ++k) {
+                RcgArgs& a = inst[(size_t)list[(size_t)(g.first + k)]];
+                a.rec = pl->rec + g.rec;
+                a.halo = pl->halo + g.halo;
+                a.xw = pl->xw + g.xw;
+            }
+    auto put = [&](void* d, const void* h, size_t bytes) {
+        if (st == NN_OK)
+            st = nn_cuda_check(ctx, cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ctx->stream), "copy");
+    };
+    put(pl->inst, inst.data(), sizeof(RcgArgs) * N);
+    put(pl->off, off, sizeof(int64_t) * N);
+    put(pl->block, block.data(), sizeof(int2) * block.size());
+    put(pl->group, group.data(), sizeof(RcgGroup) * group.size());
+    put(pl->list, list.data(), sizeof(int) * list.size());
+    if (st == NN_OK) st = batch_reset(pl, ctx->stream);
+    int coop = 0, per_sm = 0;
+    if (st == NN_OK)
+        st = nn_cuda_check(ctx, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device), "attribute");
+    if (st == NN_OK)
+        st = nn_cuda_check(ctx, cudaFuncSetAttribute(pl->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024),
+                           "cudaFuncSetAttribute(k_rcg_batch)");
+    if (st == NN_OK)
+        st = nn_cuda_check(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pl->kernel, RT, pl->smem), "occupancy");
+    if (st == NN_OK && (!coop || per_sm < 1)) st = NN_ERR_UNSUPPORTED;
+    // solves may run on other streams, and the host arrays go
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (st == NN_OK) st = nn_cuda_check(ctx, e, "nn_rcg_batch_create");
+    if (st != NN_OK) {
+        nn_rcg_batch_destroy(pl);
+        return st;
+    }
+    pl->B.inst = pl->inst;
+    pl->B.off = pl->off;
+    pl->B.block = pl->block;
+    pl->B.group = pl->group;
+    pl->B.list = pl->list;
+    *out = pl;
+    return NN_OK;
+}
+
+nn_status nn_rcg_batch_begin(nn_rcg_batch* pl, const float* d_b, float* d_x, double rtol, int max_iter, cudaStream_t cs)
+{
+    nn_ctx* ctx = pl->ctx;
+    pl->B.b = d_b;
+    pl->B.x = d_x;
+    pl->B.rtol2 = split(rtol * rtol);
+    pl->B.max_iter = max_iter;
+    void* args[] = {&pl->B};
+    NN_CUDA(ctx, cudaLaunchCooperativeKernel(pl->kernel, dim3(pl->blocks), dim3(RT), args, pl->smem, cs));
+    ctx->launches++;
+    pl->B.seq += (uint32_t)pl->longest;
+    return NN_OK;
+}
+
+// Per instance: iterations and outcome (1 converged).
+nn_status nn_rcg_batch_finish(nn_rcg_batch* pl, cudaStream_t cs, int* iters, int* flags)
+{
+    nn_ctx* ctx = pl->ctx;
+    std::vector<int> f(4 * (size_t)pl->n_inst);
+    NN_CUDA(ctx, cudaMemcpyAsync(f.data(), pl->B.flags, sizeof(int) * f.size(), cudaMemcpyDeviceToHost, cs));
+    NN_CUDA(ctx, cudaStreamSynchronize(cs));
+    for (int b = 0; b < pl->n_inst; ++b) {
+        if (f[4 * (size_t)b + 2]) {
+            NN_TRY(batch_reset(pl, cs));
+            NN_CUDA(ctx, cudaMemsetAsync(pl->B.flags, 0, sizeof(int) * f.size(), cs));
+            NN_CUDA(ctx, cudaStreamSynchronize(cs));
+            return nn_fail(ctx, NN_ERR_TIMEOUT, "k_rcg_batch: a block's wait for its neighbours gave up");
+        }
+        flags[b] = f[4 * (size_t)b];
+        iters[b] = f[4 * (size_t)b + 1];
+    }
     return NN_OK;
 }

@@ -115,3 +115,32 @@ def test_resident_solves_from_two_threads(built_lib):
     assert not errors
     for k in range(2):
         assert all(np.array_equal(r, res["alone"][0]) for r in res[k])
+
+
+@pytest.mark.parametrize("sides", [[1], [2, 1, 3], [64, 5, 33, 17, 50, 9], [7] * 200, [40] * 20 + [21] * 40 + [100]])
+def test_resident_batch_matches_oracle(ctx, orc, sides):
+    """All instances of a batch in one launch: single cells, more instances
+    than blocks (lists of several), groups of different widths."""
+    alpha_unit, beta = 3e-3, 0.02
+    bp = nn.BatchedPCG(ctx, sides, alpha_unit, beta)
+    rng = np.random.default_rng(5)
+    b = (0.01 * rng.random(int(bp.offsets[-1]))).astype(np.float32)
+    b[rng.integers(0, b.size, max(1, b.size // 300))] += 1.0
+    db, dx = ctx.to_device(b), ctx.to_device(np.zeros_like(b))
+    for guess in (0.0, 0.3):  # a second solve of the same object, from another guess
+        dx.copy_from(np.full_like(b, guess))
+        its, bad = bp.solve(db, dx, 1e-6, 5000)
+        assert bad == 0
+        x = dx.numpy()
+        for k in {0, len(sides) // 2, len(sides) - 1}:
+            g, lo, hi = sides[k], int(bp.offsets[k]), int(bp.offsets[k + 1])
+            al = alpha_unit * g * g
+            ref, rit, _ = orc.pcg7(b[lo:hi], np.full(hi - lo, guess), (g, g, g), al, beta, rtol=1e-12)
+            gap = 8 * 2.0 ** -24 * (1 + beta + 12 * al) * max(guess * (hi - lo) ** 0.5, np.linalg.norm(ref))
+            bound = 1e-6 * np.linalg.norm(b[lo:hi]) + gap
+            assert np.linalg.norm(x[lo:hi] - ref) <= bound / (1 + beta), k
+    its, bad = bp.solve(db, dx, 1e-3, 10)
+    assert bad == 0 and np.all(its == 0)
+    dx.zero()
+    its, bad = bp.solve(db, dx, 1e-6, 0)
+    assert bad == len(sides)
