@@ -24,11 +24,10 @@
 // Comput. 22 (2000) 1444), which stops at the same relative residual as
 // nn_pcg_solve.
 //
-// Kernels.  Every kernel walks grid rows (j, k) -- one division per row, none
-// per cell -- with threads along x.  On the fine level a thread owns four
-// consecutive cells (16-byte loads of the cell and its y/z neighbours, two
-// scalar x neighbours, five x-face harmonic means for four cells) when the x
-// side is a multiple of four.  Fusions on the fine level: the first two
+// Kernels.  With rows of a multiple of four cells the fine level (and coarse
+// levels of a million cells or more) runs on columns of quads, see below; the
+// other kernels walk grid rows (j, k) -- one division per row, none per cell --
+// with threads along x.  Fusions on the fine level: the first two
 // smoothing sweeps from a zero guess are one pass (the first sweep's values
 // at the neighbours are recomputed from b and 1/diag); the direction update
 // p = z + beta p runs inside the operator application (p ping-pongs between
@@ -40,13 +39,18 @@
 // the host launches the graph in chunks and reads the flag once per chunk.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "nn_internal.cuh"
+#include "nn_quad.cuh"
 
 namespace {
 
 constexpr int MG_THREADS = 256;
+constexpr int COL_BLOCKS = 4;  // resident blocks of a column kernel per SM (2: 25 % slower, 3: 3 %)
+// coarse levels of fewer cells keep a thread per cell (a sweep at 64^3: 5.2 us, by columns 8.0; at 128^3 15.2 and 10.9)
+constexpr int COL_MIN_CELLS = 1 << 20;
 #ifndef NN_MG_VEC
 #define NN_MG_VEC 4  // cells per thread on the fine level (4 or 2) when the x side allows
 #endif
@@ -575,6 +579,15 @@ __global__ void k_fcg_set(double* scal, int* flags, double rtol2, int max_iter)
     flags[F_MAXIT] = max_iter;
 }
 
+__device__ __forceinline__ void fcg_begin(const Red& red, const double (&o)[2])
+{
+    red.scal[S_BB] = o[0];
+    red.scal[S_RR] = o[1];
+    red.flags[F_ITERS] = 0;
+    red.flags[F_STATE] = isfinite(o[1]) ? 0 : 1;
+    red.flags[F_DONE] = (o[1] <= red.scal[S_TOL] * o[0] || !isfinite(o[1]) || red.flags[F_MAXIT] <= 0) ? 1 : 0;
+}
+
 // r = b - A x; (b, b), (r, r); converged at once when (r, r) <= rtol2 (b, b)
 template <int V>
 __global__ void __launch_bounds__(MG_THREADS, NN_MG_MIN_BLOCKS) k_fcg_init(Op0 op, const float* b, const float* x, float* r, Red red)
@@ -601,14 +614,7 @@ __global__ void __launch_bounds__(MG_THREADS, NN_MG_MIN_BLOCKS) k_fcg_init(Op0 o
         }
     }
     double o[2];
-    if (mg_reduce<2>(acc, red.partials, red.ticket, o) && is_tid0()) {
-        const double rtol2 = red.scal[S_TOL];
-        red.scal[S_BB] = o[0];
-        red.scal[S_RR] = o[1];
-        red.flags[F_ITERS] = 0;
-        red.flags[F_STATE] = isfinite(o[1]) ? 0 : 1;
-        red.flags[F_DONE] = (o[1] <= rtol2 * o[0] || !isfinite(o[1]) || red.flags[F_MAXIT] <= 0) ? 1 : 0;
-    }
+    if (mg_reduce<2>(acc, red.partials, red.ticket, o) && is_tid0()) fcg_begin(red, o);
 }
 
 // p = z; (r, z); beta = 0 (the first direction update keeps p = z)
@@ -654,6 +660,428 @@ __global__ void __launch_bounds__(MG_THREADS, NN_MG_MIN_BLOCKS) k_fcg_ap_dir(Op0
     }
     double o[1];
     if (mg_reduce<1>(acc, red.partials, red.ticket, o) && is_tid0()) red.scal[S_PQ] = o[0];
+}
+
+// ------------------------------------------------- fine level, by columns --
+//
+// On the fine level with rows of a multiple of four cells every stencil runs
+// on columns: a thread keeps a quad of x cells and walks up the planes of its
+// chunk, so the z neighbours and z face coefficients pass from plane to plane
+// in registers, x neighbours come by shuffle, and only the quad above and the
+// two beside it in y are loaded.  A block is whole rows (a chunk of 256 quads
+// of longer ones); the chunks in z are chosen to fill the chip about once.
+//
+// The cell field is read as v = 1 / (2 alpha D), made once a solve: a face
+// coefficient alpha 2 D D' / (D + D') is then 1 / (v + v') (two instructions
+// instead of five), and a cell's own v in the place of a neighbour outside the
+// grid gives the boundary face alpha D.
+//
+// Bound by HBM.  Row kernels that gathered the six neighbours of every quad
+// and formed all faces anew moved the same bytes at 30-45 % of the rate: the
+// fine level's seven launches of a cycle took 590 us at 256^3 with a cell
+// field, and take 374 (sweep 82 -> 48, two sweeps from zero 102 -> 65,
+// restriction 95 -> 41, prolongation 82 -> 34, A p 90 -> 66).
+
+// Launch geometry: quads a row, rows a block, blocks along x, y, z, planes a block.
+struct Cols {
+    int Q, rows, bx, by, bz, zc;
+    int blocks() const { return bx * by * bz; }
+};
+
+Cols cols_for(const nn_ctx* ctx, int nx, int ny, int nz)
+{
+    Cols c;
+    c.Q = nx / 4;
+    c.bx = (c.Q + MG_THREADS - 1) / MG_THREADS;
+    c.rows = c.bx > 1 ? 1 : std::min(ny, MG_THREADS / c.Q);
+    if (c.rows > 1) c.rows &= ~1;  // row pairs of the restriction stay in a block
+    c.by = (ny + c.rows - 1) / c.rows;
+    // one wave of blocks; chunks of at least four planes, of an even number
+    const int want = std::max(1, ctx->num_sms * COL_BLOCKS / (c.bx * c.by));
+    c.zc = std::max(4, (nz + want - 1) / want);
+    c.zc = (c.zc + 1) & ~1;
+    c.bz = (nz + c.zc - 1) / c.zc;
+    return c;
+}
+
+// A thread's column.
+struct Col {
+    int i0, j, k0, k1, c;   // first cell, rows and planes, index of the first quad
+    bool act, edge_l, edge_r;
+};
+
+__device__ __forceinline__ Col col_of(const Cols& g, int nx, int ny, int nz)
+{
+    Col t;
+    const int bx = blockIdx.x % g.bx, by = blockIdx.x / g.bx % g.by, bz = blockIdx.x / (g.bx * g.by);
+    const int w = g.bx > 1 ? MG_THREADS : g.Q;
+    const int row = threadIdx.x / w, q = bx * MG_THREADS + threadIdx.x - row * w;
+    t.act = row < g.rows && by * g.rows + row < ny && q < g.Q;
+    const int qc = min(q, g.Q - 1);
+    t.i0 = 4 * qc;
+    t.j = min(by * g.rows + min(row, g.rows - 1), ny - 1);
+    t.k0 = bz * g.zc;
+    t.k1 = min(t.k0 + g.zc, nz);
+    t.c = t.i0 + nx * (t.j + ny * t.k0);
+    const int lane = threadIdx.x & 31;
+    t.edge_l = lane == 0 || qc == 0 || threadIdx.x - row * w == 0;
+    t.edge_r = lane == 31 || qc == g.Q - 1;
+    return t;
+}
+
+// v of the cell field.  Two neighbours with D = 0 have the face coefficient
+// 0 / 0: their v is NaN.
+__global__ void __launch_bounds__(MG_THREADS) k_mg_field(int nx, int ny, int nz, const float* D, float half_ia, float* v)
+{
+    MG_ROWS(ny, nz, row)
+    {
+        const int j = row % ny, k = row / ny;
+        for (int i = threadIdx.x; i < nx; i += blockDim.x) {
+            const int c = i + nx * row;
+            const float d = D[c];
+            float o = __fdiv_rn(half_ia, d);
+            if (d == 0.0f &&
+                ((i > 0 && D[c - 1] == 0.0f) || (i < nx - 1 && D[c + 1] == 0.0f) || (j > 0 && D[c - nx] == 0.0f) ||
+                 (j < ny - 1 && D[c + nx] == 0.0f) || (k > 0 && D[c - nx * ny] == 0.0f) ||
+                 (k < nz - 1 && D[c + nx * ny] == 0.0f)))
+                o = nanf("");
+            v[c] = o;
+        }
+    }
+}
+
+struct CPlain {
+    const float* a;
+    __device__ __forceinline__ Quad quad(int c) const { return quad_ld(a + c); }
+    __device__ __forceinline__ float one(int c) const { return a[c]; }
+};
+struct CLin {  // z + beta p
+    const float *z, *p;
+    float beta;
+    __device__ __forceinline__ Quad quad(int c) const
+    {
+        const Quad a = quad_ld(z + c), b = quad_ld(p + c);
+        return {vfma(vb<2>(beta), b.a, a.a), vfma(vb<2>(beta), b.b, a.b)};
+    }
+    __device__ __forceinline__ float one(int c) const { return z[c] + beta * p[c]; }
+};
+struct CDiv {  // omega b / diag
+    const float *b, *diag;
+    float omega;
+    __device__ __forceinline__ Quad quad(int c) const
+    {
+        const Quad a = quad_ld(b + c), d = quad_ld(diag + c);
+        return {vmul(vmul(a.a, vb<2>(omega)), vrcp(d.a)), vmul(vmul(a.b, vb<2>(omega)), vrcp(d.b))};
+    }
+    __device__ __forceinline__ float one(int c) const { return b[c] * omega * nn_rcp(diag[c]); }
+};
+struct CInvd {  // omega b invd (invd null: the constant)
+    const float *b, *invd;
+    float invd_c, omega;
+    __device__ __forceinline__ Quad quad(int c) const
+    {
+        const Quad a = quad_ld(b + c);
+        if (!invd) return {vmul(a.a, vb<2>(omega * invd_c)), vmul(a.b, vb<2>(omega * invd_c))};
+        const Quad m = quad_ld(invd + c);
+        return {vmul(a.a, vmul(m.a, vb<2>(omega))), vmul(a.b, vmul(m.b, vb<2>(omega)))};
+    }
+    __device__ __forceinline__ float one(int c) const { return b[c] * ((invd ? invd[c] : invd_c) * omega); }
+};
+
+// Operators on columns: begin() before the first plane, plane() gives A u and
+// the diagonal of the quad at c from its values and neighbours.
+struct Near {
+    Quad um, uc, un, ym, yp;
+    float xl, xr;
+};
+
+struct OpConst {  // constant coefficients
+    int nx, ny, nz;
+    float alpha, onepb;
+    __device__ __forceinline__ void begin(const Col&) {}
+    __device__ __forceinline__ void plane(const Col&, int, bool, const Near& n, Quad& A, Quad& dg)
+    {
+        const V2 a = vb<2>(alpha), six = vb<2>(6.0f), minus = vb<2>(-1.0f), m = vb<2>(onepb);
+        const Quad& u = n.uc;
+        V2 na{{n.xl + u.a.v[1], u.a.v[0] + u.b.v[0]}}, nb{{u.a.v[1] + u.b.v[1], u.b.v[0] + n.xr}};
+        na = vadd(vadd(vadd(vadd(na, n.ym.a), n.yp.a), n.um.a), n.un.a);
+        nb = vadd(vadd(vadd(vadd(nb, n.ym.b), n.yp.b), n.um.b), n.un.b);
+        A = {vfma(a, vfma(six, u.a, vmul(minus, na)), vmul(m, u.a)), vfma(a, vfma(six, u.b, vmul(minus, nb)), vmul(m, u.b))};
+        dg = {vb<2>(onepb + 6.0f * alpha), vb<2>(onepb + 6.0f * alpha)};
+    }
+};
+
+struct OpField {  // the cell field as v = 1 / (2 alpha D)
+    int nx, ny, nz;
+    const float* v;
+    float onepb;
+    Quad vc, cz;  // this plane's v, the coefficients of the faces below it
+    __device__ __forceinline__ void begin(const Col& t)
+    {
+        vc = quad_ld(v + t.c);
+        const Quad vm = t.k0 > 0 ? quad_ld(v + t.c - nx * ny) : vc;
+        cz = {vrcp(vadd(vc.a, vm.a)), vrcp(vadd(vc.b, vm.b))};
+    }
+    __device__ __forceinline__ void plane(const Col& t, int c, bool hz, const Near& n, Quad& A, Quad& dg)
+    {
+        const float* d = v + c;
+        const Quad& u = n.uc;
+        const Quad vn = hz ? quad_ld(d + nx * ny) : vc, vm = t.j > 0 ? quad_ld(d - nx) : vc;
+        const Quad vp = t.j < ny - 1 ? quad_ld(d + nx) : vc;
+        float dl = __shfl_up_sync(0xffffffffu, vc.b.v[1], 1), dr = __shfl_down_sync(0xffffffffu, vc.a.v[0], 1);
+        if (t.edge_l) dl = t.i0 > 0 ? d[-1] : vc.a.v[0];
+        if (t.edge_r) dr = t.i0 + 4 < nx ? d[4] : vc.b.v[1];
+        const float c0 = nn_rcp(dl + vc.a.v[0]), c1 = nn_rcp(vc.a.v[0] + vc.a.v[1]);
+        const float c2 = nn_rcp(vc.a.v[1] + vc.b.v[0]), c3 = nn_rcp(vc.b.v[0] + vc.b.v[1]);
+        const float c4 = nn_rcp(vc.b.v[1] + dr);
+        const float f0 = c0 * (u.a.v[0] - n.xl), f1 = c1 * (u.a.v[0] - u.a.v[1]), f2 = c2 * (u.a.v[1] - u.b.v[0]);
+        const float f3 = c3 * (u.b.v[0] - u.b.v[1]), f4 = c4 * (u.b.v[1] - n.xr);
+        const V2 m = vb<2>(onepb);
+        auto half = [&](const V2& cx, const V2& fx, const V2& u0, const V2& ym, const V2& yp, const V2& um, const V2& un,
+                        const V2& v0, const V2& vm1, const V2& vp1, const V2& vn1, V2& czh, V2& A1, V2& d1) {
+            const V2 cm = vrcp(vadd(v0, vm1)), cp = vrcp(vadd(v0, vp1)), cn = vrcp(vadd(v0, vn1));
+            V2 acc = vfma(cm, vsub(u0, ym), fx);
+            acc = vfma(cp, vsub(u0, yp), acc);
+            acc = vfma(czh, vsub(u0, um), acc);
+            acc = vfma(cn, vsub(u0, un), acc);
+            A1 = vfma(m, u0, acc);
+            d1 = vadd(vadd(vadd(vadd(vadd(cx, cm), cp), czh), cn), m);
+            czh = cn;
+        };
+        half({{c0 + c1, c1 + c2}}, {{f0 + f1, f2 - f1}}, u.a, n.ym.a, n.yp.a, n.um.a, n.un.a, vc.a, vm.a, vp.a, vn.a,
+             cz.a, A.a, dg.a);
+        half({{c2 + c3, c3 + c4}}, {{f3 - f2, f4 - f3}}, u.b, n.ym.b, n.yp.b, n.um.b, n.un.b, vc.b, vm.b, vp.b, vn.b,
+             cz.b, A.b, dg.b);
+        vc = vn;
+    }
+};
+
+struct OpFaces {  // a coarse level: stored conductances and diagonal (see OpF)
+    int nx, ny, nz;
+    const float *wx, *wy, *wz, *diag;
+    Quad cz;
+    __device__ __forceinline__ void begin(const Col& t) { cz = t.k0 > 0 ? quad_ld(wz + t.c - nx * ny) : quad_zero(); }
+    __device__ __forceinline__ void plane(const Col& t, int c, bool, const Near& n, Quad& A, Quad& dg)
+    {
+        const Quad ex = quad_ld(wx + c), cp = quad_ld(wy + c), cn = quad_ld(wz + c);
+        const Quad cm = t.j > 0 ? quad_ld(wy + c - nx) : quad_zero();
+        dg = quad_ld(diag + c);
+        float c0 = __shfl_up_sync(0xffffffffu, ex.b.v[1], 1);
+        if (t.edge_l) c0 = t.i0 > 0 ? wx[c - 1] : 0.0f;
+        const Quad& u = n.uc;
+        auto half = [&](const V2& west, const V2& w, const V2& east, const V2& e, const V2& ym, const V2& yp, const V2& um,
+                        const V2& un, const V2& cm1, const V2& cp1, const V2& cz1, const V2& cn1, const V2& u0,
+                        const V2& d1) {
+            V2 s = vmul(west, w);
+            s = vfma(east, e, s);
+            s = vfma(cm1, ym, s);
+            s = vfma(cp1, yp, s);
+            s = vfma(cz1, um, s);
+            s = vfma(cn1, un, s);
+            return vfma(d1, u0, vmul(vb<2>(-1.0f), s));
+        };
+        A.a = half({{c0, ex.a.v[0]}}, {{n.xl, u.a.v[0]}}, ex.a, {{u.a.v[1], u.b.v[0]}}, n.ym.a, n.yp.a, n.um.a, n.un.a,
+                   cm.a, cp.a, cz.a, cn.a, u.a, dg.a);
+        A.b = half({{ex.a.v[1], ex.b.v[0]}}, {{u.a.v[1], u.b.v[0]}}, ex.b, {{u.b.v[1], n.xr}}, n.ym.b, n.yp.b, n.um.b,
+                   n.un.b, cm.b, cp.b, cz.b, cn.b, u.b, dg.b);
+        cz = cn;
+    }
+};
+
+// out(k, c, u, A u, diag, in) for every plane of the column; in: what `more`
+// loads at the quad, issued with the plane's other loads
+template <class Op, class F, class More, class Out>
+__device__ __forceinline__ void walk(Op op, const Col& t, const F& f, More more, Out out)
+{
+    const int sy = op.nx, sz = op.nx * op.ny;
+    int c = t.c;
+    Near n;
+    n.um = t.k0 > 0 ? f.quad(c - sz) : quad_zero();
+    n.uc = f.quad(c);
+    op.begin(t);
+    const bool ly = t.j > 0, hy = t.j < op.ny - 1, lx = t.i0 > 0, hx = t.i0 + 4 < op.nx;
+#pragma unroll 1
+    for (int k = t.k0; k < t.k1; ++k, c += sz) {
+        const bool hz = k < op.nz - 1;
+        const auto in = more(c);
+        n.un = hz ? f.quad(c + sz) : quad_zero();
+        n.ym = ly ? f.quad(c - sy) : quad_zero();
+        n.yp = hy ? f.quad(c + sy) : quad_zero();
+        n.xl = __shfl_up_sync(0xffffffffu, n.uc.b.v[1], 1);
+        n.xr = __shfl_down_sync(0xffffffffu, n.uc.a.v[0], 1);
+        if (t.edge_l) n.xl = lx ? f.one(c - 1) : 0.0f;
+        if (t.edge_r) n.xr = hx ? f.one(c + 4) : 0.0f;
+        Quad A, dg;
+        op.plane(t, c, hz, n, A, dg);
+        out(k, c, n.uc, A, dg, in);
+        n.um = n.uc;
+        n.uc = n.un;
+    }
+}
+
+// u + omega (b - A u) / diag
+__device__ __forceinline__ Quad relax(const Quad& u, const Quad& A, const Quad& dg, const Quad& b, float omega)
+{
+    const V2 o = vb<2>(omega);
+    return {vfma(vmul(o, vrcp(dg.a)), vsub(b.a, A.a), u.a), vfma(vmul(o, vrcp(dg.b)), vsub(b.b, A.b), u.b)};
+}
+__device__ __forceinline__ float dot(const Quad& x, const Quad& y, float acc)
+{
+    const V2 s = vfma(x.b, y.b, vmul(x.a, y.a));
+    return acc + (s.v[0] + s.v[1]);
+}
+
+  // a SM
+
+// Two sweeps from zero: the first, omega b / diag, is formed at the neighbours
+// as b is read.
+template <class Op, class F>
+__global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_pre2(Op op, Cols g, F f, float* y, const int* flags)
+{
+    if (flags && flags[F_DONE]) return;
+    const Col t = col_of(g, op.nx, op.ny, op.nz);
+    walk(op, t, f, [&](int c) { return quad_ld(f.b + c); },
+              [&](int, int c, const Quad& u, const Quad& A, const Quad& dg, const Quad& b) {
+                  if (t.act) quad_st(y + c, relax(u, A, dg, b, f.omega));
+              });
+}
+
+// y = x + omega D^-1 (b - A x); DOTS as in k_mg_jacobi
+template <class Op, bool DOTS>
+__global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_jacobi(Op op, Cols g, const float* b, const float* x,
+                                                                      float omega, float* y, const int* flags,
+                                                                      const float* q, Red red)
+{
+    if (flags && flags[F_DONE]) return;
+    const Col t = col_of(g, op.nx, op.ny, op.nz);
+    float acc[2] = {0.0f, 0.0f};
+    struct In {
+        Quad b, q;
+    };
+    walk(op, t, CPlain{x}, [&](int c) { return In{quad_ld(b + c), DOTS ? quad_ld(q + c) : quad_zero()}; },
+              [&](int, int c, const Quad& u, const Quad& A, const Quad& dg, const In& in) {
+                  if (!t.act) return;
+                  const Quad o = relax(u, A, dg, in.b, omega);
+                  quad_st(y + c, o);
+                  if (DOTS) {
+                      acc[0] = dot(in.b, o, acc[0]);
+                      acc[1] = dot(o, in.q, acc[1]);
+                  }
+              });
+    if constexpr (DOTS) {
+        double o[2];
+        if (mg_reduce<2>(acc, red.partials, red.ticket, o) && is_tid0()) {
+            red.scal[S_RZ] = o[0];
+            red.scal[S_BETA] = -o[1] / red.scal[S_PQ];
+        }
+    }
+}
+
+// bc = R (b - A x): a thread sums its quad's residuals of two planes into two
+// coarse cells, the odd row of a pair hands its sums to the even one.
+template <class Op>
+__global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_restrict(Op op, Cols g, const float* b, const float* x,
+                                                                        float* bc, const int* flags)
+{
+    __shared__ float2 part[MG_THREADS];
+    if (flags && flags[F_DONE]) return;
+    const Col t = col_of(g, op.nx, op.ny, op.nz);
+    const int cx = op.nx / 2, cy = op.ny / 2;
+    float2 s = make_float2(0.0f, 0.0f);
+    walk(op, t, CPlain{x}, [&](int c) { return quad_ld(b + c); },
+              [&](int k, int, const Quad&, const Quad& A, const Quad&, const Quad& r) {
+                  const V2 ra = vsub(r.a, A.a), rb = vsub(r.b, A.b);
+                  s.x += ra.v[0] + ra.v[1];
+                  s.y += rb.v[0] + rb.v[1];
+                  if (!(k & 1)) return;
+                  if (t.j & 1) part[threadIdx.x] = s;
+                  __syncthreads();
+                  if (t.act && !(t.j & 1)) {
+                      const float2 o = part[threadIdx.x + g.Q];
+                      *reinterpret_cast<float2*>(bc + t.i0 / 2 + cx * (t.j / 2 + cy * (k / 2))) =
+                          make_float2(s.x + o.x, s.y + o.y);
+                  }
+                  __syncthreads();
+                  s = make_float2(0.0f, 0.0f);
+              });
+}
+
+// r = b - A x; (b, b), (r, r), as k_fcg_init
+template <class Op>
+__global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_init(Op op, Cols g, const float* b, const float* x,
+                                                                    float* r, Red red)
+{
+    const Col t = col_of(g, op.nx, op.ny, op.nz);
+    float acc[2] = {0.0f, 0.0f};
+    walk(op, t, CPlain{x}, [&](int c) { return quad_ld(b + c); },
+              [&](int, int c, const Quad&, const Quad& A, const Quad&, const Quad& bv) {
+                  if (!t.act) return;
+                  const Quad rv{vsub(bv.a, A.a), vsub(bv.b, A.b)};
+                  quad_st(r + c, rv);
+                  acc[0] = dot(bv, bv, acc[0]);
+                  acc[1] = dot(rv, rv, acc[1]);
+              });
+    double o[2];
+    if (mg_reduce<2>(acc, red.partials, red.ticket, o) && is_tid0()) fcg_begin(red, o);
+}
+
+// p_new = z + beta p_old; q = A p_new; (p_new, q)
+template <class Op>
+__global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_ap_dir(Op op, Cols g, const float* z, const float* p_old,
+                                                                      float* p_new, float* q, Red red)
+{
+    if (red.flags[F_DONE]) return;
+    const Col t = col_of(g, op.nx, op.ny, op.nz);
+    float acc[1] = {0.0f};
+    walk(op, t, CLin{z, p_old, (float)red.scal[S_BETA]}, [](int) { return 0; },
+              [&](int, int c, const Quad& u, const Quad& A, const Quad&, int) {
+                  if (!t.act) return;
+                  quad_st(p_new + c, u);
+                  quad_st(q + c, A);
+                  acc[0] = dot(u, A, acc[0]);
+              });
+    double o[1];
+    if (mg_reduce<1>(acc, red.partials, red.ticket, o) && is_tid0()) red.scal[S_PQ] = o[0];
+}
+
+// x += P xc, two rows and two planes of a quad per thread: the nine coarse
+// rows around them are read once for sixteen fine cells.
+__global__ void __launch_bounds__(MG_THREADS) k_col_prolong(int nx, int ny, int nz, const float* xc, float* x,
+                                                            const int* flags)
+{
+    if (flags && flags[F_DONE]) return;
+    const int Q = nx / 4, cx = nx / 2, cy = ny / 2, cz = nz / 2;
+    const int n = Q * cy * cz;
+    for (int w = blockIdx.x * MG_THREADS + threadIdx.x; w < n; w += gridDim.x * MG_THREADS) {
+        const int q = w % Q, J = w / Q % cy, K = w / (Q * cy), I = 2 * q;
+        // rows interpolated along x: fine cells 4q .. 4q + 3 from coarse I - 1 .. I + 2
+        Quad e[3][3];
+#pragma unroll
+        for (int dk = 0; dk < 3; ++dk)
+#pragma unroll
+            for (int dj = 0; dj < 3; ++dj) {
+                const int j = J + dj - 1, k = K + dk - 1;
+                e[dk][dj] = quad_zero();
+                if (j < 0 || j >= cy || k < 0 || k >= cz) continue;
+                const float* r = xc + I + cx * (j + cy * k);
+                const float2 m = *reinterpret_cast<const float2*>(r);
+                const float l = I > 0 ? r[-1] : 0.0f, h = I + 2 < cx ? r[2] : 0.0f;
+                e[dk][dj] = {{{0.75f * m.x + 0.25f * l, 0.75f * m.x + 0.25f * m.y}},
+                             {{0.75f * m.y + 0.25f * m.x, 0.75f * m.y + 0.25f * h}}};
+            }
+        const V2 near = vb<2>(0.75f), far = vb<2>(0.25f);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int fj = b & 1, fk = b >> 1;
+            auto mix = [&](const Quad& a, const Quad& c) -> Quad {
+                return {vfma(far, c.a, vmul(near, a.a)), vfma(far, c.b, vmul(near, a.b))};
+            };
+            const Quad p = mix(mix(e[1][1], e[1][2 * fj]), mix(e[2 * fk][1], e[2 * fk][2 * fj]));
+            float* at = x + 4 * q + nx * (2 * J + fj + ny * (2 * K + fk));
+            const Quad u = quad_ld(at);
+            quad_st(at, {vadd(u.a, p.a), vadd(u.b, p.b)});
+        }
+    }
 }
 
 // a = (r, z) / (p, q); x += a p; r -= a q; (r, r); convergence and limit tests
@@ -797,7 +1225,9 @@ struct MgLevel {
     float mass = 0.0f;
     float *wx = nullptr, *wy = nullptr, *wz = nullptr, *wb = nullptr, *diag = nullptr;  // levels >= 1
     float *b = nullptr, *x = nullptr, *t = nullptr;                                     // work
+    Cols cols{};                 // nx % 4 == 0
     OpF op() const { return OpF{nx, ny, nz, wx, wy, wz, wb, diag}; }
+    OpFaces faces() const { return OpFaces{nx, ny, nz, wx, wy, wz, diag}; }
 };
 
 struct nn_mg {
@@ -805,6 +1235,7 @@ struct nn_mg {
     nn_pcg* pc = nullptr;
     Op0 op0{};
     int vec0 = 1;                // cells per thread on the fine level (4 when nx % 4 == 0)
+    float* v = nullptr;          // vec0 == 4 and a cell field: 1 / (2 alpha D)
     std::vector<MgLevel> lv;
     float omega = 0.8f;
     int nu = 2, coarse_sweeps = 8;
@@ -861,32 +1292,86 @@ nn_status launch_smooth0(nn_mg* mg, const Op& op, const float* b, float* y, cons
     return NN_OK;
 }
 
-template <int V, class Op>
-nn_status launch_pre2(nn_mg* mg, const Op& op, const float* b, float* y, const int* flags)
+// The column form of level l's operator: fn(op).
+template <class Fn>
+void with_cols(const nn_mg* mg, int l, Fn fn)
 {
+    const Op0& o = mg->op0;
+    if (l > 0) fn(mg->lv[l].faces());
+    else if (mg->v) fn(OpField{o.nx, o.ny, o.nz, mg->v, o.onepb});
+    else fn(OpConst{o.nx, o.ny, o.nz, o.alpha, o.onepb});
+}
+
+template <int V, class Op>
+nn_status launch_pre2(nn_mg* mg, int l, const Op& op, const float* b, float* y, const int* flags)
+{
+    if constexpr (V == 4) {
+        const Cols& g = mg->lv[l].cols;
+        cudaStream_t cs = mg->ctx->stream;
+        with_cols(mg, l, [&](auto o) {
+            if (l > 0)
+                k_col_pre2<<<g.blocks(), MG_THREADS, 0, cs>>>(o, g, CDiv{b, mg->lv[l].diag, mg->omega}, y, flags);
+            else
+                k_col_pre2<<<g.blocks(), MG_THREADS, 0, cs>>>(o, g, CInvd{b, mg->op0.invd, mg->op0.invd_c, mg->omega}, y, flags);
+        });
+        NN_CHECK_LAUNCH(mg->ctx, "k_col_pre2");
+        return NN_OK;
+    } else {
     const Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
     k_mg_pre2<V, Op><<<s.grid, s.block, 0, mg->ctx->stream>>>(op, b, mg->omega, y, flags);
     NN_CHECK_LAUNCH(mg->ctx, "k_mg_pre2");
     return NN_OK;
+    }
 }
 
 template <int V, bool DOTS, class Op>
-nn_status launch_jacobi(nn_mg* mg, const Op& op, const float* b, const float* x, float* y, const int* flags,
+nn_status launch_jacobi(nn_mg* mg, int l, const Op& op, const float* b, const float* x, float* y, const int* flags,
                         const float* q = nullptr)
 {
+    if constexpr (V == 4) {
+        const Cols& g = mg->lv[l].cols;
+        with_cols(mg, l, [&](auto o) {
+            k_col_jacobi<decltype(o), DOTS><<<g.blocks(), MG_THREADS, 0, mg->ctx->stream>>>(o, g, b, x, mg->omega, y, flags,
+                                                                                           q, red_of(mg));
+        });
+        NN_CHECK_LAUNCH(mg->ctx, "k_col_jacobi");
+        return NN_OK;
+    } else {
     Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
     if (DOTS) s.grid = dim3(mg->nblocks);  // the partials buffer holds nblocks entries
     k_mg_jacobi<V, DOTS, Op><<<s.grid, s.block, 0, mg->ctx->stream>>>(op, b, x, mg->omega, y, flags, q, red_of(mg));
     NN_CHECK_LAUNCH(mg->ctx, "k_mg_jacobi");
     return NN_OK;
+    }
 }
 
-template <int VC, class Op>
-nn_status launch_restrict(nn_mg* mg, const Op& op, const float* b, const float* x, float* bc, const int* flags)
+template <int V, class Op>
+nn_status launch_restrict(nn_mg* mg, int l, const Op& op, const float* b, const float* x, float* bc, const int* flags)
 {
+    const Cols& g = mg->lv[l].cols;
+    // (pairs of rows longer than half a block lie in different blocks)
+    if (V == 4 && g.rows >= 2) {
+        with_cols(mg, l, [&](auto o) {
+            k_col_restrict<<<g.blocks(), MG_THREADS, 0, mg->ctx->stream>>>(o, g, b, x, bc, flags);
+        });
+        NN_CHECK_LAUNCH(mg->ctx, "k_col_restrict");
+        return NN_OK;
+    }
+    constexpr int VC = V == 4 ? 2 : 1;
     const Shape s = shape_for(mg->ctx, op.nx / 2 / VC, (op.ny / 2) * (op.nz / 2));
     k_mg_restrict<VC, Op><<<s.grid, s.block, 0, mg->ctx->stream>>>(op, b, x, bc, flags);
     NN_CHECK_LAUNCH(mg->ctx, "k_mg_restrict");
+    return NN_OK;
+}
+
+// v from the cell field as it is now (every solve and every single cycle)
+nn_status refresh_field(nn_mg* mg)
+{
+    if (!mg->v) return NN_OK;
+    const Op0& op = mg->op0;
+    const Shape s = shape_for(mg->ctx, op.nx, op.ny * op.nz);
+    k_mg_field<<<s.grid, s.block, 0, mg->ctx->stream>>>(op.nx, op.ny, op.nz, op.D, 0.5f / op.alpha, mg->v);
+    NN_CHECK_LAUNCH(mg->ctx, "k_mg_field");
     return NN_OK;
 }
 
@@ -907,7 +1392,7 @@ nn_status vlevel(nn_mg* mg, int l, const Op& op, const float* b, float* out, con
         NN_TRY(mg->hook_fn(mg->hook_user, b, cur));
         for (int s = 0; s < mg->hook_sweeps; ++s) {
             float* dst = (s == mg->hook_sweeps - 1 && out != cur) ? out : oth;
-            NN_TRY((launch_jacobi<V, false>(mg, op, b, cur, dst, flags)));
+            NN_TRY((launch_jacobi<V, false>(mg, l, op, b, cur, dst, flags)));
             oth = cur;
             cur = dst;
         }
@@ -921,10 +1406,10 @@ nn_status vlevel(nn_mg* mg, int l, const Op& op, const float* b, float* out, con
     const int after_first = sweeps >= 2 ? sweeps - 2 : sweeps - 1;
     float* cur = (after_first % 2) ? L.t : L.x;
     float* oth = (after_first % 2) ? L.x : L.t;
-    if (sweeps >= 2) NN_TRY((launch_pre2<V>(mg, op, b, cur, flags)));
+    if (sweeps >= 2) NN_TRY((launch_pre2<V>(mg, l, op, b, cur, flags)));
     else NN_TRY(launch_smooth0(mg, op, b, cur, flags));
     for (int s = 0; s < after_first; ++s) {
-        NN_TRY((launch_jacobi<V, false>(mg, op, b, cur, oth, flags)));
+        NN_TRY((launch_jacobi<V, false>(mg, l, op, b, cur, oth, flags)));
         std::swap(cur, oth);
     }
     if (coarsest) {
@@ -933,10 +1418,13 @@ nn_status vlevel(nn_mg* mg, int l, const Op& op, const float* b, float* out, con
         return NN_OK;
     }
     MgLevel& C = mg->lv[l + 1];
-    if (V == 4 && (op.nx / 2) % 2 == 0) NN_TRY((launch_restrict<2>(mg, op, b, cur, C.b, flags)));
-    else NN_TRY((launch_restrict<1>(mg, op, b, cur, C.b, flags)));
+    NN_TRY((launch_restrict<V>(mg, l, op, b, cur, C.b, flags)));
     NN_TRY(vcycle(mg, l + 1, C.b, C.x, flags, nullptr));
-    {
+    if (V == 4) {
+        const int n = L.nx / 4 * (L.ny / 2) * (L.nz / 2);
+        k_col_prolong<<<(n + MG_THREADS - 1) / MG_THREADS, MG_THREADS, 0, mg->ctx->stream>>>(L.nx, L.ny, L.nz, C.x, cur, flags);
+        NN_CHECK_LAUNCH(mg->ctx, "k_col_prolong");
+    } else {
         const Shape s = shape_for(mg->ctx, L.nx, L.ny * L.nz);
         k_mg_prolong_add<<<s.grid, s.block, 0, mg->ctx->stream>>>(L.nx, L.ny, L.nz, C.x, cur, flags);
         NN_CHECK_LAUNCH(mg->ctx, "k_mg_prolong_add");
@@ -945,8 +1433,8 @@ nn_status vlevel(nn_mg* mg, int l, const Op& op, const float* b, float* out, con
     for (int s = 0; s < mg->nu; ++s) {
         const bool last = s == mg->nu - 1;
         float* dst = (last && out != cur) ? out : oth;
-        if (last && dots_q) NN_TRY((launch_jacobi<V, true>(mg, op, b, cur, dst, flags, dots_q)));
-        else NN_TRY((launch_jacobi<V, false>(mg, op, b, cur, dst, flags)));
+        if (last && dots_q) NN_TRY((launch_jacobi<V, true>(mg, l, op, b, cur, dst, flags, dots_q)));
+        else NN_TRY((launch_jacobi<V, false>(mg, l, op, b, cur, dst, flags)));
         oth = cur;
         cur = dst;
     }
@@ -962,6 +1450,7 @@ nn_status vcycle(nn_mg* mg, int l, const float* b, float* out, const int* flags,
         if (mg->vec0 == 2) return vlevel<2>(mg, 0, mg->op0, b, out, flags, dots_q);
         return vlevel<1>(mg, 0, mg->op0, b, out, flags, dots_q);
     }
+    if (mg->lv[l].cols.Q > 0) return vlevel<4>(mg, l, mg->lv[l].op(), b, out, flags, nullptr);
     return vlevel<1>(mg, l, mg->lv[l].op(), b, out, flags, nullptr);
 }
 
@@ -972,10 +1461,17 @@ nn_status enqueue_iteration_v(nn_mg* mg, float* x, int parity)
     cudaStream_t cs = ctx->stream;
     const MgLevel& L = mg->lv[0];
     const Red red = red_of(mg);
-    const dim3 blk = shape_for(ctx, L.nx / V, L.ny * L.nz).block;
     float* p_old = mg->p[parity];
     float* p_new = mg->p[1 - parity];
-    k_fcg_ap_dir<V><<<mg->nblocks, blk, 0, cs>>>(mg->op0, mg->z, p_old, p_new, mg->q, red);
+    if constexpr (V == 4) {
+        with_cols(mg, 0, [&](auto o) {
+            if constexpr (!std::is_same_v<decltype(o), OpFaces>)
+                k_col_ap_dir<<<L.cols.blocks(), MG_THREADS, 0, cs>>>(o, L.cols, mg->z, p_old, p_new, mg->q, red);
+        });
+    } else {
+        const dim3 blk = shape_for(ctx, L.nx / V, L.ny * L.nz).block;
+        k_fcg_ap_dir<V><<<mg->nblocks, blk, 0, cs>>>(mg->op0, mg->z, p_old, p_new, mg->q, red);
+    }
     NN_CHECK_LAUNCH(ctx, "k_fcg_ap_dir");
     k_fcg_update<V><<<mg->nblocks, dim3(MG_THREADS), 0, cs>>>(x, mg->r, p_new, mg->q, L.G, red);
     NN_CHECK_LAUNCH(ctx, "k_fcg_update");
@@ -1037,7 +1533,7 @@ extern "C" nn_status nn_mg_destroy(nn_mg* mg)
     drop_graph(mg);
     for (MgLevel& L : mg->lv)
         for (float* v : {L.wx, L.wy, L.wz, L.wb, L.diag, L.b, L.x, L.t}) cudaFree(v);
-    for (float* v : {mg->r, mg->z, mg->q, mg->p[0], mg->p[1]}) cudaFree(v);
+    for (float* v : {mg->r, mg->z, mg->q, mg->p[0], mg->p[1], mg->v}) cudaFree(v);
     cudaFree(mg->scal);
     cudaFree(mg->flags);
     cudaFree(mg->partials);
@@ -1108,7 +1604,12 @@ extern "C" nn_status nn_mg_create(nn_pcg* pc, int levels, nn_mg** out)
     mg->nblocks = std::max(1, std::min((G + MG_THREADS - 1) / MG_THREADS, ctx->num_sms * 8));
     if (st == NN_OK) st = nn_alloc(ctx, &mg->scal, S_COUNT);
     if (st == NN_OK) st = nn_alloc(ctx, &mg->flags, F_COUNT);
-    if (st == NN_OK) st = nn_alloc(ctx, &mg->partials, (size_t)2 * std::max(mg->nblocks, ctx->num_sms * 8));
+    for (MgLevel& L : mg->lv)
+        if (L.nx % 4 == 0 && (&L == &mg->lv[0] || L.G >= COL_MIN_CELLS)) L.cols = cols_for(ctx, L.nx, L.ny, L.nz);
+    if (st == NN_OK && mg->vec0 == 4 && D) st = nn_alloc(ctx, &mg->v, G);
+    if (st == NN_OK)
+        st = nn_alloc(ctx, &mg->partials,
+                      (size_t)2 * std::max({mg->nblocks, ctx->num_sms * 8, mg->vec0 == 4 ? mg->lv[0].cols.blocks() : 0}));
     if (st == NN_OK) st = nn_alloc(ctx, &mg->ticket, 1);
     if (st == NN_OK)
         st = nn_cuda_check(ctx, cudaMallocHost((void**)&mg->h_flags, sizeof(int) * F_COUNT), "cudaMallocHost");
@@ -1147,6 +1648,7 @@ extern "C" nn_status nn_mg_levels(nn_mg* mg, int* levels)
 extern "C" nn_status nn_mg_apply(nn_mg* mg, const float* d_r, float* d_z)
 {
     if (!mg || !d_r || !d_z) return NN_ERR_INVALID_ARG;
+    NN_TRY(refresh_field(mg));
     NN_TRY(vcycle(mg, 0, d_r, d_z, nullptr, nullptr));
     return nn_cuda_check(mg->ctx, cudaStreamSynchronize(mg->ctx->stream), "nn_mg_apply");
 }
@@ -1166,7 +1668,12 @@ extern "C" nn_status nn_mg_solve(nn_mg* mg, const float* d_b, float* d_x, double
     k_fcg_set<<<1, 1, 0, cs>>>(mg->scal, mg->flags, rtol2, max_iter);
     NN_CHECK_LAUNCH(ctx, "k_fcg_set");
     const dim3 blk = shape_for(ctx, L.nx / mg->vec0, L.ny * L.nz).block;
-    if (mg->vec0 == 4) k_fcg_init<4><<<mg->nblocks, blk, 0, cs>>>(mg->op0, d_b, d_x, mg->r, red);
+    NN_TRY(refresh_field(mg));
+    if (mg->vec0 == 4)
+        with_cols(mg, 0, [&](auto o) {
+            if constexpr (!std::is_same_v<decltype(o), OpFaces>)
+                k_col_init<<<L.cols.blocks(), MG_THREADS, 0, cs>>>(o, L.cols, d_b, d_x, mg->r, red);
+        });
     else if (mg->vec0 == 2) k_fcg_init<2><<<mg->nblocks, blk, 0, cs>>>(mg->op0, d_b, d_x, mg->r, red);
     else k_fcg_init<1><<<mg->nblocks, blk, 0, cs>>>(mg->op0, d_b, d_x, mg->r, red);
     NN_CHECK_LAUNCH(ctx, "k_fcg_init");
