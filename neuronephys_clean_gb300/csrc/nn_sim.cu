@@ -69,6 +69,8 @@ struct nn_sim {
     int dsl_slotw = 0;             // words per slot
     int dsl_cmax = 0;              // most chunks of one block
     int dsl_dmax = 0;              // longest delay of the layout
+    int dsl_group = 1;             // delays per chunk (small networks)
+    uint32_t* dsl_zero = nullptr;  // [words] staged in the place of a delay that is not live
     // paracrine
     int grid = 0;
     int64_t G = 0;
@@ -160,6 +162,8 @@ struct PullArgs {
     const float* dsl_w;
     uint2* dsl_hits;
     int dsl_cols, dsl_ring, dsl_slotw, dsl_cmax, dsl_dmax;
+    int dsl_group;
+    const uint32_t* dsl_zero;
     // automatic delivery: only ring rows with rowflag set hold pull spikes
     // (the others were pushed), and the gather adds to the ring slot, which
     // pushed spikes may already have reached (null / 0: every row, overwrite)
@@ -235,7 +239,8 @@ __global__ void __launch_bounds__(DELIV_THREADS) k_deliver_pull(PullArgs a)
 // (postsynaptic neurons).  Its synapses are stored as one run per block,
 // ordered by delay and, within a delay, by source bucket (DSL_BUCKET_WORDS
 // bitmap words = 16,384 consecutive source neurons), and cut into chunks of
-// at most DSL_CHUNK entries that span at most DSL_SPAN buckets.  An entry is
+// at most DSL_CHUNK entries that span at most DSL_SPAN buckets (small
+// networks: the whole rows of several delays, see build_sliced).  An entry is
 // one 32-bit word: the source's offset from the chunk's first bucket (18
 // bits), the column offset within the block (13 bits) and the inhibitory bit.
 // A chunk of delay d needs only its buckets' words of the spike bitmap of step
@@ -278,9 +283,24 @@ static_assert(DSL_SPAN * DSL_BUCKET_WORDS * 32 <= (1 << 18), "source offsets tak
 
 // Stage chunk m = {first entry, entries, first word, words << 8 | delay}: its
 // bitmap words of the row of step t + 1 - d, then its entries (a multiple of
-// four words; the layout pads every chunk).
-__device__ __forceinline__ void dsl_issue(const PullArgs& a, int s1, int4 m, uint32_t* dst, uint64_t* bar)
+// four words; the layout pads every chunk).  A chunk of several delays stages
+// the whole rows of its delays one behind the other, zeros for those that are
+// not live (beyond dlast, or rows of pushed steps).
+__device__ __forceinline__ void dsl_issue(const PullArgs& a, int s1, int dlast, int4 m, uint32_t* dst, uint64_t* bar)
 {
+    if (a.dsl_group > 1) {
+        const int d0 = m.w & 255, cnt = min(a.dsl_group, a.dsl_dmax - d0 + 1);
+        const uint32_t bw = (uint32_t)a.words * 4u, be = (uint32_t)((m.y + 3) & ~3) * 4u;
+        nn_mbar_expect_tx(bar, cnt * bw + be);
+        nn_bulk_g2s(dst + a.dsl_slotw, a.dsl_ent + m.x, be, bar);
+        for (int j = 0; j < cnt; ++j) {
+            int hs = s1 - d0 - j;
+            if (hs < 0) hs += a.D;
+            const bool live = d0 + j <= dlast && (!a.rowflag || a.rowflag[hs]);
+            nn_bulk_g2s(dst + j * a.words, live ? a.bitmap + (size_t)hs * a.words : a.dsl_zero, bw, bar);
+        }
+        return;
+    }
     int hs = s1 - (m.w & 255);
     if (hs < 0) hs += a.D;
     const uint32_t bw = (uint32_t)(m.w >> 8) * 4u;
@@ -358,7 +378,13 @@ __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(Pul
                     if (hs < 0) hs += a.D;
                     const int c0 = cp[d - 1];
                     s_cp[d] = c0;  // first chunk of delay d
-                    if (a.rowflag[hs]) len[h] = cp[d] - c0;
+                    if (a.dsl_group == 1) {
+                        if (a.rowflag[hs]) len[h] = cp[d] - c0;
+                    } else if ((d - 1) % a.dsl_group == 0) {
+                        // a group's chunks stand at its first delay
+                        for (int j = 0; j < a.dsl_group && d + j <= dlast; ++j)
+                            if (a.rowflag[hs - j < 0 ? hs - j + a.D : hs - j]) len[h] = cp[d] - c0;
+                    }
                 }
             }
             int run = 0;
@@ -416,7 +442,7 @@ __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(Pul
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 }
                 last[slot] = c;
-                dsl_issue(a, s1, tab[c], ring + (size_t)slot * SL, &full[slot]);
+                dsl_issue(a, s1, dlast, tab[c], ring + (size_t)slot * SL, &full[slot]);
             }
     } else {
         uint2* hq = hitq + warp * DSL_HITCAP;
@@ -605,8 +631,8 @@ __global__ void k_dsl_count(const int64_t* col_ptr, const uint32_t* csc_src, con
 // atomics and may differ between builds -- the fixed-point sums do not depend
 // on it) ...
 __global__ void k_dsl_fill(const int64_t* col_ptr, const uint32_t* csc_src, const float* csc_w, const uint8_t* csc_d,
-                           int n, int cols, int dmax, int nb, unsigned int* cursor, uint32_t* out_src, float* out_w,
-                           uint16_t* out_col)
+                           int n, int cols, int dmax, int nb, int group, int words, unsigned int* cursor,
+                           uint32_t* out_src, float* out_w, uint16_t* out_col)
 {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
         for (int64_t e = col_ptr[k]; e < col_ptr[k + 1]; ++e) {
@@ -614,7 +640,8 @@ __global__ void k_dsl_fill(const int64_t* col_ptr, const uint32_t* csc_src, cons
             if (d < 1 || d > dmax) continue;
             const uint32_t sw = csc_src[e];
             const unsigned int q = atomicAdd(&cursor[dsl_key(k, cols, dmax, nb, d, sw)], 1u);
-            out_src[q] = sw;
+            // (delays of one chunk: their rows are staged one behind the other)
+            out_src[q] = sw + (uint32_t)((d - 1) % group) * (uint32_t)words * 32u;
             out_w[q] = csc_w[e];
             out_col[q] = (uint16_t)(k % cols);
         }
@@ -1194,6 +1221,7 @@ static PullArgs pull_args(nn_sim* s, int q, bool hybrid)
     a.dsl_ent = s->dsl_ent; a.dsl_w = s->dsl_w; a.dsl_hits = s->dsl_hits;
     a.dsl_cols = s->dsl_cols; a.dsl_ring = s->dsl_ring; a.dsl_slotw = s->dsl_slotw;
     a.dsl_cmax = s->dsl_cmax; a.dsl_dmax = s->dsl_dmax;
+    a.dsl_group = s->dsl_group; a.dsl_zero = s->dsl_zero;
     a.err = s->err;
     return a;
 }
@@ -1337,6 +1365,7 @@ static void free_network(nn_sim* s)
     nn_release(s->row_ptr); nn_release(s->col); nn_release(s->weight); nn_release(s->delay);
     nn_release(s->col_ptr); nn_release(s->csc_src); nn_release(s->csc_w); nn_release(s->csc_d);
     nn_release(s->dsl_chunk); nn_release(s->dsl_cptr); nn_release(s->dsl_ent); nn_release(s->dsl_w); nn_release(s->dsl_hits);
+    nn_release(s->dsl_zero);
     s->nnz = 0;
 }
 
@@ -1391,7 +1420,21 @@ static nn_status build_sliced(nn_sim* s)
     const int nblk = (s->n + cols - 1) / cols;
     const int dmax = s->D - 1;
     const int nb = (s->words + DSL_BUCKET_WORDS - 1) / DSL_BUCKET_WORDS;
-    const int slotw = std::min(s->words, DSL_SPAN * DSL_BUCKET_WORDS);
+    // Delays per chunk.  A chunk costs about 0.9 us whatever it holds, and a
+    // network of 50k neurons and 5e6 synapses has 1,650 entries per block and
+    // delay: 20 chunks, 18 us a step.  So chunks hold as many delays as fill
+    // them on average, while source offsets over all their rows stay below
+    // 2^18; networks of more than 131k neurons, or with full chunks, keep one.
+    int group = 1;
+    {
+        const double per = 1.1 * (double)s->nnz / ((double)nblk * std::max(dmax, 1)) + 1.0;
+        const int fit = std::min({(1 << 18) / (32 * s->words), (int)(DSL_CHUNK / per), dmax});
+        if (fit > 1) {
+            const int groups = (dmax + fit - 1) / fit;
+            group = (dmax + groups - 1) / groups;
+        }
+    }
+    const int slotw = group > 1 ? group * s->words : std::min(s->words, DSL_SPAN * DSL_BUCKET_WORDS);
     if (s->nnz <= 0 || dsl_smem_bytes(2, slotw, cols, 0) > (size_t)smem_max || cols > DSL_MAX_COLS || dmax < 1 ||
         dmax > DSL_MAX_DELAY || s->nnz >= INT32_MAX / 2 || (s->words % 4))
         return NN_OK;
@@ -1432,14 +1475,14 @@ static nn_status build_sliced(nn_sim* s)
         for (int b = 0; b < nblk; ++b) {
             const size_t c_b = chunks.size();
             cptr[(size_t)b * (dmax + 1)] = (int32_t)c_b;
+            bool open = false;
+            int64_t start = 0;
+            int len = 0, b0 = 0, b1 = 0;
             for (int d = 1; d <= dmax; ++d) {
-                bool open = false;
-                int64_t start = 0;
-                int len = 0, b0 = 0, b1 = 0;
                 auto close = [&]() {
-                    const int w0 = b0 * DSL_BUCKET_WORDS;
-                    const int w1 = std::min((b1 + 1) * DSL_BUCKET_WORDS, s->words);
-                    chunks.push_back(make_int4((int)ppos, len, w0, ((w1 - w0) << 8) | d));
+                    const int w0 = group > 1 ? 0 : b0 * DSL_BUCKET_WORDS;
+                    const int w1 = group > 1 ? s->words : std::min((b1 + 1) * DSL_BUCKET_WORDS, s->words);
+                    chunks.push_back(make_int4((int)ppos, len, w0, ((w1 - w0) << 8) | (d - (d - 1) % group)));
                     ustart.push_back((int32_t)start);
                     ppos += (len + 3) & ~3;
                     open = false;
@@ -1449,7 +1492,7 @@ static nn_status build_sliced(nn_sim* s)
                     int64_t left = h[key];
                     h[key] = (unsigned int)pos;
                     while (left > 0) {
-                        if (open && (len == DSL_CHUNK || bk - b0 >= DSL_SPAN)) close();
+                        if (open && (len == DSL_CHUNK || (group == 1 && bk - b0 >= DSL_SPAN))) close();
                         if (!open) {
                             open = true;
                             start = pos;
@@ -1463,8 +1506,9 @@ static nn_status build_sliced(nn_sim* s)
                         b1 = bk;
                     }
                 }
+                if (d % group && d < dmax) continue;  // the group goes on
                 if (open) close();
-                cptr[(size_t)b * (dmax + 1) + d] = (int32_t)chunks.size();
+                for (int e = d - (d - 1) % group; e <= d; ++e) cptr[(size_t)b * (dmax + 1) + e] = (int32_t)chunks.size();
             }
             cmax = std::max(cmax, (int)(chunks.size() - c_b));
         }
@@ -1494,6 +1538,11 @@ static nn_status build_sliced(nn_sim* s)
     if (st == NN_OK) st = nn_alloc(ctx, &s->dsl_ent, (size_t)ppos);
     if (st == NN_OK) st = nn_alloc(ctx, &s->dsl_w, (size_t)ppos);
     if (st == NN_OK) st = nn_alloc(ctx, &s->dsl_hits, (size_t)ppos);
+    if (st == NN_OK && group > 1) {
+        st = nn_alloc(ctx, &s->dsl_zero, (size_t)s->words);
+        if (st == NN_OK)
+            st = nn_cuda_check(ctx, nn_zero_async(ctx, s->dsl_zero, sizeof(uint32_t) * s->words), "build_sliced");
+    }
     if (st == NN_OK)
         st = nn_cuda_check(ctx, nn_copy_sync(ctx, s->dsl_chunk, chunks.data(), sizeof(int4) * chunks.size(),
                                              cudaMemcpyHostToDevice), "build_sliced");
@@ -1505,7 +1554,7 @@ static nn_status build_sliced(nn_sim* s)
                                              cudaMemcpyHostToDevice), "build_sliced");
     if (st == NN_OK) {
         k_dsl_fill<<<nn_grid_for(ctx, s->n, 128, 8), 128, 0, ctx->stream>>>(
-            s->col_ptr, s->csc_src, s->csc_w, s->csc_d, s->n, cols, dmax, nb, cnt, t_src, t_w, t_col);
+            s->col_ptr, s->csc_src, s->csc_w, s->csc_d, s->n, cols, dmax, nb, group, s->words, cnt, t_src, t_w, t_col);
         st = nn_cuda_check(ctx, cudaGetLastError(), "k_dsl_fill");
     }
     if (st == NN_OK) {
@@ -1531,6 +1580,7 @@ static nn_status build_sliced(nn_sim* s)
     cudaFree(d_ustart);
     if (st != NN_OK) {
         nn_release(s->dsl_chunk); nn_release(s->dsl_cptr); nn_release(s->dsl_ent); nn_release(s->dsl_w); nn_release(s->dsl_hits);
+    nn_release(s->dsl_zero);
         return st;
     }
     s->dsl_cols = cols;
@@ -1538,6 +1588,7 @@ static nn_status build_sliced(nn_sim* s)
     s->dsl_slotw = slotw;
     s->dsl_cmax = cmax;
     s->dsl_dmax = dmax;
+    s->dsl_group = group;
     return NN_OK;
 }
 
@@ -1573,6 +1624,7 @@ static nn_status after_network(nn_sim* s)
     drop_graph(s);
     nn_release(s->col_ptr); nn_release(s->csc_src); nn_release(s->csc_w); nn_release(s->csc_d);
     nn_release(s->dsl_chunk); nn_release(s->dsl_cptr); nn_release(s->dsl_ent); nn_release(s->dsl_w); nn_release(s->dsl_hits);
+    nn_release(s->dsl_zero);
     if (s->cfg.delivery == NN_DELIVERY_PULL || s->cfg.delivery == NN_DELIVERY_AUTO) NN_TRY(build_csc(s));
     return NN_OK;
 }
