@@ -70,6 +70,7 @@ struct nn_sim {
     int dsl_cmax = 0;              // most chunks of one block
     int dsl_dmax = 0;              // longest delay of the layout
     int dsl_group = 1;             // delays per chunk (small networks)
+    int dsl_direct = 0;            // sums beside the slots (narrow blocks)
     uint32_t* dsl_zero = nullptr;  // [words] staged in the place of a delay that is not live
     // paracrine
     int grid = 0;
@@ -164,6 +165,7 @@ struct PullArgs {
     int dsl_cols, dsl_ring, dsl_slotw, dsl_cmax, dsl_dmax;
     int dsl_group;
     const uint32_t* dsl_zero;
+    int dsl_direct;  // the sums have shared memory of their own beside the slots
     // automatic delivery: only ring rows with rowflag set hold pull spikes
     // (the others were pushed), and the gather adds to the ring slot, which
     // pushed spikes may already have reached (null / 0: every row, overwrite)
@@ -310,9 +312,18 @@ __device__ __forceinline__ void dsl_issue(const PullArgs& a, int s1, int dlast, 
     nn_bulk_g2s(dst + a.dsl_slotw, a.dsl_ent + m.x, be, bar);
 }
 
+// One hit into the fixed-point sums.
+__device__ __forceinline__ void dsl_add(uint32_t word, float w, unsigned long long* acc_e, unsigned long long* acc_i)
+{
+    atomicAdd(((word >> 31) ? acc_i : acc_e) + ((word >> 18) & 0x1fffu),
+              (unsigned long long)llrintf(w * (float)DSL_FIX));
+}
+
 // Move a warp's queued hits {entry, word} to the block's hit list: each lane
-// loads its weights, then stores {word, weight bits} pairs at out[0, cnt).
-__device__ __forceinline__ void dsl_flush(const uint2* q, int cnt, int lane, const float* w, uint2* out)
+// loads its weights, then stores {word, weight bits} pairs at out[0, cnt) --
+// or, with the sums at hand (out null), adds them.
+__device__ __forceinline__ void dsl_flush(const uint2* q, int cnt, int lane, const float* w, uint2* out,
+                                          unsigned long long* acc_e, unsigned long long* acc_i)
 {
     constexpr int PER = DSL_HITCAP / 32;
     uint32_t ew[PER];
@@ -330,7 +341,10 @@ __device__ __forceinline__ void dsl_flush(const uint2* q, int cnt, int lane, con
     }
 #pragma unroll
     for (int k = 0; k < PER; ++k)
-        if (lane + 32 * k < cnt) out[lane + 32 * k] = make_uint2(ew[k], __float_as_uint(wv[k]));
+        if (lane + 32 * k < cnt) {
+            if (out) out[lane + 32 * k] = make_uint2(ew[k], __float_as_uint(wv[k]));
+            else dsl_add(ew[k], wv[k], acc_e, acc_i);
+        }
 }
 
 __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(PullArgs a)
@@ -338,11 +352,12 @@ __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(Pul
     extern __shared__ __align__(128) unsigned char dsl_smem[];
     const int R = a.dsl_ring, SW = a.dsl_slotw, SL = a.dsl_slotw + DSL_CHUNK;  // slot: bitmap words, entries
     uint32_t* ring = reinterpret_cast<uint32_t*>(dsl_smem);
-    // after the sweep the slots hold the sums
-    unsigned long long* acc_e = reinterpret_cast<unsigned long long*>(dsl_smem);
+    // after the sweep the slots hold the sums (dsl_direct: they lie behind them)
+    const size_t ring_bytes = (size_t)R * SL * 4, sum_bytes = (size_t)a.dsl_cols * 16;
+    unsigned long long* acc_e = reinterpret_cast<unsigned long long*>(dsl_smem + (a.dsl_direct ? ring_bytes : 0));
     unsigned long long* acc_i = acc_e + a.dsl_cols;
     uint2* hitq = reinterpret_cast<uint2*>(
-        dsl_smem + max((size_t)R * SL * 4, (size_t)a.dsl_cols * 16));  // [DSL_WARPS][DSL_HITCAP]
+        dsl_smem + (a.dsl_direct ? ring_bytes + sum_bytes : max(ring_bytes, sum_bytes)));  // [DSL_WARPS][DSL_HITCAP]
     int4* tab = reinterpret_cast<int4*>(hitq + DSL_WARPS * DSL_HITCAP);
     uint64_t* full = reinterpret_cast<uint64_t*>(tab + a.dsl_cmax);
     uint64_t* empty = full + R;
@@ -417,6 +432,8 @@ __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(Pul
     }
     // the block's hit list starts at its first entry: it has room for every entry
     uint2* hits = a.dsl_hits + (C > 0 ? a.dsl_chunk[cfirst].x : 0);
+    if (a.dsl_direct)
+        for (int k = tid; k < a.dsl_cols; k += blockDim.x) acc_e[k] = acc_i[k] = 0ull;
     if (tid == 0) {
         abort_flag = 0;
         hit_count = 0;
@@ -502,10 +519,10 @@ __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(Pul
                     if (!b) continue;
                     if (hcnt + __popc(b) > DSL_HITCAP) {
                         int hb = 0;
-                        if (lane == 0) hb = atomicAdd(&hit_count, hcnt);
+                        if (lane == 0 && !a.dsl_direct) hb = atomicAdd(&hit_count, hcnt);
                         hb = __shfl_sync(0xffffffffu, hb, 0);
                         __syncwarp();
-                        dsl_flush(hq, hcnt, lane, a.dsl_w, hits + hb);
+                        dsl_flush(hq, hcnt, lane, a.dsl_w, a.dsl_direct ? nullptr : hits + hb, acc_e, acc_i);
                         __syncwarp();
                         hcnt = 0;
                     }
@@ -523,10 +540,10 @@ __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(Pul
         }
         if (!abort_flag && hcnt > 0) {
             int hb = 0;
-            if (lane == 0) hb = atomicAdd(&hit_count, hcnt);
+            if (lane == 0 && !a.dsl_direct) hb = atomicAdd(&hit_count, hcnt);
             hb = __shfl_sync(0xffffffffu, hb, 0);
             __syncwarp();
-            dsl_flush(hq, hcnt, lane, a.dsl_w, hits + hb);
+            dsl_flush(hq, hcnt, lane, a.dsl_w, a.dsl_direct ? nullptr : hits + hb, acc_e, acc_i);
         }
     }
     __syncthreads();
@@ -541,14 +558,15 @@ __global__ void __launch_bounds__(DSL_THREADS + 32, 1) k_deliver_pull_sliced(Pul
     // every staged chunk was consumed, so no copy into the slots is pending:
     // sum the hit list (written by this block, read back through L2) into
     // the slots' bytes
-    for (int k = tid; k < a.dsl_cols; k += blockDim.x) acc_e[k] = acc_i[k] = 0ull;
-    __syncthreads();
-    for (int i = tid; i < hit_count; i += blockDim.x) {
-        const uint2 h = __ldcg(hits + i);
-        atomicAdd(((h.x >> 31) ? acc_i : acc_e) + ((h.x >> 18) & 0x1fffu),
-                  (unsigned long long)llrintf(__uint_as_float(h.y) * (float)DSL_FIX));
+    if (!a.dsl_direct) {
+        for (int k = tid; k < a.dsl_cols; k += blockDim.x) acc_e[k] = acc_i[k] = 0ull;
+        __syncthreads();
+        for (int i = tid; i < hit_count; i += blockDim.x) {
+            const uint2 h = __ldcg(hits + i);
+            dsl_add(h.x, __uint_as_float(h.y), acc_e, acc_i);
+        }
+        __syncthreads();
     }
-    __syncthreads();
     float2* out = reinterpret_cast<float2*>(a.ring + (size_t)(t1 % (uint64_t)a.D) * a.n_pad * 2);
     for (int k = tid; k < k1 - k0; k += blockDim.x) {
         const float2 v = make_float2((float)((double)(long long)acc_e[k] / DSL_FIX),
@@ -1221,18 +1239,19 @@ static PullArgs pull_args(nn_sim* s, int q, bool hybrid)
     a.dsl_ent = s->dsl_ent; a.dsl_w = s->dsl_w; a.dsl_hits = s->dsl_hits;
     a.dsl_cols = s->dsl_cols; a.dsl_ring = s->dsl_ring; a.dsl_slotw = s->dsl_slotw;
     a.dsl_cmax = s->dsl_cmax; a.dsl_dmax = s->dsl_dmax;
-    a.dsl_group = s->dsl_group; a.dsl_zero = s->dsl_zero;
+    a.dsl_group = s->dsl_group; a.dsl_zero = s->dsl_zero; a.dsl_direct = s->dsl_direct;
     a.err = s->err;
     return a;
 }
 
 // Dynamic shared memory of k_deliver_pull_sliced: the slots (slotw bitmap
-// words and a chunk of entries each) during the sweep, the same bytes as two
-// 64-bit sums per column after it; the warps' hit queues, the block's chunk
+// words and a chunk of entries each) during the sweep, two 64-bit sums per
+// column behind them (direct) or in the same bytes after it; the warps' hit queues, the block's chunk
 // table, and per slot two mbarriers (full, empty) and the last chunk issued.
-static size_t dsl_smem_bytes(int ring, int slotw, int cols, int cmax)
+static size_t dsl_smem_bytes(int ring, int slotw, int cols, int cmax, bool direct)
 {
-    return std::max((size_t)ring * (slotw + DSL_CHUNK) * 4, (size_t)cols * 16) + (size_t)DSL_WARPS * DSL_HITCAP * 8 +
+    const size_t slots = (size_t)ring * (slotw + DSL_CHUNK) * 4, sums = (size_t)cols * 16;
+    return (direct ? slots + sums : std::max(slots, sums)) + (size_t)DSL_WARPS * DSL_HITCAP * 8 +
            (size_t)cmax * 16 + (size_t)ring * 20;
 }
 
@@ -1244,7 +1263,7 @@ static nn_status launch_pull(nn_sim* s, const PullArgs& d, cudaStream_t cs)
     if (s->dsl_chunk) {
         const int blocks = (s->n + s->dsl_cols - 1) / s->dsl_cols;
         k_deliver_pull_sliced<<<blocks, DSL_THREADS + 32,
-                                dsl_smem_bytes(s->dsl_ring, s->dsl_slotw, s->dsl_cols, s->dsl_cmax), cs>>>(d);
+                                dsl_smem_bytes(s->dsl_ring, s->dsl_slotw, s->dsl_cols, s->dsl_cmax, s->dsl_direct != 0), cs>>>(d);
         NN_CHECK_LAUNCH(ctx, "k_deliver_pull_sliced");
         return NN_OK;
     }
@@ -1422,7 +1441,7 @@ static nn_status build_sliced(nn_sim* s)
     const int nb = (s->words + DSL_BUCKET_WORDS - 1) / DSL_BUCKET_WORDS;
     // Delays per chunk.  A chunk costs about 0.9 us whatever it holds, and a
     // network of 50k neurons and 5e6 synapses has 1,650 entries per block and
-    // delay: 20 chunks, 18 us a step.  So chunks hold as many delays as fill
+    // delay: 20 chunks, 18 us a step (13 us with them merged, launch included).  So chunks hold as many delays as fill
     // them on average, while source offsets over all their rows stay below
     // 2^18; networks of more than 131k neurons, or with full chunks, keep one.
     int group = 1;
@@ -1435,7 +1454,7 @@ static nn_status build_sliced(nn_sim* s)
         }
     }
     const int slotw = group > 1 ? group * s->words : std::min(s->words, DSL_SPAN * DSL_BUCKET_WORDS);
-    if (s->nnz <= 0 || dsl_smem_bytes(2, slotw, cols, 0) > (size_t)smem_max || cols > DSL_MAX_COLS || dmax < 1 ||
+    if (s->nnz <= 0 || dsl_smem_bytes(2, slotw, cols, 0, false) > (size_t)smem_max || cols > DSL_MAX_COLS || dmax < 1 ||
         dmax > DSL_MAX_DELAY || s->nnz >= INT32_MAX / 2 || (s->words % 4))
         return NN_OK;
     // fixed-point range: |sum| <= longest column x largest |weight| < 2^31
@@ -1516,7 +1535,13 @@ static nn_status build_sliced(nn_sim* s)
     // slots: as many as fit, up to DSL_MAX_RING (at least two)
     int ring = DSL_MAX_RING;
     if (const char* r = std::getenv("NN_PULL_RING")) ring = std::max(2, std::min(DSL_MAX_RING, std::atoi(r)));
-    while (ring >= 2 && dsl_smem_bytes(ring, slotw, cols, cmax) > (size_t)smem_max) --ring;
+    while (ring >= 2 && dsl_smem_bytes(ring, slotw, cols, cmax, false) > (size_t)smem_max) --ring;
+    // sums beside the slots where that costs no slot that the chunks would use:
+    // the hits of narrow blocks then go straight into them instead of through
+    // the list in global memory (200 steps of 50k neurons with delays 1-20:
+    // 3455 us against 3545)
+    while (ring > 2 && ring > cmax) --ring;
+    const bool direct = dsl_smem_bytes(ring, slotw, cols, cmax, true) <= (size_t)smem_max;
     if (st != NN_OK || pos > s->nnz || ppos >= INT32_MAX || chunks.empty() || ring < 2) {
         cudaFree(cnt);
         return st;
@@ -1567,7 +1592,7 @@ static nn_status build_sliced(nn_sim* s)
             s->dsl_chunk, d_ustart, nc, t_src, t_col, t_w, s->dsl_ent, s->dsl_w);
         st = nn_cuda_check(ctx, cudaGetLastError(), "k_dsl_pack");
     }
-    const size_t smem = dsl_smem_bytes(ring, slotw, cols, cmax);
+    const size_t smem = dsl_smem_bytes(ring, slotw, cols, cmax, direct);
     if (st == NN_OK)
         st = nn_cuda_check(ctx, cudaFuncSetAttribute(k_deliver_pull_sliced,
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -1580,7 +1605,7 @@ static nn_status build_sliced(nn_sim* s)
     cudaFree(d_ustart);
     if (st != NN_OK) {
         nn_release(s->dsl_chunk); nn_release(s->dsl_cptr); nn_release(s->dsl_ent); nn_release(s->dsl_w); nn_release(s->dsl_hits);
-    nn_release(s->dsl_zero);
+        nn_release(s->dsl_zero);
         return st;
     }
     s->dsl_cols = cols;
@@ -1589,6 +1614,7 @@ static nn_status build_sliced(nn_sim* s)
     s->dsl_cmax = cmax;
     s->dsl_dmax = dmax;
     s->dsl_group = group;
+    s->dsl_direct = direct ? 1 : 0;
     return NN_OK;
 }
 

@@ -223,6 +223,49 @@ def test_chunked_pull_many_buckets(ctx, monkeypatch):
     np.testing.assert_allclose(a[1], u[1], rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("n,k,dmax", [(1024, 8, 1), (1025, 20, 2), (4100, 30, 7), (20000, 100, 23), (2744, 200, 63),
+                                      (131072, 40, 5), (131200, 40, 5)])
+def test_pull_chunks_of_several_delays(ctx, monkeypatch, n, k, dmax):
+    """Pull gathers whose chunks hold one delay, some or all of them: a group
+    that does not divide dmax, rows of the first and last steps that are not
+    live, 131,072 neurons (two delays' offsets fill 18 bits) and one bitmap row
+    more (one delay a chunk).  Against the warp-per-column kernel: same
+    spikes; inputs are sums of at most a few hundred positive weights in another
+    order, a few hundred roundings of 2^-24 at most: 1e-4."""
+    rng = np.random.default_rng(n + dmax)
+    m = n * k
+    col = rng.integers(0, n, m).astype(np.int32)
+    rp = np.arange(n + 1, dtype=np.int64) * k
+    w = np.exp(rng.normal(-1.0, 1.0, m)).astype(np.float32)
+    d = rng.integers(1, dmax + 1, m).astype(np.uint8)
+    inh = (rng.random(n) < 0.2).astype(np.uint8)
+    v = rng.uniform(-65, -35, n).astype(np.float32)
+
+    def run(unsliced):
+        if unsliced:
+            monkeypatch.setenv("NN_PULL_UNSLICED", "1")
+        else:
+            monkeypatch.delenv("NN_PULL_UNSLICED", raising=False)
+        c = nn.default_config(n)
+        c.seed, c.max_delay, c.raster_capacity, c.delivery = 5, dmax, 2_000_000, 1
+        s = nn.Simulation(ctx, c)
+        s.set_network(rp, col, w, d, inh)
+        assert s.pull_info()[0] == (not unsliced)
+        s.init_state(-65.0, 6.0, 12.0)
+        s.set_field("V", v)
+        s.step(3)
+        early = np.stack([s.get_field("GE"), s.get_field("GI")])
+        s.step(97)
+        return raster_set(*s.raster()), early, np.stack([s.get_field("GE"), s.get_field("GI")])
+
+    a, b, u = run(False), run(False), run(True)
+    assert len(a[0]) > 100
+    assert a[0] == b[0] and np.array_equal(a[1], b[1]) and np.array_equal(a[2], b[2])
+    assert a[0] == u[0]
+    np.testing.assert_allclose(a[1], u[1], rtol=1e-4, atol=1e-5)
+    np.testing.assert_allclose(a[2], u[2], rtol=1e-4, atol=1e-5)
+
+
 def test_delays_parity(ctx, orc):
     """Gaussian network with delays U{1..20}: raster and state vs the oracle."""
     n, seed = 2744, 31
