@@ -251,8 +251,8 @@ nn_status nn_rcg_batch_begin(nn_rcg_batch* pl, const float* d_b, float* d_x, dou
 nn_status nn_rcg_batch_finish(nn_rcg_batch* pl, cudaStream_t cs, int* iters, int* flags);
 
 struct nn_cg_plan;
-nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D,
-                            const float* invdv, bool lazy, nn_cg_plan** out);
+nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D, bool lazy,
+                            nn_cg_plan** out);
 void nn_cg_plan_destroy(nn_cg_plan* pl);
 nn_status nn_cg_run(nn_cg_plan* pl, const float* d_b, float* d_x, double rtol, int max_iter, int* iters,
                     double* relres, int* converged);

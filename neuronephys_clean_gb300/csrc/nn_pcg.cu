@@ -39,7 +39,7 @@ struct nn_pcg {
     std::vector<cudaEvent_t> ev_a, ev_b;
     float last_ms = 0.0f;
     int last_iters = 0;
-    // single-kernel TMA iteration (nx % 4 == 0, aligned D); null: two-kernel path
+    // single-kernel iteration; null: two-kernel path
     nn_cg_plan* fast = nullptr;
     // whole solve in one kernel, for grids that fit on the chip; null: a
     // launch per iteration (or two)
@@ -350,13 +350,13 @@ extern "C" nn_status nn_pcg_create(nn_ctx* ctx, int nx, int ny, int nz, double a
     }
     st = nn_cuda_check(ctx, cudaGetLastError(), "nn_pcg_create");
     if (st == NN_OK && !std::getenv("NN_PCG_TWO_KERNEL")) {
-        // the resident solve where the grid fits, and the single-kernel TMA
-        // iteration where supported (beside the resident solve only the tile
-        // autotuner uses it, which allocates its vectors then)
+        // the resident solve where the grid fits, and the single-kernel
+        // iteration (beside the resident solve only the tile autotuner uses it,
+        // which allocates its vectors then)
         nn_status fs = nn_rcg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, &pc->res);
         if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
         if (st == NN_OK) {
-            fs = nn_cg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, pc->invd, pc->res != nullptr, &pc->fast);
+            fs = nn_cg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, pc->res != nullptr, &pc->fast);
             if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
         }
         ctx->last_error.clear();
@@ -522,13 +522,17 @@ nn_status nn_pcg_async_finish(nn_pcg* pc, int* iters, double* relres, int* conve
 
 bool nn_pcg_async_supported(const nn_pcg* pc) { return pc->fast != nullptr || pc->res != nullptr; }
 
-// The resident solve when the grid fits, the single-kernel TMA iteration when
-// its rows allow it, else two kernels.
+// Grids of whole aligned quads: their solves want x aligned too, and their tile
+// depth can be tuned.
+static bool tunable(const nn_pcg* pc) { return pc->fast && pc->nx % 4 == 0 && !((uintptr_t)pc->Dcell & 15); }
+
+// The resident solve when the grid fits, else the single-kernel iteration, else
+// (2^31 cells and more) two kernels.
 nn_status nn_pcg_run_best(nn_pcg* pc, const float* d_b, float* d_x, double rtol, int max_iter, int* iters,
                           double* relres, int* converged)
 {
     if (pc->res) {
-        if (pc->fast && ((uintptr_t)d_x & 15))
+        if (tunable(pc) && ((uintptr_t)d_x & 15))
             return nn_fail(pc->ctx, NN_ERR_INVALID_ARG, "PCG: x must be a 16-byte aligned device vector");
         NN_TRY(nn_rcg_begin(pc->res, d_b, d_x, rtol, max_iter, pc->ctx->stream));
         return nn_rcg_finish(pc->res, pc->ctx->stream, iters, relres, converged);
@@ -545,19 +549,19 @@ __global__ void k_pcg_trial_rhs(float* b, int64_t G)
         b[i] = 0.5f + (float)(((uint32_t)i * 2654435761u) >> 22) * (1.0f / 1024.0f);
 }
 
-// Tile depth of the single-kernel iteration (0: the grid runs the two-kernel PCG).
-int nn_pcg_tile_depth(const nn_pcg* pc) { return pc->fast ? nn_cg_plan_tile_depth(pc->fast) : 0; }
+// Tile depth of the single-kernel iteration (0: not tunable).
+int nn_pcg_tile_depth(const nn_pcg* pc) { return tunable(pc) ? nn_cg_plan_tile_depth(pc->fast) : 0; }
 void nn_pcg_set_tile_depth(nn_pcg* pc, int zc)
 {
-    if (pc->fast && zc >= 4) nn_cg_plan_set_tile_depth(pc->fast, zc);
+    if (tunable(pc) && zc >= 4) nn_cg_plan_set_tile_depth(pc->fast, zc);
 }
 
 // Tile autotuner of the single-kernel iteration (nn_cg_plan_autotune) on
-// scratch vectors; NN_ERR_UNSUPPORTED when the grid runs the two-kernel PCG.
+// scratch vectors; NN_ERR_UNSUPPORTED on grids that it does not take.
 nn_status nn_pcg_autotune_tiles(nn_pcg* pc, int iters, int* tile_z, float* ms_per_iter)
 {
     if (!pc || iters < 1) return NN_ERR_INVALID_ARG;
-    if (!pc->fast) return NN_ERR_UNSUPPORTED;
+    if (!tunable(pc)) return NN_ERR_UNSUPPORTED;
     nn_ctx* ctx = pc->ctx;
     const int64_t G = (int64_t)pc->nx * pc->ny * pc->nz;
     float *b = nullptr, *x = nullptr;

@@ -1,0 +1,73 @@
+"""The CG of one kernel an iteration, on grids too large for the resident
+solve: tiles cut short, rows that end inside a quad, several tiles along a row,
+single planes and cells a row, odd and even iteration counts.
+
+Tolerance of a solve: the recurrence's relative residual <= rtol.  The true
+residual may exceed it by the rounding of the FP32 recurrences: 2^-24 |A| |x|
+an iteration, adding up like sqrt(100) = 10 over the iterations here, with
+|A| <= 1 + beta + 12 alpha max D and |x| <= the larger of guess and solution.
+The error is at most the residual over the smallest eigenvalue, 1 + beta."""
+import numpy as np
+import pytest
+
+import neuronephys_clean_gb300 as nn
+
+pytestmark = pytest.mark.gpu
+
+HETERO = [(80, 66, 260), (109, 111, 113), (400, 700, 5), (37, 37, 1030), (2, 3, 240001), (9000, 2, 80)]
+CONST = [(136, 135, 137), (900, 1000, 3), (2, 1100, 1152)]
+
+
+def _problem(shape, hetero, seed=3):
+    rng = np.random.default_rng(seed)
+    G = int(np.prod(shape))
+    D = rng.lognormal(0.0, 0.7, shape).astype(np.float32) if hetero else None
+    b = (0.01 * rng.random(G)).astype(np.float32)
+    b[rng.integers(0, G, max(1, G // 300))] += 1.0
+    return D, b, rng.random(G).astype(np.float32)
+
+
+@pytest.mark.parametrize("shape,hetero", [(s, True) for s in HETERO] + [(s, False) for s in CONST])
+def test_streamed_solve_matches_oracle(ctx, orc, shape, hetero):
+    nz, ny, nx = shape
+    D, b, x0 = _problem(shape, hetero)
+    alpha, beta = 1.5, 0.2
+    pc = nn.PCG(ctx, nx, ny, nz, alpha, beta, ctx.to_device(D.ravel()) if hetero else None)
+    db = ctx.to_device(b)
+    norm = 1 + beta + 12 * alpha * (1.0 if D is None else float(D.max()))
+    for guess, rtol in ((np.zeros_like(b), 1e-5), (x0, 1e-6)):  # a second solve of the same object
+        dx = ctx.to_device(guess)
+        it, rel = pc.solve(db, dx, rtol=rtol, max_iter=500)
+        assert 0 < it <= 100 and rel <= rtol
+        x = dx.numpy()
+        gap = 10 * 2.0 ** -24 * norm * max(np.linalg.norm(guess), np.linalg.norm(x))
+        bound = rtol * np.linalg.norm(b) + gap
+        assert np.linalg.norm(b - orc.apply7(x, shape, alpha, beta, D)) <= bound
+    it, rel = pc.solve(db, dx, rtol=1e-4, max_iter=10)  # recognised without an iteration
+    assert it == 0 and rel <= 1e-4 and np.array_equal(dx.numpy(), x)
+
+
+@pytest.mark.parametrize("shape,hetero", [((70, 131, 153), True), ((130, 140, 136), False)])
+def test_streamed_iterates_match_two_kernels(ctx, monkeypatch, shape, hetero):
+    """x after n iterations, n odd and even, against the two-kernel solver's.
+    Both run the same recurrence in FP32 from x = 0: the rounding of some ten
+    operations an iteration, 1e-5 of the iterate with room."""
+    nz, ny, nx = shape
+    D, b, _ = _problem(shape, hetero)
+    dD, db = ctx.to_device(D.ravel()) if hetero else None, ctx.to_device(b)
+    got = []
+    for env in (False, True):
+        if env:
+            monkeypatch.setenv("NN_PCG_TWO_KERNEL", "1")
+        pc = nn.PCG(ctx, nx, ny, nz, 2.0, 0.1, dD)
+        monkeypatch.delenv("NN_PCG_TWO_KERNEL", raising=False)
+        xs = []
+        for n in (0, 1, 2, 3, 4, 17, 18):
+            dx = ctx.to_device(np.zeros_like(b))
+            with pytest.raises(nn.NNError) as e:
+                pc.solve(db, dx, rtol=1e-12, max_iter=n)
+            assert e.value.status == nn.NN_ERR_NOT_CONVERGED
+            xs.append(dx.numpy())
+        got.append(xs)
+    for n, (x, y) in enumerate(zip(*got)):
+        assert np.linalg.norm(x - y) <= 1e-5 * np.linalg.norm(y), n
