@@ -113,3 +113,20 @@ def test_weight_gradient_many_tiles(ctx, cin, cout):
     nn.conv3d_wgrad(ctx, to_act(ctx, x), to_act(ctx, gy), dw, None)
     rdw, _ = U.conv3d_weight_grad(x, gy)
     np.testing.assert_allclose(dw.numpy(), rdw, rtol=1e-5, atol=1e-5 * np.abs(rdw).max())
+
+
+@pytest.mark.parametrize("cin", [16, 32, 48])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 2, 130), (2, 126, 1), (40, 48, 64)])
+def test_weight_gradient_16_channels(ctx, cin, shape):
+    """The weight gradient of 16-channel layers (all taps in one CTA): a single
+    voxel, one tile and a bit, rows of one cell, several tiles per CTA (more
+    than its copy slots).  dw is added to.  A CTA's sums are FP32 over at most
+    eight tiles, then 152 of them: 1e-5 of the largest gradient as above."""
+    rng = np.random.default_rng(cin + shape[2])
+    x, gy = rand_act(rng, cin, shape), rand_act(rng, 16, shape)
+    d0 = rng.standard_normal((27, cin, 16)).astype(np.float32)
+    dw, db = ctx.to_device(d0), ctx.to_device(np.zeros(16, np.float32))
+    nn.conv3d_wgrad(ctx, to_act(ctx, x), to_act(ctx, gy), dw, db)
+    rdw, rdb = U.conv3d_weight_grad(x, gy)
+    np.testing.assert_allclose(dw.numpy(), d0 + rdw, rtol=1e-5, atol=1e-5 * np.abs(rdw).max())
+    np.testing.assert_allclose(db.numpy(), rdb, rtol=1e-5, atol=1e-5 * np.abs(rdb).max())
