@@ -23,6 +23,8 @@
 // channels have a kernel of their own (k_conv3_wgrad16).
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "nn_conv.cuh"
 #include "nn_ptx.cuh"
 
@@ -107,6 +109,48 @@ __device__ __forceinline__ bool interior(const nn_act_geom& g, int64_t o, int& z
     y = (int)(rem / g.R);
     x = (int)(rem - (int64_t)y * g.R);
     return z >= 1 && z <= g.nz && y >= 1 && y <= g.ny && x >= 1 && x <= g.nx;
+}
+
+template <int COUT>
+__device__ __forceinline__ void load_mask(const ConvArgs& a, int64_t o, uint4 (&mk)[COUT / 8])
+{
+    if (!a.mask) return;
+#pragma unroll
+    for (int gb = 0; gb < COUT / 8; ++gb) mk[gb] = a.mask[gb * a.g.S + a.g.GD + o];
+}
+
+// The epilogue of one voxel: accumulators v (and masks mk, if a.mask) to the
+// outputs; (z, y, x) its interior coordinates when in.
+template <int COUT>
+__device__ __forceinline__ void store_voxel(const ConvArgs& a, int64_t o, bool in, int z, int y, int x, const float* v,
+                                            const uint4 (&mk)[COUT / 8])
+{
+#pragma unroll
+    for (int gb = 0; gb < COUT / 8; ++gb) {
+        float t[8], m[8];
+        if (a.mask) unpack_bf16x8(mk[gb], m);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float q = v[gb * 8 + i] + (a.bias ? a.bias[gb * 8 + i] : 0.0f);
+            if (a.relu) q = fmaxf(q, 0.0f);
+            if (a.mask && !(m[i] > 0.0f)) q = 0.0f;
+            t[i] = in ? q : 0.0f;
+        }
+        const uint4 pk = pack_bf16x8(t);
+        a.y[gb * a.g.S + a.g.GD + o] = pk;
+        if (a.up && in) {
+            // the eight children of interior voxel (z, y, x) (1-based) in the finer grid
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const int64_t fz = 2 * (z - 1) + (c >> 2) + 1, fy = 2 * (y - 1) + ((c >> 1) & 1) + 1,
+                              fx = 2 * (x - 1) + (c & 1) + 1;
+                a.up[gb * a.gu.S + a.gu.GD + fz * a.gu.P + fy * a.gu.R + fx] = pk;
+            }
+        }
+        if (gb == 0 && a.y32 && in)
+            a.y32[((int64_t)(z - 1) * a.g.ny + (y - 1)) * a.g.nx + (x - 1)] =
+                a.y32_scale ? t[0] * (float)a.y32_scale[0] : t[0];
+    }
 }
 
 template <int CIN, int COUT>
@@ -201,39 +245,171 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3(ConvArgs a)
         const int64_t o = o0 + tid;  // TMEM lane == tile row == voxel
         int z, y, x;
         const bool in = interior(a.g, o, z, y, x);
+        uint4 mk[COUT / 8];
+        load_mask<COUT>(a, o, mk);
         float v[COUT];
 #pragma unroll
         for (int c0 = 0; c0 < COUT; c0 += 16) nn_tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0, v + c0);
-#pragma unroll
-        for (int gb = 0; gb < COUT / 8; ++gb) {
-            float t[8], mk[8];
-            if (a.mask) unpack_bf16x8(a.mask[gb * a.g.S + a.g.GD + o], mk);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float q = v[gb * 8 + i] + (a.bias ? a.bias[gb * 8 + i] : 0.0f);
-                if (a.relu) q = fmaxf(q, 0.0f);
-                if (a.mask && !(mk[i] > 0.0f)) q = 0.0f;
-                t[i] = in ? q : 0.0f;
-            }
-            const uint4 pk = pack_bf16x8(t);
-            a.y[gb * a.g.S + a.g.GD + o] = pk;
-            if (a.up && in) {
-                // the eight children of interior voxel (z, y, x) (1-based) in the finer grid
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int64_t fz = 2 * (z - 1) + (c >> 2) + 1, fy = 2 * (y - 1) + ((c >> 1) & 1) + 1,
-                                  fx = 2 * (x - 1) + (c & 1) + 1;
-                    a.up[gb * a.gu.S + a.gu.GD + fz * a.gu.P + fy * a.gu.R + fx] = pk;
-                }
-            }
-            if (gb == 0 && a.y32 && in)
-                a.y32[((int64_t)(z - 1) * a.g.ny + (y - 1)) * a.g.nx + (x - 1)] =
-                    a.y32_scale ? t[0] * (float)a.y32_scale[0] : t[0];
-        }
+        store_voxel<COUT>(a, o, in, z, y, x, v, mk);
     }
     nn_tc_fence_before();
     __syncthreads();
     if (warp == 0) {
+        nn_tc_fence_after();
+        nn_tmem_dealloc(tmem, C::TMEM_COLS);
+    }
+}
+
+// The same for layers of 16 input channels on grids of many tiles, with the same
+// sums in the same order.  k_conv3 reads its weights again for every tile (as many
+// bytes as its windows or more) and does copies, MMAs and epilogue of a tile one
+// after another.  Here a CTA keeps all weights in shared memory and walks over
+// pairs of tiles; one warp issues the copies, one for each tile the MMAs, eight
+// the epilogue of the pair before.  A commit drains the MMAs before it, so there
+// is one for the nine of a dz.
+// Time in us, before and here: 16 -> 16 and 48 on 64^3 voxels 22.6 and 39, 16 and
+// 22; 16 -> 48 on 72 x 80 x 96 75 and 40.  Wider layers stay with k_conv3: their
+// MMAs read 4 KB of A for few columns, about 30 ns each, which bounds both (48 ->
+// 16 on 72 x 80 x 96: 70 and 75; 32 -> 16 on 64^3 1.1 times slower here).
+template <int CIN, int COUT>
+struct StreamCfg {
+    static constexpr int G_IN = CIN / 8;
+    static constexpr int W_BYTES = 27 * CIN * COUT * 2;
+    static constexpr int WIN = (2 * TILE + 2) * 16;
+    static constexpr int STAGE = (3 * G_IN * WIN + 127) / 128 * 128;  // the three dy of a dz
+    static constexpr int PER_SM = 110 * 1024 - W_BYTES >= 3 * STAGE ? 2 : 1;
+    static constexpr int STAGES = std::min(8, ((PER_SM == 2 ? 110 : 220) * 1024 - W_BYTES) / STAGE);
+    static constexpr int SMEM = 128 + W_BYTES + STAGES * STAGE;
+    static constexpr uint32_t TMEM_COLS = 4 * COUT <= 64 ? 64 : 4 * COUT <= 128 ? 128 : 256;  // [buffer][tile]
+    static_assert(STAGES >= 3 && 4 * COUT <= 256 && W_BYTES % 128 == 0, "stages and accumulators");
+};
+constexpr int STREAM_THREADS = 352;
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(STREAM_THREADS) k_conv3_stream(const __grid_constant__ ConvArgs a)
+{
+    using C = StreamCfg<CIN, COUT>;
+    constexpr int S = C::STAGES;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* const wsm = align128(smem_raw);
+    unsigned char* const win = wsm + C::W_BYTES;
+    __shared__ uint64_t full[S], empty[S], wbar, acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int tiles = (int)a.g.tiles, npairs = (tiles + 1) / 2;
+    const int n = (npairs - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;  // at most npairs CTAs
+    // first tile of the CTA's j-th pair; of an odd number the last pair repeats a tile
+    auto first = [&](int j) { return min(2 * ((int)blockIdx.x + j * (int)gridDim.x), tiles - 2); };
+    if (tid == 0) {
+        for (int q = 0; q < S; ++q) {
+            nn_mbar_init(&full[q], 1);
+            nn_mbar_init(&empty[q], 2);
+        }
+        nn_mbar_init(&wbar, 1);
+        for (int q = 0; q < 2; ++q) {
+            nn_mbar_init(&acc_full[q], 2);
+            nn_mbar_init(&acc_empty[q], 8);
+        }
+        nn_mbar_fence_init();
+        abort_flag = 0;
+    }
+    if (warp == 1) nn_tmem_alloc(&tmem_slot, C::TMEM_COLS);
+    nn_tc_fence_before();
+    __syncthreads();
+    nn_tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    // the kernel before this one has finished with the activations
+    nn_grid_dep_wait();
+    auto wait = [&](uint64_t* bar, int phase) -> bool {
+        if (!nn_mbar_wait(bar, (uint32_t)(phase & 1), CONV_WAIT_LIMIT)) abort_flag = 1;
+        return !abort_flag;
+    };
+
+    int issued = 0;
+    if (tid == 0) {
+        nn_mbar_expect_tx(&wbar, C::W_BYTES);
+        nn_bulk_g2s(wsm, a.w, C::W_BYTES, &wbar);
+        bool ok = true;
+        for (int j = 0; ok && j < n; ++j) {
+            const uint4* src0 = a.x + a.g.GD + a.g.o_first + (int64_t)first(j) * TILE - 1;
+            for (int dz = 0; dz < 3; ++dz, ++issued) {
+                const int q = issued % S;
+                if (issued >= S && !(ok = wait(&empty[q], issued / S - 1))) break;
+                nn_mbar_expect_tx(&full[q], 3 * C::G_IN * C::WIN);
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy) {
+                    const uint4* src = src0 + (dz - 1) * a.g.P + (dy - 1) * a.g.R;
+#pragma unroll
+                    for (int gi = 0; gi < C::G_IN; ++gi)
+                        nn_bulk_g2s(win + q * C::STAGE + (dy * C::G_IN + gi) * C::WIN, src + gi * a.g.S, C::WIN, &full[q]);
+                }
+            }
+        }
+    } else if (warp == 1 || warp == 2) {
+        const int h = warp - 1;
+        const uint32_t lead = nn_elect();
+        constexpr uint32_t idesc = nn_umma_idesc_bf16(128, COUT);
+        const uint32_t wbase0 = nn_smem_u32(wsm), win0 = nn_smem_u32(win);
+        bool ok = wait(&wbar, 0);
+        for (int j = 0, it = 0; ok && j < n; ++j) {
+            if (j >= 2 && !(ok = wait(&acc_empty[j & 1], j / 2 - 1))) break;
+            nn_tc_fence_after();
+            const uint32_t acc = tmem + (j & 1) * 2 * COUT;
+            for (int dz = 0; dz < 3; ++dz, ++it) {
+                const int q = it % S;
+                if (!(ok = wait(&full[q], it / S))) break;
+                nn_tc_fence_after();
+                const uint32_t abase = win0 + q * C::STAGE, wbase = wbase0 + dz * (C::W_BYTES / 3);
+#pragma unroll
+                for (int t = 0; t < 9; ++t)  // (dy, dx)
+#pragma unroll
+                    for (int kc = 0; kc < CIN / 16; ++kc) {
+                        const uint64_t bd = nn_umma_sdesc(wbase + (t * (CIN / 16) + kc) * 2 * COUT * 16, COUT * 16, 128);
+                        const uint64_t ad = nn_umma_sdesc(
+                            abase + (t / 3 * C::G_IN + 2 * kc) * C::WIN + (t % 3 + h * TILE) * 16, C::WIN, 128);
+                        nn_umma_bf16_lead(lead, acc + h * COUT, ad, bd, idesc, (dz | t | kc) != 0);
+                    }
+                if (lead) nn_umma_commit(&empty[q]);
+                __syncwarp();
+            }
+            if (lead) nn_umma_commit(&acc_full[j & 1]);
+            __syncwarp();
+        }
+    } else if (warp >= 3) {
+        const int h = (warp - 3) >> 2, row = 32 * (warp & 3) + lane;  // a warp reads the TMEM lanes of its number modulo four
+        const int R = (int)a.g.R, P = (int)a.g.P;
+        for (int j = 0; j < n; ++j) {
+            const int o = (int)a.g.o_first + (first(j) + h) * TILE + row;
+            const int z = o / P, rem = o - z * P, y = rem / R, x = rem - y * R;
+            const bool in = z >= 1 && z <= a.g.nz && y >= 1 && y <= a.g.ny && x >= 1 && x <= a.g.nx;
+            uint4 mk[COUT / 8];
+            load_mask<COUT>(a, o, mk);
+            const bool ok = lane != 0 || wait(&acc_full[j & 1], j / 2);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            nn_tc_fence_after();
+            float v[COUT];
+#pragma unroll
+            for (int c0 = 0; c0 < COUT; c0 += 16)
+                nn_tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + ((j & 1) * 2 + h) * COUT + c0, v + c0);
+            nn_tc_fence_before();
+            __syncwarp();
+            if (lane == 0) nn_mbar_arrive(&acc_empty[j & 1]);
+            store_voxel<COUT>(a, o, in, z, y, x, v, mk);
+        }
+    }
+    __syncwarp();
+    nn_tc_fence_before();
+    __syncthreads();
+    if (abort_flag && tid == 0) {
+        // let copies already in flight land before the CTA leaves
+        nn_mbar_wait(&wbar, 0, CONV_WAIT_LIMIT);
+        for (int i = issued > S ? issued - S : 0; i < issued; ++i)
+            nn_mbar_wait(&full[i % S], (uint32_t)((i / S) & 1), CONV_WAIT_LIMIT);
+        atomicExch(a.err, 1);
+    }
+    __syncthreads();
+    if (warp == 1) {
         nn_tc_fence_after();
         nn_tmem_dealloc(tmem, C::TMEM_COLS);
     }
@@ -417,7 +593,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
 // rows of a fourth MMA.  N = CIN, K = voxels; x is loaded once a tile.  One CTA
 // per SM; one warp issues the copies, another the MMAs.
 // Bound by the copies, about 5 TB/s from L2.  48 -> 16 channels on 72 x 80 x 96
-// voxels: 43 us against 213; 16 -> 16 on 64^3: 22 against 41.
+// voxels: 40 us against 213; 16 -> 16 on 64^3: 19 against 41.
 constexpr int W16_PAIRS = 8;
 constexpr int W16_LAST = 6 * WG_BLOCK;                // the ninth pair: [dx][channel block]
 constexpr int W16_WIN = 2 * W16_PAIRS * WIN_BYTES;    // [channel block][pair]
@@ -444,7 +620,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad16(const uint4* __res
     __shared__ uint64_t full[S], done[S], acc_bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int64_t ntiles = (g.tiles - 1 - (int64_t)blockIdx.x) / gridDim.x + 1;  // the grid has at most g.tiles CTAs
     if (tid == 0) {
         for (int q = 0; q < S; ++q) {
@@ -484,7 +660,8 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad16(const uint4* __res
                 nn_bulk_g2s(buf + W16_LAST + W16_WIN + cb * WG_BLOCK, x + cb * g.S + g.GD + o0, WG_BLOCK, &full[q]);
         }
     }
-    if (tid == 0) {
+    if (warp == 0) {
+        const uint32_t lead = nn_elect();
         // A and B both MN-major (bits 15, 16 of the instruction descriptor)
         constexpr uint32_t idesc = nn_umma_idesc_bf16(WG_MP, CIN) | (1u << 15) | (1u << 16);
         for (int64_t j = 0; j < ntiles; ++j) {
@@ -500,13 +677,14 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad16(const uint4* __res
                 const uint64_t bd = nn_umma_sdesc(xs + kk * 256, 128, WG_BLOCK);
 #pragma unroll
                 for (int dx = 0; dx < 3; ++dx)
-                    nn_umma_bf16(tmem + dx * CIN, nn_umma_sdesc(win + (kk * 16 + 2 - dx) * 16, 128, WIN_BYTES), bd, idesc,
+                    nn_umma_bf16_lead(lead, tmem + dx * CIN, nn_umma_sdesc(win + (kk * 16 + 2 - dx) * 16, 128, WIN_BYTES), bd, idesc,
                                  (j | kk) != 0);
-                nn_umma_bf16(tmem + 3 * CIN, nn_umma_sdesc(last + kk * 256, 128, WG_BLOCK), bd, idesc, (j | kk) != 0);
+                nn_umma_bf16_lead(lead, tmem + 3 * CIN, nn_umma_sdesc(last + kk * 256, 128, WG_BLOCK), bd, idesc, (j | kk) != 0);
             }
-            nn_umma_commit(&done[q]);
+            if (lead) nn_umma_commit(&done[q]);
+            __syncwarp();
         }
-        nn_umma_commit(&acc_bar);
+        if (lead) nn_umma_commit(&acc_bar);
     }
     // (lanes 1-31 wait for their warp's issuing lane; then one thread waits for
     // the accumulators, as above)
@@ -630,6 +808,24 @@ __global__ void k_act_unpack(const uint4* act, nn_act_geom g, int C, float* dens
 template <int CIN, int COUT>
 nn_status launch_fwd(nn_ctx* ctx, const ConvArgs& a)
 {
+    // many tiles per SM (see k_conv3_stream)
+    if constexpr (CIN == 16) {
+        using W = StreamCfg<CIN, COUT>;
+        if (a.g.tiles > (int64_t)ctx->num_sms * 4 && a.g.S < INT32_MAX) {
+            static bool set = false;
+            if (!set) {
+                NN_CUDA(ctx, cudaFuncSetAttribute(k_conv3_stream<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  W::SMEM));
+                NN_CUDA(ctx, cudaFuncSetAttribute(k_conv3_stream<CIN, COUT>,
+                                                  cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+                set = true;
+            }
+            NN_CUDA(ctx, nn_launch_pdl(k_conv3_stream<CIN, COUT>, dim3(W::PER_SM * ctx->num_sms), dim3(STREAM_THREADS),
+                                       (size_t)W::SMEM, ctx->stream, a));
+            ctx->launches++;
+            return NN_OK;
+        }
+    }
     using C = ConvCfg<CIN, COUT>;
     static bool attr_set = false;  // per process; kernels are per device but the attribute is a function property
     if (!attr_set) {

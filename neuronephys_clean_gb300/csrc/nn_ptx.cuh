@@ -97,6 +97,27 @@ __device__ __forceinline__ void nn_umma_bf16(uint32_t tmem_d, uint64_t adesc, ui
         : "memory");
 }
 
+// The same for a converged warp, issued by the lane with lead != 0: the loop
+// around it then runs on uniform registers, which the descriptors are passed in
+// (a loop of one thread moves each of them there: 50 ns an MMA, here 31).
+__device__ __forceinline__ void nn_umma_bf16_lead(uint32_t lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                                  uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+        : "memory");
+}
+
+// One lane of a converged warp (the same at every call).
+__device__ __forceinline__ uint32_t nn_elect()
+{
+    uint32_t lead;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(lead));
+    return lead;
+}
+
 // Arrive on the mbarrier once all previously issued MMAs of this thread completed.
 __device__ __forceinline__ void nn_umma_commit(uint64_t* bar)
 {

@@ -130,3 +130,21 @@ def test_weight_gradient_16_channels(ctx, cin, shape):
     rdw, rdb = U.conv3d_weight_grad(x, gy)
     np.testing.assert_allclose(dw.numpy(), d0 + rdw, rtol=1e-5, atol=1e-5 * np.abs(rdw).max())
     np.testing.assert_allclose(db.numpy(), rdb, rtol=1e-5, atol=1e-5 * np.abs(rdb).max())
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (16, 48), (48, 16)])
+@pytest.mark.parametrize("shape", [(2, 1, 39000), (290, 9, 23), (27, 50, 61)])
+def test_streamed_forward_matches_oracle(ctx, cin, cout, shape):
+    """The forward kernels of grids with many tiles (of 16-channel inputs with the
+    weights kept in shared memory): odd numbers of tiles, two rows, a last tile that is mostly past the grid, several tiles
+    per CTA; bias, ReLU, mask and the dense output at once."""
+    assert ((np.prod(np.add(shape, 2)) - 2 * (shape[1] + 2) * (shape[2] + 2)) / 128) > 608
+    rng = np.random.default_rng(cin * 100 + cout)
+    x, w, m = rand_act(rng, cin, shape), rand_w(rng, cin, cout), rand_act(rng, cout, shape)
+    b = rng.standard_normal(cout).astype(np.float32) * 0.1
+    wp = nn.conv3d_pack_weights(ctx, ctx.to_device(w), cin, cout)
+    ay, y32 = nn.Activation(ctx, shape, cout), ctx.empty(shape, np.float32)
+    nn.conv3d_forward(ctx, to_act(ctx, x), wp, ay, bias=ctx.to_device(b), relu=True, mask=to_act(ctx, m), y32=y32)
+    ref = np.maximum(U.conv3d(x, w, b), 0.0) * (m > 0)
+    assert_bf16_close(ay.unpack(), ref)
+    np.testing.assert_allclose(y32.numpy(), U.bf16(ref[0]), rtol=2.0 ** -7, atol=1e-6 * np.abs(ref).max())
