@@ -82,6 +82,7 @@ void nn_ctx_release(nn_ctx* ctx)
     cudaStreamSynchronize(ctx->stream);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+    nn_release(ctx->conv_err);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }

@@ -1003,25 +1003,31 @@ extern "C" nn_status nn_conv3d_pack_weights(nn_ctx* ctx, int cin, int cout, cons
     return nn_conv_pack(ctx, cin, cout, d_w, adjoint, d_packed);
 }
 
+// The error word of one call: the context's (a context belongs to one host
+// thread, and every call returns with it read).
+static nn_status conv_err_clear(nn_ctx* ctx)
+{
+    if (!ctx->conv_err) NN_TRY(nn_alloc(ctx, &ctx->conv_err, 1));
+    return nn_cuda_check(ctx, cudaMemsetAsync(ctx->conv_err, 0, sizeof(int), ctx->stream), "memset");
+}
+
+static nn_status conv_err_check(nn_ctx* ctx, const char* kernel)
+{
+    int h = 0;
+    NN_CUDA(ctx, nn_copy_sync(ctx, &h, ctx->conv_err, sizeof(int), cudaMemcpyDeviceToHost));
+    return h ? nn_fail(ctx, NN_ERR_TIMEOUT, "%s: a pipeline wait timed out", kernel) : NN_OK;
+}
+
 extern "C" nn_status nn_conv3d_forward(nn_ctx* ctx, int nz, int ny, int nx, int cin, int cout, const void* d_x,
                                        const void* d_wpacked, const float* d_bias, int relu, const void* d_mask,
                                        void* d_y, float* d_y32)
 {
     if (!ctx || !d_x || !d_wpacked || !d_y || nz < 1 || ny < 1 || nx < 1) return NN_ERR_INVALID_ARG;
     if (!nn_conv_supported(cin, cout)) return nn_fail(ctx, NN_ERR_UNSUPPORTED, "conv3d %d -> %d", cin, cout);
-    int* err = nullptr;
-    NN_TRY(nn_alloc(ctx, &err, 1));
-    nn_status st = nn_cuda_check(ctx, cudaMemsetAsync(err, 0, sizeof(int), ctx->stream), "memset");
-    if (st == NN_OK)
-        st = nn_conv_forward(ctx, nn_act_geometry(nz, ny, nx), cin, cout, d_x, d_wpacked, d_bias, relu, d_mask, d_y,
-                             d_y32, err);
-    int h_err = 0;
-    if (st == NN_OK) st = nn_cuda_check(ctx, cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost,
-                                                             ctx->stream), "memcpy");
-    if (st == NN_OK) st = nn_cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "conv3d");
-    nn_release(err);
-    if (st == NN_OK && h_err) st = nn_fail(ctx, NN_ERR_TIMEOUT, "k_conv3: a pipeline wait timed out");
-    return st;
+    NN_TRY(conv_err_clear(ctx));
+    NN_TRY(nn_conv_forward(ctx, nn_act_geometry(nz, ny, nx), cin, cout, d_x, d_wpacked, d_bias, relu, d_mask, d_y, d_y32,
+                           ctx->conv_err));
+    return conv_err_check(ctx, "k_conv3");
 }
 
 extern "C" nn_status nn_conv3d_wgrad(nn_ctx* ctx, int nz, int ny, int nx, int cin, int cout, const void* d_x,
@@ -1029,15 +1035,7 @@ extern "C" nn_status nn_conv3d_wgrad(nn_ctx* ctx, int nz, int ny, int nx, int ci
 {
     if (!ctx || !d_x || !d_gy || !d_dw) return NN_ERR_INVALID_ARG;
     if (!nn_conv_supported(cin, cout)) return nn_fail(ctx, NN_ERR_UNSUPPORTED, "conv3d wgrad %d -> %d", cin, cout);
-    int* err = nullptr;
-    NN_TRY(nn_alloc(ctx, &err, 1));
-    nn_status st = nn_cuda_check(ctx, cudaMemsetAsync(err, 0, sizeof(int), ctx->stream), "memset");
-    if (st == NN_OK) st = nn_conv_wgrad(ctx, nn_act_geometry(nz, ny, nx), cin, cout, d_x, d_gy, d_dw, d_db, err);
-    int h_err = 0;
-    if (st == NN_OK) st = nn_cuda_check(ctx, cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost,
-                                                             ctx->stream), "memcpy");
-    if (st == NN_OK) st = nn_cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "conv3d wgrad");
-    nn_release(err);
-    if (st == NN_OK && h_err) st = nn_fail(ctx, NN_ERR_TIMEOUT, "k_conv3_wgrad: a pipeline wait timed out");
-    return st;
+    NN_TRY(conv_err_clear(ctx));
+    NN_TRY(nn_conv_wgrad(ctx, nn_act_geometry(nz, ny, nx), cin, cout, d_x, d_gy, d_dw, d_db, ctx->conv_err));
+    return conv_err_check(ctx, "k_conv3_wgrad");
 }

@@ -19,6 +19,7 @@ struct nn_ctx {
     std::string last_error;
     int64_t launches = 0;  // kernels launched on behalf of the caller
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // nn_ctx_time_begin/end
+    int* conv_err = nullptr;  // device error word of the convolution entry points (allocated by the first)
     // Objects created on a context hold a reference, so destroying the context
     // before them (in any order) never leaves them with a dangling pointer.
     int refs = 1;

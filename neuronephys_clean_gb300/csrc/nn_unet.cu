@@ -396,11 +396,13 @@ struct nn_unet {
     nn_act_geom g[3];
     int64_t G0 = 0;
     struct Layer {
-        float *w = nullptr, *b = nullptr, *gw = nullptr, *gb = nullptr;
-        float *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;
+        float *w = nullptr, *b = nullptr, *gw = nullptr, *gb = nullptr;  // parts of params and grads
         void *wp = nullptr, *wpa = nullptr;
         int64_t nw = 0;
     } L[NL];
+    // parameters, gradients and Adam's moments of all layers: w, b of each in turn
+    int64_t np = 0;
+    float *params = nullptr, *grads = nullptr, *mom1 = nullptr, *mom2 = nullptr;
     // activations
     void *I0 = nullptr, *E0a = nullptr, *CAT0 = nullptr, *D0a = nullptr, *D0b = nullptr, *OUT = nullptr;
     void *P1 = nullptr, *E1a = nullptr, *CAT1 = nullptr, *D1a = nullptr, *D1b = nullptr;
@@ -471,18 +473,21 @@ nn_status nn_unet_make(nn_ctx* ctx, int nz, int ny, int nx, uint64_t seed, nn_un
     u->g[2] = nn_act_geometry(nz / 4, ny / 4, nx / 4);
     u->G0 = (int64_t)nz * ny * nx;
     nn_status st = NN_OK;
+    for (int l = 0; l < NL; ++l) {
+        u->L[l].nw = 27LL * LCIN[l] * LCOUT[l];
+        u->np += u->L[l].nw + LCOUT[l];
+    }
+    for (float** p : {&u->params, &u->grads, &u->mom1, &u->mom2})
+        if (st == NN_OK) st = buf_alloc(u, p, (size_t)u->np);
+    int64_t off = 0;
     for (int l = 0; l < NL && st == NN_OK; ++l) {
         auto& L = u->L[l];
-        L.nw = 27LL * LCIN[l] * LCOUT[l];
+        L.w = u->params + off;
+        L.gw = u->grads + off;
+        L.b = L.w + L.nw;
+        L.gb = L.gw + L.nw;
+        off += L.nw + LCOUT[l];
         unsigned char *wp = nullptr, *wpa = nullptr;
-        st = buf_alloc(u, &L.w, L.nw);
-        if (st == NN_OK) st = buf_alloc(u, &L.gw, L.nw);
-        if (st == NN_OK) st = buf_alloc(u, &L.mw, L.nw);
-        if (st == NN_OK) st = buf_alloc(u, &L.vw, L.nw);
-        if (st == NN_OK) st = buf_alloc(u, &L.b, LCOUT[l]);
-        if (st == NN_OK) st = buf_alloc(u, &L.gb, LCOUT[l]);
-        if (st == NN_OK) st = buf_alloc(u, &L.mb, LCOUT[l]);
-        if (st == NN_OK) st = buf_alloc(u, &L.vb, LCOUT[l]);
         if (st == NN_OK) st = buf_alloc(u, &wp, nn_conv_packed_weight_bytes(LCIN[l], LCOUT[l]));
         if (st == NN_OK) st = buf_alloc(u, &wpa, nn_conv_packed_weight_bytes(LCIN[l], LCOUT[l]));
         L.wp = wp;
@@ -661,12 +666,8 @@ static nn_status unet_adam(nn_unet* u, float lr)
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     u->adam_t++;
     const float c1 = 1.0f / (1.0f - powf(b1, (float)u->adam_t)), c2 = 1.0f / (1.0f - powf(b2, (float)u->adam_t));
-    for (int l = 0; l < NL; ++l) {
-        auto& L = u->L[l];
-        NN_TRY(launch(ctx, L.nw, "k_adam", k_adam, L.w, L.gw, L.mw, L.vw, L.nw, lr, b1, b2, eps, c1, c2));
-        NN_TRY(launch(ctx, LCOUT[l], "k_adam", k_adam, L.b, L.gb, L.mb, L.vb, (int64_t)LCOUT[l], lr, b1, b2, eps, c1, c2));
-        NN_TRY(unet_repack(u, l));
-    }
+    NN_TRY(launch(ctx, u->np, "k_adam", k_adam, u->params, u->grads, u->mom1, u->mom2, u->np, lr, b1, b2, eps, c1, c2));
+    for (int l = 0; l < NL; ++l) NN_TRY(unet_repack(u, l));
     return NN_OK;
 }
 
@@ -902,9 +903,7 @@ extern "C" nn_status nn_learned_solve(nn_learned* lp, const float* d_b, float* d
 extern "C" nn_status nn_learned_num_params(nn_learned* lp, int64_t* n)
 {
     if (!lp || !n) return NN_ERR_INVALID_ARG;
-    int64_t s = 0;
-    for (int l = 0; l < NL; ++l) s += lp->net->L[l].nw + LCOUT[l];
-    *n = s;
+    *n = lp->net->np;
     return NN_OK;
 }
 
@@ -912,15 +911,7 @@ extern "C" nn_status nn_learned_get_params(nn_learned* lp, float* h_out)
 {
     if (!lp || !h_out) return NN_ERR_INVALID_ARG;
     nn_ctx* ctx = lp->ctx;
-    NN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    int64_t off = 0;
-    for (int l = 0; l < NL; ++l) {
-        const auto& L = lp->net->L[l];
-        NN_CUDA(ctx, nn_copy_sync(ctx, h_out + off, L.w, sizeof(float) * L.nw, cudaMemcpyDeviceToHost));
-        off += L.nw;
-        NN_CUDA(ctx, nn_copy_sync(ctx, h_out + off, L.b, sizeof(float) * LCOUT[l], cudaMemcpyDeviceToHost));
-        off += LCOUT[l];
-    }
+    NN_CUDA(ctx, nn_copy_sync(ctx, h_out, lp->net->params, sizeof(float) * lp->net->np, cudaMemcpyDeviceToHost));
     return NN_OK;
 }
 
@@ -928,16 +919,8 @@ extern "C" nn_status nn_learned_set_params(nn_learned* lp, const float* h_in)
 {
     if (!lp || !h_in) return NN_ERR_INVALID_ARG;
     nn_ctx* ctx = lp->ctx;
-    NN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    int64_t off = 0;
-    for (int l = 0; l < NL; ++l) {
-        auto& L = lp->net->L[l];
-        NN_CUDA(ctx, nn_copy_sync(ctx, L.w, h_in + off, sizeof(float) * L.nw, cudaMemcpyHostToDevice));
-        off += L.nw;
-        NN_CUDA(ctx, nn_copy_sync(ctx, L.b, h_in + off, sizeof(float) * LCOUT[l], cudaMemcpyHostToDevice));
-        off += LCOUT[l];
-        NN_TRY(unet_repack(lp->net, l));
-    }
+    NN_CUDA(ctx, nn_copy_sync(ctx, lp->net->params, h_in, sizeof(float) * lp->net->np, cudaMemcpyHostToDevice));
+    for (int l = 0; l < NL; ++l) NN_TRY(unet_repack(lp->net, l));
     return nn_cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "nn_learned_set_params");
 }
 
@@ -952,30 +935,21 @@ extern "C" nn_status nn_learned_net_gradient(nn_learned* lp, const float* d_rc, 
     nn_ctx* ctx = lp->ctx;
     nn_unet* u = lp->net;
     NN_CUDA(ctx, cudaMemsetAsync(u->err, 0, sizeof(int), ctx->stream));
-    for (int l = 0; l < NL; ++l) {
-        NN_CUDA(ctx, cudaMemsetAsync(u->L[l].gw, 0, sizeof(float) * u->L[l].nw, ctx->stream));
-        NN_CUDA(ctx, cudaMemsetAsync(u->L[l].gb, 0, sizeof(float) * LCOUT[l], ctx->stream));
-    }
+    NN_CUDA(ctx, cudaMemsetAsync(u->grads, 0, sizeof(float) * u->np, ctx->stream));
     NN_TRY(unet_forward(u, d_rc, lp->logd));
     NN_CUDA(ctx, cudaMemsetAsync(u->scal + 1, 0, sizeof(double), ctx->stream));
     NN_TRY(launch(ctx, u->G0, "k_net_loss", k_net_loss, (const float*)u->y32, d_target, (const double*)u->scal,
                   (uint4*)u->gOUT, u->g[0], u->scal + 1));
     NN_TRY(unet_backward(u));
     NN_TRY(check_err(u));
-    if (d_y) NN_CUDA(ctx, nn_copy_sync(ctx, d_y, u->y32, sizeof(float) * u->G0, cudaMemcpyDeviceToDevice));
+    if (d_y)
+        NN_CUDA(ctx, cudaMemcpyAsync(d_y, u->y32, sizeof(float) * u->G0, cudaMemcpyDeviceToDevice, ctx->stream));
     double l2 = 0.0;
-    NN_CUDA(ctx, nn_copy_sync(ctx, &l2, u->scal + 1, sizeof(double), cudaMemcpyDeviceToHost));
+    NN_CUDA(ctx, cudaMemcpyAsync(&l2, u->scal + 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    if (h_grad)
+        NN_CUDA(ctx, cudaMemcpyAsync(h_grad, u->grads, sizeof(float) * u->np, cudaMemcpyDeviceToHost, ctx->stream));
+    NN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (loss) *loss = 0.5 * l2;
-    if (h_grad) {
-        int64_t off = 0;
-        for (int l = 0; l < NL; ++l) {
-            const auto& L = u->L[l];
-            NN_CUDA(ctx, nn_copy_sync(ctx, h_grad + off, L.gw, sizeof(float) * L.nw, cudaMemcpyDeviceToHost));
-            off += L.nw;
-            NN_CUDA(ctx, nn_copy_sync(ctx, h_grad + off, L.gb, sizeof(float) * LCOUT[l], cudaMemcpyDeviceToHost));
-            off += LCOUT[l];
-        }
-    }
     return NN_OK;
 }
 
