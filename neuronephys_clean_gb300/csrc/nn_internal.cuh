@@ -105,6 +105,9 @@ inline cudaError_t nn_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, 
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 __device__ __forceinline__ void nn_grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the programmatic dependent of this kernel start once every block has
+// called this or left (it still waits, as above, for this kernel's end).
+__device__ __forceinline__ void nn_grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 inline int nn_grid_for(const nn_ctx* ctx, int64_t work, int threads, int per_sm = 8)
 {

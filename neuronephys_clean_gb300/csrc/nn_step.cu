@@ -1,5 +1,6 @@
 // The neuron update: one RK4 step of every neuron with threshold detection,
 // compaction and push delivery (see the kernel comment).
+#include "nn_internal.cuh"
 #include "nn_step.cuh"
 
 namespace {
@@ -26,8 +27,28 @@ namespace {
 template <int NPT, bool UNI, bool EL>
 __global__ void __launch_bounds__(256, NN_HH_MIN_BLOCKS) k_hh_step(StepArgs a)
 {
+    nn_grid_dep_launch();
     const uint64_t t = *a.base + (uint64_t)a.q;
     const int slot = (int)(t % (uint64_t)a.D);
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int chunk = 32 * NPT;
+    // noise: one Philox draw and one Box-Muller per neuron pair
+    float Z[NPT];
+    auto noise = [&](int ch) {
+        const int i0 = ch * chunk + lane * NPT;
+        if (NPT == 1) {
+            Z[0] = nn_normal(a.seed, (uint32_t)i0, t);
+        } else {
+#pragma unroll
+            for (int q = 0; q < NPT; q += 2) nn_normal_pair(a.seed, (uint32_t)(i0 + q) >> 1, t, Z[q], Z[q + 1]);
+        }
+    };
+    // a programmatic dependent of the step before: its launch and the first
+    // chunk's noise, which need nothing that steps write, overlap that step's end
+    noise(warp);
+    nn_grid_dep_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.counts[(t + 1) & 1] = 0;  // next step's count
         if (a.rowflag) a.rowflag[slot] = a.bitmap != nullptr;
@@ -39,10 +60,6 @@ __global__ void __launch_bounds__(256, NN_HH_MIN_BLOCKS) k_hh_step(StepArgs a)
     int* list = a.list + (size_t)(t & 1) * a.n_pad;
     int* cnt = a.counts + (t & 1);
     uint32_t* bm = a.bitmap ? a.bitmap + (size_t)slot * a.words : nullptr;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int chunk = 32 * NPT;
     // electrode sample of this step (nullptr: none)
     float* el_v = EL && s_el >= 0 ? a.el_val + (size_t)s_el * a.el_members : nullptr;
     uint8_t* el_s = EL && s_el >= 0 ? a.el_spk + (size_t)s_el * a.el_members : nullptr;
@@ -79,14 +96,7 @@ __global__ void __launch_bounds__(256, NN_HH_MIN_BLOCKS) k_hh_step(StepArgs a)
 #pragma unroll
             for (int q = 0; q < NPT; ++q) UP[q] = 0.0f;
         }
-        // noise: one Philox draw and one Box-Muller per neuron pair
-        float Z[NPT];
-        if (NPT == 1) {
-            Z[0] = nn_normal(a.seed, (uint32_t)i0, t);
-        } else {
-#pragma unroll
-            for (int q = 0; q < NPT; q += 2) nn_normal_pair(a.seed, (uint32_t)(i0 + q) >> 1, t, Z[q], Z[q + 1]);
-        }
+        if (ch != warp) noise(ch);
         uint32_t mask = 0;
         bool bad = false;
         bool any_in = false;
@@ -227,26 +237,29 @@ __global__ void __launch_bounds__(256, NN_HH_MIN_BLOCKS) k_hh_step(StepArgs a)
 
 }  // namespace
 
-cudaError_t nn_launch_hh_step(const StepArgs& a, int npt, int blocks, int tpb, cudaStream_t cs)
+cudaError_t nn_launch_hh_step(const StepArgs& a, int npt, int blocks, int tpb, cudaStream_t cs, bool pdl)
 {
     // uniform when no per-neuron gNa scale is loaded and the field does not
     // feed back (g_par = 0 or no density input): then ngna = -gNa and
     // ngpu = 0 (or -0) for every neuron, as the general form computes them
     const bool uni = !a.gna_scale && (!a.upar || a.p.g_par == 0.0f);
     const bool el = a.el_every > 0;
+    void (*f)(StepArgs) = nullptr;
     switch (npt * 4 + (uni ? 2 : 0) + (el ? 1 : 0)) {
-        case 4: k_hh_step<1, false, false><<<blocks, tpb, 0, cs>>>(a); break;
-        case 5: k_hh_step<1, false, true><<<blocks, tpb, 0, cs>>>(a); break;
-        case 6: k_hh_step<1, true, false><<<blocks, tpb, 0, cs>>>(a); break;
-        case 7: k_hh_step<1, true, true><<<blocks, tpb, 0, cs>>>(a); break;
-        case 8: k_hh_step<2, false, false><<<blocks, tpb, 0, cs>>>(a); break;
-        case 9: k_hh_step<2, false, true><<<blocks, tpb, 0, cs>>>(a); break;
-        case 10: k_hh_step<2, true, false><<<blocks, tpb, 0, cs>>>(a); break;
-        case 11: k_hh_step<2, true, true><<<blocks, tpb, 0, cs>>>(a); break;
-        case 16: k_hh_step<4, false, false><<<blocks, tpb, 0, cs>>>(a); break;
-        case 17: k_hh_step<4, false, true><<<blocks, tpb, 0, cs>>>(a); break;
-        case 18: k_hh_step<4, true, false><<<blocks, tpb, 0, cs>>>(a); break;
-        default: k_hh_step<4, true, true><<<blocks, tpb, 0, cs>>>(a); break;
+        case 4: f = k_hh_step<1, false, false>; break;
+        case 5: f = k_hh_step<1, false, true>; break;
+        case 6: f = k_hh_step<1, true, false>; break;
+        case 7: f = k_hh_step<1, true, true>; break;
+        case 8: f = k_hh_step<2, false, false>; break;
+        case 9: f = k_hh_step<2, false, true>; break;
+        case 10: f = k_hh_step<2, true, false>; break;
+        case 11: f = k_hh_step<2, true, true>; break;
+        case 16: f = k_hh_step<4, false, false>; break;
+        case 17: f = k_hh_step<4, false, true>; break;
+        case 18: f = k_hh_step<4, true, false>; break;
+        default: f = k_hh_step<4, true, true>; break;
     }
+    if (pdl) return nn_launch_pdl(f, dim3(blocks), dim3(tpb), 0, cs, a);
+    f<<<blocks, tpb, 0, cs>>>(a);
     return cudaPeekAtLastError();
 }

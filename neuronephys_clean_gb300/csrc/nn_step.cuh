@@ -107,4 +107,6 @@ __device__ __forceinline__ void nn_push_row(const StepArgs& a, int64_t beg, int6
 }
 
 // One step of every neuron on stream cs (NPT neurons per thread: 1, 2 or 4).
-cudaError_t nn_launch_hh_step(const StepArgs& a, int npt, int blocks, int tpb, cudaStream_t cs);
+// pdl: as a programmatic dependent of the kernel before it, which has to be a
+// kernel of the step before that leaves *a.base as it is.
+cudaError_t nn_launch_hh_step(const StepArgs& a, int npt, int blocks, int tpb, cudaStream_t cs, bool pdl);
