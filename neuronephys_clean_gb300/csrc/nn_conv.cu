@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
 // lie at equal distances and make 128 rows, read at byte offsets 0, 16, 32 for
 // the three dx.  The ninth pair's three taps are staged one by one and make 48
 // rows of a fourth MMA.  N = CIN, K = voxels; x is loaded once a tile.  One CTA
-// per SM; one warp issues the copies, another the MMAs.
+// per SM; one warp issues the copies, another the MMAs, the other two sum db.
 // Bound by the copies, about 5 TB/s from L2.  48 -> 16 channels on 72 x 80 x 96
 // voxels: 40 us against 213; 16 -> 16 on 64^3: 19 against 41.
 constexpr int W16_PAIRS = 8;
@@ -611,7 +611,7 @@ struct W16Cfg {
 
 template <int CIN>
 __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad16(const uint4* __restrict__ x, const uint4* __restrict__ gy,
-                                                              nn_act_geom g, float* dw, int* err)
+                                                              nn_act_geom g, float* dw, float* db, int* err)
 {
     using C = W16Cfg<CIN>;
     constexpr int S = C::STAGES, COUT = 16;
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad16(const uint4* __res
     if (tid == 0) {
         for (int q = 0; q < S; ++q) {
             nn_mbar_init(&full[q], 1);
-            nn_mbar_init(&done[q], 1);
+            nn_mbar_init(&done[q], 3);  // the MMAs, and the two warps of db
         }
         nn_mbar_init(&acc_bar, 1);
         nn_mbar_fence_init();
@@ -685,6 +685,39 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad16(const uint4* __res
             __syncwarp();
         }
         if (lead) nn_umma_commit(&acc_bar);
+    }
+    if (warp >= 2) {
+        // db of channel block warp - 2 from the unshifted tile, window 4's middle:
+        // four voxels a lane and tile, added in two floats
+        const int cb = warp - 2, lane = tid & 31;
+        float h[8] = {}, l[8] = {};
+        for (int64_t j = 0; j < ntiles; ++j) {
+            const int q = (int)(j % S);
+            if (!nn_mbar_wait(&full[q], (uint32_t)((j / S) & 1), CONV_WAIT_LIMIT)) break;
+            const uint4* t = reinterpret_cast<const uint4*>(sm + q * C::SLOT + W16_LAST + (cb * W16_PAIRS + 4) * WIN_BYTES);
+            float s[8] = {};
+#pragma unroll
+            for (int v = 0; v < TILE / 32; ++v) {
+                float f[8];
+                unpack_bf16x8(t[1 + lane + 32 * v], f);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) s[c] += f[c];
+            }
+            __syncwarp();
+            if (lane == 0) nn_mbar_arrive(&done[q]);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const float a = __fadd_rn(h[c], s[c]), b = __fsub_rn(a, h[c]);
+                l[c] = __fadd_rn(l[c], __fadd_rn(__fsub_rn(h[c], __fsub_rn(a, b)), __fsub_rn(s[c], b)));
+                h[c] = a;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            float a = h[c] + l[c];
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (db && lane == 0) atomicAdd(db + 8 * cb + c, a);
+        }
     }
     // (lanes 1-31 wait for their warp's issuing lane; then one thread waits for
     // the accumulators, as above)
@@ -869,7 +902,8 @@ nn_status launch_wgrad(nn_ctx* ctx, const nn_act_geom& g, const void* x, const v
 }
 
 template <int CIN>
-nn_status launch_wgrad16(nn_ctx* ctx, const nn_act_geom& g, const void* x, const void* gy, float* dw, int* err)
+nn_status launch_wgrad16(nn_ctx* ctx, const nn_act_geom& g, const void* x, const void* gy, float* dw, float* db,
+                         int* err)
 {
     using C = W16Cfg<CIN>;
     static bool attr_set = false;
@@ -878,7 +912,7 @@ nn_status launch_wgrad16(nn_ctx* ctx, const nn_act_geom& g, const void* x, const
         attr_set = true;
     }
     const unsigned grid = (unsigned)std::min<int64_t>(g.tiles, ctx->num_sms);
-    k_conv3_wgrad16<CIN><<<grid, WG_THREADS, C::SMEM, ctx->stream>>>((const uint4*)x, (const uint4*)gy, g, dw, err);
+    k_conv3_wgrad16<CIN><<<grid, WG_THREADS, C::SMEM, ctx->stream>>>((const uint4*)x, (const uint4*)gy, g, dw, db, err);
     NN_CHECK_LAUNCH(ctx, "k_conv3_wgrad16");
     return NN_OK;
 }
@@ -930,14 +964,14 @@ nn_status nn_conv_wgrad(nn_ctx* ctx, const nn_act_geom& g, int cin, int cout, co
     nn_status st = NN_ERR_UNSUPPORTED;
 #define NN_X(ci, co) \
     if (st == NN_ERR_UNSUPPORTED && cin == ci && cout == co) { \
-        if constexpr (co == 16) st = launch_wgrad16<ci>(ctx, g, x, gy, dw, err); \
+        if constexpr (co == 16) st = launch_wgrad16<ci>(ctx, g, x, gy, dw, db, err); \
         else st = launch_wgrad<ci, co>(ctx, g, x, gy, dw, err); \
     }
     NN_CONV_SHAPES(NN_X)
 #undef NN_X
     if (st == NN_ERR_UNSUPPORTED) return nn_fail(ctx, st, "conv3d wgrad %d -> %d is not instantiated", cin, cout);
     if (st != NN_OK) return st;
-    if (db) {
+    if (db && cout != 16) {
         dim3 grid((unsigned)std::min<int64_t>(g.tiles, (int64_t)ctx->num_sms * 4), cout / 8);
         k_bias_grad<<<grid, 256, 0, ctx->stream>>>((const uint4*)gy, g, cout, db);
         NN_CHECK_LAUNCH(ctx, "k_bias_grad");
