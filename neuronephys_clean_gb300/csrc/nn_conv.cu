@@ -11,7 +11,7 @@
 // K-major operand layout (8-row x 16-byte core matrices, rows 16 bytes
 // apart) allows.  Up to nine stages are in flight at once (all nine when
 // they fit in 96 KB, so a small grid pays one copy round trip, not nine); one
-// thread issues CIN/16 MMAs (K = 16) per tap, commits them to an mbarrier,
+// warp issues CIN/16 MMAs (K = 16) per tap, commits them to an mbarrier,
 // and the epilogue (bias, ReLU, optional gradient mask, BF16 store with zeros
 // on pads) reads the accumulator back with tcgen05.ld.
 //
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3(ConvArgs a)
     __shared__ uint64_t full[C::STAGES_BIG], done[C::STAGES_BIG], acc_bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int64_t o0 = a.g.o_first + (int64_t)blockIdx.x * TILE;
 
     if (tid == 0) {
@@ -183,9 +183,13 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3(ConvArgs a)
     // the kernel before this one has finished with the activations
     nn_grid_dep_wait();
 
-    if (tid == 0) {
+    // (a converged warp, its elected lane issues: see nn_umma_bf16_lead)
+    if (warp == 0) {
+        const uint32_t lead = nn_elect();
         int issued = 0;
         auto issue = [&](int st) {
+            ++issued;
+            if (!lead) return;
             const int q = st % S;
             unsigned char* buf = sm + q * C::STAGE_STRIDE;
             const int dz = st / 3 - 1, dy = st % 3 - 1;
@@ -195,9 +199,9 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3(ConvArgs a)
             for (int gi = 0; gi < C::G_IN; ++gi)
                 nn_bulk_g2s(buf + gi * WIN_BYTES, a.x + gi * a.g.S + a.g.GD + start, WIN_BYTES, &full[q]);
             nn_bulk_g2s(buf + C::ACT_BYTES, a.w + (size_t)st * C::W_BYTES, C::W_BYTES, &full[q]);
-            ++issued;
         };
         for (int st = 0; st < S; ++st) issue(st);
+        __syncwarp();
         constexpr uint32_t idesc = nn_umma_idesc_bf16(128, COUT);
         bool ok = true;
         int consumed = 0;
@@ -215,26 +219,27 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3(ConvArgs a)
                 for (int kc = 0; kc < CIN / 16; ++kc) {
                     const uint64_t ad = nn_umma_sdesc(abase + 2 * kc * WIN_BYTES + dx * 16, WIN_BYTES, 128);
                     const uint64_t bd = nn_umma_sdesc(wbase + (dx * (CIN / 16) + kc) * 2 * COUT * 16, COUT * 16, 128);
-                    nn_umma_bf16(tmem, ad, bd, idesc, (st | dx | kc) != 0);
+                    nn_umma_bf16_lead(lead, tmem, ad, bd, idesc, (st | dx | kc) != 0);
                 }
-            nn_umma_commit(&done[b]);
+            if (lead) nn_umma_commit(&done[b]);
+            __syncwarp();
             if (st + S < 9) {
                 ok = nn_mbar_wait(&done[b], (st / S) & 1, CONV_WAIT_LIMIT);
                 if (!ok) break;
                 issue(st + S);
+                __syncwarp();
             }
         }
-        nn_umma_commit(&acc_bar);
+        if (lead) nn_umma_commit(&acc_bar);
+        __syncwarp();
         if (!ok) {
             abort_flag = 1;
             // let copies already in flight land before the CTA leaves
             for (int st = consumed; st < issued; ++st) nn_mbar_wait(&full[st % S], (st / S) & 1, CONV_WAIT_LIMIT);
         }
     }
-    // lanes 1-31 of warp 0 wait here for lane 0's issue loop (spinning on
-    // the mbarrier beside it would stall that loop at every wait); one thread
-    // then waits for the accumulator and the block barrier releases the rest,
-    // whose polls would otherwise take issue slots from the other CTAs
+    // one thread waits for the accumulator and the block barrier releases the
+    // rest, whose polls would otherwise take issue slots from the other CTAs
     __syncwarp();
     if (tid == 0 && !nn_mbar_wait(&acc_bar, 0, CONV_WAIT_LIMIT)) abort_flag = 1;
     __syncthreads();
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3(ConvArgs a)
 // Time in us, before and here: 16 -> 16 and 48 on 64^3 voxels 22.6 and 39, 16 and
 // 22; 16 -> 48 on 72 x 80 x 96 75 and 40.  Wider layers stay with k_conv3: their
 // MMAs read 4 KB of A for few columns, about 30 ns each, which bounds both (48 ->
-// 16 on 72 x 80 x 96: 70 and 75; 32 -> 16 on 64^3 1.1 times slower here).
+// 16 on 72 x 80 x 96: 65 and 75; 32 -> 16 on 64^3 1.1 times slower here).
 template <int CIN, int COUT>
 struct StreamCfg {
     static constexpr int G_IN = CIN / 8;
@@ -467,7 +472,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
     __shared__ uint64_t full[S], done[S], acc_bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int st9 = blockIdx.y, dz = st9 / 3 - 1, dy = st9 % 3 - 1;
     const int64_t ntiles =
         (int64_t)blockIdx.x < g.tiles ? (g.tiles - 1 - (int64_t)blockIdx.x) / gridDim.x + 1 : 0;
@@ -486,10 +491,13 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
     nn_tc_fence_after();
     const uint32_t tmem = tmem_slot;
 
-    if (tid == 0) {
+    if (warp == 0) {
+        const uint32_t lead = nn_elect();
         int64_t issued = 0, consumed = 0;
         // tile j into slot j % S: the gradient blocks, then x at shifts dx = 0, 1, 2
         auto issue = [&](int64_t j) {
+            ++issued;
+            if (!lead) return;
             const int q = (int)(j % S);
             const int64_t o0 = g.o_first + (blockIdx.x + j * gridDim.x) * TILE;
             const int64_t start = o0 + dz * g.P + dy * g.R - 1;
@@ -510,12 +518,12 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
                 for (int cb = 0; cb < CIN / 8; ++cb)
                     nn_bulk_g2s(buf + C::A_BYTES + cb * WIN_BYTES, x + cb * g.S + g.GD + start, WIN_BYTES, &full[q]);
             }
-            ++issued;
         };
         // A and B both MN-major (bits 15, 16 of the instruction descriptor)
         constexpr uint32_t idesc = nn_umma_idesc_bf16(WG_MP, C::NM) | (1u << 15) | (1u << 16);
         bool ok = true;
         for (int64_t j = 0; j < S && j < ntiles; ++j) issue(j);
+        __syncwarp();
         for (int64_t j = 0; j < ntiles; ++j) {
             const int q = (int)(j % S);
             ok = nn_mbar_wait(&full[q], (uint32_t)((j / S) & 1), CONV_WAIT_LIMIT);
@@ -533,16 +541,19 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
                     const uint32_t boff = C::MERGE ? kk * 256 : (kk * 16 + h) * 16;
                     const uint64_t ad = nn_umma_sdesc(abase + kk * 256, 128, WG_BLOCK);
                     const uint64_t bd = nn_umma_sdesc(bbase + boff, 128, C::B_BSTRIDE);
-                    nn_umma_bf16(tmem + h * C::NM, ad, bd, idesc, (j | kk) != 0);
+                    nn_umma_bf16_lead(lead, tmem + h * C::NM, ad, bd, idesc, (j | kk) != 0);
                 }
-            nn_umma_commit(&done[q]);
+            if (lead) nn_umma_commit(&done[q]);
+            __syncwarp();
             if (j + S < ntiles) {
                 ok = nn_mbar_wait(&done[q], (uint32_t)((j / S) & 1), CONV_WAIT_LIMIT);
                 if (!ok) break;
                 issue(j + S);
+                __syncwarp();
             }
         }
-        nn_umma_commit(&acc_bar);
+        if (lead) nn_umma_commit(&acc_bar);
+        __syncwarp();
         if (!ok) {
             abort_flag = 1;
             // let copies already in flight land before the CTA leaves
@@ -550,10 +561,8 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
                 nn_mbar_wait(&full[j % S], (uint32_t)((j / S) & 1), CONV_WAIT_LIMIT);
         }
     }
-    // lanes 1-31 of warp 0 wait here for lane 0's issue loop (spinning on
-    // the mbarrier beside it would stall that loop at every wait); one thread
-    // then waits for the accumulator and the block barrier releases the rest,
-    // whose polls would otherwise take issue slots from the other CTAs
+    // one thread waits for the accumulator and the block barrier releases the
+    // rest, whose polls would otherwise take issue slots from the other CTAs
     __syncwarp();
     if (tid == 0 && !nn_mbar_wait(&acc_bar, 0, CONV_WAIT_LIMIT)) abort_flag = 1;
     __syncthreads();

@@ -86,20 +86,10 @@ __host__ __device__ constexpr uint32_t nn_umma_idesc_bf16(int M, int N)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A * B^T; issued by one thread.
-__device__ __forceinline__ void nn_umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate)
-{
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// The same for a converged warp, issued by the lane with lead != 0: the loop
-// around it then runs on uniform registers, which the descriptors are passed in
-// (a loop of one thread moves each of them there: 50 ns an MMA, here 31).
+// D[tmem] (+)= A * B^T, called by a converged warp and issued by its lane with
+// lead != 0: the loop around it then runs on uniform registers, which the
+// descriptors are passed in (a loop of one thread moves each of them there: 50 ns
+// an MMA, this one 31).
 __device__ __forceinline__ void nn_umma_bf16_lead(uint32_t lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                                   uint32_t idesc, uint32_t accumulate)
 {
