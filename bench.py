@@ -82,8 +82,8 @@ HH_FP32_OPS_PER_NEURON_STEP = 340
 # and log, sqrt, sin, cos per neuron pair for the noise
 HH_TRANSCENDENTALS_PER_NEURON_STEP = 26
 FP32_LANES_PER_SM = 128            # FP32 lanes per SM (sm_100 family), one fused multiply-add (2 ops) per lane and clock
-PCG_BYTES_PER_CELL_ITER = 40       # k_cg_iter R: r,w,s,p,x; W: r,w,s,p,x -> 10 floats per cell
-PCG_HET_BYTES_PER_CELL_ITER = 48   # k_cg_iter<HET>: + D and 1/diag reads
+PCG_BYTES_PER_CELL_ITER = 24       # k_cg_iter R: u,t; W: u,t; R, W: p,x in every second iteration
+PCG_HET_BYTES_PER_CELL_ITER = 28   # k_cg_iter<HET>: + 1/(2 alpha D)
 PUSH_BYTES_PER_EVENT = 13          # 4 B target + 4 B weight + 1 B delay + 4 B ring read-modify-write
 PULL_CSC_BYTES_PER_SYNAPSE = 9     # full CSC sweep: 4 B source + 4 B weight + 1 B delay
 
@@ -91,7 +91,8 @@ PULL_CSC_BYTES_PER_SYNAPSE = 9     # full CSC sweep: 4 B source + 4 B weight + 1
 # (dram__bytes_read.sum + dram__bytes_write.sum per launch / units per launch).
 NCU_TRAFFIC_PER_UNIT = {
     "hh_step": 36.03,        # 36.03 MB read + 0 MB written per 1M-neuron launch (writes stay in L2)
-    "pcg_iteration": 20.2,   # 41.99 MB read + 0.45 MB written per 128^3 launch (the rest hits L2)
+    "pcg_iteration": None,   # one launch a solve on grids that fit on the chip
+    "pcg_het_iteration": 25.8,  # 279 MB read + 153 MB written per 256^3 launch
 }
 
 
@@ -318,7 +319,8 @@ def run_ours(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
                "algorithmic_bytes": n * HH_BYTES_PER_NEURON_STEP, "launch_ms": hh_ms,
                "launch_ms_of": "median launch of the last period of one bench step after the timed region, solves in line",
                "peak_source": peak_kind}
-    pcg_roof = {"bound": "hbm", "kernel": "k_cg_iter (one PCG iteration)", "achieved": pcg_ach,
+    pcg_roof = {"bound": "hbm", "kernel": "one PCG iteration (k_rcg, its vectors on the chip; larger grids k_cg_iter)",
+                "achieved": pcg_ach,
                 "peak": hbm_peak, "unit": "GB/s", "frac": pcg_ach / hbm_peak if pcg_ach else None,
                 "traffic": (NCU_TRAFFIC_PER_UNIT["pcg_iteration"] * G) if NCU_TRAFFIC_PER_UNIT["pcg_iteration"] else None,
                 "algorithmic_bytes": G * PCG_BYTES_PER_CELL_ITER, "launch_ms": it_ms, "peak_source": peak_kind}
@@ -370,7 +372,7 @@ def run_ours(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
         "data": "synthetic (seeded counter-based generators)",
         "config": workload_config(wl, nnz, args.delivery),
         "delivery": delivery_info,
-        "autotuned": {"cg_tile": f"32 x 16 x {cg_tile[0]}", "trial_ms_per_timestep": cg_tile[1],
+        "autotuned": {"cg_tile_depth": cg_tile[0], "trial_ms_per_timestep": cg_tile[1],
                       "how": "each tile depth timed over six periods with the solve overlapping the neuron "
                              "updates, from a snapshot restored afterwards"},
         "electrodes": el_info,
@@ -896,11 +898,12 @@ def run_cg(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
         "warmup": args.warmup, "ms_per_step": ms_solve, "higher_is_better": False, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32 (FP64 reductions)", "data": "synthetic (seeded lognormal D, Poisson sources)",
         "config": {"workload": wl["workload"], "grid": wl["grid"], "alpha": alpha, "beta": beta,
-                   "preconditioner": "jacobi", "l2": "inputs larger than L2 (9 x 67 MB vectors)"},
+                   "preconditioner": "jacobi", "l2": "inputs larger than L2 (8 x 67 MB vectors)"},
         "cg": {"iterations": it_mean, "relres": rel, "ms_per_iteration": it_ms,
                "solution_norm": float(np.linalg.norm(x.astype(np.float64)))},
         "roofline": {"bound": "hbm", "kernel": "k_cg_iter<HET> (one PCG iteration)", "achieved": ach,
-                     "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak, "traffic": None,
+                     "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
+                     "traffic": G * NCU_TRAFFIC_PER_UNIT["pcg_het_iteration"],
                      "algorithmic_bytes": G * PCG_HET_BYTES_PER_CELL_ITER, "launch_ms": it_ms,
                      "peak_source": peak_kind},
         "gpu_launches": int(launches),
