@@ -357,6 +357,8 @@ extern "C" nn_status nn_pcg_create(nn_ctx* ctx, int nx, int ny, int nz, double a
         if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
         if (st == NN_OK) {
             fs = nn_cg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, pc->res != nullptr, &pc->fast);
+            // rows that have to be padded take three vectors more than two kernels
+            if (fs == NN_ERR_OOM && (nx % 4 || ((uintptr_t)d_Dcell & 15))) fs = NN_ERR_UNSUPPORTED;
             if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
         }
         ctx->last_error.clear();
