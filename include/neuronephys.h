@@ -302,8 +302,8 @@ NN_API nn_status nn_sim_set_instances(nn_sim* s, int n_inst, const int* h_offset
  * state, keeps the fastest and restores the state the trials touched. */
 NN_API nn_status nn_sim_autotune(nn_sim* s, int trial_steps, int* best_tpb, int* best_npt, float* best_ms);
 /* Autotuner of the field solver's block shape: for a single grid the z-depth
- * of the 32 x 16 tiles of the one-kernel PCG iteration (4 .. 32;
- * NN_ERR_UNSUPPORTED when the grid runs the two-kernel PCG), for a batch the
+ * of the tiles of the one-kernel PCG iteration (4 .. 32; NN_ERR_UNSUPPORTED
+ * on grids whose rows or field are not whole aligned quads), for a batch the
  * batched PCG's cells per block.  When the solve overlaps the neuron updates
  * (par_overlap, no field feedback) each shape is timed over six whole periods
  * from a snapshot of the simulation, which is restored afterwards;

@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_cg_pad(int nx, int nq, int rows,
 
 // v = 1 / (2 alpha D) with a ghost row and plane on every side and behind the
 // row, where it is that of the nearest cell.  Two neighbours with D = 0 have the
-// face coefficient 0 / 0: their v is NaN.
+// face coefficient 0 / 0, an infinite D inf / inf: their v is NaN.
 __global__ void __launch_bounds__(CG_THREADS) k_cg_field(int nx, int ny, int nz, int nq, const float* D, float half_ia,
                                                          float* v)
 {
@@ -553,6 +553,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_cg_field(int nx, int ny, int nz,
             ((x > 0 && D[c - 1] == 0.0f) || (x < nx - 1 && D[c + 1] == 0.0f) || (j > 0 && D[c - nx] == 0.0f) ||
              (j < ny - 1 && D[c + nx] == 0.0f) || (k > 0 && D[c - sz] == 0.0f) || (k < nz - 1 && D[c + sz] == 0.0f)))
             o = nanf("");
+        if (isinf(d)) o = nanf("");
         v[i] = o;
     }
 }

@@ -730,7 +730,7 @@ __device__ __forceinline__ Col col_of(const Cols& g, int nx, int ny, int nz)
 }
 
 // v of the cell field.  Two neighbours with D = 0 have the face coefficient
-// 0 / 0: their v is NaN.
+// 0 / 0, an infinite D inf / inf: their v is NaN.
 __global__ void __launch_bounds__(MG_THREADS) k_mg_field(int nx, int ny, int nz, const float* D, float half_ia, float* v)
 {
     MG_ROWS(ny, nz, row)
@@ -745,6 +745,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_field(int nx, int ny, int nz,
                  (j < ny - 1 && D[c + nx] == 0.0f) || (k > 0 && D[c - nx * ny] == 0.0f) ||
                  (k < nz - 1 && D[c + nx * ny] == 0.0f)))
                 o = nanf("");
+            if (isinf(d)) o = nanf("");
             v[c] = o;
         }
     }

@@ -208,6 +208,7 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
                     if (HET) {
                         const float d = a.D[c];
                         at(v, e) = __fdiv_rn(a.half_ia, d);
+                        poison |= isinf(d);  // 2 D1 D2 / (D1 + D2) = inf / inf
                         if (d == 0.0f)
                             poison |= (i0 + e > 0 && a.D[c - 1] == 0.0f) || (i0 + e < a.nx - 1 && a.D[c + 1] == 0.0f) ||
                                       (y0 + j > 0 && a.D[c - a.nx] == 0.0f) ||

@@ -91,3 +91,21 @@ def test_streamed_solve_overlaps_as_in_line(ctx, grid):
         got.append((s.get_density(), s.get_field("V")))
     assert np.linalg.norm(got[0][0]) > 0
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("n", [12, 112])
+@pytest.mark.parametrize("solver", ["cg", "two kernels", "multigrid"])
+def test_infinite_diffusivity_does_not_converge(ctx, monkeypatch, n, solver):
+    """A cell with infinite diffusion has the face coefficients inf / inf: no
+    solver converges, on the chip, streamed or with multigrid."""
+    D = np.ones((n, n, n), np.float32)
+    D[5, 6, 7] = np.inf
+    b = ctx.to_device(np.random.default_rng(0).random(n ** 3).astype(np.float32))
+    dD = ctx.to_device(D.ravel())
+    if solver == "two kernels":
+        monkeypatch.setenv("NN_PCG_TWO_KERNEL", "1")
+    pc = nn.PCG(ctx, n, n, n, 4.0, 0.1, dD)
+    s = nn.MultigridPCG(pc) if solver == "multigrid" else pc
+    with pytest.raises(nn.NNError) as e:
+        s.solve(b, ctx.to_device(np.zeros(n ** 3, np.float32)), rtol=1e-6, max_iter=200)
+    assert e.value.status in (nn.NN_ERR_NOT_CONVERGED, 5)  # 5: non-finite state
