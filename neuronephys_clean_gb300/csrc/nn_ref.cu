@@ -259,10 +259,19 @@ __global__ void __launch_bounds__(LF_THREADS) k_leapfrog(LFVars s, int n, float 
 {
     const int lane = threadIdx.x & 31;
     const Pair tab = lf_exp_table[lane];
+    const int first = blockIdx.x * blockDim.x + threadIdx.x - lane;
+    // The step's kernels (this one, the coupling's two and the paracrine's) are
+    // programmatic dependents of whatever is before them on the stream, which
+    // hides their launches; the first noise needs no memory.  Ten steps of 14,638
+    // neurons with a field solve: 289 -> 231 us; of a million 937 -> 861.
+    nn_grid_dep_launch();
+    const float z0 = EXT_Z ? 0.0f : nn_normal(seed, (uint32_t)min(first + lane, n - 1), step);
+    nn_grid_dep_wait();
     // whole warps: lanes past the last neuron repeat it
-    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += gridDim.x * blockDim.x) {
+    for (int i0 = first; i0 < n; i0 += gridDim.x * blockDim.x) {
         const int i = min(i0 + lane, n - 1);
-        lf_neuron(s, i, timestep, p, EXT_Z ? z[i] : nn_normal(seed, (uint32_t)i, step), tab, i0 + lane < n);
+        lf_neuron(s, i, timestep, p, EXT_Z ? z[i] : i0 == first ? z0 : nn_normal(seed, (uint32_t)i, step), tab,
+                  i0 + lane < n);
     }
 }
 
@@ -277,8 +286,8 @@ nn_status leapfrog_launch(nn_ctx* ctx, float* const* vars, int n, float dt, cons
         s.v[q] = vars[q];
     }
     const int grid = nn_grid_for(ctx, n, LF_THREADS, 64);
-    if (d_z) k_leapfrog<true><<<grid, LF_THREADS, 0, ctx->stream>>>(s, n, dt, *p, seed, step, d_z);
-    else k_leapfrog<false><<<grid, LF_THREADS, 0, ctx->stream>>>(s, n, dt, *p, seed, step, nullptr);
+    NN_CUDA(ctx, nn_launch_pdl(d_z ? k_leapfrog<true> : k_leapfrog<false>, dim3(grid), dim3(LF_THREADS), 0, ctx->stream, s,
+                               n, dt, *p, seed, step, d_z));
     NN_CHECK_LAUNCH(ctx, "k_leapfrog");
     return NN_OK;
 }
@@ -409,6 +418,8 @@ __global__ void __launch_bounds__(CMP_THREADS) k_cmp_count_zero(const float* out
                                                                 int* sub_before, float* inputs)
 {
     __shared__ int cnt[CMP_TILE / 32];  // firing neurons of 32 consecutive neurons
+    nn_grid_dep_launch();
+    nn_grid_dep_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < CMP_ITEMS; ++q) {
@@ -450,6 +461,8 @@ __global__ void __launch_bounds__(CMP_THREADS) k_cmp_write_push(const float* out
     __shared__ int64_t red[CMP_THREADS / 32];
     __shared__ int s_list[CMP_SUB];
     __shared__ int wt[CMP_SUB / 32];
+    nn_grid_dep_launch();
+    nn_grid_dep_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * CMP_SUB + threadIdx.x;
     const bool f = threadIdx.x < CMP_SUB && i < n && fires(out[i]);
@@ -580,12 +593,13 @@ extern "C" nn_status nn_coupling_run(nn_coupling* c, const int* d_indices, const
     nn_ctx* ctx = c->ctx;
     // two launches: threshold counts with the inputs zeroed, then the ordered
     // list, the count and the scatter
-    k_cmp_count_zero<<<c->nblocks, CMP_THREADS, 0, ctx->stream>>>(d_outputs, c->n, c->block_counts, c->sub_before,
-                                                                  d_inputs);
+    NN_CUDA(ctx, nn_launch_pdl(k_cmp_count_zero, dim3(c->nblocks), dim3(CMP_THREADS), 0, ctx->stream, d_outputs, c->n,
+                               c->block_counts, c->sub_before, d_inputs));
     NN_CHECK_LAUNCH(ctx, "k_cmp_count_zero");
     const int subs = (c->n - 1) / CMP_SUB + 1;
-    k_cmp_write_push<<<subs, CMP_THREADS, 0, ctx->stream>>>(d_outputs, c->n, c->block_counts, c->sub_before, c->firing,
-                                                            c->count, d_indices, d_offsets, d_inputs, signal_mode);
+    NN_CUDA(ctx, nn_launch_pdl(k_cmp_write_push, dim3(subs), dim3(CMP_THREADS), 0, ctx->stream, d_outputs, c->n,
+                               c->block_counts, c->sub_before, c->firing, c->count, d_indices, d_offsets, d_inputs,
+                               signal_mode));
     NN_CHECK_LAUNCH(ctx, "k_cmp_write_push");
     return coupling_readback(c, num_firing);
 }
@@ -854,6 +868,8 @@ __global__ void k_interp(int n, const int* idx8, const float* w8, const float* g
 // update_on_fine_timescale (src/paracrine.cuh:246-253)
 __global__ void k_fine(int n, const int* list, const int* count, float* gen, float coup, int quirk)
 {
+    nn_grid_dep_launch();
+    nn_grid_dep_wait();
     if (quirk) {
         // transform_if with the compacted index buffer as the stencil
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -1096,8 +1112,8 @@ extern "C" nn_status nn_paracrine_ref_fine(nn_paracrine* pm, const nn_coupling* 
     if (!pm || !c || c->n != pm->n) return nn_fail(pm ? pm->ctx : nullptr, NN_ERR_INVALID_ARG, "nn_paracrine_ref_fine: bad argument");
     if (pm->n == 0) return NN_OK;
     nn_ctx* ctx = pm->ctx;
-    k_fine<<<nn_grid_for(ctx, pm->n, 256, 16), 256, 0, ctx->stream>>>(pm->n, c->firing, c->count, pm->generated,
-                                                                       pm->p.coup_strength, pm->p.quirk_firing_list);
+    NN_CUDA(ctx, nn_launch_pdl(k_fine, dim3(nn_grid_for(ctx, pm->n, 256, 16)), dim3(256), 0, ctx->stream, pm->n, c->firing,
+                               c->count, pm->generated, pm->p.coup_strength, pm->p.quirk_firing_list));
     NN_CHECK_LAUNCH(ctx, "k_fine");
     return NN_OK;
 }
