@@ -362,6 +362,15 @@ struct Red {
     int* flags;
 };
 
+// The kernels of an iteration, but for the first, are programmatic dependents of
+// each other: the launches of the small levels' 2-5 us kernels overlap (256^3 3 %
+// less time, 128 x 112 x 176 10 %).  Called before anything else.
+__device__ __forceinline__ void mg_chain()
+{
+    nn_grid_dep_launch();
+    nn_grid_dep_wait();
+}
+
 __device__ __forceinline__ bool is_tid0() { return threadIdx.x == 0 && threadIdx.y == 0; }
 
 // ---------------------------------------------------------------- V-cycle --
@@ -371,6 +380,7 @@ template <class Op>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_smooth0(Op op, const float* b, float omega, float* y,
                                                            const int* flags)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     MG_ROWS(op.ny, op.nz, row)
     {
@@ -391,6 +401,7 @@ template <int V, class Op>
 __global__ void __launch_bounds__(MG_THREADS, NN_MG_MIN_BLOCKS) k_mg_pre2(Op op, const float* b, float omega, float* y,
                                                         const int* flags)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     const int gx = op.nx / V;
     MG_ROWS(op.ny, op.nz, row)
@@ -416,6 +427,7 @@ template <int V, bool DOTS, class Op>
 __global__ void __launch_bounds__(MG_THREADS, NN_MG_MIN_BLOCKS) k_mg_jacobi(Op op, const float* b, const float* x, float omega,
                                                           float* y, const int* flags, const float* q, Red red)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     const int gx = op.nx / V;
     float acc[2] = {0.0f, 0.0f};
@@ -458,6 +470,7 @@ template <int VC, class Op>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(Op op, const float* b, const float* x, float* bc,
                                                             const int* flags)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     constexpr int V = 2 * VC;
     const int cx = op.nx / 2, cy = op.ny / 2, cz = op.nz / 2;
@@ -491,6 +504,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(Op op, const float* 
 __global__ void __launch_bounds__(MG_THREADS) k_mg_prolong_add(int nx, int ny, int nz, const float* xc, float* x,
                                                                const int* flags)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
     MG_ROWS(ny, nz, row)
@@ -639,6 +653,7 @@ template <int V>
 __global__ void __launch_bounds__(MG_THREADS, NN_MG_MIN_BLOCKS) k_fcg_ap_dir(Op0 op, const float* z, const float* p_old, float* p_new,
                                                            float* q, Red red)
 {
+    nn_grid_dep_launch();
     if (red.flags[F_DONE]) return;
     const float beta = (float)red.scal[S_BETA];
     const int gx = op.nx / V;
@@ -939,6 +954,7 @@ __device__ __forceinline__ float dot(const Quad& x, const Quad& y, float acc)
 template <class Op, class F>
 __global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_pre2(Op op, Cols g, F f, float* y, const int* flags)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     const Col t = col_of(g, op.nx, op.ny, op.nz);
     walk(op, t, f, [&](int c) { return quad_ld(f.b + c); },
@@ -953,6 +969,7 @@ __global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_jacobi(Op op, Co
                                                                       float omega, float* y, const int* flags,
                                                                       const float* q, Red red)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     const Col t = col_of(g, op.nx, op.ny, op.nz);
     float acc[2] = {0.0f, 0.0f};
@@ -984,6 +1001,7 @@ template <class Op>
 __global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_restrict(Op op, Cols g, const float* b, const float* x,
                                                                         float* bc, const int* flags)
 {
+    mg_chain();
     __shared__ float2 part[MG_THREADS];
     if (flags && flags[F_DONE]) return;
     const Col t = col_of(g, op.nx, op.ny, op.nz);
@@ -1031,6 +1049,7 @@ template <class Op>
 __global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_ap_dir(Op op, Cols g, const float* z, const float* p_old,
                                                                       float* p_new, float* q, Red red)
 {
+    nn_grid_dep_launch();
     if (red.flags[F_DONE]) return;
     const Col t = col_of(g, op.nx, op.ny, op.nz);
     float acc[1] = {0.0f};
@@ -1050,6 +1069,7 @@ __global__ void __launch_bounds__(MG_THREADS, COL_BLOCKS) k_col_ap_dir(Op op, Co
 __global__ void __launch_bounds__(MG_THREADS) k_col_prolong(int nx, int ny, int nz, const float* xc, float* x,
                                                             const int* flags)
 {
+    mg_chain();
     if (flags && flags[F_DONE]) return;
     const int Q = nx / 4, cx = nx / 2, cy = ny / 2, cz = nz / 2;
     const int n = Q * cy * cz;
@@ -1090,6 +1110,7 @@ template <int V>
 __global__ void __launch_bounds__(MG_THREADS) k_fcg_update(float* x, float* r, const float* p, const float* q, int G,
                                                            Red red)
 {
+    mg_chain();
     if (red.flags[F_DONE]) return;
     const double pq = red.scal[S_PQ];
     const float a = pq > 0.0 ? (float)(red.scal[S_RZ] / pq) : 0.0f;
@@ -1284,11 +1305,18 @@ Shape shape_for(const nn_ctx* ctx, int gx, int rows)
 
 Red red_of(const nn_mg* mg) { return Red{mg->partials, mg->ticket, mg->scal, mg->flags}; }
 
+// A kernel that begins with mg_chain (errors are read behind the launch).
+template <class... KA, class... A>
+void chain(const nn_mg* mg, void (*kern)(KA...), dim3 grid, dim3 block, A... args)
+{
+    nn_launch_pdl(kern, grid, block, 0, mg->ctx->stream, args...);
+}
+
 template <class Op>
 nn_status launch_smooth0(nn_mg* mg, const Op& op, const float* b, float* y, const int* flags)
 {
     const Shape s = shape_for(mg->ctx, op.nx, op.ny * op.nz);
-    k_mg_smooth0<Op><<<s.grid, s.block, 0, mg->ctx->stream>>>(op, b, mg->omega, y, flags);
+    chain(mg, k_mg_smooth0<Op>, s.grid, s.block, op, b, mg->omega, y, flags);
     NN_CHECK_LAUNCH(mg->ctx, "k_mg_smooth0");
     return NN_OK;
 }
@@ -1308,18 +1336,20 @@ nn_status launch_pre2(nn_mg* mg, int l, const Op& op, const float* b, float* y, 
 {
     if constexpr (V == 4) {
         const Cols& g = mg->lv[l].cols;
-        cudaStream_t cs = mg->ctx->stream;
         with_cols(mg, l, [&](auto o) {
+            using O = decltype(o);
             if (l > 0)
-                k_col_pre2<<<g.blocks(), MG_THREADS, 0, cs>>>(o, g, CDiv{b, mg->lv[l].diag, mg->omega}, y, flags);
+                chain(mg, k_col_pre2<O, CDiv>, dim3(g.blocks()), dim3(MG_THREADS), o, g,
+                      CDiv{b, mg->lv[l].diag, mg->omega}, y, flags);
             else
-                k_col_pre2<<<g.blocks(), MG_THREADS, 0, cs>>>(o, g, CInvd{b, mg->op0.invd, mg->op0.invd_c, mg->omega}, y, flags);
+                chain(mg, k_col_pre2<O, CInvd>, dim3(g.blocks()), dim3(MG_THREADS), o, g,
+                      CInvd{b, mg->op0.invd, mg->op0.invd_c, mg->omega}, y, flags);
         });
         NN_CHECK_LAUNCH(mg->ctx, "k_col_pre2");
         return NN_OK;
     } else {
     const Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
-    k_mg_pre2<V, Op><<<s.grid, s.block, 0, mg->ctx->stream>>>(op, b, mg->omega, y, flags);
+    chain(mg, k_mg_pre2<V, Op>, s.grid, s.block, op, b, mg->omega, y, flags);
     NN_CHECK_LAUNCH(mg->ctx, "k_mg_pre2");
     return NN_OK;
     }
@@ -1332,15 +1362,15 @@ nn_status launch_jacobi(nn_mg* mg, int l, const Op& op, const float* b, const fl
     if constexpr (V == 4) {
         const Cols& g = mg->lv[l].cols;
         with_cols(mg, l, [&](auto o) {
-            k_col_jacobi<decltype(o), DOTS><<<g.blocks(), MG_THREADS, 0, mg->ctx->stream>>>(o, g, b, x, mg->omega, y, flags,
-                                                                                           q, red_of(mg));
+            chain(mg, k_col_jacobi<decltype(o), DOTS>, dim3(g.blocks()), dim3(MG_THREADS), o, g, b, x, mg->omega, y, flags,
+                  q, red_of(mg));
         });
         NN_CHECK_LAUNCH(mg->ctx, "k_col_jacobi");
         return NN_OK;
     } else {
     Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
     if (DOTS) s.grid = dim3(mg->nblocks);  // the partials buffer holds nblocks entries
-    k_mg_jacobi<V, DOTS, Op><<<s.grid, s.block, 0, mg->ctx->stream>>>(op, b, x, mg->omega, y, flags, q, red_of(mg));
+    chain(mg, k_mg_jacobi<V, DOTS, Op>, s.grid, s.block, op, b, x, mg->omega, y, flags, q, red_of(mg));
     NN_CHECK_LAUNCH(mg->ctx, "k_mg_jacobi");
     return NN_OK;
     }
@@ -1353,14 +1383,14 @@ nn_status launch_restrict(nn_mg* mg, int l, const Op& op, const float* b, const 
     // (pairs of rows longer than half a block lie in different blocks)
     if (V == 4 && g.rows >= 2) {
         with_cols(mg, l, [&](auto o) {
-            k_col_restrict<<<g.blocks(), MG_THREADS, 0, mg->ctx->stream>>>(o, g, b, x, bc, flags);
+            chain(mg, k_col_restrict<decltype(o)>, dim3(g.blocks()), dim3(MG_THREADS), o, g, b, x, bc, flags);
         });
         NN_CHECK_LAUNCH(mg->ctx, "k_col_restrict");
         return NN_OK;
     }
     constexpr int VC = V == 4 ? 2 : 1;
     const Shape s = shape_for(mg->ctx, op.nx / 2 / VC, (op.ny / 2) * (op.nz / 2));
-    k_mg_restrict<VC, Op><<<s.grid, s.block, 0, mg->ctx->stream>>>(op, b, x, bc, flags);
+    chain(mg, k_mg_restrict<VC, Op>, s.grid, s.block, op, b, x, bc, flags);
     NN_CHECK_LAUNCH(mg->ctx, "k_mg_restrict");
     return NN_OK;
 }
@@ -1423,11 +1453,11 @@ nn_status vlevel(nn_mg* mg, int l, const Op& op, const float* b, float* out, con
     NN_TRY(vcycle(mg, l + 1, C.b, C.x, flags, nullptr));
     if (V == 4) {
         const int n = L.nx / 4 * (L.ny / 2) * (L.nz / 2);
-        k_col_prolong<<<(n + MG_THREADS - 1) / MG_THREADS, MG_THREADS, 0, mg->ctx->stream>>>(L.nx, L.ny, L.nz, C.x, cur, flags);
+        chain(mg, k_col_prolong, dim3((n + MG_THREADS - 1) / MG_THREADS), dim3(MG_THREADS), L.nx, L.ny, L.nz, C.x, cur, flags);
         NN_CHECK_LAUNCH(mg->ctx, "k_col_prolong");
     } else {
         const Shape s = shape_for(mg->ctx, L.nx, L.ny * L.nz);
-        k_mg_prolong_add<<<s.grid, s.block, 0, mg->ctx->stream>>>(L.nx, L.ny, L.nz, C.x, cur, flags);
+        chain(mg, k_mg_prolong_add, s.grid, s.block, L.nx, L.ny, L.nz, C.x, cur, flags);
         NN_CHECK_LAUNCH(mg->ctx, "k_mg_prolong_add");
     }
     // post-smoothing: nu sweeps, the last one into out (never in place)
@@ -1474,7 +1504,7 @@ nn_status enqueue_iteration_v(nn_mg* mg, float* x, int parity)
         k_fcg_ap_dir<V><<<mg->nblocks, blk, 0, cs>>>(mg->op0, mg->z, p_old, p_new, mg->q, red);
     }
     NN_CHECK_LAUNCH(ctx, "k_fcg_ap_dir");
-    k_fcg_update<V><<<mg->nblocks, dim3(MG_THREADS), 0, cs>>>(x, mg->r, p_new, mg->q, L.G, red);
+    chain(mg, k_fcg_update<V>, dim3(mg->nblocks), dim3(MG_THREADS), x, mg->r, p_new, mg->q, L.G, red);
     NN_CHECK_LAUNCH(ctx, "k_fcg_update");
     return vcycle(mg, 0, mg->r, mg->z, mg->flags, mg->q);
 }
