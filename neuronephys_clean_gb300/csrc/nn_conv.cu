@@ -490,6 +490,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const uint4* __restr
     __syncthreads();
     nn_tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    nn_grid_dep_wait();  // the kernel before this one has finished with the activations
 
     if (warp == 0) {
         const uint32_t lead = nn_elect();
@@ -645,6 +646,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad16(const uint4* __res
     __syncthreads();
     nn_tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    nn_grid_dep_wait();  // the kernel before this one has finished with the activations
 
     if (tid == 32) {
         for (int64_t j = 0; j < ntiles; ++j) {
@@ -774,6 +776,7 @@ __global__ void k_bias_grad(const uint4* __restrict__ gy, nn_act_geom g, int cou
 {
     __shared__ float part[64][8];
     const int gb = blockIdx.y;
+    nn_grid_dep_wait();
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int64_t o = g.o_first + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o <= g.o_last;
          o += (int64_t)gridDim.x * blockDim.x) {
@@ -904,8 +907,8 @@ nn_status launch_wgrad(nn_ctx* ctx, const nn_act_geom& g, const void* x, const v
     // one wave of persistent CTAs over the 9 (dz, dy) pairs
     const int64_t per_y = std::max<int64_t>(1, std::min<int64_t>(g.tiles, ((int64_t)ctx->num_sms * per_sm) / 9));
     dim3 grid((unsigned)per_y, 9);
-    k_conv3_wgrad<CIN, COUT>
-        <<<grid, WG_THREADS, C::SMEM, ctx->stream>>>((const uint4*)x, (const uint4*)gy, g, dw, err);
+    NN_CUDA(ctx, nn_launch_pdl(k_conv3_wgrad<CIN, COUT>, grid, dim3(WG_THREADS), (size_t)C::SMEM, ctx->stream,
+                               (const uint4*)x, (const uint4*)gy, g, dw, err));
     NN_CHECK_LAUNCH(ctx, "k_conv3_wgrad");
     return NN_OK;
 }
@@ -921,7 +924,8 @@ nn_status launch_wgrad16(nn_ctx* ctx, const nn_act_geom& g, const void* x, const
         attr_set = true;
     }
     const unsigned grid = (unsigned)std::min<int64_t>(g.tiles, ctx->num_sms);
-    k_conv3_wgrad16<CIN><<<grid, WG_THREADS, C::SMEM, ctx->stream>>>((const uint4*)x, (const uint4*)gy, g, dw, db, err);
+    NN_CUDA(ctx, nn_launch_pdl(k_conv3_wgrad16<CIN>, dim3(grid), dim3(WG_THREADS), (size_t)C::SMEM, ctx->stream,
+                               (const uint4*)x, (const uint4*)gy, g, dw, db, err));
     NN_CHECK_LAUNCH(ctx, "k_conv3_wgrad16");
     return NN_OK;
 }
@@ -982,7 +986,7 @@ nn_status nn_conv_wgrad(nn_ctx* ctx, const nn_act_geom& g, int cin, int cout, co
     if (st != NN_OK) return st;
     if (db && cout != 16) {
         dim3 grid((unsigned)std::min<int64_t>(g.tiles, (int64_t)ctx->num_sms * 4), cout / 8);
-        k_bias_grad<<<grid, 256, 0, ctx->stream>>>((const uint4*)gy, g, cout, db);
+        NN_CUDA(ctx, nn_launch_pdl(k_bias_grad, grid, dim3(256), 0, ctx->stream, (const uint4*)gy, g, cout, db));
         NN_CHECK_LAUNCH(ctx, "k_bias_grad");
     }
     return NN_OK;
