@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <string>
@@ -253,6 +254,17 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
 void nn_rcg_batch_destroy(nn_rcg_batch* pl);
 nn_status nn_rcg_batch_begin(nn_rcg_batch* pl, const float* d_b, float* d_x, double rtol, int max_iter, cudaStream_t cs);
 nn_status nn_rcg_batch_finish(nn_rcg_batch* pl, cudaStream_t cs, int* iters, int* flags);
+
+// The power of two c by which the CG kernels scale u = c M r (M = 1/diag).  With
+// constant coefficients they sum u u for (r, u) and (r, r), smaller than these by
+// the diagonal and its square; with c near the diagonal's root u u has the
+// magnitude of r u, so small right-hand sides do not underflow earlier, nor
+// large ones overflow.  1 with a cell field, where the sums are of r u and r r.
+inline float nn_jacobi_scale(double alpha, double beta, bool field)
+{
+    const double diag = 1.0 + beta + 6.0 * alpha;
+    return field || !(diag > 0.0) || diag > 1e30 ? 1.0f : (float)std::exp2(std::round(0.5 * std::log2(diag)));
+}
 
 struct nn_cg_plan;
 nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, double beta, const float* D, bool lazy,

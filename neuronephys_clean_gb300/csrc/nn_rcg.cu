@@ -9,14 +9,21 @@
 // so that the preconditioner is needed only inside the stencil pass, where
 // the diagonal is the sum of the face coefficients at hand.
 //
-// What bounds it.  A launch per iteration (nn_cg.cu) moves ten vectors through
-// L2 and pays a grid's start, tail and reduction: 22 us an iteration at 128^3,
-// 5 us at 32^3, and 54 us at 97 x 83 x 150 in the two-kernel form of nn_pcg.cu
-// (rows that no TMA box can hold).  Here nothing but the bricks' faces and the
-// three sums leaves the SM: an iteration costs one exchange between the blocks
-// (3 us) and the arithmetic on the block's own cells.  Measured per iteration:
-// 2.8 us at 32^3, 3.4 at 48^3, 3.9 at 64^3, 9 at 128^3 (solve to 1e-6: 2.13 ms
-// -> 0.87), 9.3 at 97 x 83 x 150 with a cell field (9.8 ms -> 1.8).
+// What bounds it.  A launch per iteration that moved ten vectors through L2 and
+// paid a grid's start, tail and reduction took 22 us an iteration at 128^3 and
+// 5 us at 32^3; two launches an iteration (nn_pcg.cu) 54 us at 97 x 83 x 150.
+// Here nothing but the bricks' faces and the three sums leaves the SM: an
+// iteration costs one exchange between the blocks (3 us) and the arithmetic on
+// the block's own cells.  Measured per iteration: 3.2 us at 32^3, 4.2 at 64^3,
+// 9.0 at 128^3 (solve to 1e-6: 2.13 ms -> 0.85), and with a cell field 4.5 at
+// 48^3, 9.0 at 97 x 83 x 150 (9.8 ms -> 1.8).
+//
+// Precision.  The cells are FP32, and so are the sums within a warp; across
+// warps and blocks the sums are FP64, as are the scalars and the convergence
+// test.  The FP64 pipe's latencies (65 cycles an addition, 570 a division) lie
+// between the exchange and the next update, 0.6 us an iteration more than sums
+// and scalars in pairs of floats would take; divisions as such took 0.6 us more
+// (8^3: 2.45 us in pairs, 3.65 with plain divisions, 3.0).
 //
 // Layout.  A block owns a brick of whole x rows, by x bz of them.  A thread
 // owns one quad of four x cells in each of the brick's bz planes, so p and
@@ -41,7 +48,6 @@
 
 #include "nn_hh.cuh"
 #include "nn_internal.cuh"
-#include "nn_pair.cuh"
 #include "nn_quad.cuh"
 
 namespace {
@@ -92,17 +98,31 @@ __device__ __forceinline__ bool tagged(const ulonglong2& v, uint32_t tag)
     return (uint32_t)(v.x >> 32) == tag && (uint32_t)(v.y >> 32) == tag;
 }
 
-// Sums and scalars as unevaluated pairs of floats (48 bits).  The addends are
-// FP32 warp sums, so FP64 would carry no more information, and its chains of
-// dependent additions and divisions are slow on this chip: an iteration on
-// 8^3 cells took 5.1 us with FP64 sums and scalars and takes 3.1 us with pairs
-// (the solutions' errors against FP64 are the same).  Sums are kept scaled by
-// SUM_SCALE, so that adding thousands of warps does not overflow.
-constexpr float SUM_SCALE = 1.0f / 4096.0f;
-
-__device__ __forceinline__ Pair pair_shfl(const Pair& x, int o)
+// A double as the two data words of a tagged pair.
+__device__ __forceinline__ void st_tagged(ulonglong2* p, double v, uint32_t tag)
 {
-    return {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o)};
+    st_tagged(p, (uint32_t)__double2loint(v), (uint32_t)__double2hiint(v), tag);
+}
+__device__ __forceinline__ double tagged_double(const ulonglong2& v)
+{
+    return __hiloint2double((int)(uint32_t)v.y, (int)(uint32_t)v.x);
+}
+
+// n / d.  The FP64 pipe has a latency of 65 cycles (a division takes 570), so a
+// float's reciprocal of the mantissa (error e < 2^-21) is refined once, by
+// Halley's third-order step x (1 + e + e e), whose error e^3 is below FP64's
+// rounding; the exponent goes to n, beside that chain.
+__device__ __forceinline__ double fast_div(double n, double d)
+{
+    const int hi = __double2hiint(d), lo = __double2loint(d), e = hi >> 20 & 0x7ff;
+    if (e < 2 || e > 2044) return n / d;  // zero, subnormal, non-finite, or of an extreme reciprocal
+    const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, lo);
+    const float s = nn_rcp(__int_as_float((hi & 0xfffff) << 3 | (unsigned)lo >> 29 | 0x3f800000));  // (0.5, 1]
+    const unsigned b = __float_as_uint(s);
+    const double x = __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
+    const double r = fma(-m, x, 1.0);
+    const double ns = n * __hiloint2double((hi & (int)0x80000000) | (2046 - e) << 20, 0);
+    return ns * fma(x, fma(r, r, r), x);
 }
 
 struct RcgArgs {
@@ -111,13 +131,14 @@ struct RcgArgs {
     int quads, pitch, hq;      // quads a row, shared row pitch, halo quads of a brick
     float op_alpha, onepb, invd;
     float half_ia;             // 1 / (2 alpha)
-    Pair diag;                 // constant coefficients: 1 / invd
-    Pair rtol2;
+    float c, inv_c;            // u = c M r, c a power of two (nn_jacobi_scale)
+    double diag;               // constant coefficients: 1 / invd
+    double rtol2;
     const float* b;
     float* x;
     const float* D;
     float4* xw;                // x during the solve: [block][plane][thread]
-    ulonglong2* rec;           // [2][nb][4]: tagged pairs g, d, rho, (b, b)
+    ulonglong2* rec;           // [2][nb][4]: tagged g, d, rho, (b, b)
     Tagged4* halo;             // [2][nb][hq]: tagged w' of a brick's faces
     unsigned* epoch;           // first tag of the next solve
     double* scal;              // out: rho, (b, b)
@@ -131,8 +152,10 @@ template <int NZ, bool HET>
 __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, const uint32_t base, float4* smem4,
                                               bool& fail)
 {
-    __shared__ float ws[4][RT / 32];
-    __shared__ Pair wp[4][8];
+    __shared__ __align__(16) float ws[4][RT / 32];
+    __shared__ double wp[4][MAX_BLOCKS / 32];
+    __shared__ double s_gamma, s_den, s_lim, s_bb, s_rr;  // the first thread's, kept out of everyone's registers
+    static_assert(MAX_BLOCKS == 160, "five groups of 32 blocks");
     __shared__ float sc_alpha, sc_beta;
     __shared__ int sc_stop, sc_fail;
     const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -155,7 +178,7 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
     const bool full = i0 + 4 <= a.nx;
     // halo duty is on all warps but the first (there are two or more), which
     // polls the sums
-    const int ht = tid - 32, hstep = T - 32, nw = T >> 5;
+    const int ht = tid - 32, hstep = T - 32;
     const int yq = a.bz * a.quads, zq = a.by * a.quads;  // halo quads: y-, y+ (yq each), z-, z+ (zq each)
 
     // halo quad h: its place in shared memory, the brick and face slot it
@@ -193,6 +216,8 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
     // cell's own v outside the grid gives the boundary face alpha D
     for (int c = tid; c < (a.bz + 2) * psz / 4; c += T) reinterpret_cast<float4*>(U)[c] = make_float4(0, 0, 0, 0);
     if (tid == 0) sc_fail = 0;
+    if (tid < 4 * (RT / 32)) (&ws[0][0])[tid] = 0.0f;
+    if (tid < 4 * (MAX_BLOCKS / 32)) (&wp[0][0])[tid] = 0.0;
     __syncthreads();
     bool poison = false;  // two neighbours with D = 0: their face coefficient is 0 / 0
     if (act) {
@@ -367,7 +392,7 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
         for (int e = 0; e < 4; ++e)
             if (i0 + e < a.nx) {
                 const float bv = a.b[g0 + k * gsz + e];
-                at(S[k], e) = HET ? __fdividef(bv - at(A, e), at(dg, e)) : (bv - at(A, e)) * a.invd;
+                at(S[k], e) = HET ? __fdividef(bv - at(A, e), at(dg, e)) : (bv - at(A, e)) * (a.c * a.invd);
                 if (poison) at(S[k], e) = nanf("");
                 acc_b += bv * bv;
             }
@@ -385,8 +410,7 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
     receive(base + 1, [&](int, int sm, float4 v) { *reinterpret_cast<float4*>(U + sm) = v; });
 
     uint32_t tag = base + 2;
-    Pair gamma{0, 0}, alpha{0, 0}, bb{0, 0}, rr{0, 0};  // thread 0
-    int it = -1, stop = 0;
+    int it = -1;
     float al_prev = 0.0f;
     bool owed = false;  // x lacks the last direction, al_prev P
     for (;; ++tag) {
@@ -418,7 +442,7 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
                 ad = vfma(A.b, u.b, vfma(A.a, u.a, ad));
             }
         });
-        // block sums: FP32 within a warp, pairs across warps and blocks
+        // block sums: FP32 within a warp, FP64 across warps and blocks
         const float v0 = nn_warp_sumf(ag.v[0] + ag.v[1]), v1 = nn_warp_sumf(ad.v[0] + ad.v[1]);
         const float v2 = HET ? nn_warp_sumf(ar.v[0] + ar.v[1]) : 0.0f;
         const float v3 = it < 0 ? nn_warp_sumf(acc_b) : 0.0f;
@@ -432,14 +456,15 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
         const int hl = lane & 15, up = lane >> 4;  // lanes 0-15: g, rho; 16-31: d, (b, b)
         const int np = (HET || it < 0) ? 2 : 1;    // pairs of sums to exchange: {g, d} and {rho, (b, b)}
         ulonglong2* rec = a.rec + 4 * (size_t)(tag & 1) * a.nb;
-        if (warp == 0)
-            for (int pr = 0; pr < np; ++pr) {
-                Pair s0{hl < nw ? ws[2 * pr + up][hl] * SUM_SCALE : 0.0f, 0.0f};
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) s0 = pair_add(s0, pair_shfl(s0, o));
-                if (hl == 0)
-                    st_tagged(rec + 4 * rank + 2 * pr + up, __float_as_uint(s0.h), __float_as_uint(s0.l), tag);
-            }
+        if (warp == 0) {
+            // lanes 4 w .. 4 w + 3: sum w, four warps each
+            const int w = lane >> 2 & 3;
+            const float4 v = *reinterpret_cast<const float4*>(&ws[w][4 * (lane & 3)]);
+            double s0 = ((double)v.x + (double)v.y) + ((double)v.z + (double)v.w);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+            if (lane == 4 * w && w < 2 * np) st_tagged(rec + 4 * rank + w, s0, tag);
+        }
         // x takes two directions every second iteration: loaded here, behind
         // the wait
         Quad X[NZ];
@@ -449,15 +474,23 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
                 if (k < bzn) X[k] = quad_ldcg(xw + k * T);
         receive(tag, [&](int h, int, float4 v) { WH[h] = v; });
         // every block adds all blocks' sums in the same order: a record a
-        // thread, then warps, then the first warp
+        // thread, then warps (without the steps that would add zeros), then the
+        // first warp
+        // (rgamma, factor: 1 / g and 1 / (g a) = den / g^2 of the last iteration,
+        // formed while the first thread waits)
+        double rgamma = 0.0, factor = 0.0;
         for (int c0 = 32 * warp; c0 < a.nb; c0 += T) {
             const int c = c0 + lane;
-            Pair t[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+            double t[4] = {0.0, 0.0, 0.0, 0.0};
             if (c < a.nb) {
                 ulonglong2 v[4];
 #pragma unroll
                 for (int w = 0; w < 4; ++w)
                     if (w < 2 * np) v[w] = ld_tagged(rec + 4 * c + w);
+                if (c == 0 && it >= 0) {
+                    rgamma = 1.0 / s_gamma;
+                    factor = s_den != 0.0 ? rgamma * rgamma * s_den : (double)INFINITY;
+                }
 #pragma unroll
                 for (int w = 0; w < 4; ++w)
                     if (w < 2 * np) {
@@ -469,48 +502,54 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
                             }
                             v[w] = ld_tagged(rec + 4 * c + w);
                         }
-                        t[w] = Pair{__uint_as_float((uint32_t)v[w].x), __uint_as_float((uint32_t)v[w].y)};
+                        t[w] = tagged_double(v[w]);
                     }
             }
             __syncwarp();
-            for (int pr = 0; pr < np; ++pr) {
-                const Pair t0 = pr ? t[2] : t[0], t1 = pr ? t[3] : t[1];
-                Pair r = pair_add(up ? t1 : t0, pair_shfl(up ? t0 : t1, 16));
 #pragma unroll
-                for (int o = 8; o > 0; o >>= 1) r = pair_add(r, pair_shfl(r, o));
+            for (int pr = 0; pr < 2; ++pr) {
+                if (pr >= np) break;
+                const double t0 = t[2 * pr], t1 = t[2 * pr + 1];
+                double r = (up ? t1 : t0) + __shfl_xor_sync(0xffffffffu, up ? t0 : t1, 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+                    if (o < a.nb) r += __shfl_xor_sync(0xffffffffu, r, o);
                 if (hl == 0) wp[2 * pr + up][c0 >> 5] = r;
             }
         }
         __syncthreads();
         if (warp == 0) {
-            // lane 8 w + i: sum w of the group of blocks i
-            const int w = lane >> 3, i = lane & 7, groups = (a.nb + 31) >> 5;
-            Pair r = i < groups && w < 2 * np ? wp[w][i] : Pair{0, 0};
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) r = pair_add(r, pair_shfl(r, o));
-            const Pair d = pair_shfl(r, 8), r2 = pair_shfl(r, 16), r3 = pair_shfl(r, 24);  // lane 0's
+            // lane w: sum w
+            const double* t = wp[lane & 3];
+            const double r = ((t[0] + t[1]) + (t[2] + t[3])) + t[4];
+            const double d = __shfl_sync(0xffffffffu, r, 1);
+            const double r2 = np > 1 ? __shfl_sync(0xffffffffu, r, 2) : 0.0;
+            const double r3 = np > 1 ? __shfl_sync(0xffffffffu, r, 3) : 0.0;
             if (lane == 0) {
-                const Pair g = HET ? r : pair_mul(r, a.diag);  // constant coefficients: r = diag u
-                rr = HET ? r2 : pair_mul(g, a.diag);
-                if (it < 0) bb = r3;
-                const Pair lim = pair_mul(a.rtol2, bb);
-                const bool met = rr.h < lim.h || (rr.h == lim.h && rr.l <= lim.l);
-                Pair al{0, 0}, be{0, 0};
+                // g = (r, u); with constant coefficients r holds (c r = diag u)
+                // g / diag, which be and den, ratios of g, may use as it is
+                const double g = HET ? r : r * a.diag;
+                const double rr = HET ? r2 : g * a.diag;
+                double den = d, be = 0.0;
                 if (it < 0) {
-                    if (d.h != 0.0f) al = pair_div(g, d);
-                    stop = met ? 1 : a.max_iter <= 0 ? 2 : 0;
+                    s_bb = r3;
+                    s_lim = a.rtol2 * ((double)a.c * a.c * r3);
                 } else {
-                    be = pair_div(g, gamma);
-                    const Pair m = pair_div(pair_mul(be, g), alpha);
-                    const Pair den = pair_add(d, Pair{-m.h, -m.l});
-                    if (den.h != 0.0f) al = pair_div(g, den);
-                    stop = met ? 1 : it + 1 >= a.max_iter ? 2 : !(isfinite(al.h) && isfinite(be.h)) ? 3 : 0;
+                    be = r * rgamma;
+                    den = fma(-(r * r), factor, d);  // d - be g / a
                 }
-                sc_alpha = al.h;
-                sc_beta = be.h;
+                const double al = den != 0.0 ? fast_div(g, den) : 0.0;
+                const int stop = rr <= s_lim                       ? 1
+                                 : it + 1 >= a.max_iter            ? 2
+                                 : it < 0                          ? 0
+                                 : !(isfinite(al) && isfinite(be)) ? 3
+                                                                   : 0;
+                s_gamma = r;
+                s_den = den;
+                s_rr = rr;
+                sc_alpha = (float)al;
+                sc_beta = (float)be;
                 sc_stop = stop;
-                gamma = g;
-                alpha = al;
             }
         }
         __syncthreads();
@@ -519,7 +558,7 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
         // ---- s', p, x, u (own cells and halo)
         const float al = sc_alpha, be = sc_beta;
         if (act) {
-            const V2 al2 = vb<2>(al), nal2 = vb<2>(-al), be2 = vb<2>(be), ap2 = vb<2>(al_prev);
+            const V2 al2 = vb<2>(al * a.inv_c), nal2 = vb<2>(-al), be2 = vb<2>(be), ap2 = vb<2>(al_prev * a.inv_c);
 #pragma unroll
             for (int k = 0; k < NZ; ++k) {
                 if (k >= bzn) break;
@@ -555,7 +594,7 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
         for (int k = 0; k < NZ; ++k) {
             if (k >= bzn) break;
             Quad x = quad_ldcg(xw + k * T);
-            if (owed) x = {vfma(vb<2>(al_prev), P[k].a, x.a), vfma(vb<2>(al_prev), P[k].b, x.b)};
+            if (owed) x = {vfma(vb<2>(al_prev * a.inv_c), P[k].a, x.a), vfma(vb<2>(al_prev * a.inv_c), P[k].b, x.b)};
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 if (i0 + e < a.nx) a.x[g0 + k * gsz + e] = at(x, e);
@@ -567,11 +606,11 @@ __device__ __forceinline__ uint32_t rcg_solve(const RcgArgs& a, const int rank, 
             a.flags[2] = 1;
             a.flags[0] = 3;
         } else if (rank == 0) {
-            a.flags[0] = stop;
+            a.flags[0] = sc_stop;
             a.flags[1] = it;
             a.flags[2] = 0;
-            a.scal[0] = ((double)rr.h + rr.l) / SUM_SCALE;
-            a.scal[1] = ((double)bb.h + bb.l) / SUM_SCALE;
+            a.scal[0] = s_rr * a.inv_c * a.inv_c;
+            a.scal[1] = s_bb;
         }
     }
     return tag;
@@ -610,7 +649,7 @@ struct RcgBatchArgs {
     unsigned* epoch;           // per group
     double* scal;              // [instances][2]
     int* flags;                // [instances][4]
-    Pair rtol2;
+    double rtol2;
     int max_iter;
 };
 
@@ -701,19 +740,15 @@ const void* kernel_of(int nz)
 }
 }  // namespace
 
-static Pair split(double v)
+static void rcg_operator(RcgArgs& a, double alpha, double beta, bool het)
 {
-    const float h = (float)v;
-    return {h, (float)(v - (double)h)};
-}
-
-static void rcg_operator(RcgArgs& a, double alpha, double beta)
-{
+    a.c = nn_jacobi_scale(alpha, beta, het);
+    a.inv_c = 1.0f / a.c;
     a.op_alpha = (float)alpha;
     a.onepb = (float)(1.0 + beta);
     a.invd = (float)(1.0 / (1.0 + beta + 6.0 * alpha));
     a.half_ia = (float)(0.5 / alpha);
-    a.diag = split(1.0 / (double)a.invd);
+    a.diag = 1.0 / (double)a.invd;
 }
 
 struct nn_rcg_plan {
@@ -808,7 +843,7 @@ nn_status nn_rcg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, 
     int per_sm = 0;
     NN_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     if (!coop || per_sm < 1) return NN_ERR_UNSUPPORTED;
-    rcg_operator(a, alpha, beta);
+    rcg_operator(a, alpha, beta, D != nullptr);
     a.D = D;
     nn_rcg_plan* pl = new nn_rcg_plan();
     pl->ctx = ctx;
@@ -853,7 +888,7 @@ nn_status nn_rcg_begin(nn_rcg_plan* pl, const float* d_b, float* d_x, double rto
     nn_ctx* ctx = pl->ctx;
     pl->a.b = d_b;
     pl->a.x = d_x;
-    pl->a.rtol2 = split(rtol * rtol);
+    pl->a.rtol2 = rtol * rtol;
     pl->a.max_iter = max_iter;
     if (pl->timing && !pl->e0) {
         NN_CUDA(ctx, cudaEventCreate(&pl->e0));
@@ -1031,7 +1066,7 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
         for (int b : c.list) {
             const Shape& s = shape(sides[b], c.width);
             RcgArgs a = s.a;
-            rcg_operator(a, alpha_unit * sides[b] * sides[b], beta);
+            rcg_operator(a, alpha_unit * sides[b] * sides[b], beta, false);
             nz = std::max(nz, a.bz);
             pl->smem = std::max(pl->smem, s.smem);
             halo = std::max(halo, 2 * (size_t)a.nb * a.hq);
@@ -1109,7 +1144,7 @@ nn_status nn_rcg_batch_begin(nn_rcg_batch* pl, const float* d_b, float* d_x, dou
     nn_ctx* ctx = pl->ctx;
     pl->B.b = d_b;
     pl->B.x = d_x;
-    pl->B.rtol2 = split(rtol * rtol);
+    pl->B.rtol2 = rtol * rtol;
     pl->B.max_iter = max_iter;
     void* args[] = {&pl->B};
     NN_CUDA(ctx, cudaLaunchCooperativeKernel(pl->kernel, dim3(pl->blocks), dim3(RT), args, pl->smem, cs));
