@@ -69,6 +69,7 @@ struct CgArgs {
     int rows, rp;                 // rows of a tile: owned; computed by NR
     int ntx, nty, zc;             // tiles in x and y; planes of a tile
     float op_alpha, onepb, invd;  // invd: 1/diag for constant coefficients
+    float c, inv_c;               // u = c M r, t = c M s, c a power of two (nn_jacobi_scale)
     int frame;                    // a quad beside the tile is loaded on both sides (more than one tile in x)
     float *u_out, *t_out;
     float *p, *x;                 // x: rows of 4 nq cells
@@ -141,8 +142,8 @@ struct CgSum {
 // The sums' scalars, by one thread of the last block to arrive.
 __device__ void cg_scalars(const CgArgs& a, bool init, const double* out)
 {
-    const double g = out[0], d = out[1], rr = out[2];
-    a.scal[C_RR] = rr;
+    const double g = out[0], d = out[1], rr = out[2], c2 = (double)a.c * a.c;  // g, d and rr times c2
+    a.scal[C_RR] = rr / c2;
     a.scal[C_DELTA] = d;
     if (init) {
         a.scal[C_BB] = out[3];
@@ -153,7 +154,7 @@ __device__ void cg_scalars(const CgArgs& a, bool init, const double* out)
         a.scal[C_BETA_P] = 0.0;
         a.flags[1] = 0;
         a.flags[2] = 0;
-        a.flags[0] = (rr <= a.rtol2 * out[3]) ? 1 : 0;
+        a.flags[0] = (rr <= a.rtol2 * c2 * out[3]) ? 1 : 0;
         return;
     }
     const int it = a.flags[1] + 1;
@@ -165,7 +166,7 @@ __device__ void cg_scalars(const CgArgs& a, bool init, const double* out)
     a.scal[C_BETA] = bnew;
     a.scal[C_ALPHA] = denom != 0.0 ? g / denom : 0.0;
     a.scal[C_GAMMA] = g;
-    if (rr <= a.rtol2 * a.scal[C_BB]) a.flags[0] = 1;
+    if (rr <= a.rtol2 * c2 * a.scal[C_BB]) a.flags[0] = 1;
     else if (it >= a.max_iter) a.flags[0] = 2;
     else if (!(std::isfinite(a.scal[C_ALPHA]) && std::isfinite(a.scal[C_BETA]))) a.flags[0] = 3;
 }
@@ -285,6 +286,7 @@ __global__ void __launch_bounds__(CG_MAX_THREADS, 1)
     }
     const float alpha = INIT ? 0.0f : (float)a.scal[C_ALPHA], beta = INIT ? 0.0f : (float)a.scal[C_BETA];
     const float alpha_p = INIT ? 0.0f : (float)a.scal[C_ALPHA_P], beta_p = INIT ? 0.0f : (float)a.scal[C_BETA_P];
+    const float ax = HET ? alpha : alpha * a.inv_c, axp = HET ? alpha_p : alpha_p * a.inv_c;  // of x
     const Quad onepb = quad_all(a.onepb);
 
     // registers carried along the march: u and v here; the faces and fluxes to
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(CG_MAX_THREADS, 1)
                     Quad po = fma(quad_all(alpha_p), tC[h], uC[h]);
                     if (has_p) po = fma(quad_all(beta_p), quad_of(slot_p[so + h * cq]), po);
                     const Quad pn = fma(quad_all(beta), po, uC[h]);
-                    const Quad xn = fma(quad_all(alpha), pn, fma(quad_all(alpha_p), po, quad_of(slot_x[so + h * cq])));
+                    const Quad xn = fma(quad_all(ax), pn, fma(quad_all(axp), po, quad_of(slot_x[so + h * cq])));
                     *reinterpret_cast<float4*>(a.p + g + h * sy) = float4_of(pn);
                     *reinterpret_cast<float4*>(a.x + g + h * sy) = float4_of(xn);
                 }
@@ -427,7 +429,7 @@ __global__ void __launch_bounds__(CG_MAX_THREADS, 1)
 #pragma unroll
                         for (int e = 1; e < 4; ++e)
                             if (e >= pad) at(rv, e) = 0.0f;
-                    wN[h] = mi * rv;
+                    wN[h] = (HET ? mi : quad_all(a.c * a.invd)) * rv;
                 } else {
                     tv = fma(quad_all(beta), tC[h], mi * w);
                     if (pad < 4)
@@ -445,8 +447,8 @@ __global__ void __launch_bounds__(CG_MAX_THREADS, 1)
                     // the mass term and the energies of the faces inside the
                     // quad, to the plane behind and on the grid's near sides
                     const Quad uu = nu * nu, dz = nu - wP[h];
-                    e_g += sum(HET || INIT ? rv * nu : uu);
-                    e_r += sum(HET || INIT ? rv * rv : uu);
+                    e_g += sum(HET ? rv * nu : uu);
+                    e_r += sum(HET ? rv * rv : uu);
                     if (INIT) e_b += sum(tC[h] * tC[h]);
                     Quad s = HET ? fma(onepb, uu, fzP[h] * dz * dz) : dz * dz;
                     if (k == (dir > 0 ? a.nz - 1 : 0)) s = HET ? fma(fzN, uu, s) : s + uu;
@@ -501,7 +503,7 @@ __global__ void __launch_bounds__(CG_MAX_THREADS, 1)
         return;
     }
     if (live) sd.add(across(n - 1));
-    const double scale = HET || INIT ? 1.0 : (double)a.onepb + 6.0 * (double)a.op_alpha;
+    const double scale = HET ? 1.0 : (double)a.onepb + 6.0 * (double)a.op_alpha;  // r = scale u
     const double sums[4] = {scale * sg.value(), sd.value(), scale * scale * sr.value(), sbb.value()};
     double out[4];
     if (cg_reduce(INIT ? 4 : 3, sums, a.partials, a.ticket, out) && tid == 0) cg_scalars(a, INIT, out);
@@ -512,7 +514,7 @@ __global__ void __launch_bounds__(CG_MAX_THREADS, 1)
 __global__ void __launch_bounds__(CG_THREADS) k_cg_flush(const __grid_constant__ CgArgs a, const float* u, const float* t,
                                                          float* x)
 {
-    const float al = (float)a.scal[C_ALPHA_P], be = (float)a.scal[C_BETA_P];
+    const float al = (float)a.scal[C_ALPHA_P], be = (float)a.scal[C_BETA_P], ax = al * a.inv_c;
     const bool same = x == a.x;  // then only those planes are touched
     const int first = same ? (a.it + 1) & 1 : 0, step = same ? 2 : 1;
     const int planes = (a.nz - first + step - 1) / step, psz = a.nx * a.ny;
@@ -521,7 +523,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_cg_flush(const __grid_constant__
         const int k = first + step * (int)(i / psz), row = (int)(i % psz) / a.nx + k * a.ny, e = (int)(i % psz) % a.nx;
         const int c = row * 4 * a.nq + e;
         float v = a.x[c];
-        if (a.it > 0 && ((k + a.it) & 1)) v += al * (u[c] + al * t[c] + (a.it > 1 ? be * a.p[c] : 0.0f));
+        if (a.it > 0 && ((k + a.it) & 1)) v += ax * (u[c] + al * t[c] + (a.it > 1 ? be * a.p[c] : 0.0f));
         x[(int64_t)row * a.nx + e] = v;
     }
 }
@@ -594,7 +596,7 @@ struct nn_cg_plan {
     nn_ctx* ctx = nullptr;
     int nx = 0, ny = 0, nz = 0, nq = 0;
     size_t cells = 0;              // of a padded vector
-    float op_alpha = 0, onepb = 0, invd = 0, half_ia = 0;
+    float op_alpha = 0, onepb = 0, invd = 0, half_ia = 0, c = 1;
     const float* D = nullptr;      // caller's cell field (HET), not owned
     float *u[2] = {}, *t[2] = {}, *p = nullptr, *v = nullptr;
     float* xp = nullptr;           // x in rows of whole quads where the caller's is not
@@ -750,6 +752,7 @@ nn_status nn_cg_plan_create(nn_ctx* ctx, int nx, int ny, int nz, double alpha, d
     pl->onepb = (float)(1.0 + beta);
     pl->invd = (float)(1.0 / (1.0 + beta + 6.0 * alpha));
     pl->half_ia = 0.5f / pl->op_alpha;
+    pl->c = nn_jacobi_scale(alpha, beta, D != nullptr);
     pl->D = D;
     pl->elem_blocks = nn_grid_for(ctx, (int64_t)pl->cells, CG_THREADS, 8);
     // (the reduction's static shared memory is beside the tile's)
@@ -783,6 +786,7 @@ static CgArgs cg_args(nn_cg_plan* pl, float* x, double rtol, int max_iter, int i
     a.wq = pl->wq; a.cq = pl->cq; a.rows = pl->rows; a.rp = pl->rp;
     a.ntx = pl->ntx; a.nty = pl->nty; a.zc = pl->zc;
     a.op_alpha = pl->op_alpha; a.onepb = pl->onepb; a.invd = pl->invd;
+    a.c = pl->c; a.inv_c = 1.0f / pl->c;
     a.frame = pl->ntx > 1;
     a.u_out = pl->u[pin ^ 1];
     a.t_out = pl->t[pin ^ 1];

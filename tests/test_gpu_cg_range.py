@@ -20,7 +20,9 @@ BETA = 0.05
 # shape (nz, ny, nx), cell field, alpha, exponents
 CASES = [((40, 44, 48), False, 6.0, (-40, 50)), ((40, 44, 48), True, 6.0, (-40, 50)),
          ((5, 4, 7), False, 1.5, (-40, 50)), ((5, 4, 7), True, 1.5, (-40, 50)),
-         ((21, 33, 35), True, 6.0, (-40, 50)), ((48, 48, 48), False, 2000.0, (-46, 45))]
+         ((21, 33, 35), True, 6.0, (-40, 50)), ((48, 48, 48), False, 2000.0, (-46, 45)),
+         ((134, 130, 136), False, 6.0, (-40, 50)), ((134, 130, 136), False, 2000.0, (-46, 45)),
+         ((110, 109, 112), True, 6.0, (-40, 50))]
 
 
 def _bound(b, x, norm, it):
