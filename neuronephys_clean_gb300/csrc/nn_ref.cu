@@ -3,6 +3,7 @@
 // and chunked lists, and the ParacrineModule (trilinear scatter/interpolation
 // + Crank-Nicolson 27-point CG).  Each function cites the reference code whose
 // behaviour it reproduces.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -890,10 +891,24 @@ __global__ void k_fine(int n, const int* list, const int* count, float* gen, flo
 // buffers), which saves a third barrier.
 //
 // Barrier: a counter that every block adds to, behind a fence; each block's
-// first thread polls it (bounded).  Sums: FP64 per thread, block partials,
-// added by every block in the same order after the barrier.
+// first thread polls it (bounded), and its second fence lets the block's plain
+// loads, L1 included, see what the others wrote.  Sums: FP64 per thread, block
+// partials, added by every block in the same order after the barrier.
+//
+// Large grids are bound by the latency of the 27 x 2 loads a cell, small ones by
+// the barriers, whose cost grows with the blocks.  us a solve by blocks a SM, 1 /
+// 2 / 3: 48^3 83 / 93 / 93, 80^3 173 / 156 / 170, 100^3 246 / 204 / 218, 150^3
+// 698 / 464 / 450, 300^3 6549 / 3611 / 3005 (with loads past L1 and one block
+// 10190, as separate launches 4998).
 constexpr int CN_THREADS = 512;
 constexpr int CN_POLLS = 1 << 22;  // some seconds
+
+// Blocks a SM: by the cells of a thread at one.
+int cn_blocks_per_sm(const nn_ctx* ctx, int64_t G)
+{
+    const int64_t cells = G / ((int64_t)ctx->num_sms * CN_THREADS);
+    return cells < 5 ? 1 : cells < 25 ? 2 : 3;
+}
 
 struct CnArgs {
     int nx, ny, nz, max_iter;
@@ -970,8 +985,6 @@ __global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
                 }
         return acc;
     };
-    // written by other blocks during this launch: read past L1
-    auto cg = [](const float* p) { return __ldcg(p); };
 
     for (I c = c0; c < G; c += stride) {
         auto val = [&](I n) { return q.u[n] + q.dep[n]; };
@@ -983,7 +996,7 @@ __global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
     barrier(false, 0.0);
     double acc = 0.0;
     for (I c = c0; c < G; c += stride) {
-        const float rv = q.b[c] - conv(c, q.A, [&](I n) { return cg(q.x + n); });
+        const float rv = q.b[c] - conv(c, q.A, [&](I n) { return q.x[n]; });
         q.r[c] = rv;
         acc += (double)rv * rv;
     }
@@ -995,7 +1008,7 @@ __global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
     while (!done && it < q.max_iter && !fail) {
         acc = 0.0;
         for (I c = c0; c < G; c += stride) {
-            auto val = [&](I n) { return it ? cg(q.r + n) + beta * cg(p_old + n) : cg(q.r + n); };
+            auto val = [&](I n) { return it ? q.r[n] + beta * p_old[n] : q.r[n]; };
             const float pv = val(c), ap = conv(c, q.A, val);
             p_new[c] = pv;
             q.Ap[c] = ap;
@@ -1037,6 +1050,11 @@ __global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
         }
     }
 }
+
+const void* cn_kernel(int64_t G)
+{
+    return G <= INT32_MAX / 2 ? (const void*)k_cn_solve<int> : (const void*)k_cn_solve<int64_t>;
+}
 }  // namespace
 
 extern "C" nn_status nn_paracrine_ref_create(nn_ctx* ctx, const nn_paracrine_ref_params* p, int n, const float* d_x,
@@ -1053,8 +1071,11 @@ extern "C" nn_status nn_paracrine_ref_create(nn_ctx* ctx, const nn_paracrine_ref
     pm->G = (int64_t)p->nx * p->ny * p->nz;
     pm->g_out = d_g_paracrine;
     const size_t G = (size_t)pm->G, N = (size_t)(n > 0 ? n : 1);
-    pm->nparts = nn_grid_for(ctx, pm->G, CN_THREADS, 1);  // co-resident: one block a SM at most
-    nn_status st = NN_OK;
+    // co-resident blocks only
+    const void* cn = cn_kernel(pm->G);
+    int per_sm = 0;
+    nn_status st = nn_cuda_check(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cn, CN_THREADS, 0), "k_cn_solve");
+    pm->nparts = nn_grid_for(ctx, pm->G, CN_THREADS, std::max(1, std::min(per_sm, cn_blocks_per_sm(ctx, pm->G))));
 #define PM_ALLOC(ptr, cnt) if (st == NN_OK) st = nn_alloc(ctx, &pm->ptr, cnt)
     PM_ALLOC(idx8, 8 * N); PM_ALLOC(w8, 8 * N);
     PM_ALLOC(u, G); PM_ALLOC(Ax, G); PM_ALLOC(un, G); PM_ALLOC(x, G); PM_ALLOC(b, G);
@@ -1159,8 +1180,7 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
     q.done = pm->done;
     NN_CUDA(ctx, cudaMemsetAsync(pm->bar, 0, sizeof(unsigned), s));
     void* args[] = {&q};
-    NN_CUDA(ctx, cudaLaunchCooperativeKernel(G <= INT32_MAX / 2 ? (const void*)k_cn_solve<int> : (const void*)k_cn_solve<int64_t>,
-                                             dim3(pm->nparts), dim3(CN_THREADS), args, 0, s));
+    NN_CUDA(ctx, cudaLaunchCooperativeKernel(cn_kernel(G), dim3(pm->nparts), dim3(CN_THREADS), args, 0, s));
     ctx->launches++;
     // interpolate, reset sources, copy out (src/paracrine.cuh:259-264)
     if (pm->n > 0) {

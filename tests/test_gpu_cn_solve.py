@@ -48,3 +48,21 @@ def test_coupling_scatter_edges(ctx, orc, n, frac):
     assert nf == rnf
     assert np.array_equal(ins.numpy(), rin)
     assert np.array_equal(cp.get_firing_neurons()[:nf], rfire)
+
+
+@pytest.mark.parametrize("shape", [(61, 79, 80), (90, 100, 110), (130, 125, 128)])
+def test_cn_solve_blocks_per_sm(ctx, orc, shape):
+    """One, two and three blocks an SM, whose blocks read what others wrote
+    through L1; bounds as above."""
+    p = nn.ParacrineModule.default_params()
+    p.nz, p.ny, p.nx = shape
+    p.h, p.D, p.decay, p.par_dt, p.max_iter = 1.0, 5.0, 3e-4, 1.0, 20
+    zero = ctx.to_device(np.zeros(1, np.float32))
+    pm = nn.ParacrineModule(ctx, ctx.empty((1,), np.float32), 1, p, zero, zero, zero)
+    u = np.random.default_rng(4).random(int(np.prod(shape))).astype(np.float32)
+    pm.set_density(u)
+    it, _ = pm.update_on_own_timescale()
+    ref, rit, _ = orc.paracrine_cn_solve(u.astype(np.float64), shape, 1.0, p.D, p.decay, 1.0, 1e-6, 20, 1)
+    assert it == rit
+    guess = u.max() * (1 + p.D * 256 / 30)
+    assert np.abs(pm.density().astype(np.float64) - ref).max() <= 1e-5 * max(1.0, np.abs(ref).max(), guess)
