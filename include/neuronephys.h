@@ -195,7 +195,9 @@ NN_API nn_status nn_paracrine_destroy(nn_paracrine* pm);
 NN_API nn_status nn_paracrine_ref_fine(nn_paracrine* pm, const nn_coupling* c);
 /* update_on_own_timescale() (src/paracrine.cuh:255-265): scatter, CN solve,
  * interpolate, reset sources, copy to d_g_paracrine.  iters/final_rr (host)
- * may be NULL. */
+ * may be NULL; with both NULL the call does not wait for the GPU, and a solve
+ * whose grid barrier gave up (NN_ERR_TIMEOUT: the density is undefined, the
+ * sources are gone) is reported by the module's next update, fine or own. */
 NN_API nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* final_rr);
 /* get_grid().density() (src/paracrine.cuh:266, :170-172): device pointer to
  * the nx*ny*nz density (x fastest). */

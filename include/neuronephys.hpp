@@ -313,7 +313,8 @@ public:
     }
     void update_on_own_timescale()
     {
-        ctx().check(nn_paracrine_ref_own(pm_, nullptr, nullptr), "update_on_own_timescale");
+        int iters = 0;  // asked for, so that this call reports its own solve
+        ctx().check(nn_paracrine_ref_own(pm_, &iters, nullptr), "update_on_own_timescale");
         ctx().finish("update_on_own_timescale");
     }
     // get_grid().density(): device pointer, x fastest

@@ -786,7 +786,9 @@ struct nn_paracrine {
     double* scal = nullptr;         // [0]=rr [1]=pAp [2]=rr_new
     double* partials = nullptr;     // [2][nparts]
     unsigned int* bar = nullptr;    // grid barrier of k_cn_solve
-    int* done = nullptr;            // [0] outcome [1] iterations [2] a wait gave up
+    int* done = nullptr;            // [0] outcome [1] iterations
+    int* h_gave_up = nullptr;       // pinned, set by k_cn_solve: a wait gave up; cleared when reported
+    int polls = 0;                  // limit of its waits
     int nparts = 0;                 // blocks of k_cn_solve
 };
 
@@ -901,7 +903,7 @@ __global__ void k_fine(int n, const int* list, const int* count, float* gen, flo
 // 698 / 464 / 450, 300^3 6549 / 3611 / 3005 (with loads past L1 and one block
 // 10190, as separate launches 4998).
 constexpr int CN_THREADS = 512;
-constexpr int CN_POLLS = 1 << 22;  // some seconds
+constexpr int CN_POLLS = 1 << 22;  // some seconds (NN_CN_POLLS sets another limit)
 
 // Blocks a SM: by the cells of a thread at one.
 int cn_blocks_per_sm(const nn_ctx* ctx, int64_t G)
@@ -921,7 +923,9 @@ struct CnArgs {
     double* scal;              // out: [0] rr of the last direction [1] pAp [2] rr
     double* partials;          // [2][blocks]
     unsigned* bar;
-    int* done;                 // out: [0] 1 converged, 2 nothing to do  [1] iterations  [2] a wait gave up
+    int* done;                 // out: [0] 1 converged, 2 nothing to do  [1] iterations
+    int* gave_up;              // out (host memory): a wait gave up
+    int polls;
 };
 
 template <class I>
@@ -944,7 +948,7 @@ __global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
         }
         __syncthreads();
         ++phase;
-        if (tid == 0) {
+        if (tid == 0 && !fail) {  // (a block that gave up arrives nowhere any more)
             if (sum) {
                 double s = 0.0;
                 for (int k = 0; k < CN_THREADS / 32; ++k) s += ws[k];
@@ -954,7 +958,7 @@ __global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
             atomicAdd(q.bar, 1u);
             int n = 0;
             while (*(volatile unsigned*)q.bar < phase * gridDim.x)
-                if (++n > CN_POLLS) {
+                if (++n > q.polls) {
                     fail = 1;
                     break;
                 }
@@ -1037,17 +1041,21 @@ __global__ void __launch_bounds__(CN_THREADS) k_cn_solve(CnArgs q)
             p_new = t;
         }
     }
+    if (fail) {
+        if (tid == 0) {
+            *(volatile int*)q.gave_up = 1;
+            __threadfence_system();
+        }
+        return;  // the block's cells keep their density
+    }
     // density = x unless the initial residual already met the tolerance (src/paracrine.cu:114-116)
     for (I c = c0; c < G; c += stride) q.u[c] = done == 2 ? q.un[c] : q.x[c];
-    if (tid == 0) {
-        if (fail) q.done[2] = 1;
-        if (blockIdx.x == 0) {
-            q.done[0] = done;
-            q.done[1] = it;
-            q.scal[0] = rr;
-            q.scal[1] = pap;
-            q.scal[2] = rr_new;
-        }
+    if (tid == 0 && blockIdx.x == 0) {
+        q.done[0] = done;
+        q.done[1] = it;
+        q.scal[0] = rr;
+        q.scal[1] = pap;
+        q.scal[2] = rr_new;
     }
 }
 
@@ -1081,17 +1089,22 @@ extern "C" nn_status nn_paracrine_ref_create(nn_ctx* ctx, const nn_paracrine_ref
     PM_ALLOC(u, G); PM_ALLOC(Ax, G); PM_ALLOC(un, G); PM_ALLOC(x, G); PM_ALLOC(b, G);
     PM_ALLOC(r, G); PM_ALLOC(p0, G); PM_ALLOC(p1, G); PM_ALLOC(Ap, G);
     PM_ALLOC(at_neurons, N); PM_ALLOC(generated, N);
-    PM_ALLOC(scal, 4); PM_ALLOC(partials, 2 * (size_t)pm->nparts); PM_ALLOC(bar, 1); PM_ALLOC(done, 3);
+    PM_ALLOC(scal, 4); PM_ALLOC(partials, 2 * (size_t)pm->nparts); PM_ALLOC(bar, 1); PM_ALLOC(done, 2);
 #undef PM_ALLOC
+    if (st == NN_OK)
+        st = nn_cuda_check(ctx, cudaHostAlloc((void**)&pm->h_gave_up, sizeof(int), cudaHostAllocMapped), "cudaHostAlloc");
     if (st != NN_OK) {
         nn_paracrine_destroy(pm);
         return st;
     }
+    *pm->h_gave_up = 0;
+    const char* polls = std::getenv("NN_CN_POLLS");
+    pm->polls = polls ? std::atoi(polls) : CN_POLLS;
     cudaStream_t s = ctx->stream;
     cudaMemsetAsync(pm->u, 0, sizeof(float) * G, s);
     cudaMemsetAsync(pm->generated, 0, sizeof(float) * N, s);
     cudaMemsetAsync(pm->at_neurons, 0, sizeof(float) * N, s);
-    cudaMemsetAsync(pm->done, 0, 3 * sizeof(int), s);
+    cudaMemsetAsync(pm->done, 0, 2 * sizeof(int), s);
     if (n > 0) {
         k_trilinear<<<nn_grid_for(ctx, n, 256, 16), 256, 0, s>>>(n, d_x, d_y, d_z, p->nx, p->ny, p->nz, p->h, pm->idx8,
                                                                   pm->w8);
@@ -1119,6 +1132,7 @@ extern "C" nn_status nn_paracrine_destroy(nn_paracrine* pm)
     nn_release(pm->Ap);
     nn_release(pm->at_neurons); nn_release(pm->generated); nn_release(pm->scal); nn_release(pm->partials);
     nn_release(pm->bar); nn_release(pm->done);
+    if (pm->h_gave_up) cudaFreeHost(pm->h_gave_up);
     nn_ctx* ctx = pm->ctx;
     delete pm;
     nn_ctx_release(ctx);
@@ -1128,9 +1142,19 @@ extern "C" nn_status nn_paracrine_destroy(nn_paracrine* pm)
 extern "C" float* nn_paracrine_density(nn_paracrine* pm) { return pm ? pm->u : nullptr; }
 extern "C" float* nn_paracrine_sources(nn_paracrine* pm) { return pm ? pm->generated : nullptr; }
 
+// Reports a solve whose wait gave up, once.
+static nn_status cn_gave_up(nn_paracrine* pm)
+{
+    volatile int* f = pm->h_gave_up;
+    if (!*f) return NN_OK;
+    *f = 0;
+    return nn_fail(pm->ctx, NN_ERR_TIMEOUT, "k_cn_solve: a grid barrier gave up");
+}
+
 extern "C" nn_status nn_paracrine_ref_fine(nn_paracrine* pm, const nn_coupling* c)
 {
     if (!pm || !c || c->n != pm->n) return nn_fail(pm ? pm->ctx : nullptr, NN_ERR_INVALID_ARG, "nn_paracrine_ref_fine: bad argument");
+    NN_TRY(cn_gave_up(pm));
     if (pm->n == 0) return NN_OK;
     nn_ctx* ctx = pm->ctx;
     NN_CUDA(ctx, nn_launch_pdl(k_fine, dim3(nn_grid_for(ctx, pm->n, 256, 16)), dim3(256), 0, ctx->stream, pm->n, c->firing,
@@ -1142,6 +1166,7 @@ extern "C" nn_status nn_paracrine_ref_fine(nn_paracrine* pm, const nn_coupling* 
 extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* final_rr)
 {
     if (!pm) return NN_ERR_INVALID_ARG;
+    NN_TRY(cn_gave_up(pm));
     nn_ctx* ctx = pm->ctx;
     cudaStream_t s = ctx->stream;
     const auto& p = pm->p;
@@ -1178,6 +1203,8 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
     q.partials = pm->partials;
     q.bar = pm->bar;
     q.done = pm->done;
+    NN_CUDA(ctx, cudaHostGetDevicePointer((void**)&q.gave_up, pm->h_gave_up, 0));
+    q.polls = pm->polls;
     NN_CUDA(ctx, cudaMemsetAsync(pm->bar, 0, sizeof(unsigned), s));
     void* args[] = {&q};
     NN_CUDA(ctx, cudaLaunchCooperativeKernel(cn_kernel(G), dim3(pm->nparts), dim3(CN_THREADS), args, 0, s));
@@ -1189,7 +1216,7 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
         NN_CUDA(ctx, cudaMemsetAsync(pm->generated, 0, sizeof(float) * (size_t)pm->n, s));
     }
     if (std::getenv("NN_DEBUG_PARACRINE")) {
-        int h_done[3];
+        int h_done[2];
         double h_scal[3];
         std::vector<float> hu((size_t)G), hx((size_t)G), hax((size_t)G);
         cudaMemcpyAsync(h_done, pm->done, sizeof h_done, cudaMemcpyDeviceToHost, s);
@@ -1204,15 +1231,12 @@ extern "C" nn_status nn_paracrine_ref_own(nn_paracrine* pm, int* iters, float* f
                 h_done[0], h_done[1], h_scal[0], h_scal[1], h_scal[2], su, sx, sa);
     }
     if (iters || final_rr) {
-        int h_done[3];
+        int h_done[2];
         double h_scal[3];
         NN_CUDA(ctx, cudaMemcpyAsync(h_done, pm->done, sizeof h_done, cudaMemcpyDeviceToHost, s));
         NN_CUDA(ctx, cudaMemcpyAsync(h_scal, pm->scal, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
         NN_CUDA(ctx, cudaStreamSynchronize(s));
-        if (h_done[2]) {
-            NN_CUDA(ctx, cudaMemsetAsync(pm->done, 0, 3 * sizeof(int), s));
-            return nn_fail(ctx, NN_ERR_TIMEOUT, "k_cn_solve: a grid barrier gave up");
-        }
+        NN_TRY(cn_gave_up(pm));
         if (iters) *iters = h_done[1];
         if (final_rr) *final_rr = (float)(h_done[1] == 0 ? h_scal[0] : (h_done[0] == 1 ? h_scal[2] : h_scal[0]));
     }

@@ -11,6 +11,7 @@ import pytest
 import neuronephys_clean_gb300 as nn
 
 pytestmark = pytest.mark.gpu
+TIMEOUT = 6  # NN_ERR_TIMEOUT
 
 
 @pytest.mark.parametrize("shape", [(2, 2, 2), (3, 2, 7), (5, 31, 33), (9, 64, 97), (70, 80, 90)])
@@ -66,3 +67,31 @@ def test_cn_solve_blocks_per_sm(ctx, orc, shape):
     assert it == rit
     guess = u.max() * (1 + p.D * 256 / 30)
     assert np.abs(pm.density().astype(np.float64) - ref).max() <= 1e-5 * max(1.0, np.abs(ref).max(), guess)
+
+
+def test_cn_solve_reports_a_barrier_that_gave_up(ctx, monkeypatch):
+    """With no polls allowed the barrier's waits run out at once: a call that
+    reads the outcome reports it, one that does not leaves it to the module's
+    next update, each once; the density stays, and the context is usable."""
+    p = nn.ParacrineModule.default_params()
+    p.nx = p.ny = p.nz = 64
+    zero, g = ctx.to_device(np.zeros(1, np.float32)), ctx.empty((1,), np.float32)
+    monkeypatch.setenv("NN_CN_POLLS", "0")
+    pm = nn.ParacrineModule(ctx, g, 1, p, zero, zero, zero)
+    monkeypatch.delenv("NN_CN_POLLS")
+    u = np.random.default_rng(1).random(64 ** 3).astype(np.float32)
+    pm.set_density(u)
+    with pytest.raises(nn.NNError) as e:
+        pm.update_on_own_timescale()
+    assert e.value.status == TIMEOUT
+    own, fine = nn.lib().nn_paracrine_ref_own, nn.lib().nn_paracrine_ref_fine
+    cp = nn.AtomicCoupling(ctx, 1)
+    for later in (lambda: own(pm.handle, None, None), lambda: fine(pm.handle, cp.handle)):
+        assert own(pm.handle, None, None) == 0
+        ctx.synchronize()
+        assert later() == TIMEOUT
+    assert fine(pm.handle, cp.handle) == 0
+    assert np.array_equal(pm.density(), u)
+    ok = nn.ParacrineModule(ctx, g, 1, p, zero, zero, zero)
+    ok.set_density(u)
+    assert ok.update_on_own_timescale()[0] > 0
