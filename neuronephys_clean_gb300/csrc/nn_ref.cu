@@ -446,60 +446,89 @@ __global__ void __launch_bounds__(CMP_THREADS) k_cmp_count_zero(const float* out
     }
 }
 
-// The second launch, a block per sub-tile: the sub-tile's offset in the
-// ascending firing list (the earlier tiles' counts and the tile's own before
-// it), its entries written, the total stored by the last block, and its firing
-// neurons scattered (signal_spikes_kernel), a warp per firing neuron with four
-// targets per lane loaded before their reductions.  With a block per tile of
-// 2,048 neurons a network of 14,638 neurons had 8 blocks whose warps scattered
-// up to a dozen rows each in turn: 38 us, with 115 blocks 7.6 us.  A million
-// neurons went from 84 to 67 us, where the L2 reductions set the time.
+// The second launch, a block for per_block consecutive stretches of SUB neurons:
+// the stretch's offset in the ascending firing list (the earlier tiles' counts
+// and the tile's own before it; later stretches go on from there), its entries
+// written, the total stored by the last one, and its firing neurons scattered
+// (signal_spikes_kernel), a warp per firing neuron with four targets per lane
+// loaded before their reductions.
+// Short stretches spread the scatter: with 2,048 neurons a block a network of
+// 14,638 had 8 blocks whose warps scattered up to a dozen rows each in turn, 38
+// us; with 128 115 blocks and 7.6 us.  Long ones save the fixed cost of a block.
+// us of the two launches at 2 % firing with 10 targets / 50 % with 100, SUB = 128
+// and 512: 300k neurons 8.4 / 82 and 7.6 / 119, 1M 18 / 240 and 11 / 254, 4M 60 /
+// 912 and 28 / 931 (2,048: 39 / 1002).  So 512 from five waves of blocks of 128
+// on.  The offset's sum costs more than the stretch from some 64 blocks an SM on:
+// 16M neurons 152 us with a stretch a block, 133 with three.
+template <int SUB>
 __global__ void __launch_bounds__(CMP_THREADS) k_cmp_write_push(const float* out, int n, const int64_t* block_counts,
-                                                                const int* sub_before, int* list, int* count,
+                                                                const int* sub_before, int per_block, int* list, int* count,
                                                                 const int* indices, const int* offsets, float* inputs,
                                                                 int signal_mode)
 {
     __shared__ int64_t red[CMP_THREADS / 32];
-    __shared__ int s_list[CMP_SUB];
-    __shared__ int wt[CMP_SUB / 32];
+    __shared__ int s_list[SUB];
+    __shared__ int wt[SUB / 32];
     nn_grid_dep_launch();
     nn_grid_dep_wait();
+    constexpr int ITEMS = SUB < CMP_THREADS ? 1 : SUB / CMP_THREADS, WARPS = CMP_THREADS / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int i = blockIdx.x * CMP_SUB + threadIdx.x;
-    const bool f = threadIdx.x < CMP_SUB && i < n && fires(out[i]);
-    const unsigned b = __ballot_sync(0xffffffffu, f);
-    if (w < CMP_SUB / 32 && lane == 0) wt[w] = __popc(b);
-    const int tile = blockIdx.x / CMP_SUBS;
-    int64_t acc = 0;
-    for (int q = threadIdx.x; q < tile; q += CMP_THREADS) acc += block_counts[q];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) red[w] = acc;
-    __syncthreads();
-    int64_t boff = sub_before[blockIdx.x];
-    for (int q = 0; q < CMP_THREADS / 32; ++q) boff += red[q];
-    int nf = 0, pos = __popc(b & ((1u << lane) - 1u));
-    for (int q = 0; q < CMP_SUB / 32; ++q) {
-        if (q < w) pos += wt[q];
-        nf += wt[q];
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count = (int)(boff + nf);
-    if (f) {
-        list[boff + pos] = i;
-        s_list[pos] = i;
-    }
-    __syncthreads();
-    for (int k = w; k < nf; k += CMP_THREADS / 32) {
-        const int pre = s_list[k];
-        const float sig = signal_mode ? out[pre] : 1.0f;
-        const int beg = offsets[pre], end = offsets[pre + 1];
-        for (int e0 = beg + lane; e0 < end; e0 += 128) {
-            int post[4];
+    const int subs = (n - 1) / SUB + 1;
+    int64_t boff = 0;
+    for (int s = blockIdx.x * per_block; s < min((int)(blockIdx.x + 1) * per_block, subs); ++s) {
+        bool f[ITEMS];
+        unsigned b[ITEMS];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) post[u] = e0 + 32 * u < end ? indices[e0 + 32 * u] : -1;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if ((unsigned)post[u] < (unsigned)n) atomicAdd(inputs + post[u], sig);
+        for (int q = 0; q < ITEMS; ++q) {
+            const int i = s * SUB + q * CMP_THREADS + (int)threadIdx.x;
+            f[q] = threadIdx.x < SUB && i < n && fires(out[i]);
+            b[q] = __ballot_sync(0xffffffffu, f[q]);
+            if (q * WARPS + w < SUB / 32 && lane == 0) wt[q * WARPS + w] = __popc(b[q]);
         }
+        if (s == (int)blockIdx.x * per_block) {
+            const int tile = (int)((int64_t)s * SUB / CMP_TILE);
+            int64_t acc = 0;
+            for (int q = threadIdx.x; q < tile; q += CMP_THREADS) acc += block_counts[q];
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) red[w] = acc;
+            __syncthreads();
+            boff = sub_before[s * (SUB / CMP_SUB)];
+            for (int q = 0; q < WARPS; ++q) boff += red[q];
+        } else {
+            __syncthreads();
+        }
+        int nf = 0, before[ITEMS] = {};
+#pragma unroll
+        for (int q = 0; q < SUB / 32; ++q) {
+#pragma unroll
+            for (int r = 0; r < ITEMS; ++r)
+                if (q < r * WARPS + w) before[r] += wt[q];
+            nf += wt[q];
+        }
+        if (s == subs - 1 && threadIdx.x == 0) *count = (int)(boff + nf);
+#pragma unroll
+        for (int q = 0; q < ITEMS; ++q)
+            if (f[q]) {
+                const int pos = before[q] + __popc(b[q] & ((1u << lane) - 1u)), i = s * SUB + q * CMP_THREADS + (int)threadIdx.x;
+                list[boff + pos] = i;
+                s_list[pos] = i;
+            }
+        boff += nf;
+        __syncthreads();
+        for (int k = w; k < nf; k += CMP_THREADS / 32) {
+            const int pre = s_list[k];
+            const float sig = signal_mode ? out[pre] : 1.0f;
+            const int beg = offsets[pre], end = offsets[pre + 1];
+            for (int e0 = beg + lane; e0 < end; e0 += 128) {
+                int post[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) post[u] = e0 + 32 * u < end ? indices[e0 + 32 * u] : -1;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if ((unsigned)post[u] < (unsigned)n) atomicAdd(inputs + post[u], sig);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -597,10 +626,11 @@ extern "C" nn_status nn_coupling_run(nn_coupling* c, const int* d_indices, const
     NN_CUDA(ctx, nn_launch_pdl(k_cmp_count_zero, dim3(c->nblocks), dim3(CMP_THREADS), 0, ctx->stream, d_outputs, c->n,
                                c->block_counts, c->sub_before, d_inputs));
     NN_CHECK_LAUNCH(ctx, "k_cmp_count_zero");
-    const int subs = (c->n - 1) / CMP_SUB + 1;
-    NN_CUDA(ctx, nn_launch_pdl(k_cmp_write_push, dim3(subs), dim3(CMP_THREADS), 0, ctx->stream, d_outputs, c->n,
-                               c->block_counts, c->sub_before, c->firing, c->count, d_indices, d_offsets, d_inputs,
-                               signal_mode));
+    const bool many = c->n > 5 * 8 * ctx->num_sms * CMP_SUB;
+    const int subs = (c->n - 1) / (many ? 512 : CMP_SUB) + 1, per_block = std::max(1, subs / (64 * ctx->num_sms));
+    NN_CUDA(ctx, nn_launch_pdl(many ? k_cmp_write_push<512> : k_cmp_write_push<CMP_SUB>, dim3((subs - 1) / per_block + 1),
+                               dim3(CMP_THREADS), 0, ctx->stream, d_outputs, c->n, c->block_counts, c->sub_before,
+                               per_block, c->firing, c->count, d_indices, d_offsets, d_inputs, signal_mode));
     NN_CHECK_LAUNCH(ctx, "k_cmp_write_push");
     return coupling_readback(c, num_firing);
 }

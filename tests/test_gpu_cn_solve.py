@@ -95,3 +95,20 @@ def test_cn_solve_reports_a_barrier_that_gave_up(ctx, monkeypatch):
     ok = nn.ParacrineModule(ctx, g, 1, p, zero, zero, zero)
     ok.set_density(u)
     assert ok.update_on_own_timescale()[0] > 0
+
+
+@pytest.mark.parametrize("n", [778_240, 778_241, 1_000_003, 10_100_001])
+@pytest.mark.parametrize("frac", [0.01, 1.0])
+def test_coupling_scatter_of_many_neurons(ctx, orc, n, frac):
+    """Longer stretches a block, and several of them; whole counts, equal."""
+    rng = np.random.default_rng(n)
+    off = np.concatenate([[0], np.cumsum(rng.integers(0, 4, n))]).astype(np.int32)
+    idx = rng.integers(0, n, int(off[-1])).astype(np.int32)
+    out = np.where(rng.random(n) < frac, 0.5, 0.05).astype(np.float32)
+    cp = nn.AtomicCoupling(ctx, n)
+    ins = ctx.to_device(np.full(n, 7.0, np.float32))
+    nf = cp(nn.AdjacencyList(ctx.to_device(idx), ctx.to_device(off)), ins, ctx.to_device(out))
+    rnf, rin, rfire = orc.coupling_push(idx, off, out, nn.NN_SIGNAL_COUNT)
+    assert nf == rnf
+    assert np.array_equal(ins.numpy(), rin)
+    assert np.array_equal(cp.get_firing_neurons()[:nf], rfire)
