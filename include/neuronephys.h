@@ -465,7 +465,8 @@ NN_API nn_status nn_bpcg_solve(nn_bpcg* bp, const float* d_b, float* d_x, double
 /* Block-size autotuner: times iterations with 512, 1,024, 2,048 and 4,096
  * cells per block (2, 4, 8, 16 per thread) on the batch's own operators,
  * right-hand side d_b and d_x as scratch (overwritten), and keeps the fastest
- * layout for later solves. */
+ * layout for later solves.  A batch that is solved on the chip in one launch
+ * has no such layout: the set value stays, *ms_per_iter is its iteration time. */
 NN_API nn_status nn_bpcg_autotune(nn_bpcg* bp, const float* d_b, float* d_x, int trial_iters, int* cells_per_block,
                                   float* ms_per_iter);
 /* Fix the block layout instead: 512, 1024, 2048 (the default) or 4096 cells per block. */

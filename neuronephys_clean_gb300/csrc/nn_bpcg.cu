@@ -1,9 +1,10 @@
-// Batches whose instances fit on the chip (sides up to about 130) are solved
-// by the resident kernel of nn_rcg.cu, all instances in one launch.  With two
-// launches an iteration over all cells, 24 networks of 120k neurons in all with
-// grids of 32^3 to 51^3 took 1,277 us a period of 100 steps and its solve, with
-// the resident kernel 811.  The rest of this file serves larger instances and
-// the block-size autotuner.
+// Batches whose instances fit on the chip (sides up to 128) are solved by the
+// resident kernel of nn_rcg.cu, all instances in one launch.  With two launches
+// an iteration over all cells, 24 networks of 120k neurons in all with grids of
+// 32^3 to 51^3 took 1,277 us a period of 100 steps and its solve, with the
+// resident kernel 811.  The rest of this file serves larger instances, and all
+// with NN_PCG_TWO_KERNEL set in the environment; its tables and vectors are
+// allocated where it runs.
 //
 // Batched Jacobi-PCG: many independent cubic 7-point backward-Euler systems
 // (one per network instance of a batch, each with its own side g_b and
@@ -26,6 +27,7 @@
 // its launch.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <vector>
 
 #include "nn_internal.cuh"
@@ -331,6 +333,10 @@ extern "C" nn_status nn_bpcg_destroy(nn_bpcg* bp)
 static nn_status set_layout(nn_bpcg* bp, int vpt)
 {
     nn_ctx* ctx = bp->ctx;
+    if (bp->res) {  // no solve uses it
+        bp->vpt = vpt;
+        return NN_OK;
+    }
     const int64_t cpb = (int64_t)BT * vpt;
     std::vector<int> first((size_t)bp->n_inst + 1, 0), binst;
     for (int b = 0; b < bp->n_inst; ++b) {
@@ -345,6 +351,40 @@ static nn_status set_layout(nn_bpcg* bp, int vpt)
     bp->nblocks = first.back();
     bp->h_first = first;
     return NN_OK;
+}
+
+// Tables and vectors of the two-launch iteration.
+static nn_status two_kernel_tables(nn_bpcg* bp, const std::vector<float>& al, const std::vector<float>& iv)
+{
+    nn_ctx* ctx = bp->ctx;
+    const int n_inst = bp->n_inst;
+    const size_t G = (size_t)bp->G;
+    nn_status st = NN_OK;
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->side, (size_t)n_inst);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->off, (size_t)n_inst + 1);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->alpha, (size_t)n_inst);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->invd, (size_t)n_inst);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->blk_inst, (size_t)bp->max_blocks);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->blk_first, (size_t)n_inst + 1);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->work, (size_t)bp->max_blocks);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->flags, (size_t)n_inst);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->iters, (size_t)n_inst);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->running, 1);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->scal, (size_t)n_inst * S_COUNT);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->partials, (size_t)3 * bp->max_blocks);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->ticket, (size_t)n_inst);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->r, G);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->p0, G);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->p1, G);
+    if (st == NN_OK) st = nn_alloc(ctx, &bp->Ap, G);
+    if (st == NN_OK) st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->side, bp->h_side.data(), sizeof(int) * n_inst, cudaMemcpyHostToDevice), "copy");
+    if (st == NN_OK)
+        st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->off, bp->h_off.data(), sizeof(int64_t) * (n_inst + 1), cudaMemcpyHostToDevice), "copy");
+    if (st == NN_OK) st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->alpha, al.data(), sizeof(float) * n_inst, cudaMemcpyHostToDevice), "copy");
+    if (st == NN_OK) st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->invd, iv.data(), sizeof(float) * n_inst, cudaMemcpyHostToDevice), "copy");
+    if (st == NN_OK) st = set_layout(bp, 8);
+    if (st == NN_OK) st = nn_cuda_check(ctx, nn_zero_async(ctx, bp->ticket, sizeof(unsigned int) * n_inst), "memset");
+    return st;
 }
 
 // sides[b] >= 1; alpha_b = alpha_unit * side_b^2 (alpha_unit = dt D on the unit cube)
@@ -376,37 +416,13 @@ extern "C" nn_status nn_bpcg_create(nn_ctx* ctx, int n_inst, const int* h_sides,
     bp->G = bp->h_off.back();
     bp->onepb = (float)(1.0 + beta);
     nn_status st = NN_OK;
-    const size_t G = (size_t)bp->G;
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->side, (size_t)n_inst);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->off, (size_t)n_inst + 1);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->alpha, (size_t)n_inst);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->invd, (size_t)n_inst);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->blk_inst, (size_t)bp->max_blocks);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->blk_first, (size_t)n_inst + 1);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->work, (size_t)bp->max_blocks);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->flags, (size_t)n_inst);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->iters, (size_t)n_inst);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->running, 1);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->scal, (size_t)n_inst * S_COUNT);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->partials, (size_t)3 * bp->max_blocks);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->ticket, (size_t)n_inst);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->r, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->p0, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->p1, G);
-    if (st == NN_OK) st = nn_alloc(ctx, &bp->Ap, G);
-    if (st == NN_OK) st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->side, h_sides, sizeof(int) * n_inst, cudaMemcpyHostToDevice), "copy");
-    if (st == NN_OK)
-        st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->off, bp->h_off.data(), sizeof(int64_t) * (n_inst + 1), cudaMemcpyHostToDevice), "copy");
-    if (st == NN_OK) st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->alpha, al.data(), sizeof(float) * n_inst, cudaMemcpyHostToDevice), "copy");
-    if (st == NN_OK) st = nn_cuda_check(ctx, nn_copy_sync(ctx, bp->invd, iv.data(), sizeof(float) * n_inst, cudaMemcpyHostToDevice), "copy");
-    if (st == NN_OK) st = set_layout(bp, 8);
-    if (st == NN_OK) st = nn_cuda_check(ctx, nn_zero_async(ctx, bp->ticket, sizeof(unsigned int) * n_inst), "memset");
+    if (!std::getenv("NN_PCG_TWO_KERNEL")) {
+        st = nn_rcg_batch_create(ctx, n_inst, h_sides, bp->h_off.data(), alpha_unit, beta, &bp->res);
+        if (st == NN_ERR_UNSUPPORTED) st = NN_OK;
+    }
+    if (st == NN_OK && !bp->res) st = two_kernel_tables(bp, al, iv);
     if (st == NN_OK) st = nn_cuda_check(ctx, cudaEventCreate(&bp->ev0), "event");
     if (st == NN_OK) st = nn_cuda_check(ctx, cudaEventCreate(&bp->ev1), "event");
-    if (st == NN_OK) {
-        const nn_status rs = nn_rcg_batch_create(ctx, n_inst, h_sides, bp->h_off.data(), alpha_unit, beta, &bp->res);
-        if (rs != NN_OK && rs != NN_ERR_UNSUPPORTED) st = rs;
-    }
     if (st != NN_OK) {
         nn_bpcg_destroy(bp);
         return st;
@@ -636,11 +652,21 @@ extern "C" nn_status nn_bpcg_autotune(nn_bpcg* bp, const float* d_b, float* d_x,
     nn_ctx* ctx = bp->ctx;
     if (bp->as_active) return nn_fail(ctx, NN_ERR_INVALID_ARG, "nn_bpcg_autotune: a solve is pending");
     cudaStream_t cs = ctx->stream;
+    const int vpt0 = bp->vpt;
+    const bool timing0 = bp->timing;
+    if (bp->res) {  // one form: its time
+        int n = 0;
+        NN_CUDA(ctx, cudaMemsetAsync(d_x, 0, sizeof(float) * (size_t)bp->G, cs));
+        bp->timing = true;
+        const nn_status st = nn_bpcg_solve(bp, d_b, d_x, 1e-30, iters, nullptr, &n, nullptr);
+        bp->timing = timing0;
+        if (cells_per_block) *cells_per_block = BT * bp->vpt;
+        if (ms_per_iter) *ms_per_iter = n > 0 ? bp->last_ms / n : 0.0f;
+        return st;
+    }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     NN_CUDA(ctx, cudaEventCreate(&e0));
     NN_CUDA(ctx, cudaEventCreate(&e1));
-    const int vpt0 = bp->vpt;
-    const bool timing0 = bp->timing;
     bp->timing = false;
     int best_vpt = vpt0;
     float best = 1e30f;

@@ -44,6 +44,7 @@
 // another, so the launch is cooperative; every poll is bounded.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <map>
 
 #include "nn_hh.cuh"
@@ -934,24 +935,16 @@ struct nn_rcg_batch {
     const void* kernel = nullptr;
     size_t smem = 0;
     RcgBatchArgs B{};
-    RcgArgs* inst = nullptr;
-    int64_t* off = nullptr;
-    int2* block = nullptr;
-    RcgGroup* group = nullptr;
-    int* list = nullptr;
-    ulonglong2* rec = nullptr;
-    Tagged4* halo = nullptr;
-    float4* xw = nullptr;
-    size_t n_rec = 0, n_halo = 0, groups = 0;
+    // everything in one allocation; the first `zero` bytes hold the tagged words
+    unsigned char* mem = nullptr;
+    size_t zero = 0;
 };
 
 void nn_rcg_batch_destroy(nn_rcg_batch* pl)
 {
     if (!pl) return;
     if (pl->ctx) cudaStreamSynchronize(pl->ctx->stream);
-    nn_release(pl->inst); nn_release(pl->off); nn_release(pl->block); nn_release(pl->group); nn_release(pl->list);
-    nn_release(pl->rec); nn_release(pl->halo); nn_release(pl->xw);
-    nn_release(pl->B.start); nn_release(pl->B.epoch); nn_release(pl->B.scal); nn_release(pl->B.flags);
+    nn_release(pl->mem);
     nn_ctx* ctx = pl->ctx;
     delete pl;
     nn_ctx_release(ctx);
@@ -959,10 +952,7 @@ void nn_rcg_batch_destroy(nn_rcg_batch* pl)
 
 static nn_status batch_reset(nn_rcg_batch* pl, cudaStream_t cs)
 {
-    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->rec, 0, sizeof(ulonglong2) * pl->n_rec, cs));
-    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->halo, 0, sizeof(Tagged4) * pl->n_halo, cs));
-    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->B.start, 0, sizeof(ulonglong2) * 2 * (size_t)pl->blocks, cs));
-    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->B.epoch, 0, sizeof(unsigned) * pl->groups, cs));
+    NN_CUDA(pl->ctx, cudaMemsetAsync(pl->mem, 0, pl->zero, cs));
     pl->B.seq = 1;
     return NN_OK;
 }
@@ -983,23 +973,27 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
         RcgArgs a{};
         size_t smem = 0;
     };
-    std::map<std::pair<int, int>, Shape> shapes;  // (side, blocks)
-    auto shape = [&](int side, int width) -> const Shape& {
-        Shape& s = shapes[{side, width}];
-        if (s.cost == 0.0) {
+    static const int widths[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 14, 16, 19, 22, 25, 30, 38, 50, 76, 152};
+    constexpr int W = sizeof widths / sizeof *widths;
+    std::map<int, std::vector<Shape>> table;  // by side: a shape a width
+    for (int b = 0; b < n_inst; ++b) table[sides[b]];
+    for (auto& e : table) {
+        e.second.resize(W);
+        for (int w = 0; w < W; ++w) {
+            Shape& s = e.second[(size_t)w];
             int threads = 0;
-            s.a.nx = s.a.ny = s.a.nz = side;
-            s.cost = rcg_shape(width, false, true, s.a, threads, s.smem) * side;
+            s.a.nx = s.a.ny = s.a.nz = e.first;
+            if (widths[w] <= sms) s.cost = rcg_shape(widths[w], false, true, s.a, threads, s.smem) * e.first;
             if (s.cost == 0.0) s.cost = -1.0;
         }
-        return s;
-    };
-    static const int widths[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 14, 16, 19, 22, 25, 30, 38, 50, 76, 152};
+    }
+    std::vector<const std::vector<Shape>*> shape((size_t)n_inst);
+    for (int b = 0; b < n_inst; ++b) shape[(size_t)b] = &table[sides[b]];
     std::vector<int> order((size_t)n_inst);
     for (int b = 0; b < n_inst; ++b) order[(size_t)b] = b;
     std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return sides[p] > sides[q]; });
     struct Column {
-        int width;
+        int w;  // of widths
         double height;
         std::vector<int> list;
     };
@@ -1008,21 +1002,21 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
         cols.clear();
         int used = 0;
         for (int b : order) {
+            const std::vector<Shape>& s = *shape[(size_t)b];
             Column* best = nullptr;
             double left = 0.0;
             for (Column& c : cols) {
-                const double cost = shape(sides[b], c.width).cost, rest = bound - c.height - cost;
+                const double cost = s[(size_t)c.w].cost, rest = bound - c.height - cost;
                 if (cost > 0.0 && rest >= 0.0 && (!best || rest < left)) {
                     best = &c;
                     left = rest;
                 }
             }
             if (!best) {
-                for (int w : widths) {
-                    if (w > sms - used) return false;
-                    const double cost = shape(sides[b], w).cost;
-                    if (cost > 0.0 && cost <= bound) {
-                        used += w;
+                for (int w = 0; w < W; ++w) {
+                    if (widths[w] > sms - used) return false;
+                    if (s[(size_t)w].cost > 0.0 && s[(size_t)w].cost <= bound) {
+                        used += widths[w];
                         cols.push_back({w, 0.0, {}});
                         best = &cols.back();
                         break;
@@ -1030,14 +1024,15 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
                 }
                 if (!best) return false;
             }
-            best->height += shape(sides[b], best->width).cost;
+            best->height += s[(size_t)best->w].cost;
             best->list.push_back(b);
         }
         return true;
     };
     double hi = 0.0;
     for (int b : order) {
-        const double c = shape(sides[b], widths[18] <= sms ? widths[18] : 76).cost;
+        const std::vector<Shape>& s = *shape[(size_t)b];
+        const double c = s[(size_t)(widths[W - 1] <= sms ? W - 1 : W - 2)].cost;
         if (c <= 0.0) return NN_ERR_UNSUPPORTED;
         hi += c;
     }
@@ -1053,18 +1048,18 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
     pl->ctx = ctx;
     nn_ctx_retain(ctx);
     pl->n_inst = n_inst;
-    pl->groups = cols.size();
     std::vector<RcgArgs> inst((size_t)n_inst);
     std::vector<RcgGroup> group;
     std::vector<int2> block;
     std::vector<int> list;
     int nz = 1;
-    size_t n_xw = 0;
+    size_t n_rec = 0, n_halo = 0, n_xw = 0;
     for (const Column& c : cols) {
-        RcgGroup g{(int)list.size(), (int)c.list.size(), c.width, (int64_t)pl->n_rec, (int64_t)pl->n_halo, (int64_t)n_xw};
+        const int width = widths[c.w];
+        RcgGroup g{(int)list.size(), (int)c.list.size(), width, (int64_t)n_rec, (int64_t)n_halo, (int64_t)n_xw};
         size_t halo = 0, xw = 0;
         for (int b : c.list) {
-            const Shape& s = shape(sides[b], c.width);
+            const Shape& s = (*shape[(size_t)b])[(size_t)c.w];
             RcgArgs a = s.a;
             rcg_operator(a, alpha_unit * sides[b] * sides[b], beta, false);
             nz = std::max(nz, a.bz);
@@ -1074,9 +1069,9 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
             inst[(size_t)b] = a;
             list.push_back(b);
         }
-        for (int r = 0; r < c.width; ++r) block.push_back({(int)group.size(), r});
-        pl->n_rec += 8 * (size_t)c.width;
-        pl->n_halo += halo;
+        for (int r = 0; r < width; ++r) block.push_back({(int)group.size(), r});
+        n_rec += 8 * (size_t)width;
+        n_halo += halo;
         n_xw += xw;
         pl->longest = std::max(pl->longest, g.count);
         group.push_back(g);
@@ -1084,35 +1079,49 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
     pl->blocks = (int)block.size();
     pl->kernel = batch_kernel_of(nz);
     const size_t N = (size_t)n_inst;
-    nn_status st = nn_alloc(ctx, &pl->rec, pl->n_rec);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->halo, pl->n_halo);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->xw, n_xw);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->inst, N);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->off, N);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->block, block.size());
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->group, group.size());
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->list, list.size());
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.start, 2 * (size_t)pl->blocks);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.epoch, group.size());
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.scal, 2 * N);
-    if (st == NN_OK) st = nn_alloc(ctx, &pl->B.flags, 4 * N);
-    if (st == NN_OK)
-        for (const RcgGroup& g : group)
-            for (int k = 0; k < g.count; ++k) {
-                RcgArgs& a = inst[(size_t)list[(size_t)(g.first + k)]];
-                a.rec = pl->rec + g.rec;
-                a.halo = pl->halo + g.halo;
-                a.xw = pl->xw + g.xw;
-            }
-    auto put = [&](void* d, const void* h, size_t bytes) {
-        if (st == NN_OK)
-            st = nn_cuda_check(ctx, cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ctx->stream), "copy");
+    size_t bytes = 0;
+    auto part = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
     };
-    put(pl->inst, inst.data(), sizeof(RcgArgs) * N);
-    put(pl->off, off, sizeof(int64_t) * N);
-    put(pl->block, block.data(), sizeof(int2) * block.size());
-    put(pl->group, group.data(), sizeof(RcgGroup) * group.size());
-    put(pl->list, list.data(), sizeof(int) * list.size());
+    const size_t o_rec = part(sizeof(ulonglong2) * n_rec), o_halo = part(sizeof(Tagged4) * n_halo);
+    const size_t o_start = part(sizeof(ulonglong2) * 2 * block.size()), o_epoch = part(sizeof(unsigned) * group.size());
+    pl->zero = bytes;
+    const size_t o_xw = part(sizeof(float4) * n_xw), o_scal = part(sizeof(double) * 2 * N), o_flags = part(sizeof(int) * 4 * N);
+    const size_t o_inst = part(sizeof(RcgArgs) * N), o_off = part(sizeof(int64_t) * N);
+    const size_t o_block = part(sizeof(int2) * block.size()), o_group = part(sizeof(RcgGroup) * group.size());
+    const size_t o_list = part(sizeof(int) * list.size());
+    nn_status st = nn_alloc(ctx, &pl->mem, bytes);
+    if (st != NN_OK) {
+        nn_rcg_batch_destroy(pl);
+        return st;
+    }
+    auto at = [&](size_t o) { return (void*)(pl->mem + o); };
+    for (const RcgGroup& g : group)
+        for (int k = 0; k < g.count; ++k) {
+            RcgArgs& a = inst[(size_t)list[(size_t)(g.first + k)]];
+            a.rec = (ulonglong2*)at(o_rec) + g.rec;
+            a.halo = (Tagged4*)at(o_halo) + g.halo;
+            a.xw = (float4*)at(o_xw) + g.xw;
+        }
+    pl->B.inst = (const RcgArgs*)at(o_inst);
+    pl->B.off = (const int64_t*)at(o_off);
+    pl->B.block = (const int2*)at(o_block);
+    pl->B.group = (const RcgGroup*)at(o_group);
+    pl->B.list = (const int*)at(o_list);
+    pl->B.start = (ulonglong2*)at(o_start);
+    pl->B.epoch = (unsigned*)at(o_epoch);
+    pl->B.scal = (double*)at(o_scal);
+    pl->B.flags = (int*)at(o_flags);
+    std::vector<unsigned char> host(bytes - o_inst);
+    auto put = [&](size_t o, const void* h, size_t n) { std::memcpy(host.data() + (o - o_inst), h, n); };
+    put(o_inst, inst.data(), sizeof(RcgArgs) * N);
+    put(o_off, off, sizeof(int64_t) * N);
+    put(o_block, block.data(), sizeof(int2) * block.size());
+    put(o_group, group.data(), sizeof(RcgGroup) * group.size());
+    put(o_list, list.data(), sizeof(int) * list.size());
+    st = nn_cuda_check(ctx, cudaMemcpyAsync(at(o_inst), host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream), "copy");
     if (st == NN_OK) st = batch_reset(pl, ctx->stream);
     int coop = 0, per_sm = 0;
     if (st == NN_OK)
@@ -1130,11 +1139,6 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
         nn_rcg_batch_destroy(pl);
         return st;
     }
-    pl->B.inst = pl->inst;
-    pl->B.off = pl->off;
-    pl->B.block = pl->block;
-    pl->B.group = pl->group;
-    pl->B.list = pl->list;
     *out = pl;
     return NN_OK;
 }
