@@ -2,9 +2,10 @@
 // resident kernel of nn_rcg.cu, all instances in one launch.  With two launches
 // an iteration over all cells, 24 networks of 120k neurons in all with grids of
 // 32^3 to 51^3 took 1,277 us a period of 100 steps and its solve, with the
-// resident kernel 811.  The rest of this file serves larger instances, and all
-// with NN_PCG_TWO_KERNEL set in the environment; its tables and vectors are
-// allocated where it runs.
+// resident kernel 811.  The rest of this file serves larger instances, batches of
+// hundreds of small ones (the rule is at nn_rcg_batch_create), and all with
+// NN_PCG_TWO_KERNEL set in the environment; its tables and vectors are allocated
+// where it runs.
 //
 // Batched Jacobi-PCG: many independent cubic 7-point backward-Euler systems
 // (one per network instance of a batch, each with its own side g_b and

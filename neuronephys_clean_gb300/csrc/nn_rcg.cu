@@ -962,7 +962,22 @@ static nn_status batch_reset(nn_rcg_batch* pl, cudaStream_t cs)
 // the least bound for which the columns fit the chip, by bisection.  An
 // instance's estimate is the cycles of an iteration on the column's blocks
 // times its side, to which its iterations are about proportional.
-// NN_ERR_UNSUPPORTED when an instance does not fit.
+//
+// NN_ERR_UNSUPPORTED when an instance does not fit, and for batches of so many
+// small instances that the two launches an iteration of nn_bpcg.cu are faster: a
+// block goes through its list one solve after another, each iteration with an
+// exchange of about 3 us, while those launches work on all instances at once.
+// Both times are estimated, in us and with as many iterations as the side (they
+// are proportional to it in both): here the list's cycles, 5,500 more an
+// iteration, and 12 us an instance; there 17 us an iteration, 14.5 ps a cell
+// (instances in whole blocks of 2,048 cells), and 100 us.  The estimates agree
+// with measured times to 30 %, so the resident form has to be 1.25 times as fast
+// by them.  Measured, resident / two launches, us: 300 of 8^3 192 / 310, 600 of
+// 8^3 356 / 334, 5000 of 8^3 2726 / 1051, 100 of 16^3 204 / 405, 600 of 16^3 1104 /
+// 659, 300 of 24^3 1094 / 1290, 600 of 32^3 4568 / 7145, 256 of 64^3 22366 / 45362.
+constexpr double EST_CYCLES_US = 1900.0, EST_EXCHANGE = 5500.0, EST_SOLVE_US = 12.0;
+constexpr double EST_TWO_US = 17.0, EST_TWO_CELL_US = 14.5e-6, EST_TWO_SOLVE_US = 100.0, EST_MARGIN = 1.25;
+
 nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const int64_t* off, double alpha_unit,
                               double beta, nn_rcg_batch** out)
 {
@@ -987,8 +1002,27 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
             if (s.cost == 0.0) s.cost = -1.0;
         }
     }
+    // the two-launch form's time; what one list would take that was spread over
+    // the chip, at the least, answers for most batches without packing
+    auto us = [](double cost, int side) { return (cost + EST_EXCHANGE * side) / EST_CYCLES_US + EST_SOLVE_US; };
+    double two = EST_TWO_SOLVE_US + EST_TWO_US * table.rbegin()->first, least = 0.0;
+    std::map<int, double> share;  // by side: blocks times time, over the chip
+    for (const auto& e : table) {
+        double s = 0.0;
+        for (int w = 0; w < W; ++w) {
+            const double c = e.second[(size_t)w].cost;
+            if (c > 0.0 && (s == 0.0 || widths[w] * us(c, e.first) < s)) s = widths[w] * us(c, e.first);
+        }
+        share[e.first] = s / sms;
+    }
     std::vector<const std::vector<Shape>*> shape((size_t)n_inst);
-    for (int b = 0; b < n_inst; ++b) shape[(size_t)b] = &table[sides[b]];
+    for (int b = 0; b < n_inst; ++b) {
+        const double g = sides[b];
+        shape[(size_t)b] = &table[sides[b]];
+        two += g * std::ceil(g * g * g / 2048.0) * 2048.0 * EST_TWO_CELL_US;
+        least += share[sides[b]];
+    }
+    if (EST_MARGIN * least > two) return NN_ERR_UNSUPPORTED;
     std::vector<int> order((size_t)n_inst);
     for (int b = 0; b < n_inst; ++b) order[(size_t)b] = b;
     std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return sides[p] > sides[q]; });
@@ -1043,6 +1077,11 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
         (pack(mid) ? hi : lo) = mid;
     }
     if (!pack(hi)) return NN_ERR_UNSUPPORTED;
+    for (const Column& c : cols) {
+        double t = 0.0;
+        for (int b : c.list) t += us((*shape[(size_t)b])[(size_t)c.w].cost, sides[b]);
+        if (EST_MARGIN * t > two) return NN_ERR_UNSUPPORTED;
+    }
 
     nn_rcg_batch* pl = new nn_rcg_batch();
     pl->ctx = ctx;

@@ -65,6 +65,15 @@ def test_side_beyond_the_resident_solve(ctx, orc):
     _check(ctx, orc, nn.BatchedPCG(ctx, sides, unit, beta), sides, unit, beta, False)
 
 
+@pytest.mark.parametrize("sides,resident", [([8] * 300, True), ([8] * 1000, False), ([16] * 100, True),
+                                            ([16] * 600, False), ([24] * 60, True), ([64] * 2 + [9] * 50, True),
+                                            ([20] * 8 + [2] * 9000, False)])
+def test_batches_of_many_small_instances(ctx, orc, sides, resident):
+    unit, beta = 1e-3, 1e-4
+    n = len(sides)
+    _check(ctx, orc, nn.BatchedPCG(ctx, sides, unit, beta), sides, unit, beta, resident, {0, 1, n // 2, n - 1})
+
+
 def test_resident_batch_holds_no_vectors(ctx):
     """A resident batch keeps buffers of the chip's size (x in use, and faces of
     32 bytes a quad, twice: some 25 MB), not the four vectors of all instances
