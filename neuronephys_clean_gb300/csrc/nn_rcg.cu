@@ -1070,6 +1070,7 @@ nn_status nn_rcg_batch_create(nn_ctx* ctx, int n_inst, const int* sides, const i
         if (c <= 0.0) return NN_ERR_UNSUPPORTED;
         hi += c;
     }
+    hi *= 1.0 + 1e-9;  // (the sum of a column's costs in another order)
     double lo = 0.0;
     if (!pack(hi)) return NN_ERR_UNSUPPORTED;
     for (int q = 0; q < 14; ++q) {

@@ -67,8 +67,9 @@ def test_side_beyond_the_resident_solve(ctx, orc):
 
 @pytest.mark.parametrize("sides,resident", [([8] * 300, True), ([8] * 1000, False), ([16] * 100, True),
                                             ([16] * 600, False), ([24] * 60, True), ([64] * 2 + [9] * 50, True),
-                                            ([20] * 8 + [2] * 9000, False)])
-def test_batches_of_many_small_instances(ctx, orc, sides, resident):
+                                            ([20] * 8 + [2] * 9000, False), ([128] * 4, True)])
+def test_form_of_a_batch(ctx, orc, sides, resident):
+    """Many small instances, and instances that each need the whole chip."""
     unit, beta = 1e-3, 1e-4
     n = len(sides)
     _check(ctx, orc, nn.BatchedPCG(ctx, sides, unit, beta), sides, unit, beta, resident, {0, 1, n // 2, n - 1})
