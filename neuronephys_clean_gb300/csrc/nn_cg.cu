@@ -85,7 +85,8 @@ struct CgArgs {
 
 // Block totals of nsum thread values (FP64 from the thread on); the last block
 // to arrive writes the grid totals to out[] in a fixed order.
-__device__ bool cg_reduce(int nsum, const double* v, double* partials, unsigned int* ticket, double* out)
+template <int nsum>
+__device__ __forceinline__ bool cg_reduce(const double* v, double* partials, unsigned int* ticket, double* out)
 {
     __shared__ double ws[4][CG_MAX_THREADS / 32];
     __shared__ bool last;
@@ -107,12 +108,13 @@ __device__ bool cg_reduce(int nsum, const double* v, double* partials, unsigned 
     __syncthreads();
     if (!last) return false;
     __threadfence();
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+        for (int q = 0; q < nsum; ++q) s[q] += __ldcg(partials + (size_t)q * gridDim.x + b);
     for (int q = 0; q < nsum; ++q) {
-        const volatile double* pp = partials + (size_t)q * gridDim.x;
-        double s = 0.0;
-        for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) s += pp[b];
-        s = nn_warp_sum(s);
-        if (lane == 0) ws[q][w] = s;
+        s[q] = nn_warp_sum(s[q]);
+        if (lane == 0) ws[q][w] = s[q];
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -506,7 +508,7 @@ __global__ void __launch_bounds__(CG_MAX_THREADS, 1)
     const double scale = HET ? 1.0 : (double)a.onepb + 6.0 * (double)a.op_alpha;  // r = scale u
     const double sums[4] = {scale * sg.value(), sd.value(), scale * scale * sr.value(), sbb.value()};
     double out[4];
-    if (cg_reduce(INIT ? 4 : 3, sums, a.partials, a.ticket, out) && tid == 0) cg_scalars(a, INIT, out);
+    if (cg_reduce<INIT ? 4 : 3>(sums, a.partials, a.ticket, out) && tid == 0) cg_scalars(a, INIT, out);
 }
 
 // x (rows of nx) from xp (rows of 4 nq, possibly x itself) after a.it
@@ -697,6 +699,16 @@ static nn_status cg_vectors(nn_cg_plan* pl)
 // planes with the least work of the busiest SM (one block each), where a block
 // computes zc + 1 planes, loads two more, and a plane costs its quads and a
 // barrier (the load of about 64 quads).
+// Two kinds of grid march too shortly, or too few quads a plane, for one block to
+// hide its copies' latency, and share an SM between blocks instead:
+// - up to eight planes: tiles of at most 256 threads (192 with a cell field),
+//   two or three to an SM by their registers.  us an iteration, the larger tile
+//   and this one: 1024 x 1024 x 8 78 and 66 (88 and 81 with a cell field), 2048 x
+//   2048 x 2 61 and 48;
+// - a plane that is one tile of at most 128 threads: chunks of 6 to 12 planes, as
+//   many as four blocks an SM take (their number counts in the reduction, so at
+//   most sixteen).  us, 152 chunks and these: 4 x 4 x 4096 20 and 11, 12 x 12 x
+//   20000 141 and 36, 32 x 32 x 4000 39 and 28.
 static bool cg_shape(nn_cg_plan* pl, int sms, size_t smem_max)
 {
     const int ny = pl->ny, nz = pl->nz;
@@ -712,6 +724,7 @@ static bool cg_shape(nn_cg_plan* pl, int sms, size_t smem_max)
         const int threads = (cq * rp + 31) / 32 * 32;
         const size_t smem = CgSmem(cq, rp, pl->ntx > 1, pl->D != nullptr).total;
         if (threads > CG_MAX_THREADS || smem > smem_max || NR * rp > 200) break;  // (box rows: at most 256)
+        if (nz <= 8 && best >= 0.0 && threads > (pl->D ? 192 : 256)) break;
         for (int waves = 1; waves <= 4; ++waves) {
             const int64_t cols = (int64_t)pl->ntx * nty;
             int64_t chunks = std::min<int64_t>(nz, std::max<int64_t>(1, (int64_t)waves * sms / cols));
@@ -728,6 +741,8 @@ static bool cg_shape(nn_cg_plan* pl, int sms, size_t smem_max)
             pl->smem = smem;
         }
     }
+    if (pl->ntx * pl->nty == 1 && pl->threads <= 128)
+        pl->zc = std::max(std::min(std::max(6, (nz + 4 * sms - 1) / (4 * sms)), 12), (nz + 16 * sms - 1) / (16 * sms));
     return best >= 0.0;
 }
 

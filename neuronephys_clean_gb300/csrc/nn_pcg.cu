@@ -45,6 +45,7 @@ struct nn_pcg {
     // launch per iteration (or two)
     nn_rcg_plan* res = nullptr;
     cudaStream_t res_stream = nullptr;  // stream of the resident solve in progress
+    bool aligned_x = false;             // solves want x on 16 bytes
 };
 
 void nn_pcg_set_timing(nn_pcg* pc, bool on)
@@ -356,7 +357,14 @@ extern "C" nn_status nn_pcg_create(nn_ctx* ctx, int nx, int ny, int nz, double a
         nn_status fs = nn_rcg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, &pc->res);
         if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
         if (st == NN_OK) {
-            fs = nn_cg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, pc->res != nullptr, &pc->fast);
+            // rows of one cell (padded to four) and single planes of more than two
+            // million cells leave the single kernel nothing of its gain: 1 x 2048 x
+            // 2048 22.3 us an iteration and 13.2 in two kernels, 2048 x 2048 x 1 18.2
+            // and 12.6, 1024 x 1024 x 1 6.3 and 7.8
+            const bool flat = !pc->res && (nx == 1 || (nz == 1 && pc->G > (1 << 21)));
+            fs = flat ? NN_ERR_UNSUPPORTED
+                      : nn_cg_plan_create(ctx, nx, ny, nz, alpha, beta, d_Dcell, pc->res != nullptr, &pc->fast);
+            pc->aligned_x = nx % 4 == 0 && !((uintptr_t)d_Dcell & 15) && (pc->fast || (flat && pc->G <= INT32_MAX));
             // rows that have to be padded take three vectors more than two kernels
             if (fs == NN_ERR_OOM && (nx % 4 || ((uintptr_t)d_Dcell & 15))) fs = NN_ERR_UNSUPPORTED;
             if (fs != NN_OK && fs != NN_ERR_UNSUPPORTED) st = fs;
@@ -524,18 +532,19 @@ nn_status nn_pcg_async_finish(nn_pcg* pc, int* iters, double* relres, int* conve
 
 bool nn_pcg_async_supported(const nn_pcg* pc) { return pc->fast != nullptr || pc->res != nullptr; }
 
-// Grids of whole aligned quads: their solves want x aligned too, and their tile
-// depth can be tuned.
+// Grids of whole aligned quads: their tile depth can be tuned.
 static bool tunable(const nn_pcg* pc) { return pc->fast && pc->nx % 4 == 0 && !((uintptr_t)pc->Dcell & 15); }
 
 // The resident solve when the grid fits, else the single-kernel iteration, else
-// (2^31 cells and more) two kernels.
+// (2^31 cells and more, a single plane, rows of one cell, or no memory for padded
+// rows) two kernels.  Grids of whole aligned quads want x aligned too, whichever
+// solver takes them.
 nn_status nn_pcg_run_best(nn_pcg* pc, const float* d_b, float* d_x, double rtol, int max_iter, int* iters,
                           double* relres, int* converged)
 {
+    if (pc->aligned_x && ((uintptr_t)d_x & 15))
+        return nn_fail(pc->ctx, NN_ERR_INVALID_ARG, "PCG: x must be a 16-byte aligned device vector");
     if (pc->res) {
-        if (tunable(pc) && ((uintptr_t)d_x & 15))
-            return nn_fail(pc->ctx, NN_ERR_INVALID_ARG, "PCG: x must be a 16-byte aligned device vector");
         NN_TRY(nn_rcg_begin(pc->res, d_b, d_x, rtol, max_iter, pc->ctx->stream));
         return nn_rcg_finish(pc->res, pc->ctx->stream, iters, relres, converged);
     }
