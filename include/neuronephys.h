@@ -311,8 +311,9 @@ NN_API nn_status nn_sim_autotune(nn_sim* s, int trial_steps, int* best_tpb, int*
  * from a snapshot of the simulation, which is restored afterwards;
  * *ms_per_iter then holds the time per timestep.  Otherwise the solver is
  * timed alone on scratch vectors and *ms_per_iter is its iteration time.
- * *shape: the chosen depth or cells per block.  A grid that fits on the chip
- * is solved by one resident kernel, which no depth affects. */
+ * *shape: the chosen depth or cells per block.  A grid or batch that is solved
+ * on the chip in one launch has no such shape: nothing is tried or changed,
+ * *shape is what is set and *ms_per_iter the solve's iteration time. */
 NN_API nn_status nn_sim_autotune_solver(nn_sim* s, int trial_iters, int* shape, float* ms_per_iter);
 /* Per-instance solver iteration counts of the last paracrine solve (n_inst entries). */
 NN_API nn_status nn_sim_instance_iterations(nn_sim* s, int* h_iters);

@@ -516,8 +516,10 @@ class Simulation:
 
     def autotune_solver(self, trial_iters: int = 20) -> tuple[int, float]:
         """Field solver block shape (single grid: tile depth of the one-kernel
-        PCG iteration; batch: cells per block), timed on scratch vectors.
-        Returns (shape, ms per iteration)."""
+        PCG iteration; batch: cells per block): (shape, ms).  Solves that
+        overlap the neuron updates are timed over whole periods (ms per
+        timestep), others on scratch vectors (ms per iteration); a field solved
+        on the chip in one launch has no shape to tune (ms per iteration)."""
         shape, ms = C.c_int(0), C.c_float(0.0)
         _check(lib().nn_sim_autotune_solver(self.handle, trial_iters, C.byref(shape), C.byref(ms)), self.ctx,
                "sim_autotune_solver")

@@ -707,6 +707,7 @@ extern "C" nn_status nn_bpcg_autotune(nn_bpcg* bp, const float* d_b, float* d_x,
 }
 
 int nn_bpcg_cells_per_block(const nn_bpcg* bp) { return BT * bp->vpt; }
+bool nn_bpcg_resident(const nn_bpcg* bp) { return bp->res != nullptr; }
 
 extern "C" nn_status nn_bpcg_set_cells_per_block(nn_bpcg* bp, int cells_per_block)
 {

@@ -236,6 +236,7 @@ nn_status nn_bpcg_async_begin(nn_bpcg* bp, const float* d_b, float* d_x, double 
                               cudaStream_t cs);
 nn_status nn_bpcg_async_finish(nn_bpcg* bp, int* h_iters, int* max_iters, int* unconverged);
 int nn_bpcg_cells_per_block(const nn_bpcg* bp);
+bool nn_bpcg_resident(const nn_bpcg* bp);
 
 // resident CG: the whole solve in one kernel (nn_rcg.cu)
 struct nn_rcg_plan;
@@ -288,6 +289,7 @@ void nn_cg_plan_set_tile_depth(nn_cg_plan* pl, int zc);
 struct nn_pcg;
 nn_status nn_pcg_autotune_tiles(nn_pcg* pc, int iters, int* tile_z, float* ms_per_iter);
 int nn_pcg_tile_depth(const nn_pcg* pc);
+bool nn_pcg_resident(const nn_pcg* pc);
 void nn_pcg_set_tile_depth(nn_pcg* pc, int zc);
 double nn_host_inv_phi(double p);
 void nn_host_gauss_table(double sigma_sites, int16_t* table4096);

@@ -567,8 +567,12 @@ void nn_pcg_set_tile_depth(nn_pcg* pc, int zc)
     if (tunable(pc) && zc >= 4) nn_cg_plan_set_tile_depth(pc->fast, zc);
 }
 
+bool nn_pcg_resident(const nn_pcg* pc) { return pc->res != nullptr; }
+
 // Tile autotuner of the single-kernel iteration (nn_cg_plan_autotune) on
-// scratch vectors; NN_ERR_UNSUPPORTED on grids that it does not take.
+// scratch vectors; NN_ERR_UNSUPPORTED on grids that it does not take.  No depth
+// affects a resident solve: its own iteration is timed, the depth that the plan
+// has is returned (as one of the autotuner's).
 nn_status nn_pcg_autotune_tiles(nn_pcg* pc, int iters, int* tile_z, float* ms_per_iter)
 {
     if (!pc || iters < 1) return NN_ERR_INVALID_ARG;
@@ -582,7 +586,23 @@ nn_status nn_pcg_autotune_tiles(nn_pcg* pc, int iters, int* tile_z, float* ms_pe
         k_pcg_trial_rhs<<<nn_grid_for(ctx, G, 256, 8), 256, 0, ctx->stream>>>(b, G);
         st = nn_cuda_check(ctx, cudaPeekAtLastError(), "k_pcg_trial_rhs");
     }
-    if (st == NN_OK) st = nn_cg_plan_autotune(pc->fast, b, x, iters, tile_z, ms_per_iter);
+    if (st == NN_OK && pc->res) {
+        int n = 0;
+        float ms = 0.0f;
+        st = nn_cuda_check(ctx, cudaMemsetAsync(x, 0, sizeof(float) * (size_t)G, ctx->stream), "memset");
+        nn_rcg_set_timing(pc->res, true);
+        if (st == NN_OK) st = nn_rcg_begin(pc->res, b, x, 1e-30, iters, ctx->stream);
+        if (st == NN_OK) st = nn_rcg_finish(pc->res, ctx->stream, nullptr, nullptr, nullptr);
+        nn_rcg_last_timing(pc->res, &ms, &n);
+        nn_rcg_set_timing(pc->res, pc->timing);
+        int depth = 4;
+        for (int zc : {6, 8, 12, 16, 24, 32})
+            if (zc <= nn_pcg_tile_depth(pc)) depth = zc;
+        if (tile_z) *tile_z = depth;
+        if (ms_per_iter) *ms_per_iter = st == NN_OK && n > 0 ? ms / n : 0.0f;
+    } else if (st == NN_OK) {
+        st = nn_cg_plan_autotune(pc->fast, b, x, iters, tile_z, ms_per_iter);
+    }
     cudaStreamSynchronize(ctx->stream);
     nn_release(b);
     nn_release(x);

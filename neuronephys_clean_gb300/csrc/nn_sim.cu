@@ -2635,12 +2635,13 @@ extern "C" nn_status nn_sim_autotune_solver(nn_sim* s, int trial_iters, int* sha
     // a pending overlapped solve owns the solver's work vectors
     NN_TRY(finish_solve(s));
     if (s->ev_solved) NN_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, s->ev_solved, 0));
+    // (a solve on the chip has no shape to try: its iteration's time)
     if (s->pcg) {
-        if (!s->row_ptr || !overlap_solve(s) || nn_pcg_tile_depth(s->pcg) == 0)
+        if (!s->row_ptr || !overlap_solve(s) || nn_pcg_tile_depth(s->pcg) == 0 || nn_pcg_resident(s->pcg))
             return nn_pcg_autotune_tiles(s->pcg, trial_iters, shape, ms_per_iter);
         return autotune_overlapped_tiles(s, shape, ms_per_iter);
     }
-    if (s->row_ptr && overlap_solve(s)) return autotune_overlapped_tiles(s, shape, ms_per_iter);
+    if (s->row_ptr && overlap_solve(s) && !nn_bpcg_resident(s->bpcg)) return autotune_overlapped_tiles(s, shape, ms_per_iter);
     float *b = nullptr, *x = nullptr;
     const int64_t G = s->G;
     NN_TRY(nn_alloc(ctx, &b, (size_t)G));
