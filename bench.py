@@ -82,6 +82,7 @@ HH_FP32_OPS_PER_NEURON_STEP = 340
 # and log, sqrt, sin, cos per neuron pair for the noise
 HH_TRANSCENDENTALS_PER_NEURON_STEP = 26
 FP32_LANES_PER_SM = 128            # FP32 lanes per SM (sm_100 family), one fused multiply-add (2 ops) per lane and clock
+RESIDENT_SIDE = 128                # largest cube whose field solve runs on the chip in one launch (k_rcg)
 PCG_BYTES_PER_CELL_ITER = 24       # k_cg_iter R: u,t; W: u,t; R, W: p,x in every second iteration
 PCG_HET_BYTES_PER_CELL_ITER = 28   # k_cg_iter<HET>: + 1/(2 alpha D)
 PUSH_BYTES_PER_EVENT = 13          # 4 B target + 4 B weight + 1 B delay + 4 B ring read-modify-write
@@ -91,7 +92,6 @@ PULL_CSC_BYTES_PER_SYNAPSE = 9     # full CSC sweep: 4 B source + 4 B weight + 1
 # (dram__bytes_read.sum + dram__bytes_write.sum per launch / units per launch).
 NCU_TRAFFIC_PER_UNIT = {
     "hh_step": 36.03,        # 36.03 MB read + 0 MB written per 1M-neuron launch (writes stay in L2)
-    "pcg_iteration": None,   # one launch a solve on grids that fit on the chip
     "pcg_het_iteration": 25.8,  # 279 MB read + 153 MB written per 256^3 launch
 }
 
@@ -247,8 +247,10 @@ def run_ours(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
     # settle: start the timed region in steady tonic firing, not at rest
     sim.step(args.settle)
     # the field solver's tile depth from the autotuner (whole periods with the
-    # solve overlapped, in the settled state; the simulation is restored)
-    cg_tile = sim.autotune_solver(10) if wl["grid"] else (0, 0.0)
+    # solve overlapped, in the settled state; the simulation is restored); a
+    # solve on the chip has none
+    resident = 0 < wl["grid"] <= RESIDENT_SIDE
+    cg_tile = sim.autotune_solver(10) if wl["grid"] and not resident else None
     for _ in range(args.warmup):  # warm-up also captures the period graph
         sim.step(P)
     ctx.synchronize()
@@ -309,7 +311,7 @@ def run_ours(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
     hh_ms = kt.hh_step_median_ms if kt.hh_step_median_ms > 0 else kt.hh_step_ms
     hh_ach = n * HH_BYTES_PER_NEURON_STEP / (hh_ms * 1e-3) / 1e9 if hh_ms > 0 else None
     it_ms = kt.solve_ms / kt.solve_iterations if kt.solve_iterations else None
-    pcg_ach = G * PCG_BYTES_PER_CELL_ITER / (it_ms * 1e-3) / 1e9 if it_ms else None
+    pcg_ach = G * PCG_BYTES_PER_CELL_ITER / (it_ms * 1e-3) / 1e9 if it_ms and not resident else None
     # time per bench step: P neuron updates and P / timescale solves
     per_period_hh = hh_ms * P
     per_period_pcg = kt.solve_ms * (P // wl["timescale"])
@@ -319,11 +321,14 @@ def run_ours(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
                "algorithmic_bytes": n * HH_BYTES_PER_NEURON_STEP, "launch_ms": hh_ms,
                "launch_ms_of": "median launch of the last period of one bench step after the timed region, solves in line",
                "peak_source": peak_kind}
-    pcg_roof = {"bound": "hbm", "kernel": "one PCG iteration (k_rcg, its vectors on the chip; larger grids k_cg_iter)",
-                "achieved": pcg_ach,
-                "peak": hbm_peak, "unit": "GB/s", "frac": pcg_ach / hbm_peak if pcg_ach else None,
-                "traffic": (NCU_TRAFFIC_PER_UNIT["pcg_iteration"] * G) if NCU_TRAFFIC_PER_UNIT["pcg_iteration"] else None,
-                "algorithmic_bytes": G * PCG_BYTES_PER_CELL_ITER, "launch_ms": it_ms, "peak_source": peak_kind}
+    if resident:  # the vectors stay on the chip: no rate of HBM bounds it
+        pcg_roof = {"bound": "latency of the exchange between blocks, and issue", "kernel": "one iteration of k_rcg",
+                    "achieved": None, "peak": None, "unit": "GB/s", "frac": None, "traffic": None,
+                    "algorithmic_bytes": None, "launch_ms": it_ms}
+    else:
+        pcg_roof = {"bound": "hbm", "kernel": "k_cg_iter (one PCG iteration)", "achieved": pcg_ach,
+                    "peak": hbm_peak, "unit": "GB/s", "frac": pcg_ach / hbm_peak if pcg_ach else None, "traffic": None,
+                    "algorithmic_bytes": G * PCG_BYTES_PER_CELL_ITER, "launch_ms": it_ms, "peak_source": peak_kind}
     dominant, other = (hh_roof, pcg_roof) if per_period_hh >= per_period_pcg else (pcg_roof, hh_roof)
     # the neuron update's own bound is FP32 arithmetic and instruction issue:
     # its algorithmic operations against the FP32 peak at the sampled clock
@@ -374,7 +379,7 @@ def run_ours(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
         "delivery": delivery_info,
         "autotuned": {"cg_tile_depth": cg_tile[0], "trial_ms_per_timestep": cg_tile[1],
                       "how": "each tile depth timed over six periods with the solve overlapping the neuron "
-                             "updates, from a snapshot restored afterwards"},
+                             "updates, from a snapshot restored afterwards"} if cg_tile else None,
         "electrodes": el_info,
         "synaptic_events_per_s": events / seconds if seconds else None,
         "spikes_in_timed_region": spikes,
@@ -747,7 +752,6 @@ def run_batch(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
     sim.set_field("IDRIVE", np.repeat(drive, sizes))
     sim.step(args.settle)
     tpb, npt, tune_ms = sim.autotune(20)
-    cpb, pcg_iter_ms = sim.autotune_solver(10)
     P = wl["total_steps"]
     for _ in range(args.warmup):
         sim.step(P)
@@ -798,10 +802,7 @@ def run_batch(args, wl: dict, dist, rank: int, local_rank: int) -> dict | None:
         "config": {"workload": wl["workload"], "instances": int(wl["n_inst"]), "neurons": n, "synapses": int(nnz),
                    "timesteps_per_step": P, "grid_cells": int(sim.field_cells()),
                    "weights": "U[0, w_b], w_b = 2 * 2.5 nS / (p_b * size_b) per instance",
-                   "autotuned": {"threads_per_block": tpb, "neurons_per_thread": npt, "trial_ms_per_step": tune_ms,
-                                 "pcg_cells_per_block": cpb, "pcg_trial_ms_per_timestep": pcg_iter_ms,
-                                 "pcg_how": "each block size timed over six periods with the batched solve "
-                                            "overlapping the neuron updates, from a snapshot restored afterwards"},
+                   "autotuned": {"threads_per_block": tpb, "neurons_per_thread": npt, "trial_ms_per_step": tune_ms},
                    "network_generation_s": t_gen, "l2": "inputs larger than L2"},
         "spikes_in_timed_region": spikes_b - spikes_a,
         "cg": {"instances": int(wl["n_inst"]), "iterations_last_solve_max": int(iters.max()),
