@@ -52,7 +52,7 @@ constexpr int COL_BLOCKS = 4;  // resident blocks of a column kernel per SM (2: 
 // coarse levels of fewer cells keep a thread per cell (a sweep at 64^3: 5.2 us, by columns 8.0; at 128^3 15.2 and 10.9)
 constexpr int COL_MIN_CELLS = 1 << 20;
 #ifndef NN_MG_VEC
-#define NN_MG_VEC 4  // cells per thread on the fine level (4 or 2) when the x side allows
+#define NN_MG_VEC 4  // fine level: columns of quads where the x side allows (2: two cells a thread, by rows)
 #endif
 #ifndef NN_MG_MIN_BLOCKS
 // resident blocks per SM the stencils are compiled for: 4 (64 registers) is
@@ -947,8 +947,6 @@ __device__ __forceinline__ float dot(const Quad& x, const Quad& y, float acc)
     return acc + (s.v[0] + s.v[1]);
 }
 
-  // a SM
-
 // Two sweeps from zero: the first, omega b / diag, is formed at the neighbours
 // as b is read.
 template <class Op, class F>
@@ -1256,7 +1254,7 @@ struct nn_mg {
     nn_ctx* ctx = nullptr;
     nn_pcg* pc = nullptr;
     Op0 op0{};
-    int vec0 = 1;                // cells per thread on the fine level (4 when nx % 4 == 0)
+    int vec0 = 1;                // cells per thread on the fine level (4, in columns, when nx % 4 == 0)
     float* v = nullptr;          // vec0 == 4 and a cell field: 1 / (2 alpha D)
     std::vector<MgLevel> lv;
     float omega = 0.8f;
@@ -1348,10 +1346,10 @@ nn_status launch_pre2(nn_mg* mg, int l, const Op& op, const float* b, float* y, 
         NN_CHECK_LAUNCH(mg->ctx, "k_col_pre2");
         return NN_OK;
     } else {
-    const Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
-    chain(mg, k_mg_pre2<V, Op>, s.grid, s.block, op, b, mg->omega, y, flags);
-    NN_CHECK_LAUNCH(mg->ctx, "k_mg_pre2");
-    return NN_OK;
+        const Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
+        chain(mg, k_mg_pre2<V, Op>, s.grid, s.block, op, b, mg->omega, y, flags);
+        NN_CHECK_LAUNCH(mg->ctx, "k_mg_pre2");
+        return NN_OK;
     }
 }
 
@@ -1368,11 +1366,11 @@ nn_status launch_jacobi(nn_mg* mg, int l, const Op& op, const float* b, const fl
         NN_CHECK_LAUNCH(mg->ctx, "k_col_jacobi");
         return NN_OK;
     } else {
-    Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
-    if (DOTS) s.grid = dim3(mg->nblocks);  // the partials buffer holds nblocks entries
-    chain(mg, k_mg_jacobi<V, DOTS, Op>, s.grid, s.block, op, b, x, mg->omega, y, flags, q, red_of(mg));
-    NN_CHECK_LAUNCH(mg->ctx, "k_mg_jacobi");
-    return NN_OK;
+        Shape s = shape_for(mg->ctx, op.nx / V, op.ny * op.nz);
+        if (DOTS) s.grid = dim3(mg->nblocks);  // the partials buffer holds nblocks entries
+        chain(mg, k_mg_jacobi<V, DOTS, Op>, s.grid, s.block, op, b, x, mg->omega, y, flags, q, red_of(mg));
+        NN_CHECK_LAUNCH(mg->ctx, "k_mg_jacobi");
+        return NN_OK;
     }
 }
 
