@@ -70,6 +70,32 @@ extern "C" nn_status nn_ctx_create(int device, nn_ctx** out)
     return NN_OK;
 }
 
+nn_status nn_pinned_word(nn_ctx* ctx, int** word)
+{
+    *word = nullptr;
+    auto c = ctx->pinned.begin();
+    while (c != ctx->pinned.end() && c->second == ~0ull) ++c;
+    if (c == ctx->pinned.end()) {
+        int* p = nullptr;
+        NN_CUDA(ctx, cudaHostAlloc((void**)&p, 64 * sizeof(int), cudaHostAllocMapped));
+        c = ctx->pinned.insert(c, {p, 0ull});
+    }
+    int k = 0;
+    while (c->second >> k & 1) ++k;
+    c->second |= 1ull << k;
+    *word = c->first + k;
+    **word = 0;
+    return NN_OK;
+}
+
+void nn_pinned_release(nn_ctx* ctx, int*& word)
+{
+    if (word)
+        for (auto& c : ctx->pinned)
+            if (word >= c.first && word < c.first + 64) c.second &= ~(1ull << (word - c.first));
+    word = nullptr;
+}
+
 void nn_ctx_retain(nn_ctx* ctx)
 {
     if (ctx) ++ctx->refs;
@@ -83,6 +109,7 @@ void nn_ctx_release(nn_ctx* ctx)
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     nn_release(ctx->conv_err);
+    for (auto& c : ctx->pinned) cudaFreeHost(c.first);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }

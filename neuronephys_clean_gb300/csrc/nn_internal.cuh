@@ -8,6 +8,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "neuronephys.h"
@@ -21,10 +22,17 @@ struct nn_ctx {
     int64_t launches = 0;  // kernels launched on behalf of the caller
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // nn_ctx_time_begin/end
     int* conv_err = nullptr;  // device error word of the convolution entry points (allocated by the first)
+    // pinned words, in chunks of 64 that the objects share (a pinned allocation
+    // takes 300 us) and the bits of those in use (nn_pinned_word)
+    std::vector<std::pair<int*, uint64_t>> pinned;
     // Objects created on a context hold a reference, so destroying the context
     // before them (in any order) never leaves them with a dangling pointer.
     int refs = 1;
 };
+
+// A word of pinned host memory, 0 at first, and its return.
+nn_status nn_pinned_word(nn_ctx* ctx, int** word);
+void nn_pinned_release(nn_ctx* ctx, int*& word);
 
 // Take / drop a reference; the last release frees the context.
 void nn_ctx_retain(nn_ctx* ctx);

@@ -1562,7 +1562,7 @@ extern "C" nn_status nn_mg_destroy(nn_mg* mg)
     drop_graph(mg);
     for (MgLevel& L : mg->lv)
         for (float* v : {L.wx, L.wy, L.wz, L.wb, L.diag, L.b, L.x, L.t}) cudaFree(v);
-    for (float* v : {mg->r, mg->z, mg->q, mg->p[0], mg->p[1], mg->v}) cudaFree(v);
+    cudaFree(mg->r);  // and z, q, p, v behind it
     cudaFree(mg->scal);
     cudaFree(mg->flags);
     cudaFree(mg->partials);
@@ -1628,14 +1628,23 @@ extern "C" nn_status nn_mg_create(nn_pcg* pc, int levels, nn_mg** out)
             if (st == NN_OK) st = nn_alloc(ctx, a, L.G);
     }
     const int G = mg->lv[0].G;
-    for (float** a : {&mg->r, &mg->z, &mg->q, &mg->p[0], &mg->p[1]})
-        if (st == NN_OK) st = nn_alloc(ctx, a, G);
+    {
+        const bool field = mg->vec0 == 4 && D;
+        const size_t V = ((size_t)G + 63) / 64 * 64;
+        if (st == NN_OK) st = nn_alloc(ctx, &mg->r, (field ? 6 : 5) * V);
+        if (st == NN_OK) {
+            mg->z = mg->r + V;
+            mg->q = mg->r + 2 * V;
+            mg->p[0] = mg->r + 3 * V;
+            mg->p[1] = mg->r + 4 * V;
+            mg->v = field ? mg->r + 5 * V : nullptr;
+        }
+    }
     mg->nblocks = std::max(1, std::min((G + MG_THREADS - 1) / MG_THREADS, ctx->num_sms * 8));
     if (st == NN_OK) st = nn_alloc(ctx, &mg->scal, S_COUNT);
     if (st == NN_OK) st = nn_alloc(ctx, &mg->flags, F_COUNT);
     for (MgLevel& L : mg->lv)
         if (L.nx % 4 == 0 && (&L == &mg->lv[0] || L.G >= COL_MIN_CELLS)) L.cols = cols_for(ctx, L.nx, L.ny, L.nz);
-    if (st == NN_OK && mg->vec0 == 4 && D) st = nn_alloc(ctx, &mg->v, G);
     if (st == NN_OK)
         st = nn_alloc(ctx, &mg->partials,
                       (size_t)2 * std::max({mg->nblocks, ctx->num_sms * 8, mg->vec0 == 4 ? mg->lv[0].cols.blocks() : 0}));

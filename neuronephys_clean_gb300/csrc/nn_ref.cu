@@ -315,7 +315,7 @@ struct nn_coupling {
     int* firing = nullptr;       // n entries; first count ascending
     int* count = nullptr;        // device int
     int64_t* block_counts = nullptr;
-    int* sub_before = nullptr;   // per sub-tile: firing neurons of its tile before it
+    int* sub_before = nullptr;   // per sub-tile: firing neurons of its tile before it (behind block_counts)
     int nblocks = 0;
 };
 
@@ -564,8 +564,8 @@ extern "C" nn_status nn_coupling_create(nn_ctx* ctx, int n, nn_coupling** out)
     if (c->nblocks < 1) c->nblocks = 1;
     nn_status st = nn_alloc(ctx, &c->firing, (size_t)(n > 0 ? n : 1));
     if (st == NN_OK) st = nn_alloc(ctx, &c->count, 1);
-    if (st == NN_OK) st = nn_alloc(ctx, &c->block_counts, (size_t)c->nblocks);
-    if (st == NN_OK) st = nn_alloc(ctx, &c->sub_before, (size_t)c->nblocks * CMP_SUBS);
+    if (st == NN_OK) st = nn_alloc(ctx, &c->block_counts, (size_t)c->nblocks * (1 + CMP_SUBS / 2));
+    if (st == NN_OK) c->sub_before = reinterpret_cast<int*>(c->block_counts + c->nblocks);
     if (st != NN_OK) {
         nn_coupling_destroy(c);
         return st;
@@ -584,7 +584,6 @@ extern "C" nn_status nn_coupling_destroy(nn_coupling* c)
     nn_release(c->firing);
     nn_release(c->count);
     nn_release(c->block_counts);
-    nn_release(c->sub_before);
     nn_ctx* ctx = c->ctx;
     delete c;
     nn_ctx_release(ctx);
@@ -807,6 +806,7 @@ struct nn_paracrine {
     int64_t G = 0;
     int* idx8 = nullptr;
     float* w8 = nullptr;
+    float* grids = nullptr;      // the allocation of the grids that follow
     float* u = nullptr;          // density
     float* Ax = nullptr;         // scatter accumulator
     float *un = nullptr, *x = nullptr, *b = nullptr, *r = nullptr, *p0 = nullptr, *p1 = nullptr, *Ap = nullptr;
@@ -1116,18 +1116,23 @@ extern "C" nn_status nn_paracrine_ref_create(nn_ctx* ctx, const nn_paracrine_ref
     pm->nparts = nn_grid_for(ctx, pm->G, CN_THREADS, std::max(1, std::min(per_sm, cn_blocks_per_sm(ctx, pm->G))));
 #define PM_ALLOC(ptr, cnt) if (st == NN_OK) st = nn_alloc(ctx, &pm->ptr, cnt)
     PM_ALLOC(idx8, 8 * N); PM_ALLOC(w8, 8 * N);
-    PM_ALLOC(u, G); PM_ALLOC(Ax, G); PM_ALLOC(un, G); PM_ALLOC(x, G); PM_ALLOC(b, G);
-    PM_ALLOC(r, G); PM_ALLOC(p0, G); PM_ALLOC(p1, G); PM_ALLOC(Ap, G);
+    const size_t V = (G + 63) / 64 * 64;
+    PM_ALLOC(grids, 9 * V);
+    if (st == NN_OK) {
+        float* v = pm->grids;
+        for (float** q : {&pm->u, &pm->Ax, &pm->un, &pm->x, &pm->b, &pm->r, &pm->p0, &pm->p1, &pm->Ap}) {
+            *q = v;
+            v += V;
+        }
+    }
     PM_ALLOC(at_neurons, N); PM_ALLOC(generated, N);
     PM_ALLOC(scal, 4); PM_ALLOC(partials, 2 * (size_t)pm->nparts); PM_ALLOC(bar, 1); PM_ALLOC(done, 2);
 #undef PM_ALLOC
-    if (st == NN_OK)
-        st = nn_cuda_check(ctx, cudaHostAlloc((void**)&pm->h_gave_up, sizeof(int), cudaHostAllocMapped), "cudaHostAlloc");
+    if (st == NN_OK) st = nn_pinned_word(ctx, &pm->h_gave_up);
     if (st != NN_OK) {
         nn_paracrine_destroy(pm);
         return st;
     }
-    *pm->h_gave_up = 0;
     const char* polls = std::getenv("NN_CN_POLLS");
     pm->polls = polls ? std::atoi(polls) : CN_POLLS;
     cudaStream_t s = ctx->stream;
@@ -1157,12 +1162,10 @@ extern "C" nn_status nn_paracrine_destroy(nn_paracrine* pm)
 {
     if (!pm) return NN_OK;
     if (pm->ctx) cudaStreamSynchronize(pm->ctx->stream);
-    nn_release(pm->idx8); nn_release(pm->w8); nn_release(pm->u); nn_release(pm->Ax); nn_release(pm->un);
-    nn_release(pm->x); nn_release(pm->b); nn_release(pm->r); nn_release(pm->p0); nn_release(pm->p1);
-    nn_release(pm->Ap);
+    nn_release(pm->idx8); nn_release(pm->w8); nn_release(pm->grids);
     nn_release(pm->at_neurons); nn_release(pm->generated); nn_release(pm->scal); nn_release(pm->partials);
     nn_release(pm->bar); nn_release(pm->done);
-    if (pm->h_gave_up) cudaFreeHost(pm->h_gave_up);
+    nn_pinned_release(pm->ctx, pm->h_gave_up);
     nn_ctx* ctx = pm->ctx;
     delete pm;
     nn_ctx_release(ctx);
