@@ -671,7 +671,6 @@ __global__ void __launch_bounds__(RT, 1) k_rcg_batch(const RcgBatchArgs B)
         ulonglong2* slot = B.start + (size_t)(s & 1) * gridDim.x + first;
         __syncthreads();
         if (tid == 0) {
-            last = 0;
             const int q = B.list[g.first + k];
             a = B.inst[q];
             a.b = B.b + B.off[q];
@@ -693,7 +692,7 @@ __global__ void __launch_bounds__(RT, 1) k_rcg_batch(const RcgBatchArgs B)
                 }
                 v = ld_tagged(slot + tid);
             }
-            atomicMax(&last, (unsigned)v.x);
+            if (tid == 0) last = (unsigned)v.x;  // the first block has a brick in every solve: its tag is the latest
         }
         __syncthreads();
         if (gave_up) {

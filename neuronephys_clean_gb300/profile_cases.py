@@ -1,8 +1,12 @@
 """Small, self-contained GPU cases for kernel profiling (ncu captures).
 
     python -m neuronephys_clean_gb300.profile_cases hh1m     # 2 steps, 1M neurons, 128^3 grid
-    python -m neuronephys_clean_gb300.profile_cases cg128    # 3 PCG iterations, 128^3, constant D
+    python -m neuronephys_clean_gb300.profile_cases cg128    # 3 PCG iterations, 128^3, constant D (on the chip)
     python -m neuronephys_clean_gb300.profile_cases cghet    # 3 PCG iterations, 128^3, lognormal D
+    python -m neuronephys_clean_gb300.profile_cases cg256    # 6 PCG iterations, 256^3, lognormal D
+    python -m neuronephys_clean_gb300.profile_cases rcg      # 32 on the chip: 128^3 constant; 97 x 83 x 150 lognormal D
+    python -m neuronephys_clean_gb300.profile_cases rcgbatch # 24 fields of 32^3 to 51^3 solved in one launch
+    python -m neuronephys_clean_gb300.profile_cases loop1m   # the reference's loop: 3 steps of 1M neurons, one 64^3 solve
     python -m neuronephys_clean_gb300.profile_cases conv128  # 3x3x3 convs (16->16, 48->16) + wgrad at 128^3
     python -m neuronephys_clean_gb300.profile_cases mg256    # multigrid FCG solve to 1e-6, 256^3, lognormal D
     python -m neuronephys_clean_gb300.profile_cases lmg256   # the same with the learned 32^3 level (20 training steps)
@@ -35,14 +39,14 @@ def hh1m(ctx):
     s.step(2)
 
 
-def _pcg(ctx, D=None):
-    n = 128
+def _pcg(ctx, D=None, shape=(128, 128, 128), iterations=3):
+    nz, ny, nx = shape
     dD = None if D is None else ctx.to_device(D.ravel())
-    pc = nn.PCG(ctx, n, n, n, 16.384, 0.0, dD)
-    b = ctx.to_device(np.random.default_rng(1).random(n ** 3).astype(np.float32))
-    x = ctx.to_device(np.zeros(n ** 3, np.float32))
+    pc = nn.PCG(ctx, nx, ny, nz, 1e-3 * max(shape) ** 2, 0.0, dD)
+    b = ctx.to_device(np.random.default_rng(1).random(nx * ny * nz).astype(np.float32))
+    x = ctx.to_device(np.zeros(nx * ny * nz, np.float32))
     try:
-        pc.solve(b, x, rtol=1e-6, max_iter=3)
+        pc.solve(b, x, rtol=1e-6, max_iter=iterations)
     except nn.NNError as e:
         if e.status != nn.NN_ERR_NOT_CONVERGED:
             raise
@@ -55,6 +59,47 @@ def cg128(ctx):
 def cghet(ctx):
     from neuronephys_clean_gb300 import fields
     _pcg(ctx, fields.lognormal_diffusivity((128, 128, 128), 1.0, 8.0, seed=1))
+
+
+def cg256(ctx):
+    from neuronephys_clean_gb300 import fields
+    shape = (256, 256, 256)
+    _pcg(ctx, fields.lognormal_diffusivity(shape, 1.0, 8.0, seed=1), shape, 6)
+
+
+def rcg(ctx):
+    from neuronephys_clean_gb300 import fields
+    _pcg(ctx, iterations=32)
+    shape = (150, 83, 97)
+    _pcg(ctx, fields.lognormal_diffusivity(shape, 1.0, 8.0, seed=1), shape, 32)
+
+
+def rcgbatch(ctx):
+    sides = np.linspace(32, 51, 24).round().astype(int).tolist()
+    bp = nn.BatchedPCG(ctx, sides, 1e-3, 1e-4)
+    b = np.random.default_rng(1).random(int(bp.offsets[-1])).astype(np.float32)
+    bp.solve(ctx.to_device(b), ctx.to_device(np.zeros_like(b)), 1e-6, 5000)
+
+
+def loop1m(ctx):
+    n, k = 1_000_000, 100
+    rng = np.random.default_rng(1)
+    e = nn.HHEphys(ctx, n, seed=1)
+    var = dict(zip(nn.SIM_PARAMS, e.vars))
+    e.set("V", rng.normal(-55, 20, n).astype(np.float32))
+    net = nn.AdjacencyList(ctx.to_device(rng.integers(0, n, n * k, np.int32)),
+                           ctx.to_device(np.arange(n + 1, dtype=np.int32) * k))
+    p = nn.ParacrineModule.default_params()
+    p.nx = p.ny = p.nz = 64
+    p.quirk_firing_list = 0
+    pos = [ctx.to_device((rng.random(n) * 62.9 - 31.45).astype(np.float32)) for _ in range(3)]
+    m = nn.ParacrineModule(ctx, ctx.empty((n,), np.float32), n, p, *pos)
+    cp = nn.AtomicCoupling(ctx, n)
+    for _ in range(3):
+        cp(net, var["EIN"], var["EOUTPUT"], read_count=False)
+        m.update_on_fine_timescale(cp)
+        e.simulate_ephys()
+    m.update_on_own_timescale()
 
 
 def conv128(ctx):
@@ -154,7 +199,8 @@ def burst1m(ctx):
     _burst_sim(ctx).step(200)
 
 
-CASES = {"hh1m": hh1m, "cg128": cg128, "cghet": cghet, "conv128": conv128, "mg256": mg256, "lmg256": lmg256,
+CASES = {"hh1m": hh1m, "cg128": cg128, "cghet": cghet, "cg256": cg256, "rcg": rcg, "rcgbatch": rcgbatch,
+         "loop1m": loop1m, "conv128": conv128, "mg256": mg256, "lmg256": lmg256,
          "pull1m": pull1m,
          "burst1m": burst1m, "burst1m_steps": burst1m_steps}
 
