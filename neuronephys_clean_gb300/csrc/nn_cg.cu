@@ -55,7 +55,7 @@
 namespace {
 constexpr int CG_THREADS = 256;      // the elementwise kernels
 constexpr int NR = 2;                // rows of a thread (256^3 with a cell field: 93 us; 1: 115, 3: 94, 4: 99)
-constexpr int CG_MAX_THREADS = 384;  // k_cg_iter: one block per SM, 128 registers a thread
+constexpr int CG_MAX_THREADS = 384;  // k_cg_iter: 154 registers a thread with a cell field, 100 without
 constexpr int STAGES = 4;            // planes of u and v in shared memory
 constexpr int CG_MAX_QUADS = 64;     // row of a TMA box: 256 cells
 constexpr uint32_t WAIT_LIMIT = 1u << 20;
