@@ -1444,8 +1444,15 @@ static nn_status build_sliced(nn_sim* s)
     nn_ctx* ctx = s->ctx;
     const char* env = std::getenv("NN_PULL_UNSLICED");
     if (env && env[0] == '1') return NN_OK;
+    // dynamic shared memory beside the kernel's own, allowed once for all
+    // simulations (the attribute is the function's: a later, smaller one must
+    // not take it from an earlier)
     int smem_max = 0;
+    cudaFuncAttributes fa;
     NN_CUDA(ctx, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    NN_CUDA(ctx, cudaFuncGetAttributes(&fa, k_deliver_pull_sliced));
+    smem_max -= (int)fa.sharedSizeBytes;
+    NN_CUDA(ctx, cudaFuncSetAttribute(k_deliver_pull_sliced, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     const int cols = (s->n + ctx->num_sms - 1) / ctx->num_sms;
     const int nblk = (s->n + cols - 1) / cols;
     const int dmax = s->D - 1;
@@ -1603,11 +1610,6 @@ static nn_status build_sliced(nn_sim* s)
             s->dsl_chunk, d_ustart, nc, t_src, t_col, t_w, s->dsl_ent, s->dsl_w);
         st = nn_cuda_check(ctx, cudaGetLastError(), "k_dsl_pack");
     }
-    const size_t smem = dsl_smem_bytes(ring, slotw, cols, cmax, direct);
-    if (st == NN_OK)
-        st = nn_cuda_check(ctx, cudaFuncSetAttribute(k_deliver_pull_sliced,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                           "cudaFuncSetAttribute");
     if (st == NN_OK) st = nn_cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "build_sliced");
     cudaFree(cnt);
     cudaFree(t_src);
