@@ -475,7 +475,8 @@ __global__ void __launch_bounds__(CMP_THREADS) k_cmp_write_push(const float* out
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int subs = (n - 1) / SUB + 1;
     int64_t boff = 0;
-    for (int s = blockIdx.x * per_block; s < min((int)(blockIdx.x + 1) * per_block, subs); ++s) {
+    const int s0 = blockIdx.x * (SUB == CMP_SUB ? 1 : per_block);
+    for (int s = s0; s < (SUB == CMP_SUB ? s0 + 1 : min(s0 + per_block, subs)); ++s) {  // (short stretches: one a block)
         bool f[ITEMS];
         unsigned b[ITEMS];
 #pragma unroll
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(CMP_THREADS) k_cmp_write_push(const float* out
             b[q] = __ballot_sync(0xffffffffu, f[q]);
             if (q * WARPS + w < SUB / 32 && lane == 0) wt[q * WARPS + w] = __popc(b[q]);
         }
-        if (s == (int)blockIdx.x * per_block) {
+        if (s == s0) {
             const int tile = (int)((int64_t)s * SUB / CMP_TILE);
             int64_t acc = 0;
             for (int q = threadIdx.x; q < tile; q += CMP_THREADS) acc += block_counts[q];
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(CMP_THREADS) k_cmp_write_push(const float* out
                     if ((unsigned)post[u] < (unsigned)n) atomicAdd(inputs + post[u], sig);
             }
         }
-        __syncthreads();
+        if (SUB != CMP_SUB) __syncthreads();
     }
 }
 
